@@ -46,6 +46,9 @@ static void free_graph(cg_graph *g) {
   cudaFree(g->tmp_parents);
   cudaFree(g->orig);
   cudaFree(g->perm);
+  cudaFree(g->check_ws);
+  cudaFree(g->scratch);
+  cudaFree(g->edge_w);
   if (g->ev0) cudaEventDestroy(g->ev0);
   if (g->ev1) cudaEventDestroy(g->ev1);
   if (g->h_stats) cudaFreeHost(g->h_stats);
@@ -72,6 +75,25 @@ static int upload(const void *src, size_t bytes, bool device_src, void **dst, cg
   if (bytes) CG_CUDA(cudaMemcpyAsync(*dst, src, bytes, device_src ? cudaMemcpyDeviceToDevice
                                                                   : cudaMemcpyHostToDevice,
                                      g->stream));
+  return CG_OK;
+}
+
+int call_scratch(cg_graph *g, size_t bytes, void **out) {
+  if (g->scratch_bytes < bytes) {
+    cudaFree(g->scratch);  // earlier users have waited for their work
+    g->scratch = nullptr;
+    g->device_bytes -= (int64_t)g->scratch_bytes;
+    g->scratch_bytes = 0;
+    const size_t take = bytes < 4096 ? 4096 : bytes;
+    if (cudaMalloc(&g->scratch, take) != cudaSuccess) {
+      cudaGetLastError();
+      g->scratch = nullptr;
+      return CG_ERR_OUT_OF_MEMORY;
+    }
+    g->scratch_bytes = take;
+    g->device_bytes += (int64_t)take;
+  }
+  *out = g->scratch;
   return CG_OK;
 }
 
@@ -367,18 +389,16 @@ int cg_count_edges(cg_graph *g, const int32_t *d_levels, int32_t k, int64_t *m_o
   if (!g || !d_levels || k <= 0 || k > 65535 || !m_out) return CG_ERR_INVALID_ARG;
   if (int r = refuse_reordered(g, "cg_count_edges")) return r;
   unsigned long long *d_m = nullptr;
-  if (cudaMallocAsync((void **)&d_m, sizeof(unsigned long long) * (size_t)k, g->stream) !=
-      cudaSuccess)
-    return CG_ERR_OUT_OF_MEMORY;
-  int rc = count_edges_launch(g, d_levels, k, d_m);
+  int rc = call_scratch(g, sizeof(unsigned long long) * (size_t)k, (void **)&d_m);
+  if (rc) return rc;
+  rc = count_edges_launch(g, d_levels, k, d_m);
   if (rc == CG_OK) {
     cudaError_t e = cudaMemcpyAsync(m_out, d_m, sizeof(int64_t) * (size_t)k,
                                     cudaMemcpyDeviceToHost, g->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
     if (e != cudaSuccess) rc = cuda_fail(e, "cg_count_edges");
   }
-  cudaFreeAsync(d_m, g->stream);
-  cudaStreamSynchronize(g->stream);
+  if (rc) cudaStreamSynchronize(g->stream);
   return rc;
 }
 

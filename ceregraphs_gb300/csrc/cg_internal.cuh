@@ -165,6 +165,11 @@ struct cg_graph {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cg_stats *h_stats = nullptr;     // page-locked copy target of d_stats
   cg::FifoState *fifo = nullptr;   // FIFO parent pass scratch (first use)
+  void *check_ws = nullptr;        // cg_validate_device workspace (first use)
+  size_t check_bytes = 0;
+  void *scratch = nullptr;         // small device scratch of calls that wait (call_scratch)
+  size_t scratch_bytes = 0;
+  uint32_t *edge_w = nullptr;      // cg_count_edges: a vertex's share of m (first use)
 };
 
 namespace cg {
@@ -173,6 +178,9 @@ int cuda_fail(cudaError_t e, const char *what);
 // Sets the text cg_last_error_string returns (a reason, not a CUDA error).
 void set_error_text(const char *text);
 int bfs_prepare(cg_graph *g);
+// `bytes` of device scratch owned by the handle, for calls that wait for the
+// stream before they return (the next call may then reuse or grow it).
+int call_scratch(cg_graph *g, size_t bytes, void **out);
 int dead_prepare(cg_graph *g);
 // CG_ERR_NOT_SUPPORTED (with a reason) while the handle's stream is being
 // captured: for set-up that has to synchronise the handle's stream.

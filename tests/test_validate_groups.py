@@ -1,0 +1,83 @@
+"""The grouped tree checks at the edges of their ranges: searches per group,
+in-lists around the thread / warp / chunk limits, levels around the byte limit."""
+import numpy as np
+import pytest
+
+from ceregraphs_gb300 import generators
+from ceregraphs_gb300.preprocess import from_edges
+
+CHECKS = ("root", "tree", "edges", "span", "tree_edge", "lowest")
+
+
+def _degrees_graph(n, seed):
+  """Directed graph with in-degrees at 1, 32/33, 128/129, 512/513, 1024/1025
+  and 2000 among random ones."""
+  rng = np.random.default_rng(seed)
+  src, dst = [], []
+  for v, d in enumerate([1, 31, 32, 33, 127, 128, 129, 511, 512, 513, 1024, 1025, 2000]):
+    at = v * 37 + 5
+    src.append(rng.choice(n, size=d, replace=False))
+    dst.append(np.full(d, at))
+  src.append(rng.integers(0, n, 4 * n))
+  dst.append(rng.integers(0, n, 4 * n))
+  return from_edges(n, np.concatenate(src), np.concatenate(dst), drop_self_loops=True)
+
+
+def _path(n):
+  i = np.arange(n - 1)
+  return from_edges(n, i, i + 1, symmetrize=True)
+
+
+def _damage(lv, pa, n, rng, many):
+  """Random mistakes in levels and parents, some far out of range."""
+  lv, pa = lv.copy(), pa.copy()
+  at = rng.integers(0, n, many)
+  lv[at] = rng.choice([-1, -5, 0, 1, 2, 3, 125], size=many)
+  at = rng.integers(0, n, many)
+  pa[at] = rng.choice([-1, -2, 0, n - 1, n, n + 9, 2 ** 31 - 1], size=many)
+  at = rng.integers(0, n, many)
+  pa[at] = rng.integers(0, n, many)
+  return lv, pa
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k", [1, 4, 5, 8, 9, 16, 17, 35])
+@pytest.mark.parametrize("kind", ["degrees", "rmat", "path126", "path127"])
+def test_groups_match_oracle(built_lib, oracle_mod, kind, k):
+  import torch
+  from ceregraphs_gb300.engine import Graph
+  a = {"degrees": lambda: _degrees_graph(3001, 3), "rmat": lambda: generators.rmat(11, 16, 4),
+       # from vertex 0 the deepest level is 125 (the last that fits) or 126
+       "path126": lambda: _path(126), "path127": lambda: _path(127)}[kind]()
+  rng = np.random.default_rng(k)
+  out_off, out_idx = a.out_lists()
+  roots = [0] + rng.integers(0, a.n, k - 1).tolist()
+  L, P = np.empty((k, a.n), np.int32), np.empty((k, a.n), np.int32)
+  for i, r in enumerate(roots):
+    L[i], P[i], _ = oracle_mod.bfs(out_off, out_idx, a.in_off, a.in_idx, r)
+    if i % 3 != 1:  # some searches stay clean
+      L[i], P[i] = _damage(L[i], P[i], a.n, rng, 1 + 7 * (i % 3))
+  with Graph(a) as g:
+    for _ in range(2):  # a second call on the kept workspace
+      got = g.validate(roots, torch.from_numpy(L).cuda(), torch.from_numpy(P).cuda())
+      for i, r in enumerate(roots):
+        want = oracle_mod.validation_counts(a.in_off, a.in_idx, r, L[i], P[i])
+        for c in CHECKS:
+          assert (got[i][c]["failures"], got[i][c]["first"]) == want[c], (i, c, got[i], want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k", [1, 15, 16, 17])
+def test_edge_counts_of_groups(built_lib, k):
+  import torch
+  from ceregraphs_gb300.engine import Graph
+  rng = np.random.default_rng(k)
+  for a in (_degrees_graph(3001, 3), generators.rmat(11, 16, 4)):
+    L = rng.integers(-1, 4, (k, a.n)).astype(np.int32)
+    with Graph(a) as g:
+      got = g.count_edges(torch.from_numpy(L).cuda(), k)
+    dst = np.repeat(np.arange(a.n), np.diff(a.in_off))
+    for i in range(k):
+      seen = L[i] >= 0
+      want = int(np.sum(seen[dst] & (a.in_idx <= dst))) if a.symmetric else int(seen[a.in_idx].sum())
+      assert got[i] == want
