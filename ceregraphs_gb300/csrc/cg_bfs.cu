@@ -62,11 +62,15 @@ struct __align__(16) WarpTile {  // 16-byte vector accesses to every member
   uint32_t found[kTileWords];
 };
 static_assert(sizeof(WarpTile) % 16 == 0 && kTileWords % 4 == 0, "16-byte tile rows");
-// Per-warp shared memory of a push round's edge spreading (gather_expand).
+// Per-warp shared memory of a push round: the edge spreading of gather_expand
+// (list starts and prefix counts fit 32 bits, nnz being below 2^32), and the
+// claimed vertices not queued yet with their out-degrees.
 struct WarpExpand {
   int32_t u[32];
-  int64_t s[32];
-  int64_t x[32];
+  uint32_t s[32];
+  uint32_t x[32];
+  int32_t claim_v[64];
+  uint32_t claim_deg[64];
 };
 __shared__ WarpTile s_tiles[kBfsWarps];
 __shared__ WarpExpand s_expand[kBfsWarps];
@@ -185,64 +189,107 @@ __device__ __forceinline__ void enqueue_claims(const BfsParams &p, bool claimed,
 
 // Edge u -> v of a push round.  Returns true for the one thread that claims
 // v, with v's out-degree in deg (its offsets are loaded with the claim, so the
-// claimer does not wait for them afterwards).
+// claimer does not wait for them afterwards).  A target claimed already gets
+// a read before its atomicMin: most of a big round's edges lead to vertices
+// that a lower source has reached, and a read costs the L2 less.
 __device__ __forceinline__ bool relax_push(const BfsParams &p, const uint32_t *cur,
                                            uint32_t *nxt, int32_t u, int32_t v, int next_level,
-                                           int64_t &deg) {
+                                           uint32_t &deg) {
   const uint32_t w = (uint32_t)v >> 5, bit = 1u << (v & 31);
   // the three words in one round trip: a claim bit seen set stays set
   const uint32_t seen = p.vis[w] | cur[w], claimed = nxt[w];
   if (seen & bit) return false;
   const int32_t ov = orig_id(p, v);
-  atomicMin(reinterpret_cast<unsigned *>(p.parents) + ov, (unsigned)orig_id(p, u));
-  if (claimed & bit) return false;
+  unsigned *par = reinterpret_cast<unsigned *>(p.parents) + ov;
+  const unsigned ou = (unsigned)orig_id(p, u);
+  if (claimed & bit) {
+    if (__ldcg(par) > ou) atomicMin(par, ou);
+    return false;
+  }
+  atomicMin(par, ou);
   const int64_t o0 = __ldg(p.out_off + v), o1 = __ldg(p.out_off + v + 1);
   const unsigned old = atomicOr(nxt + w, bit);
   if (old & bit) return false;
   p.levels[ov] = next_level;
-  deg = o1 - o0;
+  deg = (uint32_t)(o1 - o0);
   return true;
+}
+
+// Claimed vertices on their way to the next frontier's queue: a warp keeps
+// them in shared memory and queues 32 at a time, so a round makes one returning
+// atomic on the shared queue counter per 32 claims instead of one per step with
+// any claim -- at R-MAT scales that counter bounded the big push rounds -- and
+// the steps do not wait for it.  Rounds of 61,564
+// claims (R-MAT n = 100,003, top-down): 68 -> 37 us; of 862,250 (scale 23): 235
+// -> 174 us.
+struct Claims {
+  WarpExpand &X;
+  unsigned count = 0;  // entries waiting (the same in every lane), < 32 between steps
+};
+
+__device__ __forceinline__ void queue_claims(const BfsParams &p, Claims &C, unsigned n,
+                                             unsigned from, int next_parity, RoundRec *Rn,
+                                             Acc &acc) {
+  const unsigned i = from + (unsigned)lane_id();
+  const bool has = (unsigned)lane_id() < n;
+  const int32_t v = has ? C.X.claim_v[i] : 0;
+  const uint32_t d = has ? C.X.claim_deg[i] : 0u;
+  enqueue_claims(p, has, v, (int64_t)d, next_parity, Rn, acc);
 }
 
 __device__ __forceinline__ void push_step(const BfsParams &p, const uint32_t *cur, uint32_t *nxt,
                                           bool valid, int32_t u, int64_t e, int L,
-                                          int next_parity, RoundRec *Rn, Acc &acc) {
+                                          int next_parity, RoundRec *Rn, Claims &C, Acc &acc) {
   bool claimed = false;
   int32_t v = 0;
-  int64_t deg = 0;
+  uint32_t deg = 0;
   if (valid) {
     v = __ldg(p.out_idx + e);
     claimed = relax_push(p, cur, nxt, u, v, L + 1, deg);
   }
-  enqueue_claims(p, claimed, v, deg, next_parity, Rn, acc);
+  const unsigned m = __ballot_sync(kFull, claimed);
+  if (!m) return;
+  if (claimed) {
+    const unsigned at = C.count + __popc(m & ((1u << lane_id()) - 1u));
+    C.X.claim_v[at] = v;
+    C.X.claim_deg[at] = deg;
+  }
+  C.count += __popc(m);
+  __syncwarp();
+  if (C.count >= 32) {
+    C.count -= 32;  // the last 32: the entries below keep their places
+    queue_claims(p, C, 32, C.count, next_parity, Rn, acc);
+    __syncwarp();
+  }
 }
 
 // Expands up to 32 frontier vertices (one per lane, u < 0 for none) with the
 // warp's combined edge list spread evenly over its lanes.
 __device__ __forceinline__ void gather_expand(const BfsParams &p, const uint32_t *cur,
                                               uint32_t *nxt, int32_t u, int L, int next_parity,
-                                              RoundRec *Rn, Acc &acc, int32_t *s_u, int64_t *s_s,
-                                              int64_t *s_x) {
+                                              RoundRec *Rn, Claims &C, Acc &acc) {
   const int lane = lane_id();
-  int64_t s = 0, d = 0;
+  WarpExpand &X = C.X;
+  uint32_t s = 0, d = 0;
   if (u >= 0) {
-    s = __ldg(p.out_off + u);
-    d = __ldg(p.out_off + u + 1) - s;
+    const int64_t o = __ldg(p.out_off + u);
+    s = (uint32_t)o;
+    d = (uint32_t)(__ldg(p.out_off + u + 1) - o);
   }
-  int64_t incl = d;
+  uint32_t incl = d;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const int64_t t = __shfl_up_sync(kFull, incl, o);
+    const uint32_t t = __shfl_up_sync(kFull, incl, o);
     if (lane >= o) incl += t;
   }
-  const int64_t total = __shfl_sync(kFull, incl, 31);
+  const uint32_t total = __shfl_sync(kFull, incl, 31);
   if (total == 0) return;
-  s_u[lane] = u;
-  s_s[lane] = s;
-  s_x[lane] = incl - d;
+  X.u[lane] = u;
+  X.s[lane] = s;
+  X.x[lane] = incl - d;
   __syncwarp();
-  for (int64_t base = 0; base < total; base += 32) {
-    const int64_t t = base + lane;
+  for (uint32_t base = 0; base < total; base += 32) {
+    const uint32_t t = base + lane;
     const bool valid = t < total;
     int32_t uu = 0;
     int64_t e = 0;
@@ -250,22 +297,27 @@ __device__ __forceinline__ void gather_expand(const BfsParams &p, const uint32_t
       int lo = 0, hi = 31;
       while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if (s_x[mid] <= t)
+        if (X.x[mid] <= t)
           lo = mid;
         else
           hi = mid - 1;
       }
-      uu = s_u[lo];
-      e = s_s[lo] + (t - s_x[lo]);
+      uu = X.u[lo];
+      e = (int64_t)(X.s[lo] + (t - X.x[lo]));
     }
-    push_step(p, cur, nxt, valid, uu, e, L, next_parity, Rn, acc);
+    push_step(p, cur, nxt, valid, uu, e, L, next_parity, Rn, C, acc);
+    if (base + 32 < base) break;  // total within 32 of 2^32
   }
   __syncwarp();
 }
 
 // Expands frontier F_L from its queue (parity L & 1): edge-balanced chunks of
-// the big vertices' combined edge list, then the light vertices 32 to a warp.
-// Item i goes to warp i first; warps that finish take the rest from a counter.
+// the big vertices' combined edge list, then the light vertices, up to 32 to
+// a warp.  A frontier of fewer light vertices than 32 a warp is spread over
+// more warps (`group` each): a warp's steps run one after the other, about 2.6
+// us each with cold lists, so 415 vertices of degree 8 took 8 steps on 13
+// warps where one step on 415 does (29 -> 11 us a round; 26,618 vertices: 50 ->
+// 16 us).  Item i goes to warp i first; warps that finish take the rest from a counter.
 // bigw / nlight: F_L's queue sizes ((big count << 32) | big edges, light
 // count), handed over with the barrier that ended round L - 1.
 __device__ void push_round_queue(const BfsParams &p, const uint32_t *cur, uint32_t *nxt, int L,
@@ -284,7 +336,10 @@ __device__ void push_round_queue(const BfsParams &p, const uint32_t *cur, uint32
   unsigned chunk = ((big_edges / (unsigned)nwarps) + 31u) & ~31u;
   chunk = chunk < 32u ? 32u : (chunk > (unsigned)kPushChunk ? (unsigned)kPushChunk : chunk);
   const unsigned nchunks = (big_edges + chunk - 1) / chunk;
-  const unsigned nitems = nchunks + (nlight + 31u) / 32u;
+  unsigned group = 1;
+  while (group < 32u && nlight > group * (unsigned)nwarps) group <<= 1;
+  const unsigned nitems = nchunks + (nlight + group - 1) / group;
+  Claims C{s_expand[wib]};
   unsigned item = (unsigned)warp_id_global();
   while (item < nitems) {
     // the next item is claimed before this one is worked, hiding the atomic
@@ -326,16 +381,16 @@ __device__ void push_round_queue(const BfsParams &p, const uint32_t *cur, uint32
             e = __ldg(p.out_off + vn) + (int64_t)(x - endj);
           }
         }
-        push_step(p, cur, nxt, valid, u, e, L, next_parity, Rn, acc);
+        push_step(p, cur, nxt, valid, u, e, L, next_parity, Rn, C, acc);
       }
     } else {
-      const unsigned idx = (item - nchunks) * 32u + lane;
-      WarpExpand &X = s_expand[wib];
-      gather_expand(p, cur, nxt, idx < nlight ? q[idx] : -1, L, next_parity, Rn, acc, X.u, X.s,
-                    X.x);
+      const unsigned idx = (item - nchunks) * group + lane;
+      gather_expand(p, cur, nxt, (unsigned)lane < group && idx < nlight ? q[idx] : -1, L,
+                    next_parity, Rn, C, acc);
     }
     item = __shfl_sync(kFull, nextitem, 0);
   }
+  if (C.count) queue_claims(p, C, C.count, 0, next_parity, Rn, acc);
 }
 
 // Work items of a bitmap-wide round: (tile, slot) pairs; a tile holds 4096
@@ -368,7 +423,7 @@ __device__ void push_round_bitmap(const BfsParams &p, const uint32_t *cur, uint3
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int next_parity = (L + 1) & 1;
   WarpTile &T = s_tiles[wib];
-  WarpExpand &X = s_expand[wib];
+  Claims C{s_expand[wib]};
   const unsigned S = tile_slots(p.tiles, nwarps, heavy);
   const int64_t items = p.tiles * S;
   for (int64_t item = warp_id_global(); item < items; item = next_item(item, nwarps, Rc, heavy)) {
@@ -384,10 +439,11 @@ __device__ void push_round_bitmap(const BfsParams &p, const uint32_t *cur, uint3
         select_bit(T, b + lane, j, bit);
         u = (int32_t)((t * kTileWords + j) * 32 + bit);
       }
-      gather_expand(p, cur, nxt, u, L, next_parity, Rn, acc, X.u, X.s, X.x);
+      gather_expand(p, cur, nxt, u, L, next_parity, Rn, C, acc);
     }
     __syncwarp();  // T is restaged by the next item
   }
+  if (C.count) queue_claims(p, C, C.count, 0, next_parity, Rn, acc);
 }
 
 // Bottom-up round: every unvisited vertex scans its ascending in-list and
