@@ -74,6 +74,17 @@ struct RoundRec {
   unsigned long long pad[6];
 };
 
+// What block 0 hands the other blocks when its run of small rounds ends (or,
+// `still`, goes on past a bounded wait): the round to run next, the decision
+// for it and the search-wide bookkeeping.
+struct SoloExit {
+  unsigned long long visited, prev_nf, explored, next_big;
+  int pull_rounds, switches, L, still;
+  unsigned next_light, payload;
+  unsigned listed;             // frontier vertices collected from the bitmap
+  unsigned pad[17];
+};
+
 // Control block of one per-root search, zeroed before every launch.  The
 // search-wide bookkeeping (visited total, explored edges, ...) is not here:
 // every block keeps its own copy, updated from the same round totals.
@@ -82,6 +93,7 @@ struct BfsCtl {
   unsigned long long pad0[15];
   int status;                  // first error (CG_ERR_TIMEOUT, CG_ERR_LEVEL_CAP), else 0
   int pad1[31];
+  SoloExit solo;
   RoundRec rec[kRing];
 };
 
