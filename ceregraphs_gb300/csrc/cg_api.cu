@@ -36,12 +36,7 @@ static void free_graph(cg_graph *g) {
   if (g->out_idx && g->out_idx != g->in_idx) cudaFree(g->out_idx);
   cudaFree(g->in_off);
   cudaFree(g->in_idx);
-  cudaFree(g->bitmaps);
-  cudaFree(g->dead);
-  cudaFree(g->queue);
-  cudaFree(g->bigoff);
-  cudaFree(g->ctl);
-  cudaFree(g->d_stats);
+  cudaFree(g->state);
   cudaFree(g->tmp_levels);
   cudaFree(g->tmp_parents);
   cudaFree(g->orig);
@@ -76,6 +71,65 @@ static int upload(const void *src, size_t bytes, bool device_src, void **dst, cg
                                                                   : cudaMemcpyHostToDevice,
                                      g->stream));
   return CG_OK;
+}
+
+// A handle without arrays yet.
+static int graph_open(int64_t n, int64_t nnz, bool symmetric, cg_graph **out) {
+  cg_graph *g = new (std::nothrow) cg_graph();
+  if (!g) return CG_ERR_OUT_OF_MEMORY;
+  if (cudaGetDevice(&g->device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&g->num_sms, cudaDevAttrMultiProcessorCount, g->device) !=
+          cudaSuccess ||
+      cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking) != cudaSuccess) {
+    free_graph(g);
+    return CG_ERR_CUDA;
+  }
+  cudaEventCreate(&g->ev0);
+  cudaEventCreate(&g->ev1);
+  g->n = n;
+  g->nnz = nnz;
+  g->symmetric = symmetric;
+  cg_default_options(&g->opt);
+  g->opt.tau_switch_count = (int64_t)(0.15 * (double)n + 0.5);
+  *out = g;
+  return CG_OK;
+}
+
+// The handle's arrays are in place (rc 0) or could not be had: sets up its
+// per-root search state, or frees it.
+static int graph_finish(cg_graph *g, int rc, cg_graph **out) {
+  if (!rc && g->symmetric) {
+    g->out_off = g->in_off;
+    g->out_idx = g->in_idx;
+  }
+  if (!rc) rc = bfs_prepare(g);  // waits for the uploads too
+  if (rc) {
+    free_graph(g);
+    return rc;
+  }
+  *out = g;
+  return CG_OK;
+}
+
+int graph_adopt(int64_t n, int64_t nnz, int64_t *in_off, int32_t *in_idx, int64_t *out_off,
+                int32_t *out_idx, bool symmetric, cg_graph **out) {
+  cg_graph *g = nullptr;
+  const int rc = graph_open(n, nnz, symmetric, &g);
+  if (rc) {
+    cudaFree(in_off);
+    cudaFree(in_idx);
+    cudaFree(out_off);
+    cudaFree(out_idx);
+    return rc;
+  }
+  g->in_off = in_off;
+  g->in_idx = in_idx;
+  g->out_off = out_off;
+  g->out_idx = out_idx;
+  const int lists = symmetric ? 1 : 2;
+  g->device_bytes += lists * (int64_t)(sizeof(int64_t) * (size_t)(n + 1) +
+                                       sizeof(int32_t) * (size_t)nnz);
+  return graph_finish(g, CG_OK, out);
 }
 
 int call_scratch(cg_graph *g, size_t bytes, void **out) {
@@ -156,48 +210,22 @@ int cg_graph_create(int64_t n, int64_t nnz, const int64_t *in_off, const int32_t
     if (!valid_host_csr(n, nnz, in_off, in_idx)) return CG_ERR_INVALID_ARG;
     if (!sym && !valid_host_csr(n, nnz, out_off, out_idx)) return CG_ERR_INVALID_ARG;
   }
-  cg_graph *g = new (std::nothrow) cg_graph();
-  if (!g) return CG_ERR_OUT_OF_MEMORY;
-  int rc = CG_OK;
+  cg_graph *g = nullptr;
+  int rc = graph_open(n, nnz, sym, &g);
+  if (rc) return rc;
   do {
-    if (cudaGetDevice(&g->device) != cudaSuccess) { rc = CG_ERR_CUDA; break; }
-    if (cudaDeviceGetAttribute(&g->num_sms, cudaDevAttrMultiProcessorCount, g->device) !=
-        cudaSuccess) { rc = CG_ERR_CUDA; break; }
-    if (cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking) != cudaSuccess) {
-      rc = CG_ERR_CUDA;
-      break;
-    }
-    cudaEventCreate(&g->ev0);
-    cudaEventCreate(&g->ev1);
-    g->n = n;
-    g->nnz = nnz;
-    g->symmetric = sym;
-    cg_default_options(&g->opt);
-    g->opt.tau_switch_count = (int64_t)(0.15 * (double)n + 0.5);
     rc = upload(in_off, sizeof(int64_t) * (size_t)(n + 1), dev, (void **)&g->in_off, g);
     if (rc) break;
     rc = upload(in_idx, sizeof(int32_t) * (size_t)nnz, dev, (void **)&g->in_idx, g);
     if (rc) break;
-    if (sym) {
-      g->out_off = g->in_off;
-      g->out_idx = g->in_idx;
-    } else {
+    if (!sym) {
       rc = upload(out_off, sizeof(int64_t) * (size_t)(n + 1), dev, (void **)&g->out_off, g);
       if (rc) break;
       rc = upload(out_idx, sizeof(int32_t) * (size_t)nnz, dev, (void **)&g->out_idx, g);
       if (rc) break;
     }
-    rc = bfs_prepare(g);
-    if (rc) break;
-    cudaError_t e = cudaStreamSynchronize(g->stream);
-    if (e != cudaSuccess) { rc = cuda_fail(e, "cg_graph_create"); break; }
   } while (0);
-  if (rc) {
-    free_graph(g);
-    return rc;
-  }
-  *out = g;
-  return CG_OK;
+  return graph_finish(g, rc, out);
 }
 
 int cg_graph_destroy(cg_graph *g) {

@@ -1411,37 +1411,28 @@ int64_t bfs_big_capacity(int64_t n, int64_t nnz) {
   return c < n ? c : n;
 }
 
-// Vertices with in-edges: n minus the dead bits below n.
-__global__ void live_count_kernel(int64_t n, int64_t words, const uint32_t *__restrict__ dead,
-                                  unsigned long long *live) {
-  unsigned long long c = 0;
-  for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < words;
-       w += (int64_t)gridDim.x * blockDim.x)
-    c += (unsigned long long)__popc(~dead[w] & valid_bits(w, n));
-  c = warp_sum(c);
-  if (lane_id() == 0 && c) atomicAdd(live, c);
-}
-
 // Bit v of dead[v / 32]: vertex v has no in-edges, so no round reaches it
-// (bits past n are set too, through the tile padding: `words` = stride).
+// (bits past n are set too, through the tile padding: `words` = stride).  A
+// warp takes 32 words, a coalesced load of 33 offsets each.  *live: vertices
+// with in-edges.
 __global__ void dead_map_kernel(int64_t n, int64_t words, const int64_t *__restrict__ in_off,
-                                uint32_t *dead) {
-  for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < words;
-       w += (int64_t)gridDim.x * blockDim.x) {
-    uint32_t m = 0;
-    int64_t prev = w * 32 < n ? in_off[w * 32] : 0;
-    for (int b = 0; b < 32; ++b) {
-      const int64_t v = w * 32 + b;
-      if (v >= n) {
-        m |= 1u << b;
-        continue;
-      }
-      const int64_t next = in_off[v + 1];
-      if (next == prev) m |= 1u << b;
-      prev = next;
+                                uint32_t *dead, unsigned long long *live) {
+  const int lane = lane_id();
+  unsigned long long alive = 0;
+  const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t w0 = (int64_t)warp_id_global() * 32; w0 < words; w0 += warps * 32) {
+    uint32_t mine = 0;
+    for (int j = 0; j < 32 && w0 + j < words; ++j) {
+      const int64_t v = (w0 + j) * 32 + lane;
+      const bool none = v >= n || __ldg(in_off + v) == __ldg(in_off + v + 1);
+      const uint32_t m = __ballot_sync(kFull, none);
+      if (lane == j) mine = m;
     }
-    dead[w] = m;
+    if (w0 + lane < words) dead[w0 + lane] = mine;
+    if (w0 + lane < words) alive += (unsigned)__popc(~mine);
   }
+  alive = warp_sum(alive);
+  if (lane == 0 && alive) atomicAdd(live, alive);
 }
 
 int refuse_setup_in_capture(cg_graph *g) {
@@ -1452,111 +1443,53 @@ int refuse_setup_in_capture(cg_graph *g) {
   return CG_ERR_NOT_SUPPORTED;
 }
 
-// A handle's one-time per-root set-up runs on a private stream and is waited
-// for, so it is done once and at once even when the first search is issued
-// inside a capture of the handle's stream (which would only record it).  Work
-// still queued on the handle's stream (the graph upload) is waited for first.
-static int setup_stream(cg_graph *g, cudaStream_t *s) {
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  CG_CUDA(cudaStreamIsCapturing(g->stream, &cs));
-  if (cs == cudaStreamCaptureStatusNone) CG_CUDA(cudaStreamSynchronize(g->stream));
-  CG_CUDA(cudaStreamCreateWithFlags(s, cudaStreamNonBlocking));
-  return CG_OK;
-}
-
-static int setup_wait(cudaStream_t s) {
-  const cudaError_t e = cudaStreamSynchronize(s);
-  cudaStreamDestroy(s);
-  return e == cudaSuccess ? CG_OK : cuda_fail(e, "search state set-up");
-}
-
-int dead_prepare(cg_graph *g) {
-  if (g->dead) return CG_OK;
-  const int64_t words = bitmap_stride(g->n);
-  uint32_t *dead = nullptr;
-  unsigned long long *d_live = nullptr;  // the live count, read back once
-  if (cudaMalloc(&dead, sizeof(uint32_t) * (size_t)words) != cudaSuccess ||
-      cudaMalloc(&d_live, sizeof(unsigned long long)) != cudaSuccess) {
-    cudaFree(dead);
-    return CG_ERR_OUT_OF_MEMORY;
-  }
-  unsigned long long live = 0;
-  cudaStream_t s = nullptr;
-  int rc = setup_stream(g, &s);
-  if (!rc) {
-    const int64_t blocks = (words + 255) / 256;
-    const unsigned grid = (unsigned)(blocks < 4096 ? blocks : 4096);
-    cudaError_t e = cudaMemsetAsync(d_live, 0, sizeof(unsigned long long), s);
-    dead_map_kernel<<<grid, 256, 0, s>>>(g->n, words, g->in_off, dead);
-    live_count_kernel<<<grid, 256, 0, s>>>(g->n, words, dead, d_live);
-    if (e == cudaSuccess) e = cudaGetLastError();
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(&live, d_live, sizeof(live), cudaMemcpyDeviceToHost, s);
-    rc = setup_wait(s);
-    if (!rc && e != cudaSuccess) rc = cuda_fail(e, "dead-vertex map");
-  }
-  cudaFree(d_live);
-  if (rc) {
-    cudaFree(dead);
-    return rc;
-  }
-  g->dead = dead;
-  g->live = (int64_t)live;
-  g->device_bytes += sizeof(uint32_t) * words;
-  return CG_OK;
-}
-
+// The per-root search state of a new handle: one allocation, set up on the
+// handle's stream behind the upload of its arrays (the caller waits).
 int bfs_prepare(cg_graph *g) {
-  if (g->d_stats) return CG_OK;  // the last of the buffers below: all are in place
-  int rc = dead_prepare(g);
-  if (rc) return rc;
   int dev_coop = 0;
   CG_CUDA(cudaDeviceGetAttribute(&dev_coop, cudaDevAttrCooperativeLaunch, g->device));
   if (!dev_coop) return CG_ERR_NOT_SUPPORTED;
-  const int64_t words = (g->n + 31) / 32;
+  const int64_t stride = bitmap_stride(g->n);
   const int64_t bcap = bfs_big_capacity(g->n, g->nnz);
-  const size_t bytes_bm = sizeof(uint32_t) * 4 * (size_t)bitmap_stride(g->n);
-  const size_t bytes_q = sizeof(int32_t) * 2 * (size_t)g->n;
-  const size_t bytes_b = sizeof(uint32_t) * 2 * (size_t)bcap;
-  uint32_t *bitmaps = nullptr, *bigoff = nullptr;
-  int32_t *queue = nullptr;
-  BfsCtl *ctl = nullptr;
-  cg_stats *stats = nullptr;
-  if (cudaMalloc(&bitmaps, bytes_bm) != cudaSuccess || cudaMalloc(&queue, bytes_q) != cudaSuccess ||
-      cudaMalloc(&bigoff, bytes_b) != cudaSuccess || cudaMalloc(&ctl, sizeof(BfsCtl)) != cudaSuccess ||
-      cudaMalloc(&stats, sizeof(cg_stats)) != cudaSuccess) {
-    cudaFree(bitmaps);
-    cudaFree(queue);
-    cudaFree(bigoff);
-    cudaFree(ctl);
-    cudaFree(stats);
+  size_t bytes = 0;
+  auto piece = [&](size_t size) {
+    const size_t at = bytes;
+    bytes = (bytes + size + 255) & ~(size_t)255;
+    return at;
+  };
+  const size_t at_ctl = piece(sizeof(BfsCtl));
+  const size_t at_stats = piece(sizeof(cg_stats));
+  const size_t at_live = piece(sizeof(unsigned long long));
+  const size_t zeroed = bytes;
+  const size_t at_bitmaps = piece(sizeof(uint32_t) * 4 * (size_t)stride);
+  const size_t at_dead = piece(sizeof(uint32_t) * (size_t)stride);
+  const size_t at_queue = piece(sizeof(int32_t) * 2 * (size_t)g->n);
+  const size_t at_bigoff = piece(sizeof(uint32_t) * 2 * (size_t)bcap);
+  unsigned char *base = nullptr;
+  if (cudaMalloc(&base, bytes) != cudaSuccess) {
+    cudaGetLastError();
     return CG_ERR_OUT_OF_MEMORY;
   }
-  cudaStream_t s = nullptr;
-  rc = setup_stream(g, &s);
-  cudaError_t e = cudaSuccess;
-  if (!rc) {
-    e = cudaMemsetAsync(ctl, 0, sizeof(BfsCtl), s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(stats, 0, sizeof(cg_stats), s);
-    rc = setup_wait(s);
-    if (!rc && e != cudaSuccess) rc = cuda_fail(e, "search state reset");
-  }
-  if (rc) {
-    cudaFree(bitmaps);
-    cudaFree(queue);
-    cudaFree(bigoff);
-    cudaFree(ctl);
-    cudaFree(stats);
-    return rc;
-  }
-  g->words = words;
+  g->state = base;
+  g->device_bytes += (int64_t)bytes;
+  g->words = (g->n + 31) / 32;
   g->bcap = bcap;
-  g->bitmaps = bitmaps;
-  g->queue = queue;
-  g->bigoff = bigoff;
-  g->ctl = ctl;
-  g->d_stats = stats;
-  g->device_bytes += bytes_bm + bytes_q + bytes_b + sizeof(BfsCtl) + sizeof(cg_stats);
+  g->ctl = reinterpret_cast<BfsCtl *>(base + at_ctl);
+  g->d_stats = reinterpret_cast<cg_stats *>(base + at_stats);
+  g->bitmaps = reinterpret_cast<uint32_t *>(base + at_bitmaps);
+  g->dead = reinterpret_cast<uint32_t *>(base + at_dead);
+  g->queue = reinterpret_cast<int32_t *>(base + at_queue);
+  g->bigoff = reinterpret_cast<uint32_t *>(base + at_bigoff);
+  unsigned long long *d_live = reinterpret_cast<unsigned long long *>(base + at_live);
+  unsigned long long live = 0;
+  CG_CUDA(cudaMemsetAsync(base, 0, zeroed, g->stream));
+  const int64_t blocks = (stride + 255) / 256;  // 8 warps of 32 words
+  dead_map_kernel<<<(unsigned)(blocks < 4096 ? blocks : 4096), 256, 0, g->stream>>>(
+      g->n, stride, g->in_off, g->dead, d_live);
+  CG_CUDA(cudaGetLastError());
+  CG_CUDA(cudaMemcpyAsync(&live, d_live, sizeof(live), cudaMemcpyDeviceToHost, g->stream));
+  CG_CUDA(cudaStreamSynchronize(g->stream));
+  g->live = (int64_t)live;
   return CG_OK;
 }
 
@@ -1576,9 +1509,8 @@ static int bfs_grid(cg_graph *g) {
 
 int bfs_launch(cg_graph *g, int64_t root, int32_t *d_levels, int32_t *d_parents,
                int32_t *host_levels, int32_t *host_parents) {
-  int rc = bfs_prepare(g);
+  const int rc = bfs_grid(g);
   if (rc) return rc;
-  if ((rc = bfs_grid(g))) return rc;
   BfsParams p;
   p.n = g->n;
   p.nnz = g->nnz;

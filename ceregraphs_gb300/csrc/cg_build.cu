@@ -14,8 +14,17 @@
 // every quadrant test "r >= t" is done exactly on the 53-bit integer against
 // ceil(t * 2^53), computed on the host.
 //
-// CSR build: one 64-bit key (row << 32 | col) per stored entry, a CUB radix
-// sort, CUB unique, and a binary search per row for the offsets.
+// CSR build: CUB radix sorts of as few keys and as few bits as will do.  A
+// symmetrised graph sorts each undirected edge once, as (low end, high end);
+// that is the upper triangle, and its stable sort by the high end (32-bit keys)
+// is the lower one, whose entries precede the upper ones in every row.  A
+// directed graph's CSC is the stable sort of its CSR by column.  Keys hold
+// 2 * ceil(log2 n) bits, dropped loops the key 0 = (0, 0), which cannot be an
+// entry then.  Offsets come from the places where the sorted rows change.
+// Bound by the sorts' passes over memory (8 bits a pass).  R-MAT scale 20, 16.8
+// M edges: 5 passes of 16.8 M 64-bit keys and 3 of 15.7 M 32-bit pairs where one
+// sort of both directions took 7 of 33.5 M; device time 2580 -> 1620 us (with
+// one search).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -123,45 +132,126 @@ __global__ void uniform_bits_kernel(uint64_t st_hi, uint64_t st_lo, uint64_t inc
     out[e0 + j] = (uint32_t)((pcg_next(s, inc) >> 11) >> (53 - bits));
 }
 
-// one key per stored entry: row = dst, col = src (A[dst, src] = edge src -> dst)
+// One key per edge: (row = dst) << bits | (col = src), or, symmetrised, the
+// smaller end << bits | the larger one.
 __global__ void edge_keys_kernel(int64_t m, const uint32_t *__restrict__ src,
                                  const uint32_t *__restrict__ dst, int symmetrize,
-                                 int drop_loops, uint64_t sentinel, uint64_t *__restrict__ keys) {
+                                 int drop_loops, int bits, uint64_t *__restrict__ keys) {
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m;
        e += (int64_t)gridDim.x * blockDim.x) {
-    const uint64_t s = src[e], d = dst[e];
-    const bool loop = drop_loops && s == d;
-    keys[e] = loop ? sentinel : ((d << 32) | s);
-    if (symmetrize) keys[m + e] = loop ? sentinel : ((s << 32) | d);
+    const uint32_t s = src[e], d = dst[e];
+    const uint64_t hi = symmetrize ? min(s, d) : d, lo = symmetrize ? max(s, d) : s;
+    keys[e] = drop_loops && s == d ? 0ull : (hi << bits) | lo;
   }
 }
 
-__global__ void swap_halves_kernel(int64_t nnz, const uint64_t *__restrict__ in,
-                                   uint64_t *__restrict__ out) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nnz;
+// Rows without entries between two that have some, too many for one thread.
+struct Gap {
+  uint32_t first, last, at;  // rows [first, last] start at position `at`
+};
+constexpr int64_t kGapRows = 64;        // rows a thread fills itself
+constexpr int64_t kGapPiece = 1 << 16;  // rows per listed piece of a longer gap
+static int64_t gap_capacity(int64_t n) { return n / kGapRows + n / kGapPiece + 2; }
+
+// first[r] = the first position whose row is >= r, for the rows after that of
+// position i - 1 up to that of position i (every r <= n over all i <= count);
+// long gaps go on a list for fill_gaps_kernel.  Rows past n count as n.
+__device__ __forceinline__ void mark_rows(int64_t n, int64_t count, int64_t i, int64_t before,
+                                          int64_t row, uint32_t *__restrict__ first,
+                                          Gap *__restrict__ gaps, unsigned *ngaps) {
+  const int64_t r0 = i > 0 ? min(before, n) + 1 : 0, r1 = i < count ? min(row, n) : n;
+  if (r1 - r0 < kGapRows) {
+    for (int64_t r = r0; r <= r1; ++r) first[r] = (uint32_t)i;
+    return;
+  }
+  const unsigned pieces = (unsigned)((r1 - r0) / kGapPiece) + 1;
+  unsigned at = atomicAdd(ngaps, pieces);
+  for (int64_t r = r0; r <= r1; r += kGapPiece)
+    gaps[at++] = Gap{(uint32_t)r, (uint32_t)min(r + kGapPiece - 1, r1), (uint32_t)i};
+}
+
+__global__ void fill_gaps_kernel(const Gap *__restrict__ gaps, const unsigned *ngaps,
+                                 uint32_t *__restrict__ first) {
+  const unsigned count = *ngaps;
+  for (unsigned g = blockIdx.x; g < count; g += gridDim.x) {
+    const Gap x = gaps[g];
+    for (uint32_t r = x.first + threadIdx.x; r <= x.last && r >= x.first; r += blockDim.x)
+      first[r] = x.at;
+  }
+}
+
+// Row starts of the sorted keys, and each key's (column, row) for the sort by
+// column.  `loop_row`, if not negative: the column given to a loop (a
+// symmetrised graph's upper triangle holds it already).
+__global__ void split_keys_kernel(int64_t n, int64_t count, const uint64_t *__restrict__ keys,
+                                  int bits, int64_t loop_row, uint32_t *__restrict__ first,
+                                  uint32_t *__restrict__ cols, uint32_t *__restrict__ rows,
+                                  Gap *__restrict__ gaps, unsigned *ngaps) {
+  const uint64_t mask = (1ull << bits) - 1ull;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= count;
        i += (int64_t)gridDim.x * blockDim.x) {
-    const uint64_t k = in[i];
-    out[i] = (k << 32) | (k >> 32);
+    const uint64_t k = i < count ? keys[i] : 0ull;
+    const int64_t row = (int64_t)(k >> bits);
+    mark_rows(n, count, i, i > 0 ? (int64_t)(keys[i - 1] >> bits) : 0, row, first, gaps, ngaps);
+    if (i == count) continue;
+    const uint32_t col = (uint32_t)(k & mask);
+    cols[i] = loop_row >= 0 && col == row ? (uint32_t)loop_row : col;
+    rows[i] = (uint32_t)row;
   }
 }
 
-__global__ void csr_from_keys_kernel(int64_t n, int64_t nnz, const uint64_t *__restrict__ keys,
-                                     int64_t *__restrict__ off, int32_t *__restrict__ idx) {
+__global__ void row_starts_kernel(int64_t n, int64_t count, const uint32_t *__restrict__ rows,
+                                  uint32_t *__restrict__ first, Gap *__restrict__ gaps,
+                                  unsigned *ngaps) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= count;
+       i += (int64_t)gridDim.x * blockDim.x)
+    mark_rows(n, count, i, i > 0 ? rows[i - 1] : 0, i < count ? rows[i] : 0, first, gaps, ngaps);
+}
+
+// CSR of the sorted keys (first: its row starts).
+__global__ void csr_kernel(int64_t n, int64_t nnz, const uint64_t *__restrict__ keys, int bits,
+                           const uint32_t *__restrict__ first, int64_t *__restrict__ off,
+                           int32_t *__restrict__ idx) {
+  const uint64_t mask = (1ull << bits) - 1ull;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  for (int64_t i = t0; i < nnz; i += stride) idx[i] = (int32_t)(keys[i] & 0xffffffffull);
-  for (int64_t r = t0; r <= n; r += stride) {
-    const uint64_t target = (uint64_t)r << 32;
-    int64_t lo = 0, hi = nnz;
-    while (lo < hi) {
-      const int64_t mid = (lo + hi) >> 1;
-      if (keys[mid] < target)
-        lo = mid + 1;
-      else
-        hi = mid;
-    }
-    off[r] = lo;
+  for (int64_t i = t0; i < nnz; i += stride) idx[i] = (int32_t)(keys[i] & mask);
+  for (int64_t r = t0; r <= n; r += stride) off[r] = first[r];
+}
+
+// The same from (row, column) pairs sorted by row.
+__global__ void csr_pairs_kernel(int64_t n, int64_t nnz, const uint32_t *__restrict__ cols,
+                                 const uint32_t *__restrict__ first, int64_t *__restrict__ off,
+                                 int32_t *__restrict__ idx) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (int64_t i = t0; i < nnz; i += stride) idx[i] = (int32_t)cols[i];
+  for (int64_t r = t0; r <= n; r += stride) off[r] = first[r];
+}
+
+// CSR of a symmetrised graph.  up: row starts of the upper triangle's keys;
+// low: row starts of the lower triangle's pairs.  A row's lower entries come
+// first, so row r starts at up[r] + low[r]; the upper entry at position i lies
+// behind the lower entries of rows 0 .. its own, at i + low[row + 1], the lower
+// one at position j behind the upper entries of the rows before, at j + up[row].
+__global__ void csr_symmetric_kernel(int64_t n, int64_t nu, int64_t nl,
+                                     const uint64_t *__restrict__ keys, int bits,
+                                     const uint32_t *__restrict__ up,
+                                     const uint32_t *__restrict__ low_rows,
+                                     const uint32_t *__restrict__ low_cols,
+                                     const uint32_t *__restrict__ low, int64_t *__restrict__ off,
+                                     int32_t *__restrict__ idx) {
+  const uint64_t mask = (1ull << bits) - 1ull;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (int64_t i = t0; i < nu; i += stride) {
+    const uint64_t k = keys[i];
+    const int64_t row = min((int64_t)(k >> bits), n - 1);
+    idx[i + low[row + 1]] = (int32_t)(k & mask);
   }
+  for (int64_t j = t0; j < nl; j += stride)
+    idx[j + up[min((int64_t)low_rows[j], n)]] = (int32_t)low_cols[j];
+  for (int64_t r = t0; r <= n; r += stride) off[r] = (int64_t)up[r] + low[r];
 }
 
 // A == A^T exactly when the CSR and the CSC of the same entries coincide.
@@ -185,50 +275,47 @@ static int grid_for(int64_t work, int num_sms) {
   return (int)b;
 }
 
-// Sorts `count` keys in place (using `tmp` of the same size), removes
-// duplicates and sentinel keys; returns the number kept in *kept and the
-// buffer holding them in *result (keys or tmp).
-static int sort_unique(uint64_t *keys, uint64_t *tmp, int64_t count, int end_bit,
-                       uint64_t sentinel, cudaStream_t stream, uint64_t **result,
-                       int64_t *kept) {
-  size_t tb_sort = 0, tb_uniq = 0;
-  cub::DoubleBuffer<uint64_t> db(keys, tmp);
-  CG_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, tb_sort, db, count, 0, end_bit, stream));
-  int64_t *d_num = nullptr;
-  CG_CUDA(cub::DeviceSelect::Unique(nullptr, tb_uniq, keys, tmp, d_num, count, stream));
-  size_t tb = tb_sort > tb_uniq ? tb_sort : tb_uniq;
-  void *temp = nullptr;
-  if (cudaMallocAsync(&temp, tb + 16, stream) != cudaSuccess) return CG_ERR_OUT_OF_MEMORY;
-  if (cudaMallocAsync((void **)&d_num, sizeof(int64_t), stream) != cudaSuccess) {
-    cudaFreeAsync(temp, stream);
-    return CG_ERR_OUT_OF_MEMORY;
-  }
-  int rc = CG_OK;
-  do {
-    cudaError_t e = cub::DeviceRadixSort::SortKeys(temp, tb_sort, db, count, 0, end_bit, stream);
-    if (e != cudaSuccess) { rc = cuda_fail(e, "SortKeys"); break; }
-    uint64_t *sorted = db.Current();
-    uint64_t *other = db.Alternate();
-    e = cub::DeviceSelect::Unique(temp, tb_uniq, sorted, other, d_num, count, stream);
-    if (e != cudaSuccess) { rc = cuda_fail(e, "Unique"); break; }
-    int64_t nu = 0;
-    e = cudaMemcpyAsync(&nu, d_num, sizeof(int64_t), cudaMemcpyDeviceToHost, stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    if (e != cudaSuccess) { rc = cuda_fail(e, "Unique count"); break; }
-    if (nu > 0) {
-      uint64_t last = 0;
-      e = cudaMemcpyAsync(&last, other + nu - 1, sizeof(uint64_t), cudaMemcpyDeviceToHost, stream);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-      if (e != cudaSuccess) { rc = cuda_fail(e, "Unique last"); break; }
-      if (last == sentinel) --nu;
-    }
-    *result = other;
-    *kept = nu;
-  } while (0);
-  cudaFreeAsync(temp, stream);
-  cudaFreeAsync(d_num, stream);
-  return rc;
+static int value_bits(int64_t n) {  // bits of the values 0 .. n - 1, at least 1
+  int b = 1;
+  while (b < 62 && (1ll << b) < n) ++b;
+  return b;
 }
+
+// A build's device scratch: one allocation, cut into 256-byte aligned pieces.
+struct Scratch {
+  unsigned char *base = nullptr;
+  size_t used = 0;
+  template <class T>
+  T *take(int64_t count) {
+    T *p = reinterpret_cast<T *>(base + used);
+    used = (used + sizeof(T) * (size_t)count + 255) & ~(size_t)255;
+    return p;
+  }
+};
+
+// The buffers of one build, laid out in `s` (once without memory, for the
+// size).  The second sort's pairs take the space of the first's input; its
+// other set that of the unique keys when those are done with (a directed
+// graph), else space of its own.
+struct BuildSpace {
+  uint64_t *keys, *tmp;      // [m]
+  uint32_t *pairs;           // [2 m], symmetrised graphs only
+  uint32_t *first[2];        // [n + 1] row starts of the two sorts
+  Gap *gaps;
+  int64_t *count;
+  unsigned *zeros;           // two gap counts and the symmetry flag
+  void *temp;
+  BuildSpace(Scratch &s, int64_t n, int64_t m, bool sym, size_t temp_bytes) {
+    keys = s.take<uint64_t>(m);
+    tmp = s.take<uint64_t>(m);
+    pairs = s.take<uint32_t>(sym ? 2 * m : 0);
+    for (int i = 0; i < 2; ++i) first[i] = s.take<uint32_t>(n + 1);
+    gaps = s.take<Gap>(gap_capacity(n));
+    count = s.take<int64_t>(1);
+    zeros = s.take<unsigned>(3);
+    temp = s.take<unsigned char>((int64_t)temp_bytes);
+  }
+};
 
 }  // namespace cg
 
@@ -282,99 +369,159 @@ int cg_graph_from_edges(int64_t n, int64_t m, const uint32_t *d_src, const uint3
   const bool sym = (flags & CG_EDGES_SYMMETRIZE) != 0;
   const bool drop = (flags & CG_EDGES_DROP_LOOPS) != 0;
   const bool detect = (flags & CG_EDGES_DETECT_SYMMETRIC) != 0;
-  bool found_sym = false;
   int dev = 0, sms = 0;
   CG_CUDA(cudaGetDevice(&dev));
   CG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   cudaStream_t st = nullptr;
   CG_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-  const int64_t count = sym ? 2 * m : m;
-  const uint64_t sentinel = (uint64_t)n << 32;
-  int end_bit = 33;
-  while ((1ll << (end_bit - 32)) <= n) ++end_bit;
-  uint64_t *keys = nullptr, *tmp = nullptr, *res = nullptr;
-  int64_t *in_off = nullptr, *out_off = nullptr;
-  int32_t *in_idx = nullptr, *out_idx = nullptr;
+  const int bits = value_bits(n);
+  // the second sort's rows: a kept loop of a symmetrised graph gets row n there
+  const bool loops = sym && !drop;
+  const int row_bits = loops ? value_bits(n + 1) : bits;
+  Scratch mem;
+  int64_t *off[2] = {nullptr, nullptr};
+  int32_t *idx[2] = {nullptr, nullptr};
   int64_t nnz = 0;
+  bool found_sym = false;
   int rc = CG_OK;
+  auto fail = [&](cudaError_t e, const char *what) { rc = cuda_fail(e, what); };
+  auto alloc = [&](auto **p, int64_t count) {
+    if (cudaMalloc(p, sizeof(**p) * (size_t)(count > 0 ? count : 1)) == cudaSuccess) return true;
+    cudaGetLastError();
+    rc = CG_ERR_OUT_OF_MEMORY;
+    return false;
+  };
   do {
-    const size_t kb = sizeof(uint64_t) * (size_t)(count > 0 ? count : 1);
-    if (cudaMalloc(&keys, kb) != cudaSuccess || cudaMalloc(&tmp, kb) != cudaSuccess) {
-      rc = CG_ERR_OUT_OF_MEMORY;
+    if (m == 0) {
+      if (!alloc(&off[0], n + 1) || !alloc(&idx[0], 1)) break;
+      const cudaError_t e = cudaMemsetAsync(off[0], 0, sizeof(int64_t) * (size_t)(n + 1), st);
+      if (e != cudaSuccess) { fail(e, "empty offsets"); break; }
       break;
     }
-    if (count > 0) {
-      edge_keys_kernel<<<grid_for(m, sms), 256, 0, st>>>(m, d_src, d_dst, sym ? 1 : 0,
-                                                         drop ? 1 : 0, sentinel, keys);
-      cudaError_t e = cudaGetLastError();
-      if (e != cudaSuccess) { rc = cuda_fail(e, "edge_keys"); break; }
-      rc = sort_unique(keys, tmp, count, end_bit, sentinel, st, &res, &nnz);
-      if (rc) break;
+    size_t tb_keys = 0, tb_pairs = 0, tb_uniq = 0;
+    {
+      cub::DoubleBuffer<uint64_t> kb(nullptr, nullptr);
+      cub::DoubleBuffer<uint32_t> pk(nullptr, nullptr), pv(nullptr, nullptr);
+      cudaError_t e = cub::DeviceRadixSort::SortKeys(nullptr, tb_keys, kb, m, 0, 2 * bits, st);
+      if (e == cudaSuccess)
+        e = cub::DeviceRadixSort::SortPairs(nullptr, tb_pairs, pk, pv, m, 0, row_bits, st);
+      if (e == cudaSuccess)
+        e = cub::DeviceSelect::Unique(nullptr, tb_uniq, (uint64_t *)nullptr, (uint64_t *)nullptr,
+                                      (int64_t *)nullptr, m, st);
+      if (e != cudaSuccess) { fail(e, "sort sizes"); break; }
     }
-    if (cudaMalloc(&in_off, sizeof(int64_t) * (size_t)(n + 1)) != cudaSuccess ||
-        cudaMalloc(&in_idx, sizeof(int32_t) * (size_t)(nnz > 0 ? nnz : 1)) != cudaSuccess) {
-      rc = CG_ERR_OUT_OF_MEMORY;
-      break;
+    size_t tb = tb_keys > tb_pairs ? tb_keys : tb_pairs;
+    tb = tb > tb_uniq ? tb : tb_uniq;
+    Scratch size;
+    BuildSpace(size, n, m, sym, tb);
+    if (!alloc(&mem.base, (int64_t)size.used)) break;
+    BuildSpace b(mem, n, m, sym, tb);
+    cudaError_t e = cudaMemsetAsync(b.zeros, 0, 3 * sizeof(unsigned), st);
+    if (e != cudaSuccess) { fail(e, "build counters"); break; }
+    edge_keys_kernel<<<grid_for(m, sms), 256, 0, st>>>(m, d_src, d_dst, sym ? 1 : 0, drop ? 1 : 0,
+                                                       bits, b.keys);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) { fail(e, "edge_keys"); break; }
+    cub::DoubleBuffer<uint64_t> kb(b.keys, b.tmp);
+    e = cub::DeviceRadixSort::SortKeys(b.temp, tb_keys, kb, m, 0, 2 * bits, st);
+    if (e != cudaSuccess) { fail(e, "SortKeys"); break; }
+    uint64_t *const uniq = kb.Alternate();
+    e = cub::DeviceSelect::Unique(b.temp, tb_uniq, kb.Current(), uniq, b.count, m, st);
+    if (e != cudaSuccess) { fail(e, "Unique"); break; }
+    int64_t nu = 0;
+    uint64_t lowest = 1;
+    e = cudaMemcpyAsync(&nu, b.count, sizeof(nu), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(&lowest, uniq, sizeof(lowest), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) { fail(e, "Unique count"); break; }
+    const uint64_t *res = uniq;
+    if (drop && lowest == 0) {  // the dropped loops
+      ++res;
+      --nu;
     }
-    if (count > 0) {
-      csr_from_keys_kernel<<<grid_for(nnz > n ? nnz : n + 1, sms), 256, 0, st>>>(n, nnz, res,
-                                                                                in_off, in_idx);
-    } else {
-      cudaMemsetAsync(in_off, 0, sizeof(int64_t) * (size_t)(n + 1), st);
-    }
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) { rc = cuda_fail(e, "csr_from_keys"); break; }
-    if (!sym && nnz > 0) {
-      // CSC of A: the same entries keyed (col, row)
-      uint64_t *other = res == keys ? tmp : keys;
-      swap_halves_kernel<<<grid_for(nnz, sms), 256, 0, st>>>(nnz, res, other);
-      uint64_t *res2 = nullptr;
-      int64_t nnz2 = 0;
-      rc = sort_unique(other, res, nnz, 64, ~0ull, st, &res2, &nnz2);
-      if (rc) break;
-      if (cudaMalloc(&out_off, sizeof(int64_t) * (size_t)(n + 1)) != cudaSuccess ||
-          cudaMalloc(&out_idx, sizeof(int32_t) * (size_t)nnz) != cudaSuccess) {
-        rc = CG_ERR_OUT_OF_MEMORY;
-        break;
-      }
-      csr_from_keys_kernel<<<grid_for(nnz > n ? nnz : n + 1, sms), 256, 0, st>>>(n, nnz2, res2,
-                                                                                out_off, out_idx);
+    if (nu >= (1ll << 32) - (1ll << 16)) { rc = CG_ERR_NOT_SUPPORTED; break; }
+    if (sym || nu > 0) {
+      uint32_t *pair[2][2];  // [set][key, value]
+      pair[0][0] = reinterpret_cast<uint32_t *>(kb.Current());
+      pair[1][0] = sym ? b.pairs : reinterpret_cast<uint32_t *>(uniq);
+      for (int i = 0; i < 2; ++i) pair[i][1] = pair[i][0] + m;
+      split_keys_kernel<<<grid_for(nu + 1, sms), 256, 0, st>>>(
+          n, nu, res, bits, loops ? n : -1, b.first[0], pair[0][0], pair[0][1], b.gaps, b.zeros);
+      fill_gaps_kernel<<<sms, 256, 0, st>>>(b.gaps, b.zeros, b.first[0]);
       e = cudaGetLastError();
-      if (e != cudaSuccess) { rc = cuda_fail(e, "csc_from_keys"); break; }
-      if (detect) {
-        // the key buffers are free now: borrow one word of `keys` for the flag
-        unsigned *differ = reinterpret_cast<unsigned *>(keys);
-        e = cudaMemsetAsync(differ, 0, sizeof(unsigned), st);
-        if (e == cudaSuccess) {
-          same_arrays_kernel<<<grid_for(nnz > n ? nnz : n + 1, sms), 256, 0, st>>>(
-              n, nnz, in_off, in_idx, out_off, out_idx, differ);
-          e = cudaGetLastError();
-        }
-        unsigned h_differ = 1u;
-        if (e == cudaSuccess)
-          e = cudaMemcpyAsync(&h_differ, differ, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        if (e != cudaSuccess) { rc = cuda_fail(e, "symmetry check"); break; }
-        found_sym = h_differ == 0u;
+      if (e != cudaSuccess) { fail(e, "split_keys"); break; }
+      const int grid = grid_for(nu > n ? nu : n + 1, sms);
+      if (!sym) {
+        // the CSR before the second sort, which takes the keys' space
+        nnz = nu;
+        if (!alloc(&off[0], n + 1) || !alloc(&idx[0], nnz) || !alloc(&off[1], n + 1) ||
+            !alloc(&idx[1], nnz))
+          break;
+        csr_kernel<<<grid, 256, 0, st>>>(n, nnz, res, bits, b.first[0], off[0], idx[0]);
       }
+      cub::DoubleBuffer<uint32_t> pk(pair[0][0], pair[1][0]), pv(pair[0][1], pair[1][1]);
+      if (nu > 0) e = cub::DeviceRadixSort::SortPairs(b.temp, tb_pairs, pk, pv, nu, 0, row_bits, st);
+      if (e != cudaSuccess) { fail(e, "SortPairs"); break; }
+      row_starts_kernel<<<grid_for(nu + 1, sms), 256, 0, st>>>(n, nu, pk.Current(), b.first[1],
+                                                               b.gaps, b.zeros + 1);
+      fill_gaps_kernel<<<sms, 256, 0, st>>>(b.gaps, b.zeros + 1, b.first[1]);
+      e = cudaGetLastError();
+      if (e != cudaSuccess) { fail(e, "row_starts"); break; }
+      if (sym) {
+        uint32_t nl = (uint32_t)nu;  // lower triangle: all but the loops
+        if (loops) {
+          e = cudaMemcpyAsync(&nl, b.first[1] + n, sizeof(nl), cudaMemcpyDeviceToHost, st);
+          if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+          if (e != cudaSuccess) { fail(e, "loop count"); break; }
+        }
+        nnz = nu + (int64_t)nl;
+        if (nnz >= (1ll << 32) - (1ll << 16)) { rc = CG_ERR_NOT_SUPPORTED; break; }
+        if (!alloc(&off[0], n + 1) || !alloc(&idx[0], nnz)) break;
+        csr_symmetric_kernel<<<grid, 256, 0, st>>>(n, nu, nl, res, bits, b.first[0], pk.Current(),
+                                                   pv.Current(), b.first[1], off[0], idx[0]);
+      } else {
+        csr_pairs_kernel<<<grid, 256, 0, st>>>(n, nnz, pv.Current(), b.first[1], off[1], idx[1]);
+      }
+      e = cudaGetLastError();
+      if (e != cudaSuccess) { fail(e, "csr"); break; }
+      if (!sym && detect) {
+        same_arrays_kernel<<<grid, 256, 0, st>>>(n, nnz, off[0], idx[0], off[1], idx[1],
+                                                 b.zeros + 2);
+        e = cudaGetLastError();
+        unsigned differ = 1u;
+        if (e == cudaSuccess)
+          e = cudaMemcpyAsync(&differ, b.zeros + 2, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        if (e != cudaSuccess) { fail(e, "symmetry check"); break; }
+        found_sym = differ == 0u;
+      }
+    } else {
+      if (!alloc(&off[0], n + 1) || !alloc(&idx[0], 1)) break;
+      e = cudaMemsetAsync(off[0], 0, sizeof(int64_t) * (size_t)(n + 1), st);
+      if (e != cudaSuccess) { fail(e, "empty offsets"); break; }
     }
-    e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) { rc = cuda_fail(e, "cg_graph_from_edges"); break; }
-    cudaFree(keys);
-    cudaFree(tmp);
-    keys = tmp = nullptr;
-    const bool out_sym = sym || nnz == 0 || found_sym;
-    rc = cg_graph_create(n, nnz, in_off, in_idx, out_sym ? nullptr : out_off,
-                         out_sym ? nullptr : out_idx,
-                         CG_GRAPH_DEVICE_PTRS | (out_sym ? CG_GRAPH_SYMMETRIC : 0), out);
   } while (0);
-  cudaFree(keys);
-  cudaFree(tmp);
-  cudaFree(in_off);
-  cudaFree(in_idx);
-  cudaFree(out_off);
-  cudaFree(out_idx);
+  if (rc == CG_OK) {
+    const cudaError_t e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) fail(e, "cg_graph_from_edges");
+  } else {
+    cudaStreamSynchronize(st);
+  }
+  cudaFree(mem.base);
   cudaStreamDestroy(st);
+  const bool out_sym = sym || nnz == 0 || found_sym;
+  if (rc == CG_OK && out_sym) {
+    cudaFree(off[1]);
+    cudaFree(idx[1]);
+    off[1] = nullptr;
+    idx[1] = nullptr;
+  }
+  if (rc == CG_OK) return graph_adopt(n, nnz, off[0], idx[0], off[1], idx[1], out_sym, out);
+  for (int i = 0; i < 2; ++i) {
+    cudaFree(off[i]);
+    cudaFree(idx[i]);
+  }
   return rc;
 }
 

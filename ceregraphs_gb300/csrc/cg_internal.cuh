@@ -146,11 +146,11 @@ struct cg_graph {
   int32_t *out_idx = nullptr;
   cudaStream_t stream = nullptr;
   cg_options opt{};
-  // per-root search state
+  // per-root search state: pieces of one allocation
+  void *state = nullptr;
   int64_t words = 0;            // ceil(n / 32)
   uint32_t *bitmaps = nullptr;  // vis | fr0 | fr1 | fr2, 4 * bitmap_stride(n)
-  uint32_t *dead = nullptr;     // 1 bit per vertex: no in-edges (dead_prepare),
-                                // bitmap_stride(n) words
+  uint32_t *dead = nullptr;     // 1 bit per vertex: no in-edges, bitmap_stride(n) words
   int64_t live = 0;             // vertices with in-edges
   // cg_graph_reorder: resident vertex v is original vertex orig[v]; perm is
   // the inverse (both int32[n], null for a graph in its original order)
@@ -190,10 +190,13 @@ int cuda_fail(cudaError_t e, const char *what);
 // Sets the text cg_last_error_string returns (a reason, not a CUDA error).
 void set_error_text(const char *text);
 int bfs_prepare(cg_graph *g);
+// A handle that owns the given device arrays (out_off / out_idx null for a
+// symmetric graph); they are freed if it cannot be made.
+int graph_adopt(int64_t n, int64_t nnz, int64_t *in_off, int32_t *in_idx, int64_t *out_off,
+                int32_t *out_idx, bool symmetric, cg_graph **out);
 // `bytes` of device scratch owned by the handle, for calls that wait for the
 // stream before they return (the next call may then reuse or grow it).
 int call_scratch(cg_graph *g, size_t bytes, void **out);
-int dead_prepare(cg_graph *g);
 // CG_ERR_NOT_SUPPORTED (with a reason) while the handle's stream is being
 // captured: for set-up that has to synchronise the handle's stream.
 int refuse_setup_in_capture(cg_graph *g);

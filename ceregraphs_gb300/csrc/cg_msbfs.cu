@@ -920,16 +920,14 @@ static int ms_history_planes(const cg_graph *g, int lane_words) {
 }
 
 static int ms_alloc_state(cg_graph *g, int lane_words) {
-  int rc0 = dead_prepare(g);
-  if (rc0) return rc0;
   MsState *old = reinterpret_cast<MsState *>(g->ms_ctl);
   if (old && g->ms_lane_words == lane_words && old->hist_opt == g->opt.ms_history) return CG_OK;
-  rc0 = refuse_setup_in_capture(g);
-  if (rc0) return rc0;
+  int rc = refuse_setup_in_capture(g);
+  if (rc) return rc;
   ms_free_state(old);
   g->ms_ctl = nullptr;
   MsState *s = nullptr;
-  int rc = ms_create_state(g, lane_words, ms_history_planes(g, lane_words), &s);
+  rc = ms_create_state(g, lane_words, ms_history_planes(g, lane_words), &s);
   if (rc) return rc;
   s->hist_opt = g->opt.ms_history;
   g->ms_ctl = s;
