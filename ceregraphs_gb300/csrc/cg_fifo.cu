@@ -7,14 +7,24 @@
 // (rank of the parent, vertex id).
 //
 // Given the levels of a finished search, this pass recomputes the parents
-// level by level: one warp per level-(L+1) vertex takes the minimum of
-// (rank, id) over its level-L in-neighbours; a radix sort of the resulting
-// (parent rank, vertex id) keys is the queue order of level L+1, i.e. the
-// next level's ranks.  The level sizes steer the sorts from the host, so the
-// pass synchronises with the stream (and is refused inside a graph capture).
+// level by level.  A stable sort of the vertices by level (one 8-bit pass up to
+// 254 levels) lists each level in id order.  Level L's ranks reach level L+1
+// from whichever side has fewer list entries -- each vertex takes the minimum
+// over its in-list of a 4-byte rank map, or level L's out-lists push their ranks
+// by atomicMin -- and a stable sort of level L+1 by parent rank, as few bits as
+// level L has ranks, is its queue order.  After a level of one vertex nothing
+// is left to do: the search's parents stand and id order is queue order.  The
+// level sizes steer this from the host, so the pass synchronises with the
+// stream (and is refused inside a graph capture).
+//
+// Bound by the dependent launches of a level (about nine, 3 to 10 us each) and
+// by the rank gathers of the widest levels.  R-MAT scale 20, device time with
+// the search: 1319 us with a warp per vertex, 64-bit sorts and one block for
+// levels of few vertices but long lists, 418 us now.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <new>
 #include <vector>
 
 #include <cub/block/block_scan.cuh>
@@ -24,123 +34,319 @@
 
 namespace cg {
 
+constexpr int kFifoSums = 64;  // levels whose list entries are counted
+
+struct FifoSums {
+  int maxlevel;
+  unsigned counts[kFifoSums];
+  unsigned long long out[kFifoSums], in[kFifoSums];  // degrees summed
+};
+
+struct FifoLong {  // a long list: its first chunk, the vertex, its rank (out-lists)
+  uint32_t base;
+  int32_t v;
+  uint32_t rank;
+};
+
 struct FifoState {
   int64_t n = 0;
-  int32_t *rank = nullptr;              // [n] queue rank within the vertex's level
-  // [n] (level << 32) | rank and (level << 32) | FIFO parent of the vertices
-  // ranked so far in this pass (-1 elsewhere): one load tells a list entry's
-  // level and rank, or whether an out-neighbour is a given parent's child
-  unsigned long long *lr = nullptr, *pl = nullptr;
-  int32_t *order = nullptr;             // [n] vertices of levels >= 1, grouped by level
-  unsigned long long *keys = nullptr;   // [n] (parent rank, vertex) of one level
-  unsigned long long *sorted = nullptr; // [n]
-  unsigned *counts = nullptr;           // [n + 1] vertices per level
-  unsigned *cursor = nullptr;           // [n + 1] scatter cursors
-  unsigned *offs = nullptr;             // [n + 1] first slot of each level in order
-  int *maxlevel = nullptr;
-  void *temp = nullptr;                 // radix sort scratch
+  unsigned char *base = nullptr;  // the one allocation of what follows
+  FifoSums *sums = nullptr;
+  unsigned long long *nlong = nullptr;  // (lists << 32) | chunks of `longs`
+  int32_t *order = nullptr;       // [n] vertices sorted by (level, id)
+  uint32_t *rk = nullptr;         // [n] rank of the level being read, ~0 elsewhere
+  uint32_t *best = nullptr;       // [n] smallest parent rank of a vertex, ~0 none yet
+  uint32_t *key[2] = {nullptr, nullptr};  // [n] sort keys
+  int32_t *queue[3] = {nullptr, nullptr, nullptr};  // [n] a level in queue order, and sort values
+  unsigned *counts = nullptr;     // [n + 1] vertices per level
+  FifoLong *longs = nullptr;
+  void *temp = nullptr;           // radix sort scratch
   size_t temp_bytes = 0;
+  // runs of small levels: the ranks, and (level << 32) | rank and (level << 32)
+  // | FIFO parent of the vertices ranked so far in this pass (-1 elsewhere)
+  int32_t *rank = nullptr;                      // [n]
+  unsigned long long *lr = nullptr, *pl = nullptr;  // [n]
+  unsigned *offs = nullptr;       // [n + 2] first slot of each level in order
 };
 
 namespace {
 
 constexpr int kFifoBlock = 256;
-constexpr int kFifoSmemLevels = 64;
+constexpr unsigned kAll = 0xffffffffu;
+constexpr uint32_t kNoRank = 0xffffffffu;
+constexpr int64_t kFifoLane = 32;    // in-lists up to this: one thread
+constexpr int64_t kFifoWarp = 1024;  // lists up to this: the warp that meets them; above: chunks
+constexpr int64_t kFifoChunk = 512;
 
-// Vertices per level (levels >= 0) and the deepest level.
-__global__ void fifo_hist_kernel(int64_t n, const int32_t *__restrict__ levels, unsigned *counts,
-                                 int *maxlevel) {
-  __shared__ unsigned s[kFifoSmemLevels];
-  for (int i = threadIdx.x; i < kFifoSmemLevels; i += blockDim.x) s[i] = 0;
+// Vertices per level (levels >= 0), their degrees summed (the first kFifoSums
+// levels), and the deepest level.  One round of shared atomics per level
+// present in a warp.
+__global__ void __launch_bounds__(kFifoBlock) fifo_hist_kernel(
+    int64_t n, const int32_t *__restrict__ levels, const int64_t *__restrict__ in_off,
+    const int64_t *__restrict__ out_off, unsigned *counts, FifoSums *sums) {
+  __shared__ unsigned s_count[kFifoSums];
+  __shared__ unsigned long long s_out[kFifoSums], s_in[kFifoSums];
+  for (int i = threadIdx.x; i < kFifoSums; i += blockDim.x) s_count[i] = s_out[i] = s_in[i] = 0;
   __syncthreads();
+  const int lane = lane_id();
   int mx = -1;
-  for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n;
-       v += (int64_t)gridDim.x * blockDim.x) {
-    const int L = levels[v];
-    if (L < 0) continue;
-    mx = L > mx ? L : mx;
-    if (L < kFifoSmemLevels)
-      atomicAdd(&s[L], 1u);
-    else
-      atomicAdd(&counts[L], 1u);
-  }
-  mx = __reduce_max_sync(0xffffffffu, mx);
-  if ((threadIdx.x & 31) == 0 && mx >= 0) atomicMax(maxlevel, mx);
-  __syncthreads();
-  for (int i = threadIdx.x; i < kFifoSmemLevels; i += blockDim.x)
-    if (s[i]) atomicAdd(&counts[i], s[i]);
-}
-
-// order[offs[L] ..] = the vertices of level L >= 1 (in no particular order;
-// each level is sorted later).  One atomic per level present in a warp.
-__global__ void fifo_scatter_kernel(int64_t n, const int32_t *__restrict__ levels,
-                                    const unsigned *__restrict__ offs, unsigned *cursor,
-                                    int32_t *order) {
-  const int lane = threadIdx.x & 31;
   for (int64_t base = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~31ll; base < n;
        base += (int64_t)gridDim.x * blockDim.x) {
     const int64_t v = base + lane;
     const int L = v < n ? levels[v] : -1;
-    const unsigned peers = __match_any_sync(0xffffffffu, L);
-    if (L >= 1) {
-      const int leader = __ffs(peers) - 1;
-      unsigned at = 0;
-      if (lane == leader) at = atomicAdd(&cursor[L], (unsigned)__popc(peers));
-      at = __shfl_sync(peers, at, leader);
-      order[offs[L] + at + __popc(peers & ((1u << lane) - 1u))] = (int32_t)v;
+    unsigned din = 0, dout = 0;
+    if (L >= 0 && L < kFifoSums) {
+      din = (unsigned)(__ldg(in_off + v + 1) - __ldg(in_off + v));
+      dout = out_off == in_off ? din : (unsigned)(__ldg(out_off + v + 1) - __ldg(out_off + v));
     }
-  }
-}
-
-// One warp per vertex v of level L+1 (order[0 .. count)): its level-L
-// in-neighbour of smallest rank is its parent (ranks are unique within a
-// level); keys[i] = (that rank << vbits) | v, the sort key of level L+1's
-// queue order (v < 2^vbits).
-__global__ void fifo_pick_kernel(const int64_t *__restrict__ in_off,
-                                 const int32_t *__restrict__ in_idx,
-                                 const int32_t *__restrict__ levels,
-                                 const int32_t *__restrict__ rank,
-                                 const int32_t *__restrict__ order, unsigned count, int L,
-                                 int vbits, unsigned long long *keys, int32_t *parents) {
-  const int lane = threadIdx.x & 31;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < count;
-       i += nwarps) {
-    const int32_t v = order[i];
-    const int64_t s = __ldg(in_off + v), e = __ldg(in_off + v + 1);
-    unsigned long long best = ~0ull;
-    for (int64_t j = s + lane; j < e; j += 32) {
-      const int32_t u = __ldg(in_idx + j);
-      if (levels[u] == L) {
-        const unsigned long long k = ((unsigned long long)(uint32_t)rank[u] << 32) | (uint32_t)u;
-        best = k < best ? k : best;
+    mx = max(mx, L);
+    unsigned todo = __ballot_sync(kAll, L >= 0);
+    while (todo) {
+      const int l = __shfl_sync(kAll, L, __ffs(todo) - 1);
+      const unsigned m = __ballot_sync(kAll, L == l);
+      todo &= ~m;
+      if (l >= kFifoSums) {
+        if (lane == 0) atomicAdd(&counts[l], (unsigned)__popc(m));
+        continue;
+      }
+      const unsigned i = __reduce_add_sync(kAll, L == l ? din : 0u);
+      const unsigned o = out_off == in_off ? i : __reduce_add_sync(kAll, L == l ? dout : 0u);
+      if (lane == 0) {
+        atomicAdd(&s_count[l], (unsigned)__popc(m));
+        atomicAdd(&s_in[l], (unsigned long long)i);
+        atomicAdd(&s_out[l], (unsigned long long)o);
       }
     }
+  }
+  mx = __reduce_max_sync(kAll, mx);
+  if (lane == 0 && mx >= 0) atomicMax(&sums->maxlevel, mx);
+  __syncthreads();
+  for (int i = threadIdx.x; i < kFifoSums; i += blockDim.x)
+    if (s_count[i]) {
+      atomicAdd(&counts[i], s_count[i]);
+      atomicAdd(&sums->counts[i], s_count[i]);
+      atomicAdd(&sums->in[i], s_in[i]);
+      atomicAdd(&sums->out[i], s_out[i]);
+    }
+}
+
+__global__ void fifo_iota_kernel(int64_t n, int32_t *x) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x)
+    x[i] = (int32_t)i;
+}
+
+// The rank map of level L (rk is ~0 elsewhere).
+__global__ void fifo_ranks_kernel(const int32_t *__restrict__ queue, unsigned count,
+                                  uint32_t *rk) {
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
+    rk[queue[i]] = i;
+}
+
+__device__ __forceinline__ void fifo_list_long(bool is_long, int32_t v, uint32_t rank, int64_t deg,
+                                               FifoLong *longs, unsigned long long *nlong) {
+  if (!is_long) return;
+  const unsigned chunks = (unsigned)((deg + kFifoChunk - 1) / kFifoChunk);
+  const unsigned long long old = atomicAdd(nlong, (1ull << 32) | chunks);
+  longs[old >> 32] = FifoLong{(uint32_t)old, v, rank};
+}
+
+// Pull: level L+1's vertices (seg) take the smallest rank over their in-lists.
+// A warp has 32 of them: short lists by a lane each (four entries' ranks in
+// flight), longer ones by the warp (128 entries in flight), the longest listed.
+__global__ void __launch_bounds__(kFifoBlock) fifo_pull_kernel(
+    const int64_t *__restrict__ in_off, const int32_t *__restrict__ in_idx,
+    const uint32_t *__restrict__ rk, const int32_t *__restrict__ seg, unsigned count,
+    uint32_t *__restrict__ best, FifoLong *longs, unsigned long long *nlong) {
+  const int lane = lane_id();
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t base = (int64_t)warp_id_global() * 32; base < count; base += nwarps * 32) {
+    int32_t v = 0;
+    int64_t b = 0, e = 0;
+    if (base + lane < count) {
+      v = seg[base + lane];
+      b = __ldg(in_off + v);
+      e = __ldg(in_off + v + 1);
+    }
+    const int64_t deg = e - b;
+    uint32_t low = kNoRank;
+    if (deg <= kFifoLane) {
+      for (int64_t j = b; j < e; j += 4) {
+        int32_t u[4];
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-      const unsigned long long o = __shfl_xor_sync(0xffffffffu, best, d);
-      best = o < best ? o : best;
+        for (int q = 0; q < 4; ++q) u[q] = j + q < e ? __ldg(in_idx + j + q) : -1;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (u[q] >= 0) low = min(low, __ldg(rk + u[q]));
+      }
     }
-    if (lane == 0) {
-      parents[v] = best == ~0ull ? -1 : (int32_t)(uint32_t)best;
-      keys[i] = ((best >> 32) << vbits) | (uint32_t)v;
+    unsigned todo = __ballot_sync(kAll, deg > kFifoLane && deg <= kFifoWarp);
+    while (todo) {
+      const int src = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const int64_t sb = __shfl_sync(kAll, b, src), se = __shfl_sync(kAll, e, src);
+      uint32_t x = kNoRank;
+      for (int64_t j = sb + lane; j < se; j += 128) {
+        int32_t u[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) u[q] = j + 32 * q < se ? __ldg(in_idx + j + 32 * q) : -1;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (u[q] >= 0) x = min(x, __ldg(rk + u[q]));
+      }
+      x = __reduce_min_sync(kAll, x);
+      if (lane == src) low = x;
+    }
+    if (base + lane < count && deg <= kFifoWarp) best[v] = low;
+    fifo_list_long(deg > kFifoWarp, v, 0u, deg, longs, nlong);
+  }
+}
+
+__device__ __forceinline__ void fifo_offer(const int32_t *__restrict__ levels, int32_t v, int L,
+                                           uint32_t rank, uint32_t *best) {
+  // a read first: a hub's rank is low, and most targets have it already
+  if (__ldg(levels + v) == L + 1 && __ldcg(best + v) > rank) atomicMin(best + v, rank);
+}
+
+// Push: level L's vertices offer their rank to their level-(L+1)
+// out-neighbours.  A warp spreads the edges of 32 vertices over its lanes, of
+// fewer when there are not 32 for every warp, four edges a lane in flight (110
+// hubs' neighbours at R-MAT scale 20: 339 us on 4 warps, 24 us on 110); the
+// longest lists go on the list.
+__global__ void __launch_bounds__(kFifoBlock) fifo_push_kernel(
+    const int64_t *__restrict__ out_off, const int32_t *__restrict__ out_idx,
+    const int32_t *__restrict__ levels, const int32_t *__restrict__ queue, unsigned count, int L,
+    uint32_t *best, FifoLong *longs, unsigned long long *nlong) {
+  __shared__ uint32_t s_first[kFifoBlock / 32][32];
+  __shared__ int64_t s_start[kFifoBlock / 32][32];
+  const int lane = lane_id();
+  uint32_t *first = s_first[threadIdx.x >> 5];
+  int64_t *start = s_start[threadIdx.x >> 5];
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  int group = 1;
+  while (group < 32 && (int64_t)count > group * nwarps) group <<= 1;
+  for (int64_t base = (int64_t)warp_id_global() * group; base < count; base += nwarps * group) {
+    int64_t b = 0, deg = 0;
+    int32_t u = 0;
+    if (lane < group && base + lane < count) {
+      u = queue[base + lane];
+      b = __ldg(out_off + u);
+      deg = __ldg(out_off + u + 1) - b;
+    }
+    fifo_list_long(deg > kFifoWarp, u, (uint32_t)(base + lane), deg, longs, nlong);
+    const uint32_t d = deg > kFifoWarp ? 0u : (uint32_t)deg;
+    uint32_t incl = d;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(kAll, incl, o);
+      if (lane >= o) incl += t;
+    }
+    const uint32_t total = __shfl_sync(kAll, incl, 31);
+    first[lane] = incl - d;
+    start[lane] = b;
+    __syncwarp();
+    for (uint32_t t0 = lane; t0 < total; t0 += 128) {
+      int lo[4];
+      int32_t v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t t = t0 + 32 * q;
+        lo[q] = 0;  // the last of the 32 whose prefix is <= t
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1)
+          if (first[lo[q] + step] <= t) lo[q] += step;
+        v[q] = t < total ? __ldg(out_idx + start[lo[q]] + (t - first[lo[q]])) : -1;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (v[q] >= 0) fifo_offer(levels, v[q], L, (uint32_t)(base + lo[q]), best);
+    }
+    __syncwarp();
+  }
+}
+
+// The listed long lists, a warp per chunk.
+template <bool Push>
+__global__ void __launch_bounds__(kFifoBlock) fifo_long_kernel(
+    const int64_t *__restrict__ off, const int32_t *__restrict__ idx,
+    const int32_t *__restrict__ levels, const uint32_t *__restrict__ rk, int L, uint32_t *best,
+    const FifoLong *__restrict__ longs, const unsigned long long *nlong) {
+  const unsigned long long all = *nlong;
+  const unsigned lists = (unsigned)(all >> 32), chunks = (unsigned)all;
+  const int lane = lane_id();
+  const unsigned nwarps = (gridDim.x * blockDim.x) >> 5;
+  for (unsigned c = (unsigned)warp_id_global(); c < chunks; c += nwarps) {
+    unsigned lo = 0, hi = lists - 1;
+    while (lo < hi) {
+      const unsigned mid = (lo + hi + 1) >> 1;
+      if (longs[mid].base <= c)
+        lo = mid;
+      else
+        hi = mid - 1;
+    }
+    const FifoLong x = longs[lo];
+    const int64_t b = __ldg(off + x.v) + (int64_t)(c - x.base) * kFifoChunk;
+    const int64_t e = min(b + kFifoChunk, __ldg(off + x.v + 1));
+    uint32_t low = kNoRank;
+    for (int64_t j = b + lane; j < e; j += 128) {
+      int32_t u[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) u[q] = j + 32 * q < e ? __ldg(idx + j + 32 * q) : -1;
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (u[q] >= 0) {
+          if (Push)
+            fifo_offer(levels, u[q], L, x.rank, best);
+          else
+            low = min(low, __ldg(rk + u[q]));
+        }
+    }
+    if (!Push) {
+      low = __reduce_min_sync(kAll, low);
+      if (lane == 0 && low != kNoRank) atomicMin(best + x.v, low);
     }
   }
 }
 
-__global__ void fifo_rank_kernel(const unsigned long long *__restrict__ sorted, unsigned count,
-                                 int vbits, int level, int32_t *rank, unsigned long long *lr) {
-  const unsigned long long vmask = (1ull << vbits) - 1ull;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const unsigned long long v = sorted[i] & vmask;
-    rank[v] = (int32_t)i;
-    lr[v] = ((unsigned long long)level << 32) | (unsigned long long)i;
+// Level L+1 (seg) takes its parents; the sort's keys (parent ranks) and values.
+// `clear`: rk's entries of level L go back to ~0.
+__global__ void fifo_finish_kernel(const int32_t *__restrict__ seg, unsigned count,
+                                   const uint32_t *__restrict__ best,
+                                   const int32_t *__restrict__ queue, unsigned parents_count,
+                                   int clear, uint32_t *rk, uint32_t *__restrict__ keys,
+                                   int32_t *__restrict__ vals, int32_t *__restrict__ parents,
+                                   unsigned long long *nlong) {
+  const unsigned t0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+  if (t0 == 0) *nlong = 0;
+  for (unsigned i = t0; i < count; i += step) {
+    const int32_t v = seg[i];
+    const uint32_t r = best[v];
+    parents[v] = r == kNoRank ? -1 : queue[r];
+    keys[i] = r;
+    vals[i] = v;
   }
+  if (clear)
+    for (unsigned i = t0; i < parents_count; i += step) rk[queue[i]] = kNoRank;
 }
 
-// Levels of at most kSmallLevel vertices are handled by one block, many
-// levels to a launch, with no sort: level L+1's queue is level L's queue in
+// Into and out of a run of small levels: level L's ranks from its queue, and
+// its queue from its ranks (seg: its vertices).
+__global__ void fifo_enter_kernel(const int32_t *__restrict__ queue, unsigned count, int level,
+                                  int32_t *rank, unsigned long long *lr) {
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < count;
+       i += gridDim.x * blockDim.x) {
+    rank[queue[i]] = (int32_t)i;
+    lr[queue[i]] = ((unsigned long long)level << 32) | i;
+  }
+}
+__global__ void fifo_leave_kernel(const int32_t *__restrict__ seg, unsigned count,
+                                  const int32_t *__restrict__ rank, int32_t *queue) {
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
+    queue[rank[seg[i]]] = seg[i];
+}
+
+// Runs of levels of at most kSmallLevel vertices and kSmallEdges list entries
+// are handled by one block, many levels to a launch, with no sort: level L+1's queue is level L's queue in
 // order with each vertex's children (the out-neighbours whose FIFO parent it
 // is) appended in out-list order, which is ascending -- the same order the
 // sort of (parent rank, id) gives.  Per level: (1) every child picks its
@@ -156,6 +362,8 @@ __global__ void fifo_rank_kernel(const unsigned long long *__restrict__ sorted, 
 constexpr int kSmallThreads = 1024;
 constexpr int kSmallPer = 8;                                // counts a thread scans
 constexpr int kSmallLevel = kSmallThreads * kSmallPer;     // vertices per level, at most
+constexpr uint64_t kSmallEdges = 1 << 15;  // out-edges of level L, in-edges of level L + 1
+constexpr int kSmallRun = 3;    // levels worth a run: it sets up 16 bytes a vertex
 constexpr int kHeavyList = 64;  // list length above which a warp scans
 using SmallScan = cub::BlockScan<unsigned, kSmallThreads>;
 struct SmallSmem {
@@ -218,8 +426,7 @@ __global__ void __launch_bounds__(kSmallThreads) fifo_small_levels_kernel(
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   constexpr int kWarps = kSmallThreads / 32;
   int cur = 0;
-  // level L0 in queue order, from the ranks already assigned (level 0 is the
-  // root alone; order[] lists levels >= 1)
+  // level L0 in queue order, from the ranks already assigned
   if (L0 == 0) {
     if (t == 0) S.queue[0][0] = root;
   } else {
@@ -348,34 +555,56 @@ int fifo_state(cg_graph *g, FifoState **out) {
     *out = g->fifo;
     return CG_OK;
   }
-  FifoState *f = new FifoState();
+  FifoState *f = new (std::nothrow) FifoState();
+  if (!f) return CG_ERR_OUT_OF_MEMORY;
   f->n = g->n;
   const size_t n = (size_t)g->n;
-  bool ok = cudaMalloc(&f->rank, sizeof(int32_t) * n) == cudaSuccess &&
-            cudaMalloc(&f->lr, sizeof(unsigned long long) * n) == cudaSuccess &&
-            cudaMalloc(&f->pl, sizeof(unsigned long long) * n) == cudaSuccess &&
-            cudaMalloc(&f->order, sizeof(int32_t) * n) == cudaSuccess &&
-            cudaMalloc(&f->keys, sizeof(unsigned long long) * n) == cudaSuccess &&
-            cudaMalloc(&f->sorted, sizeof(unsigned long long) * n) == cudaSuccess &&
-            cudaMalloc(&f->counts, sizeof(unsigned) * (n + 1)) == cudaSuccess &&
-            cudaMalloc(&f->cursor, sizeof(unsigned) * (n + 1)) == cudaSuccess &&
-            cudaMalloc(&f->offs, sizeof(unsigned) * (n + 1)) == cudaSuccess &&
-            cudaMalloc(&f->maxlevel, sizeof(int)) == cudaSuccess;
-  if (ok)
-    ok = cudaFuncSetAttribute(fifo_small_levels_kernel,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)sizeof(SmallSmem)) == cudaSuccess;
-  if (ok) {
-    cub::DeviceRadixSort::SortKeys(nullptr, f->temp_bytes, f->keys, f->sorted, (int)n, 0, 64,
-                                   g->stream);
-    ok = cudaMalloc(&f->temp, f->temp_bytes ? f->temp_bytes : 16) == cudaSuccess;
+  {
+    cub::DoubleBuffer<uint32_t> k(nullptr, nullptr);
+    cub::DoubleBuffer<int32_t> v(nullptr, nullptr);
+    size_t by_rank = 0, by_level = 0;
+    cub::DeviceRadixSort::SortPairs(nullptr, by_rank, k, v, (int64_t)n, 0, 32, g->stream);
+    cub::DeviceRadixSort::SortPairs(nullptr, by_level, (const uint32_t *)nullptr,
+                                    (uint32_t *)nullptr, (const int32_t *)nullptr,
+                                    (int32_t *)nullptr, (int64_t)n, 0, 32, g->stream);
+    f->temp_bytes = by_rank > by_level ? by_rank : by_level;
   }
-  if (!ok) {
+  const size_t nlongs = (size_t)(g->nnz / (kFifoWarp + 1) + 1);
+  size_t bytes = 0;
+  auto piece = [&](size_t size) {
+    const size_t at = bytes;
+    bytes = (bytes + size + 255) & ~(size_t)255;
+    return at;
+  };
+  const size_t at_sums = piece(sizeof(FifoSums)), at_nlong = piece(sizeof(unsigned long long)),
+               at_longs = piece(sizeof(FifoLong) * nlongs), at_temp = piece(f->temp_bytes),
+               at_counts = piece(sizeof(unsigned) * (n + 1)),
+               at_offs = piece(sizeof(unsigned) * (n + 2)), at_lr = piece(8 * n),
+               at_pl = piece(8 * n);
+  size_t at4[9];  // 4 bytes a vertex each
+  for (size_t &x : at4) x = piece(4 * n);
+  if (cudaMalloc(&f->base, bytes) != cudaSuccess ||
+      cudaFuncSetAttribute(fifo_small_levels_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)sizeof(SmallSmem)) != cudaSuccess) {
+    cudaGetLastError();
     fifo_free(f);
     return CG_ERR_OUT_OF_MEMORY;
   }
-  g->device_bytes += (int64_t)((sizeof(int32_t) * 2 + sizeof(unsigned long long) * 4) * n +
-                               sizeof(unsigned) * 3 * (n + 1) + f->temp_bytes);
+  f->sums = reinterpret_cast<FifoSums *>(f->base + at_sums);
+  f->nlong = reinterpret_cast<unsigned long long *>(f->base + at_nlong);
+  f->longs = reinterpret_cast<FifoLong *>(f->base + at_longs);
+  f->temp = f->base + at_temp;
+  f->counts = reinterpret_cast<unsigned *>(f->base + at_counts);
+  f->offs = reinterpret_cast<unsigned *>(f->base + at_offs);
+  f->lr = reinterpret_cast<unsigned long long *>(f->base + at_lr);
+  f->pl = reinterpret_cast<unsigned long long *>(f->base + at_pl);
+  f->order = reinterpret_cast<int32_t *>(f->base + at4[0]);
+  f->rk = reinterpret_cast<uint32_t *>(f->base + at4[1]);
+  f->best = reinterpret_cast<uint32_t *>(f->base + at4[2]);
+  f->rank = reinterpret_cast<int32_t *>(f->base + at4[3]);
+  for (int i = 0; i < 2; ++i) f->key[i] = reinterpret_cast<uint32_t *>(f->base + at4[4 + i]);
+  for (int i = 0; i < 3; ++i) f->queue[i] = reinterpret_cast<int32_t *>(f->base + at4[6 + i]);
+  g->device_bytes += (int64_t)bytes;
   g->fifo = f;
   *out = f;
   return CG_OK;
@@ -385,17 +614,7 @@ int fifo_state(cg_graph *g, FifoState **out) {
 
 void fifo_free(FifoState *f) {
   if (!f) return;
-  cudaFree(f->rank);
-  cudaFree(f->lr);
-  cudaFree(f->pl);
-  cudaFree(f->order);
-  cudaFree(f->keys);
-  cudaFree(f->sorted);
-  cudaFree(f->counts);
-  cudaFree(f->cursor);
-  cudaFree(f->offs);
-  cudaFree(f->maxlevel);
-  cudaFree(f->temp);
+  cudaFree(f->base);
   delete f;
 }
 
@@ -410,60 +629,111 @@ int fifo_parents(cg_graph *g, int64_t root, const int32_t *d_levels, int32_t *d_
   int rc = fifo_state(g, &f);
   if (rc) return rc;
   const int64_t n = g->n;
+  const int sms = g->num_sms;
   cudaStream_t st = g->stream;
+  CG_CUDA(cudaMemsetAsync(f->sums, 0, sizeof(FifoSums), st));
+  CG_CUDA(cudaMemsetAsync(f->nlong, 0, sizeof(unsigned long long), st));
   CG_CUDA(cudaMemsetAsync(f->counts, 0, sizeof(unsigned) * (size_t)(n + 1), st));
-  CG_CUDA(cudaMemsetAsync(f->maxlevel, 0xff, sizeof(int), st));
-  fifo_hist_kernel<<<grid_for(n, kFifoBlock, g->num_sms), kFifoBlock, 0, st>>>(n, d_levels,
-                                                                               f->counts,
-                                                                               f->maxlevel);
+  fifo_hist_kernel<<<grid_for(n, kFifoBlock, sms), kFifoBlock, 0, st>>>(
+      n, d_levels, g->in_off, g->out_off, f->counts, f->sums);
   CG_CUDA(cudaGetLastError());
-  int maxlevel = -1;
-  CG_CUDA(cudaMemcpyAsync(&maxlevel, f->maxlevel, sizeof(int), cudaMemcpyDeviceToHost, st));
+  FifoSums sums;
+  CG_CUDA(cudaMemcpyAsync(&sums, f->sums, sizeof(sums), cudaMemcpyDeviceToHost, st));
   CG_CUDA(cudaStreamSynchronize(st));
+  const int maxlevel = sums.maxlevel;
   if (maxlevel <= 0) return CG_OK;  // only the root: its parent is itself already
-  std::vector<unsigned> counts((size_t)maxlevel + 1), offs((size_t)maxlevel + 2, 0u);
-  CG_CUDA(cudaMemcpyAsync(counts.data(), f->counts, sizeof(unsigned) * counts.size(),
-                          cudaMemcpyDeviceToHost, st));
-  CG_CUDA(cudaStreamSynchronize(st));
-  for (int L = 1; L <= maxlevel; ++L) offs[L + 1] = offs[L] + counts[L];
-  CG_CUDA(cudaMemcpyAsync(f->offs, offs.data(), sizeof(unsigned) * offs.size(),
-                          cudaMemcpyHostToDevice, st));
-  CG_CUDA(cudaMemsetAsync(f->cursor, 0, sizeof(unsigned) * (size_t)(maxlevel + 1), st));
-  fifo_scatter_kernel<<<grid_for(n, kFifoBlock, g->num_sms), kFifoBlock, 0, st>>>(
-      n, d_levels, f->offs, f->cursor, f->order);
-  CG_CUDA(cudaMemsetAsync(f->rank + root, 0, sizeof(int32_t), st));
-  CG_CUDA(cudaMemsetAsync(f->lr, 0xff, sizeof(unsigned long long) * (size_t)n, st));
-  CG_CUDA(cudaMemsetAsync(f->pl, 0xff, sizeof(unsigned long long) * (size_t)n, st));
-  CG_CUDA(cudaMemsetAsync(f->lr + root, 0, sizeof(unsigned long long), st));  // level 0, rank 0
-  // keys (parent rank << vbits) | v: only the bits in use are sorted
-  const int vbits = bits_for((uint64_t)(n - 1));
+  std::vector<unsigned> counts(sums.counts, sums.counts + kFifoSums);
+  counts.resize((size_t)maxlevel + 1);
+  if (maxlevel >= kFifoSums) {
+    CG_CUDA(cudaMemcpyAsync(counts.data(), f->counts, sizeof(unsigned) * counts.size(),
+                            cudaMemcpyDeviceToHost, st));
+    CG_CUDA(cudaStreamSynchronize(st));
+  }
+  std::vector<unsigned> offs((size_t)maxlevel + 2, 0u);
+  for (int L = 0; L <= maxlevel; ++L) offs[(size_t)L + 1] = offs[(size_t)L] + counts[(size_t)L];
+  // the vertices by level, in id order within one (unreached ones, -1, last:
+  // all bits set is past maxlevel); rk and best hold the values and the keys
+  // on their way
+  fifo_iota_kernel<<<grid_for(n, kFifoBlock, sms), kFifoBlock, 0, st>>>(
+      n, reinterpret_cast<int32_t *>(f->rk));
+  size_t tb = f->temp_bytes;
+  CG_CUDA(cub::DeviceRadixSort::SortPairs(f->temp, tb,
+                                          reinterpret_cast<const uint32_t *>(d_levels), f->best,
+                                          reinterpret_cast<const int32_t *>(f->rk), f->order, n, 0,
+                                          bits_for((uint64_t)maxlevel + 1), st));
+  CG_CUDA(cudaMemsetAsync(f->rk, 0xff, sizeof(uint32_t) * (size_t)n, st));
+  CG_CUDA(cudaMemsetAsync(f->best, 0xff, sizeof(uint32_t) * (size_t)n, st));
+  auto small = [&](int L) {  // level L to L + 1 suits a run of small levels
+    return counts[(size_t)L] <= (unsigned)kSmallLevel &&
+           counts[(size_t)L + 1] <= (unsigned)kSmallLevel && counts[(size_t)L + 1] > 0 &&
+           (L + 1 >= kFifoSums || (sums.out[L] <= kSmallEdges && sums.in[L + 1] <= kSmallEdges));
+  };
+  bool small_ready = false;
+  const int32_t *queue = f->order;  // level L in queue order: level 0 is the root alone
+  int at = 0;                       // f->queue[at], at + 1, at + 2 (mod 3): queue, free, free
   for (int L = 0; L < maxlevel; ++L) {
-    const unsigned c = counts[(size_t)L + 1];
+    const unsigned c = counts[(size_t)L + 1], p = counts[(size_t)L];
     if (c == 0) break;
-    if (c <= (unsigned)kSmallLevel && counts[(size_t)L] <= (unsigned)kSmallLevel) {
-      // a run of small levels: one launch of one block
-      int L1 = L + 1;
-      while (L1 < maxlevel && counts[(size_t)L1 + 1] > 0 &&
-             counts[(size_t)L1 + 1] <= (unsigned)kSmallLevel &&
-             counts[(size_t)L1] <= (unsigned)kSmallLevel)
-        ++L1;
+    const int32_t *seg = f->order + offs[(size_t)L + 1];
+    int L1 = L;
+    while (L1 < maxlevel && small(L1)) ++L1;
+    if (L1 - L >= kSmallRun) {
+      // levels L .. L1 in one launch of one block
+      if (!small_ready) {
+        CG_CUDA(cudaMemsetAsync(f->lr, 0xff, sizeof(unsigned long long) * (size_t)n, st));
+        CG_CUDA(cudaMemsetAsync(f->pl, 0xff, sizeof(unsigned long long) * (size_t)n, st));
+        CG_CUDA(cudaMemcpyAsync(f->offs, offs.data(), sizeof(unsigned) * offs.size(),
+                                cudaMemcpyHostToDevice, st));
+        small_ready = true;
+      }
+      fifo_enter_kernel<<<grid_for(p, kFifoBlock, sms), kFifoBlock, 0, st>>>(queue, p, L, f->rank,
+                                                                             f->lr);
       fifo_small_levels_kernel<<<1, kSmallThreads, sizeof(SmallSmem), st>>>(
           g->in_off, g->in_idx, g->out_off, g->out_idx, f->rank, f->lr, f->pl, f->order,
           f->counts, f->offs, L, L1, (int32_t)root, d_parents);
       CG_CUDA(cudaGetLastError());
+      if (L1 < maxlevel) {
+        int32_t *next = f->queue[(at + 1) % 3];
+        const unsigned c1 = counts[(size_t)L1];
+        fifo_leave_kernel<<<grid_for(c1, kFifoBlock, sms), kFifoBlock, 0, st>>>(
+            f->order + offs[(size_t)L1], c1, f->rank, next);
+        queue = next;
+        at = (at + 1) % 3;
+      }
       L = L1 - 1;
       continue;
     }
-    const unsigned parents_c = counts[(size_t)L];  // ranks of level L: 0 .. parents_c - 1
-    const int end_bit = vbits + bits_for(parents_c ? parents_c - 1 : 0);
-    fifo_pick_kernel<<<grid_for((int64_t)c * 32, kFifoBlock, g->num_sms), kFifoBlock, 0, st>>>(
-        g->in_off, g->in_idx, d_levels, f->rank, f->order + offs[(size_t)L + 1], c, L, vbits,
-        f->keys, d_parents);
-    size_t tb = f->temp_bytes;
-    CG_CUDA(cub::DeviceRadixSort::SortKeys(f->temp, tb, f->keys, f->sorted, (int)c, 0,
-                                           end_bit, st));
-    fifo_rank_kernel<<<grid_for(c, kFifoBlock, g->num_sms), kFifoBlock, 0, st>>>(
-        f->sorted, c, vbits, L + 1, f->rank, f->lr);
+    if (p == 1) {
+      // one possible parent, the search's own; queue order is id order
+      queue = seg;
+      continue;
+    }
+    // atomics count double
+    const bool push = L + 1 < kFifoSums && 2 * sums.out[L] < sums.in[L + 1];
+    if (push) {
+      fifo_push_kernel<<<grid_for((int64_t)p * 32, kFifoBlock, sms), kFifoBlock, 0, st>>>(
+          g->out_off, g->out_idx, d_levels, queue, p, L, f->best, f->longs, f->nlong);
+      fifo_long_kernel<true><<<sms * 8, kFifoBlock, 0, st>>>(g->out_off, g->out_idx, d_levels,
+                                                             f->rk, L, f->best, f->longs, f->nlong);
+    } else {
+      fifo_ranks_kernel<<<grid_for(p, kFifoBlock, sms), kFifoBlock, 0, st>>>(queue, p, f->rk);
+      fifo_pull_kernel<<<grid_for(c, kFifoBlock, sms), kFifoBlock, 0, st>>>(
+          g->in_off, g->in_idx, f->rk, seg, c, f->best, f->longs, f->nlong);
+      fifo_long_kernel<false><<<sms * 8, kFifoBlock, 0, st>>>(g->in_off, g->in_idx, d_levels, f->rk,
+                                                              L, f->best, f->longs, f->nlong);
+    }
+    int32_t *vals[2] = {f->queue[(at + 1) % 3], f->queue[(at + 2) % 3]};
+    fifo_finish_kernel<<<grid_for(c > p ? c : p, kFifoBlock, sms), kFifoBlock, 0, st>>>(
+        seg, c, f->best, queue, p, push ? 0 : 1, f->rk, f->key[0], vals[0], d_parents, f->nlong);
+    CG_CUDA(cudaGetLastError());
+    if (L + 1 == maxlevel) break;  // the last level's order is not needed
+    cub::DoubleBuffer<uint32_t> kb(f->key[0], f->key[1]);
+    cub::DoubleBuffer<int32_t> vb(vals[0], vals[1]);
+    tb = f->temp_bytes;
+    CG_CUDA(cub::DeviceRadixSort::SortPairs(f->temp, tb, kb, vb, (int64_t)c, 0, bits_for(p - 1),
+                                            st));
+    queue = vb.Current();
+    at = vb.Current() == vals[0] ? (at + 1) % 3 : (at + 2) % 3;
   }
   CG_CUDA(cudaGetLastError());
   return CG_OK;
