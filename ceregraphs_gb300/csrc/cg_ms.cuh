@@ -15,10 +15,7 @@ constexpr int kMsMaxLanes = 128;
 constexpr int kPullLight = 32;    // in-degree <= this: one thread scans the in-list
 constexpr int kHubDeg = 1024;     // in-degree > this: hub
 constexpr int kHubChunk = 1024;   // in-list entries of a hub per work item
-constexpr int kPairs = 4;         // first-hit records a light vertex's pull rounds may take,
-                                  // unless the light vertices hold under half of the edges
-                                  // (then all kRecords: see MsState::pull_records)
-constexpr int kRecords = 8;       // records per light vertex in all (pull rounds + scan pass)
+constexpr int kPosBits = 5;       // bits of a position in a light vertex's in-list
 
 struct MsRound {
   unsigned long long nf[kCounterShards];      // vertices with a nonzero frontier mask
@@ -50,8 +47,8 @@ struct MsCtl {
   int pull_rounds;
   int switches;
   unsigned exited;                // blocks past the final pass (finish time)
-  unsigned nover;                 // light vertices whose records ran out (scan pass)
   unsigned scan_work;             // scan pass: chunks of scanmap handed out
+  unsigned pad0;
   unsigned long long visited;
   unsigned long long done[2];     // lanes whose search ended (cleared by the host)
   long long t_start;
@@ -68,14 +65,13 @@ struct MsParams {
   const int32_t *__restrict__ out_idx;
   uint64_t *vis, *fr0, *fr1, *fr2;
   uint32_t *touched0, *touched1, *touched2;
-  uint32_t *scanmap;  // light vertices with lanes their records leave open (ledger)
+  uint32_t *scanmap;  // vertices whose parents the rounds leave open (ledger)
   const uint32_t *dead;  // vertices without in-edges (never reached after round 0)
   // ledger batches: vertices of in-degree 1 .. kPullLight (static), and those
   // of them a batch has finished -- every running lane visited (no lane can
   // reach them again), so later pull rounds skip them
   const uint32_t *light;
   uint32_t *fin;
-  int pull_records;    // ledger: records a light vertex's pull rounds may take (<= kRecords)
   int32_t *queue0, *queue1;
   uint32_t *bigoff0, *bigoff1;
   const int32_t *hub_slot;   // [n], -1 for non-hubs
@@ -115,12 +111,12 @@ struct MsParams {
   const uint32_t *cand_choff; // [ncand + 1] prefix of in-list chunks
   uint32_t *cand;             // [ncand][64 W], 0xFFFFFFFF = none yet
   int ncand;
-  // (source, lanes) records of light vertices: the first hits of their
-  // pull-round scans (up to kPairs), then those of the scan pass after the
-  // rounds (up to kRecords in all); record q at [q * n + v]
-  int32_t *pair_u;
-  uint64_t *pair_m;           // W words per record
-  uint8_t *pair_n;            // [n] records used
+  // ledger batches: the in-list position of each lane's parent, for light
+  // vertices, as bit slices -- bit l of pos[b][v] is bit b of lane l's position.
+  // Slice b of v counts only once bit b of pos_used[v] is set (it is stored
+  // then, not ORed: the slices need no clearing between batches)
+  uint64_t *pos;              // [kPosBits][n][W]
+  uint8_t *pos_used;          // [n]
   int gate;                   // run only if *flag is set (the fallback launch)
   int32_t roots[kMsMaxLanes];
 };
@@ -544,11 +540,9 @@ struct MsState {
   uint32_t *cand_choff = nullptr;
   uint32_t *cand = nullptr;
   int ncand = 0;
-  int32_t *pair_u = nullptr;
-  uint64_t *pair_m = nullptr;
-  uint8_t *pair_n = nullptr;
+  uint64_t *pos = nullptr;
+  uint8_t *pos_used = nullptr;
   uint32_t *lightfin = nullptr;  // [2][words]: the light map, then the finished map
-  int pull_records = kPairs;     // records a light vertex's pull rounds may take
   int64_t bcap = 0;
   int nhub = 0;
   int lane_words = 0;
@@ -581,12 +575,10 @@ inline MsParams ms_params(const cg_graph *g, const MsState *s) {
   p.cand_choff = s->cand_choff;
   p.cand = s->cand;
   p.ncand = s->ncand;
-  p.pair_u = s->pair_u;
-  p.pair_m = s->pair_m;
-  p.pair_n = s->pair_n;
+  p.pos = s->pos;
+  p.pos_used = s->pos_used;
   p.light = s->lightfin;
   p.fin = s->lightfin ? s->lightfin + p.words : nullptr;
-  p.pull_records = s->pull_records;
   p.touched0 = s->touched;
   p.scanmap = s->touched + 3 * p.words;
   p.dead = g->dead;
@@ -642,8 +634,8 @@ inline int ms_reset(const MsState *s, cudaStream_t stream) {
   return CG_OK;
 }
 
-// History launch of one batch (cg_msledger.cu): the rounds, then the scan,
-// output and fix-up passes; sets *s->flag instead if the search outgrows the
+// History launch of one batch (cg_msledger.cu): the rounds, then the scan
+// and output passes; sets *s->flag instead if the search outgrows the
 // history.
 int ms_ledger_pass(cg_graph *g, MsState *s, const int64_t *roots, int k, int32_t *d_levels,
                    int32_t *d_parents);

@@ -645,9 +645,8 @@ static void ms_free_state(MsState *s) {
   cudaFree(s->cand_vtx);
   cudaFree(s->cand_choff);
   cudaFree(s->cand);
-  cudaFree(s->pair_u);
-  cudaFree(s->pair_m);
-  cudaFree(s->pair_n);
+  cudaFree(s->pos);
+  cudaFree(s->pos_used);
   cudaFree(s->lightfin);
   delete s;
 }
@@ -768,11 +767,9 @@ __global__ void slot_map_kernel(int count, const int32_t *__restrict__ vtx, int3
 }
 
 // Bit v of light[w]: vertex v = 32 w + b has in-degree 1 .. kPullLight (the
-// vertices a ledger pull round scans one thread each); *light_edges sums
-// their in-degrees.
+// vertices a ledger pull round scans one thread each).
 __global__ void light_map_kernel(int64_t n, int64_t words, const int64_t *__restrict__ in_off,
-                                 uint32_t *light, unsigned long long *light_edges) {
-  unsigned long long e = 0;
+                                 uint32_t *light) {
   for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < words;
        w += (int64_t)gridDim.x * blockDim.x) {
     uint32_t m = 0;
@@ -780,14 +777,10 @@ __global__ void light_map_kernel(int64_t n, int64_t words, const int64_t *__rest
       const int64_t v = w * 32 + b;
       if (v >= n) break;
       const int64_t d = in_off[v + 1] - in_off[v];
-      if (d >= 1 && d <= kPullLight) {
-        m |= 1u << b;
-        e += (unsigned long long)d;
-      }
+      if (d >= 1 && d <= kPullLight) m |= 1u << b;
     }
     light[w] = m;
   }
-  if (e) atomicAdd(light_edges, e);
 }
 
 // Parent-candidate slots of the output pass of a ledger batch: every vertex of
@@ -801,36 +794,19 @@ static int ms_build_cands(cg_graph *g, MsState *s) {
       cudaMalloc(&s->cand_vtx, sizeof(int32_t) * nc) != cudaSuccess ||
       cudaMalloc(&s->cand_choff, sizeof(uint32_t) * (nc + 1)) != cudaSuccess ||
       cudaMalloc(&s->cand, sizeof(uint32_t) * nc * 64 * s->lane_words) != cudaSuccess ||
-      cudaMalloc(&s->pair_u, sizeof(int32_t) * kRecords * (size_t)g->n) != cudaSuccess ||
-      cudaMalloc(&s->pair_m, sizeof(uint64_t) * kRecords * (size_t)g->n * s->lane_words) !=
+      cudaMalloc(&s->pos, sizeof(uint64_t) * kPosBits * (size_t)g->n * s->lane_words) !=
           cudaSuccess ||
-      cudaMalloc(&s->pair_n, (size_t)((g->n + 3) / 4) * 4) != cudaSuccess ||
+      cudaMalloc(&s->pos_used, (size_t)((g->n + 3) / 4) * 4) != cudaSuccess ||
       cudaMalloc(&s->lightfin, sizeof(uint32_t) * 2 * (size_t)((g->n + 31) / 32)) != cudaSuccess)
     return CG_ERR_OUT_OF_MEMORY;
-  g->device_bytes += (sizeof(int32_t) + sizeof(uint64_t) * s->lane_words) * kRecords * g->n + g->n +
+  g->device_bytes += sizeof(uint64_t) * s->lane_words * kPosBits * g->n + g->n +
                      sizeof(uint32_t) * 2 * ((g->n + 31) / 32);
   {
-    // pull rounds may take all kRecords records where light vertices hold
-    // under half of the edges (their parents are a few hubs: R-MAT), else
-    // kPairs, leaving room for the scan pass to merge later hits into
-    // records of the same source (graphs of light vertices only: each is
-    // reached over many rounds, from the same few in-neighbours)
     const int64_t words = (g->n + 31) / 32;
     const int64_t blocks = (words + 255) / 256;
-    unsigned long long *d_le = nullptr, le = 0;
-    CG_CUDA(cudaMalloc(&d_le, sizeof(unsigned long long)));
-    cudaError_t e = cudaMemsetAsync(d_le, 0, sizeof(unsigned long long), g->stream);
-    if (e == cudaSuccess) {
-      light_map_kernel<<<(unsigned)(blocks < 4096 ? blocks : 4096), 256, 0, g->stream>>>(
-          g->n, words, g->in_off, s->lightfin, d_le);
-      e = cudaGetLastError();
-    }
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(&le, d_le, sizeof(le), cudaMemcpyDeviceToHost, g->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-    cudaFree(d_le);
-    if (e != cudaSuccess) return cuda_fail(e, "light-vertex map");
-    s->pull_records = 2 * le < (unsigned long long)g->nnz ? kRecords : kPairs;
+    light_map_kernel<<<(unsigned)(blocks < 4096 ? blocks : 4096), 256, 0, g->stream>>>(
+        g->n, words, g->in_off, s->lightfin);
+    CG_CUDA(cudaGetLastError());
   }
   CG_CUDA(cudaMemsetAsync(s->cand_slot, 0xff, sizeof(int32_t) * (size_t)g->n, g->stream));
   if (s->nmed)
@@ -1021,8 +997,8 @@ int msbfs_launch(cg_graph *g, const int64_t *roots, int32_t k, int32_t *d_levels
     int32_t *lv = d_levels + (int64_t)b * g->n;
     int32_t *pa = d_parents + (int64_t)b * g->n;
     if (s->hist_planes >= 4) {
-      // rounds on masks, then the scan, output and fix-up passes; the direct
-      // kernel runs only if the search outgrew the history
+      // rounds on masks, then the scan and output passes; the direct kernel
+      // runs only if the search outgrew the history
       rc = ms_ledger_pass(g, s, roots + b, kk, lv, pa);
       if (!rc) rc = W == 2 ? ms_launch_gated<2>(g, s, roots + b, kk, lv, pa)
                            : ms_launch_gated<1>(g, s, roots + b, kk, lv, pa);

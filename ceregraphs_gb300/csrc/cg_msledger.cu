@@ -2,9 +2,8 @@
 // mode).  The rounds advance the W-word lane masks -- vis, and the frontier
 // F_L of every round, kept as a history F_0 .. F_D in HBM -- and write no
 // per-(lane, vertex) output.  After the last round a scan pass resolves the
-// parents the rounds left open, one output pass writes every (lane, vertex)
-// output exactly once, and a fix-up pass rewrites the few parents that did
-// not fit the per-vertex records:
+// parents the rounds left open and one output pass writes every (lane, vertex)
+// output exactly once:
 //   level(l, v)  = the round L whose F_L[v] holds bit l      (-1 if none)
 //   parent(l, v) = v at level 0, roots[l] at level 1, else the lowest
 //                  in-neighbour u of v with bit l in F_{level - 1}[u]
@@ -21,12 +20,14 @@
 // candidates.  A push round relaxing u -> v takes atomicMin(slot[l], u) for
 // each new lane l (ms_relax); a pull round scans such a vertex's ascending
 // in-list with one warp (or its chunks, for hubs, with several) and records
-// each lane's first hit (or_warp_first).  Vertices of smaller in-degree keep
-// (source, lanes) records: a pull round's thread scan records each entry that
-// brings new lanes (the lowest-index parent of those lanes, the in-list being
-// ascending); the lanes pushes gave them, and those past the pull rounds'
-// records, are resolved by the scan pass (scan_in_list), which appends
-// records; lanes past all records go to the fix-up pass.
+// each lane's first hit (or_warp_first).  Vertices of smaller in-degree keep the
+// position of each lane's parent in their in-list, as kPosBits bit slices: a
+// pull round's thread scan knows it for the lanes it finds (the first entry
+// holding a lane is its lowest-index parent, the in-list being ascending), the
+// scan pass finds it for the lanes that pushes gave them.  The size is fixed
+// and no later pass has to sort overlaps out: (source, lanes) records, up to 8
+// of them, ran out on a directed graph of in-degree 8 and left 0.79 ms of
+// fix-ups and 0.59 ms of rescans of a 2.4 ms batch (n = 1 M, 100 lanes).
 //
 // Rounds: a pull round ORs the frontier masks of a vertex's in-neighbours
 // until every wanted lane is found; a push round ORs frontier masks into
@@ -53,26 +54,35 @@ namespace {
 constexpr int kOutBlock = 128;                 // output pass: 4 warps a block
 constexpr int kOutWarps = kOutBlock / 32;
 constexpr int kOutLevels = 4;                  // levels resolved per in-list scan
-// A warp's shared tile: one parent table of kTab words per thread -- 64
-// parents of its vertex (lane l at column (l - 8 t) mod 64 for thread t: the
-// 32 threads reading the same lane hit 32 different banks, the stride being
-// 9 mod 32), then the sources of its kRecords records at kTabRec + q, and -1
-// (unreached) at kTabNone.  A lane's parent is one table read at a byte index.
-constexpr int kTabRec = 64;
-constexpr int kTabNone = kTabRec + 8;
+// A warp's shared tile: one parent table of kTab words per thread.  A vertex
+// with a candidate slot has its 64 parents there, lane l at column (l - 8 t) mod
+// 64 for thread t (the 32 threads reading the same lane hit 32 different banks,
+// kTab - 8 being odd); a light vertex the in-list entries that positions point
+// at, from column 0; -1 (unreached) is at kTabNone.  A lane's parent is one
+// table read at a byte index.
+constexpr int kTabNone = 64;
 constexpr int kTab = kTabNone + 1;
-constexpr int kOutWarpBytes = 32 * kTab * 4;
-static_assert(kRecords <= 8, "record indices are 3 bit slices");
+// Behind the table, the bytes of 32 lanes' levels and table indices: word t of
+// row g has those of lanes g, g + 8, g + 16, g + 24 for thread t's vertex (rows
+// of 33 words: eight threads each on four rows read different banks).
+constexpr int kStageRow = 33;
+constexpr int kStage = 8 * kStageRow;
+constexpr int kOutWarpBytes = (32 * kTab + 2 * kStage) * 4;
+static_assert((kTab - 8) % 2 == 1, "same lane, different banks");
+static_assert((1 << kPosBits) == kPullLight, "a position in a light in-list");
 constexpr int kSlices = 7;                     // bit slices of a level (levels 0..64)
 
-// Bits 0..3 of x moved to bit 0 of bytes 0..3 (the four shifted copies do not
-// overlap, so the product has no carries).
-__device__ __forceinline__ uint32_t spread4(uint32_t x) { return (x * 0x00204081u) & 0x01010101u; }
-
-template <bool B>
-struct Flag {
-  static constexpr bool value = B;
-};
+// Four bytes from global to shared memory, asynchronously; the wait covers all
+// copies of the calling thread.
+__device__ __forceinline__ void copy_async4(void *dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
 
 template <int W>
 __device__ __forceinline__ uint64_t *plane(const MsParams &p, int L) {
@@ -98,24 +108,38 @@ __device__ __forceinline__ Mask<W> or_thread(const MsParams &p, int64_t s, int64
   return got;
 }
 
-// or_thread that also records, for light vertex v, each in-list entry that
-// brings new lanes -- their lowest-index parent, the scan being ascending --
-// as a (source, lanes) pair, up to p.pull_records per vertex over all pull rounds.
+// Adds lanes to slice b of light vertex v's positions; `used` is its pos_used.
+template <int W>
+__device__ __forceinline__ void add_slice(const MsParams &p, int64_t v, int b, const Mask<W> &a,
+                                          unsigned &used) {
+  if (!a.any()) return;
+  const int64_t at = (int64_t)b * p.n + v;
+  st_mask<W>(p.pos, at, (used >> b) & 1u ? a | ld_mask<W>(p.pos, at) : a);
+  used |= 1u << b;
+}
+
+// The scan of light vertex v's in-list in a pull round: ORs its in-neighbours'
+// frontier masks for the lanes of `want` until all are found (returned), and
+// keeps the position of each lane's first entry, its lowest-index parent.
 // `want1`, after a push round: the lanes that push gave v at this round's
 // level L, whose parents are the first entries holding them in F_{L-1}
-// (`prev`) -- found in the same pass and recorded alike, so the scan pass
-// need not rescan v.  Lanes found after the records run out (`over`) are
-// left to the scan pass.  Returns the lanes of `want` found.
+// (`prev`) -- found in the same pass, so the scan pass need not rescan v.
 template <int W>
-__device__ __forceinline__ Mask<W> or_thread_rec(const MsParams &p, int64_t v, int64_t s,
+__device__ __forceinline__ Mask<W> or_thread_pos(const MsParams &p, int64_t v, int64_t s,
                                                  int64_t e, const Mask<W> &want,
                                                  const uint64_t *cur, const uint64_t *prev,
-                                                 const Mask<W> &want1, bool &over) {
+                                                 const Mask<W> &want1) {
   constexpr int G = 4;
   Mask<W> got = Mask<W>::zero(), got1 = Mask<W>::zero();
+  // the lanes at positions with bit 0 .. 4 set; with 128 lanes the last three
+  // would spill and go to memory as they are found
+  constexpr int kKept = W == 1 ? kPosBits : 2;
+  Mask<W> A[kKept];
+#pragma unroll
+  for (int b = 0; b < kKept; ++b) A[b] = Mask<W>::zero();
+  const unsigned used0 = p.pos_used[v];
+  unsigned used = used0;
   const bool two = want1.any();
-  int used = p.pair_n[v];
-  const int first = used;
   for (int64_t i0 = s; i0 < e; i0 += G) {
     int32_t u[G];
     Mask<W> m[G], m1[G];
@@ -126,27 +150,33 @@ __device__ __forceinline__ Mask<W> or_thread_rec(const MsParams &p, int64_t v, i
       m[k] = u[k] >= 0 ? ld_mask<W>(cur, u[k]) : Mask<W>::zero();
       m1[k] = two && u[k] >= 0 ? ld_mask<W>(prev, u[k]) : Mask<W>::zero();
     }
+    // entry i0 + k is at position i0 - s + k: its low two bits are k's
+    Mask<W> four = Mask<W>::zero();
 #pragma unroll
     for (int k = 0; k < G; ++k) {
       const Mask<W> nb = (m[k] & want).andnot(got);
       const Mask<W> nb1 = (m1[k] & want1).andnot(got1);
       const Mask<W> r = nb | nb1;  // disjoint: want1 lanes are visited, want lanes are not
-      if (r.any()) {
-        if (used < p.pull_records) {
-          const int64_t at = (int64_t)used * p.n + v;
-          p.pair_u[at] = u[k];
-          st_mask<W>(p.pair_m, at, r);
-          ++used;
-        } else {
-          over = true;
-        }
-        got = got | nb;
-        got1 = got1 | nb1;
-      }
+      if (k & 1) A[0] = A[0] | r;
+      if (k & 2) A[1] = A[1] | r;
+      four = four | r;
+      got = got | nb;
+      got1 = got1 | nb1;
+    }
+    const int hi = (int)(i0 - s) >> 2;
+#pragma unroll
+    for (int b = 2; b < kPosBits; ++b) {
+      if (!((hi >> (b - 2)) & 1)) continue;
+      if (b < kKept)
+        A[b < kKept ? b : 0] = A[b < kKept ? b : 0] | four;
+      else
+        add_slice<W>(p, v, b, four, used);
     }
     if (got == want && got1 == want1) break;
   }
-  if (used != first) p.pair_n[v] = (uint8_t)used;
+#pragma unroll
+  for (int b = 0; b < kKept; ++b) add_slice<W>(p, v, b, A[b], used);
+  if (used != used0) p.pos_used[v] = (uint8_t)used;
   return got;
 }
 
@@ -262,9 +292,9 @@ template <int W>
 __device__ void lg_pull(const MsParams &p, int L, const uint64_t *cur, uint64_t *nxt,
                         const Mask<W> &active, bool after_push, MsRound *Rc, MsRound *Rn,
                         MsAcc &acc) {
-  // after a push round of level >= 1, light vertices also resolve the
-  // parents of the lanes that push gave them (F_L) against F_{L-1} (64
-  // lanes; with 128 the registers would spill, and the scan pass does it)
+  // after a push round, light vertices also resolve the parents of the lanes
+  // that push gave them (F_L) against F_{L-1} (64 lanes; with 128 the registers
+  // would spill, and the scan pass does it)
   after_push = after_push && W == 1;
   const uint64_t *prev = after_push ? plane<W>(p, L - 1) : cur;
   const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
@@ -338,12 +368,12 @@ __device__ void lg_pull(const MsParams &p, int L, const uint64_t *cur, uint64_t 
         // every running lane visited: no lane can reach v again (finished
         // lanes never run again), so later rounds skip it
         const bool done = has && !want.any();
-        bool claimed = false, over = false;
+        bool claimed = false;
         int64_t deg = 0;
         const bool scan = want.any() || want1.any();
         if (__ballot_sync(kMsFull, scan)) {
           Mask<W> got = Mask<W>::zero();
-          if (scan) got = or_thread_rec<W>(p, v, s, e, want, cur, prev, want1, over);
+          if (scan) got = or_thread_pos<W>(p, v, s, e, want, cur, prev, want1);
           claimed = got.any();
           if (claimed) {
             st_mask<W>(nxt, v, got);
@@ -351,20 +381,17 @@ __device__ void lg_pull(const MsParams &p, int L, const uint64_t *cur, uint64_t 
             deg = sym ? e - s : __ldg(p.out_off + v + 1) - __ldg(p.out_off + v);
           }
         }
-        // per word of the batch: claim bits (T_{L+1}), records overflow
-        // (scanmap), finished bits
+        // per word of the batch: claim bits (T_{L+1}), finished bits
         const unsigned mybit = 1u << (unsigned)(v & 31);
         const int wlo = __shfl_sync(kMsFull, wsel, 0);
         const int whi = __shfl_sync(kMsFull, wsel, min(31, total - 1 - b0));
         for (int j = wlo; j <= whi; ++j) {  // uniform: the whole warp
           const bool inj = has && wsel == j;
           const unsigned cb = __reduce_or_sync(kMsFull, inj && claimed ? mybit : 0u);
-          const unsigned ob = __reduce_or_sync(kMsFull, inj && over ? mybit : 0u);
           const unsigned db = __reduce_or_sync(kMsFull, inj && done ? mybit : 0u);
           if (lane == j) {
             finw |= db;
             if (cb) atomicOr(tnext + w0 + j, cb);
-            if (ob) atomicOr(p.scanmap + w0 + j, ob);
           }
         }
         ms_enqueue<false>(claimed, (int32_t)v, deg, q, p.n, boff, &Rn->nlight, &Rn->big, acc);
@@ -856,7 +883,7 @@ __global__ void __launch_bounds__(kMsBlock, 2) msbfs_ledger(MsParams p) {
     p.scanmap[w] = 0;
     p.fin[w] = 0;
   }
-  uint32_t *pn = reinterpret_cast<uint32_t *>(p.pair_n);
+  uint32_t *pn = reinterpret_cast<uint32_t *>(p.pos_used);
   for (int64_t w = gtid; w < (p.n + 3) / 4; w += nthreads) pn[w] = 0;
   bool ok = grid_wait(&ctl->wait, &ctl->status, p.timeout_ns);
   if (ok && blockIdx.x == 0 && threadIdx.x < p.k) {
@@ -906,10 +933,10 @@ __global__ void __launch_bounds__(kMsBlock, 2) msbfs_ledger(MsParams p) {
     }
     uint32_t *tclr = claims(p, L + 2);
     for (int64_t w = gtid; w < p.words; w += nthreads) tclr[w] = 0;
-    if (L >= 2 && pdir == 0 && (dir == 0 || W != 1)) {
-      // a push round gave these vertices lanes at level L >= 2 and this
-      // round is a push too (or 128 lanes): the scan pass resolves their
-      // parents (else this pull round's light scans do, or_thread_rec)
+    if (L >= 1 && pdir == 0 && (dir == 0 || W != 1)) {
+      // a push round gave these vertices lanes and this round is a push too
+      // (or 128 lanes): the scan pass resolves their parents (else this pull
+      // round's light scans do, or_thread_pos); open_levels has the same rule
       const uint32_t *tcur = claims(p, L);
       for (int64_t w = gtid; w < p.words; w += nthreads) {
         const uint32_t t = tcur[w];
@@ -920,7 +947,7 @@ __global__ void __launch_bounds__(kMsBlock, 2) msbfs_ledger(MsParams p) {
       Mask<W> active;
 #pragma unroll
       for (int i = 0; i < W; ++i) active.w[i] = *(volatile unsigned long long *)&Rc->lanes[i];
-      lg_pull<W>(p, L, cur, nxt, active, L >= 2 && pdir == 0, Rc, Rn, acc);
+      lg_pull<W>(p, L, cur, nxt, active, L >= 1 && pdir == 0, Rc, Rn, acc);
       if (p.nhub > 0) {
         if (!(ok = grid_wait(&ctl->wait, &ctl->status, p.timeout_ns))) break;
         lg_hub_merge<W>(p, L, cur, nxt, Rn, acc);
@@ -955,9 +982,9 @@ __global__ void __launch_bounds__(kMsBlock, 2) msbfs_ledger(MsParams p) {
     p.stats->status = *(volatile int *)&ctl->status;
 }
 
-// ---- scan pass, output pass, fix-up pass ------------------------------------
+// ---- scan pass, output pass ---------------------------------------------------
 
-constexpr int kScanBlock = 256;  // scan and fix-up passes: threads a block
+constexpr int kScanBlock = 256;  // scan pass: threads a block
 constexpr int kScanWords = 4;    // scan pass: scanmap words a warp takes at a time
 constexpr int kScanG = 2;        // in-list entries loaded together (most lanes resolve at the first)
 constexpr int kPre = 8;          // history planes loaded together (the output pass needs 8)
@@ -970,111 +997,33 @@ __device__ __forceinline__ int history_rounds(const MsParams &p) {
   return rounds;
 }
 
-// Lanes of `want` for which u is one level closer to the root than v: bit l
-// of Ms[k] is a lane with v at level Ls[k]; u qualifies if F_{Ls[k]-1}[u] has l.
+// Bit L: the parents of level L's light vertices were left open -- round L - 1
+// pushed, and round L was no pull round that resolves them.
 template <int W>
-__device__ __forceinline__ uint64_t parent_hits(const MsParams &p, int32_t u, int h,
-                                                const int (&Ls)[kOutLevels],
-                                                const uint64_t (&Ms)[kOutLevels], uint64_t want) {
-  uint64_t b = 0;
-#pragma unroll
-  for (int k = 0; k < kOutLevels; ++k)
-    if (Ms[k] & want) b |= Ms[k] & plane<W>(p, Ls[k] - 1)[(int64_t)u * W + h];
-  return b & want;
-}
-
-// The lanes of `todo` (half h) that light vertex v reached at a level >= 2,
-// resolved by scans of v's ascending in-list: the first entry u holding the
-// lane in F_{level - 1}[u] is the lane's parent, the lowest-index rule.  One
-// pass over the list resolves up to kOutLevels levels; hit(u, lanes) gets
-// each entry that resolves lanes.
-template <int W, int G, class Hit>
-__device__ __forceinline__ void scan_in_list(const MsParams &p, int64_t v, int h, int rounds,
-                                             int64_t s, int64_t e, uint64_t todo, Hit &&hit) {
-  int L = 2;
-  while (todo && L < rounds) {
-    int Ls[kOutLevels];
-    uint64_t Ms[kOutLevels];
-#pragma unroll
-    for (int k = 0; k < kOutLevels; ++k) {
-      Ls[k] = 1;
-      Ms[k] = 0;
-    }
-    int nl = 0;
-    uint64_t gtodo = 0;
-    while (nl < kOutLevels && L < rounds && todo) {
-      uint64_t pm[kPre];
-#pragma unroll
-      for (int j = 0; j < kPre; ++j)
-        pm[j] = L + j < rounds ? plane<W>(p, L + j)[v * W + h] : 0ull;
-      int taken = 0;
-#pragma unroll
-      for (int j = 0; j < kPre; ++j) {
-        if (nl < kOutLevels) {
-          const uint64_t m = pm[j] & todo;
-          if (m) {
-#pragma unroll
-            for (int k = 0; k < kOutLevels; ++k)
-              if (k == nl) {
-                Ls[k] = L + j;
-                Ms[k] = m;
-              }
-            ++nl;
-            todo &= ~m;
-            gtodo |= m;
-          }
-          taken = j + 1;
-        }
-      }
-      L += taken;
-    }
-    for (int64_t j0 = s; j0 < e && gtodo; j0 += G) {
-      int32_t u[G];
-      uint64_t b[G];
-#pragma unroll
-      for (int k = 0; k < G; ++k) u[k] = j0 + k < e ? __ldg(p.in_idx + j0 + k) : -1;
-#pragma unroll
-      for (int k = 0; k < G; ++k)
-        b[k] = u[k] >= 0 ? parent_hits<W>(p, u[k], h, Ls, Ms, gtodo) : 0;
-#pragma unroll
-      for (int k = 0; k < G; ++k) {
-        const uint64_t bk = b[k] & gtodo;
-        if (bk) {
-          gtodo &= ~bk;
-          hit(u[k], bk);
-        }
-      }
-    }
+__device__ __forceinline__ uint64_t open_levels(const MsParams &p, int rounds) {
+  uint64_t open = 0;
+  for (int L = 1; L < rounds && L < CG_HISTORY; ++L) {
+    const bool pushed = p.stats->direction_history[L - 1] == 0;
+    const bool resolved = W == 1 && p.stats->direction_history[L] == 1;
+    if (pushed && !resolved) open |= 1ull << L;
   }
-}
-
-// OR of the masks of records [0, np) of vertex v, half h (np <= kRecords).
-template <int W>
-__device__ __forceinline__ uint64_t records_mask(const MsParams &p, int64_t v, int h, int np) {
-  uint64_t m = 0;
-#pragma unroll
-  for (int q = 0; q < kRecords; ++q)
-    if (q < np) m |= p.pair_m[((int64_t)q * p.n + v) * W + h];
-  return m;
+  return open;
 }
 
 // Scan pass, between the rounds and the output pass, over the light vertices
 // (in-degree 1 .. kPullLight; heavier ones have candidate slots) that the
-// rounds marked in scanmap: reached by a push round at a level >= 2, or with
-// more pull-round first hits than records.  A warp takes kScanWords words of
-// the map at a time (the first by its index, the next from a counter, claimed
-// before the current chunk is worked), compacts their marked vertices in
-// shared memory, and gives each thread one.
-// The lanes a vertex's records leave open are resolved by scan_in_list and
-// appended as records; a vertex that runs out of records goes on a list
-// (queue0, free once the rounds are over) for the fix-up pass.
+// rounds marked in scanmap.  A warp takes kScanWords words of the map at a time
+// (the first by its index, the next from a counter, claimed before the current
+// chunk is worked), compacts their marked vertices in shared memory, and gives
+// each thread one, whose in-list it scans for the parents of up to kOutLevels
+// open levels at once: the first entry u holding a lane of F_L in F_{L-1} is
+// its parent, and its position joins the vertex's slices.
 template <int W>
 __global__ void __launch_bounds__(kScanBlock) msbfs_scan(MsParams p) {
   __shared__ int32_t s_list[kScanBlock / 32][kScanWords * 32];
-  __shared__ int32_t s_ru[kScanBlock][kRecords + 1];  // a thread's record sources
   if (*(volatile int *)p.flag || *(volatile int *)&p.ctl->status != 0) return;
-  const int rounds = history_rounds(p);
-  if (rounds <= 2) return;
+  const uint64_t open = open_levels<W>(p, history_rounds(p));
+  if (!open) return;
   const int lane = lane_id();
   int32_t *list = s_list[threadIdx.x >> 5];
   const unsigned nwarps = gridDim.x * (kScanBlock / 32);
@@ -1085,7 +1034,8 @@ __global__ void __launch_bounds__(kScanBlock) msbfs_scan(MsParams p) {
     if (lane == 0) next = nwarps + atomicAdd(&p.ctl->scan_work, 1u);
     const int64_t w0 = (int64_t)chunk * kScanWords;
     const int64_t wi = w0 + lane;
-    uint32_t bits = lane < kScanWords && wi < p.words ? p.scanmap[wi] : 0u;
+    uint32_t bits =
+        lane < kScanWords && wi < p.words ? p.scanmap[wi] & __ldg(p.light + wi) : 0u;
     const int c = __popc(bits);
     int incl = c;
 #pragma unroll
@@ -1099,108 +1049,80 @@ __global__ void __launch_bounds__(kScanBlock) msbfs_scan(MsParams p) {
     for (int i = lane; i < total; i += 32) {
       const int64_t v = list[i];
       const int64_t s = __ldg(p.in_off + v), e = __ldg(p.in_off + v + 1);
-      if (e == s || e - s > kPullLight) continue;
-      const int np0 = p.pair_n[v];
-      int np = np0;
-      bool over = false;
-      // the records' sources: a hit from a source already recorded joins its
-      // record (pull rounds record a source again in each round it serves)
-      int32_t *ru = s_ru[threadIdx.x];
-      for (int q = 0; q < np0; ++q) ru[q] = p.pair_u[(int64_t)q * p.n + v];
-      for (int h = 0; h < W && 64 * h < p.k; ++h) {
-        const uint64_t covered = records_mask<W>(p, v, h, np0);
-        scan_in_list<W, kScanG>(p, v, h, rounds, s, e, ~covered, [&](int32_t u, uint64_t m) {
-          int found = -1;
-          for (int q = 0; q < np && found < 0; ++q)
-            if (ru[q] == u) found = q;
-          if (found >= 0) {
-            p.pair_m[((int64_t)found * p.n + v) * W + h] |= m;
-          } else if (np < kRecords) {
-            const int64_t at = (int64_t)np * p.n + v;
-            p.pair_u[at] = u;
+      Mask<W> A[kPosBits];
 #pragma unroll
-            for (int w = 0; w < W; ++w) p.pair_m[at * W + w] = w == h ? m : 0ull;
-            ru[np] = u;
-            ++np;
-          } else {
-            over = true;
+      for (int b = 0; b < kPosBits; ++b) A[b] = Mask<W>::zero();
+      for (uint64_t left = open; left;) {
+        int Ls[kOutLevels];
+        Mask<W> Ms[kOutLevels], todo = Mask<W>::zero();
+#pragma unroll
+        for (int k = 0; k < kOutLevels; ++k) {
+          Ls[k] = left ? __ffsll((long long)left) - 1 : 0;
+          left &= left ? left - 1 : 0ull;
+          Ms[k] = Ls[k] ? ld_mask<W>(plane<W>(p, Ls[k]), v) : Mask<W>::zero();
+        }
+#pragma unroll
+        for (int k = 0; k < kOutLevels; ++k) todo = todo | Ms[k];
+        for (int64_t j0 = s; j0 < e && todo.any(); j0 += kScanG) {
+          int32_t u[kScanG];
+          Mask<W> hit[kScanG];
+#pragma unroll
+          for (int q = 0; q < kScanG; ++q) {
+            u[q] = j0 + q < e ? __ldg(p.in_idx + j0 + q) : -1;
+            hit[q] = Mask<W>::zero();
           }
-        });
+#pragma unroll
+          for (int q = 0; q < kScanG; ++q)
+#pragma unroll
+            for (int k = 0; k < kOutLevels; ++k)
+              if (u[q] >= 0 && (Ms[k] & todo).any())
+                hit[q] = hit[q] | (Ms[k] & ld_mask<W>(plane<W>(p, Ls[k] - 1), u[q]));
+#pragma unroll
+          for (int q = 0; q < kScanG; ++q) {
+            const Mask<W> r = hit[q] & todo;
+            const int pos = (int)(j0 - s) + q;
+            if (!r.any()) continue;
+            todo = todo.andnot(r);
+#pragma unroll
+            for (int b = 0; b < kPosBits; ++b)
+              if ((pos >> b) & 1) A[b] = A[b] | r;
+          }
+        }
       }
-      if (np != np0) p.pair_n[v] = (uint8_t)np;
-      if (over) p.queue0[atomicAdd(&p.ctl->nover, 1u)] = (int32_t)v;
+      const unsigned used0 = p.pos_used[v];
+      unsigned used = used0;
+#pragma unroll
+      for (int b = 0; b < kPosBits; ++b) add_slice<W>(p, v, b, A[b], used);
+      if (used != used0) p.pos_used[v] = (uint8_t)used;
     }
     __syncwarp();
     chunk = __shfl_sync(kMsFull, next, 0);
   }
 }
 
-// Fix-up pass, after the output pass: the lanes of the listed vertices that
-// no record covers (a vertex with more distinct parents than kRecords) get
-// their parents written one by one.  One warp a vertex, 32 in-list entries
-// at a time in ascending order: lane j holds entry j of the chunk and gathers
-// that entry's history masks for up to kPre levels at once; the 32 x 64 hit
-// matrix is transposed a 32-lane word at a time (warp_transpose32), so warp
-// lane b finds the chunk's first entry -- the lowest-index parent, earlier
-// chunks having had no hit -- of lane b of that word.
-template <int W>
-__global__ void __launch_bounds__(kScanBlock, W == 1 ? 6 : 4) msbfs_fixup(MsParams p) {
-  if (*(volatile int *)p.flag || *(volatile int *)&p.ctl->status != 0) return;
-  const unsigned cnt = *(volatile unsigned *)&p.ctl->nover;
-  if (cnt == 0) return;
-  const int rounds = history_rounds(p);
-  const int lane = lane_id();
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t i = warp_id_global(); i < cnt; i += nwarps) {
-    const int64_t v = p.queue0[i];
-    const int64_t s = __ldg(p.in_off + v), e = __ldg(p.in_off + v + 1);
-    const int np = min((int)p.pair_n[v], kRecords);
-    for (int h = 0; h < W && 64 * h < p.k; ++h) {
-      // the lanes no record covers; those reached at a level >= 2 get parents
-      uint64_t todo = ~records_mask<W>(p, v, h, np);
-      for (int64_t c0 = s; c0 < e && todo; c0 += 32) {  // uniform: the whole warp
-        const bool has = c0 + lane < e;
-        const int32_t u = has ? __ldg(p.in_idx + c0 + lane) : 0;
-        for (int L0 = 2; L0 < rounds && todo; L0 += kPre) {
-          uint64_t pm[kPre];
-#pragma unroll
-          for (int j = 0; j < kPre; ++j)
-            pm[j] = L0 + j < rounds ? plane<W>(p, L0 + j)[v * W + h] & todo : 0ull;
-          uint64_t hit = 0, batch = 0;
-#pragma unroll
-          for (int j = 0; j < kPre; ++j) {
-            batch |= pm[j];
-            if (pm[j] && has) hit |= pm[j] & plane<W>(p, L0 + j - 1)[(int64_t)u * W + h];
-          }
-          if (!batch) continue;
-          uint64_t found = 0;
-#pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            const uint32_t t = warp_transpose32((uint32_t)(hit >> (32 * half)));
-            const int first = t ? __ffs(t) - 1 : 0;
-            const int32_t par = __shfl_sync(kMsFull, u, first);
-            if (t) p.parents[(int64_t)(64 * h + 32 * half + lane) * p.n + v] = par;
-            found |= (uint64_t)__ballot_sync(kMsFull, t != 0) << (32 * half);
-          }
-          todo &= ~found;
-        }
-      }
-    }
-  }
-}
-
 // Output pass.  Each warp takes 32 consecutive vertices (one per thread).  Per
 // 64-lane half of the batch a thread reads its vertex's history masks once
-// and keeps each lane's level as bit slices in registers; parents of levels
-// >= 2 come from the slot's candidates (in-degree > kPullLight), copied by
-// the warp into the parent row of the vertex's shared table, or from the
-// vertex's (source, lanes) records: their sources in the same table, each
-// lane's record index as bit slices like the levels.  Then, lane by lane,
-// the warp writes the tile's 32 levels and 32 parents as two 128-byte rows,
-// each parent one table read; parents of levels 0 and 1 are the vertex and
-// the lane's root.
+// and keeps each lane's level as bit slices in registers; the parents of a
+// vertex with a slot are its candidates (in-degree > kPullLight), copied by
+// the warp into the vertex's row of the shared table, those of a light vertex
+// the in-list entries at its lanes' positions, bit slices like the levels.
+// The bytes of four lanes (levels, table indices) come out of the slices
+// together: lanes g, g + 8, g + 16 and g + 24 lie under the same 0x01010101
+// mask, one shift and one logic operation a slice.  They are turned round in
+// shared memory, so that a thread has four vertices of a lane and writes 16
+// bytes at a time, eight threads a 128-byte row piece.  Where rows do not all
+// start on 16 bytes (n no multiple of 4), tiles overlap: a tile has the four
+// vertices before its own 28 as well, and a row that starts r elements past 16
+// bytes (the four lanes of a word share r) gets the 28 from r vertices earlier,
+// so every store is still 16 aligned bytes.  Writing such a tile's ends element
+// by element instead took 545 us where this takes 289 (n = 1,000,003, 100
+// lanes).  Lanes at level 0 are their own vertex's and are written last.
+//
+// Integer issue bound it when each thread wrote its vertex's values one by one
+// (3,900 instructions per tile of 32 vertices and 64 lanes, 2,000 now).  R-MAT
+// scale 23, 64 lanes: 1345 -> 1077 us for 5.3 GB; scale 18: 50 -> 34 us.
 template <int W>
-__global__ void __launch_bounds__(kOutBlock) msbfs_outputs(MsParams p) {
+__global__ void __launch_bounds__(kOutBlock, 5) msbfs_outputs(MsParams p) {
   extern __shared__ __align__(16) unsigned char s_tile[];
   __shared__ unsigned s_cnt[CG_HISTORY + 1];  // lane discoveries per level
   MsCtl *ctl = p.ctl;
@@ -1216,104 +1138,83 @@ __global__ void __launch_bounds__(kOutBlock) msbfs_outputs(MsParams p) {
   const int rounds = history_rounds(p);
   for (int i = threadIdx.x; i <= CG_HISTORY; i += blockDim.x) s_cnt[i] = 0;
   __syncthreads();
+  constexpr uint32_t kOne = 0x01010101u;
   const int lane = lane_id();
   const int wib = threadIdx.x >> 5;
   int32_t *tab = reinterpret_cast<int32_t *>(s_tile + wib * kOutWarpBytes);
-  int32_t *my_tab = tab + lane * kTab;  // lane l at my_tab[(l - 8 * lane) & 63]
+  int32_t *my_tab = tab + lane * kTab;
+  uint32_t *s_level = reinterpret_cast<uint32_t *>(tab) + 32 * kTab, *s_index = s_level + kStage;
   my_tab[kTabNone] = -1;
+  unsigned found[kPre];  // lanes of my vertices at levels 0 .. kPre - 1
+#pragma unroll
+  for (int j = 0; j < kPre; ++j) found[j] = 0;
   int nsl = 1;  // bit slices needed for levels 0 .. rounds - 1
   while (nsl < kSlices && (rounds - 1) >> nsl) ++nsl;
   const int64_t nwarps = (int64_t)gridDim.x * kOutWarps;
-  // a tile's slot and record count are loaded one tile ahead: the tile's
-  // history, candidate and record loads then all go out at its start
+  // rows aligned alike in both outputs (else they are written one by one), and
+  // whether any is off 16 bytes: then tiles are 28 vertices and the 4 before
+  const bool same_align = ((reinterpret_cast<uintptr_t>(p.levels) ^
+                            reinterpret_cast<uintptr_t>(p.parents)) & 15u) == 0;
+  const int before = (p.n & 3) || (reinterpret_cast<uintptr_t>(p.levels) & 15u) ? 4 : 0;
+  const int own_tile = 32 - before;  // vertices of a tile
+  const int64_t tiles = (p.n + (before ? 3 : 0) + own_tile - 1) / own_tile;
+  // a tile's slots, position flags and list bounds are loaded one tile ahead:
+  // the tile's history, candidate and list loads then all go out at its start
   int64_t tile = (int64_t)blockIdx.x * kOutWarps + wib;
-  int next_slot = -1, next_np = 0;
-  if (tile * 32 + lane < p.n) {
-    next_slot = p.cand_slot[tile * 32 + lane];
-    next_np = p.pair_n[tile * 32 + lane];
-  }
-  for (; tile * 32 < p.n; tile += nwarps) {
-    const int64_t v = tile * 32 + lane;
-    const bool valid = v < p.n;
-    const int slot = next_slot;
-    const int np = slot < 0 ? min(next_np, kRecords) : 0;
-    const int64_t vn = (tile + nwarps) * 32 + lane;
+  int next_slot = -1;
+  unsigned next_used = 0, next_deg = 0;
+  int64_t next_s = 0;
+  auto look_ahead = [&](int64_t v) {
     next_slot = -1;
-    next_np = 0;
-    if (vn < p.n) {
-      next_slot = p.cand_slot[vn];
-      next_np = p.pair_n[vn];
+    next_used = next_deg = 0;
+    if (v >= 0 && v < p.n) {
+      next_slot = p.cand_slot[v];
+      next_used = p.pos_used[v];
+      next_s = __ldg(p.in_off + v);
+      next_deg = (unsigned)min(__ldg(p.in_off + v + 1) - next_s, (int64_t)kPullLight);
     }
+  };
+  look_ahead(tile * own_tile - before + lane);
+  for (; tile < tiles; tile += nwarps) {
+    const int64_t v = tile * own_tile - before + lane;
+    const bool valid = v >= 0 && v < p.n;
+    const int slot = next_slot;
+    const unsigned used = slot < 0 ? next_used : 0u;
+    const int64_t s = next_s;
+    // entries that positions can point at: 2^(slices in use), within the list
+    const unsigned entries = slot < 0 ? min(next_deg, 1u << (32 - __clz(used))) : 0u;
+    const unsigned tile_used = __reduce_or_sync(kMsFull, used);
+    look_ahead((tile + nwarps) * own_tile - before + lane);
 #pragma unroll 1
     for (int h = 0; h < W && 64 * h < p.k; ++h) {
-      // the first kPre history planes: independent of the slot and record
-      // loads below, so they are issued first and their latency overlaps
+      // the first kPre history planes: independent of the loads below, so they
+      // are issued first and their latency overlaps
       uint64_t pm0[kPre];
 #pragma unroll
       for (int j = 0; j < kPre; ++j)
         pm0[j] = valid && j < rounds ? plane<W>(p, j)[v * W + h] : 0ull;
-      // parents of levels >= 2 of the tile's slotted vertices: the warp copies
-      // each slot's 256-byte candidate row into the vertex's tile row, four
-      // rows' loads in flight
-      {
-        unsigned pend = __ballot_sync(kMsFull, slot >= 0);
-        while (pend) {
-          int src[4];
-          uint2 x[4];
+      uint64_t Q[kPosBits];  // bit l of Q[b]: bit b of lane l's position
 #pragma unroll
-          for (int r = 0; r < 4; ++r) {
-            src[r] = pend ? __ffs(pend) - 1 : -1;
-            if (pend) pend &= pend - 1;
-          }
-#pragma unroll
-          for (int r = 0; r < 4; ++r) {
-            const int ss = src[r] >= 0 ? __shfl_sync(kMsFull, slot, src[r]) : -1;
-            x[r] = ss >= 0 ? __ldg(reinterpret_cast<const uint2 *>(p.cand + (int64_t)ss * (64 * W) +
-                                                                  64 * h) + lane)
-                           : make_uint2(0u, 0u);
-          }
-#pragma unroll
-          for (int r = 0; r < 4; ++r) {
-            if (src[r] >= 0) {
-              int32_t *t = tab + src[r] * kTab + ((2 * lane - 8 * src[r]) & 63);
-              t[0] = (int32_t)x[r].x;
-              t[1] = (int32_t)x[r].y;
-            }
-          }
-        }
-      }
-      // a light vertex's records (pull rounds, then the scan pass), four
-      // records' loads in flight: sources into the thread's table, each
-      // lane's record index as three bit slices rq (the masks are disjoint)
-      uint64_t rq[3] = {0ull, 0ull, 0ull}, cov = 0;
-      for (int q0 = 0; q0 < np; q0 += 4) {
-        int32_t pu[4];
-        uint64_t pmk[4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          pu[r] = 0;
-          pmk[r] = 0;
-          if (q0 + r < np) {
-            const int64_t at = (int64_t)(q0 + r) * p.n + v;
-            pu[r] = p.pair_u[at];
-            pmk[r] = p.pair_m[at * W + h];
-          }
-        }
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-          if (q0 + r < np) my_tab[kTabRec + q0 + r] = pu[r];
-        const uint64_t all4 = pmk[0] | pmk[1] | pmk[2] | pmk[3];
-        cov |= all4;
-        rq[0] |= pmk[1] | pmk[3];
-        rq[1] |= pmk[2] | pmk[3];
-        if (q0 & 4) rq[2] |= all4;
+      for (int b = 0; b < kPosBits; ++b)
+        Q[b] = (used >> b) & 1u ? p.pos[((int64_t)b * p.n + v) * W + h] : 0ull;
+      // a light vertex's list entries, and the 256-byte candidate rows of the
+      // tile's slotted vertices (by the warp), go into the table while the
+      // slices are made: asynchronous copies, all in flight at once
+      if (h == 0)
+        for (unsigned q = 0; q < entries; ++q) copy_async4(my_tab + q, p.in_idx + s + q);
+      for (unsigned pend = __ballot_sync(kMsFull, slot >= 0); pend; pend &= pend - 1) {
+        const int src = __ffs(pend) - 1;
+        const uint32_t *row =
+            p.cand + (int64_t)__shfl_sync(kMsFull, slot, src) * (64 * W) + 64 * h;
+        int32_t *t = tab + src * kTab;
+        copy_async4(t + ((lane - 8 * src) & 63), row + lane);
+        copy_async4(t + ((lane + 32 - 8 * src) & 63), row + lane + 32);
       }
       // each lane's level as bit slices: bit l of S[b] = bit b of lane l's level
-      uint64_t S[kSlices], reached = 0, m01[2] = {0ull, 0ull};
+      uint64_t S[kSlices], reached = 0;
 #pragma unroll
       for (int b = 0; b < kSlices; ++b) S[b] = 0;
-      m01[0] = pm0[0];
-      m01[1] = pm0[1];
+      const uint64_t own = pm0[0];  // lanes whose root is v
       for (int L0 = 0; L0 < rounds; L0 += kPre) {  // uniform: the whole warp
         uint64_t pm[kPre];
 #pragma unroll
@@ -1327,8 +1228,13 @@ __global__ void __launch_bounds__(kOutBlock) msbfs_outputs(MsParams p) {
 #pragma unroll
         for (int j = 0; j < kPre; ++j) {
           const uint64_t m = pm[j];
-          const unsigned c = __reduce_add_sync(kMsFull, (unsigned)__popcll(m));
-          if (lane == 0 && c) atomicAdd(&s_cnt[L0 + j], c);
+          const unsigned mine = lane >= before ? (unsigned)__popcll(m) : 0u;  // once a vertex
+          if (L0 == 0) {
+            found[j] += mine;
+          } else {
+            const unsigned c = __reduce_add_sync(kMsFull, mine);
+            if (lane == 0 && c) atomicAdd(&s_cnt[L0 + j], c);
+          }
           batch |= m;
 #pragma unroll
           for (int b = 0; b < 3; ++b)
@@ -1339,74 +1245,120 @@ __global__ void __launch_bounds__(kOutBlock) msbfs_outputs(MsParams p) {
         for (int b = 3; b < kSlices; ++b)
           if ((L0 >> b) & 1) S[b] |= batch;
       }
+      copy_async_wait();
       __syncwarp();  // the candidate rows copied by the warp are in place
-      // levels 0 and 1 (rare): the vertex itself, the lane's root
-      for (uint64_t x = m01[0]; x; x &= x - 1)
-        my_tab[(__ffsll((long long)x) - 1 - 8 * lane) & 63] = (int32_t)v;
-      for (uint64_t x = m01[1]; x; x &= x - 1) {
-        const int b = __ffsll((long long)x) - 1;
-        my_tab[(b - 8 * lane) & 63] = p.roots[64 * h + b];
-      }
-      __syncwarp();
       // rows: lane l of this half, vertices tile*32 .. tile*32 + 31, a 32-lane
-      // word of the masks at a time; four lanes' levels are built as the
-      // bytes of a word (0xFF unreached, which sign-extends to -1)
+      // word of the masks at a time
       const int lanes = min(64, p.k - 64 * h);
       const int64_t n = p.n;
+      const uint32_t slotted = slot >= 0 ? ~0u : 0u;
 #pragma unroll 1
       for (int hw = 0; hw < 2 && 32 * hw < lanes; ++hw) {
-        uint32_t sl[kSlices];
+        uint32_t sl[kSlices], qs[kPosBits];
 #pragma unroll
         for (int b = 0; b < kSlices; ++b) sl[b] = (uint32_t)(S[b] >> (32 * hw));
+#pragma unroll
+        for (int b = 0; b < kPosBits; ++b) qs[b] = (uint32_t)(Q[b] >> (32 * hw));
         const uint32_t rw = (uint32_t)(reached >> (32 * hw));
-        const uint32_t cw = (uint32_t)(cov >> (32 * hw));
-        uint32_t qs[3];
+        // table columns of lanes 0, 8, 16, 24 of the word (a slotted vertex):
+        // multiples of 8, so lane l + 8 i's is l more, without a wrap
+        const uint32_t col =
+            ((((uint32_t)(32 * hw - 8 * lane) & 63u) * kOne + 0x18100800u) & 0x3f3f3f3fu) & slotted;
+        // bit g + 8 i of x at bit b of byte i
+        auto bits_at = [](uint32_t x, int g, int b) {
+          return (g >= b ? x >> (g - b) : x << (b - g)) & (kOne << b);
+        };
 #pragma unroll
-        for (int b = 0; b < 3; ++b) qs[b] = (uint32_t)(rq[b] >> (32 * hw));
-        const int lend = min(32, lanes - 32 * hw);
-        // rows of lane 64 h + 32 hw, advanced one row per lane written
-        int32_t *pl = p.levels + (int64_t)(64 * h + 32 * hw) * n + v;
-        int32_t *pp = p.parents + (int64_t)(64 * h + 32 * hw) * n + v;
-        auto group = [&](int l4, auto checked) {
-          // bytes of four lanes: 0xFF where unreached (um), where a record
-          // covers the lane (cm), its level (0xFF unreached sign-extends to -1)
-          const uint32_t um = spread4(~(rw >> l4) & 0xFu) * 0xFFu;
-          const uint32_t cm = spread4((cw >> l4) & 0xFu) * 0xFFu;
-          uint32_t word = um;
+        for (int g = 0; g < 8; ++g) {
+          // lanes g + 8 i, i = 0..3, in byte i: 0xFF where unreached (um), the
+          // level (0xFF unreached sign-extends to -1), the table index
+          const uint32_t um = bits_at(~rw, g, 0) * 0xFFu;
+          uint32_t word = um, pos = 0;
 #pragma unroll
-          for (int b = 0; b < kSlices; ++b)
-            if (b < nsl) word |= spread4((sl[b] >> l4) & 0xFu) << b;
-          // each lane's table index: its record's source, -1 when unreached,
-          // else its column of the parent row ((l - 8 lane) mod 64 never
-          // wraps inside an aligned group of four)
-          const uint32_t qw = spread4((qs[0] >> l4) & 0xFu) | (spread4((qs[1] >> l4) & 0xFu) << 1) |
-                              (spread4((qs[2] >> l4) & 0xFu) << 2);
-          const uint32_t col = ((uint32_t)((32 * hw + l4 - 8 * lane) & 63) * 0x01010101u) | 0x03020100u;
-          const uint32_t idx = (col & ~(cm | um)) | ((qw | (0x01010101u * kTabRec)) & cm) |
-                               ((0x01010101u * kTabNone) & um);
+          for (int b = 0; b < 3; ++b) word |= bits_at(sl[b], g, b);
+          if (nsl > 3) {
+#pragma unroll
+            for (int b = 3; b < kSlices; ++b) word |= bits_at(sl[b], g, b);
+          }
+#pragma unroll
+          for (int b = 0; b < 3; ++b) pos |= bits_at(qs[b], g, b);
+          if (tile_used >> 3) {
+#pragma unroll
+            for (int b = 3; b < kPosBits; ++b) pos |= bits_at(qs[b], g, b);
+          }
+          const uint32_t at = pos | ((col + (uint32_t)g * kOne) & slotted);
+          s_level[kStageRow * g + lane] = word;
+          s_index[kStageRow * g + lane] = (at & ~um) | (kTabNone * kOne & um);
+        }
+        __syncwarp();
+        // thread (g, j): four vertices of lanes g + 8 i
+        const int j = lane & 7;
+        const int64_t v0 = tile * own_tile;
+        const bool inner = same_align && v0 >= before && v0 + own_tile <= n;
+#pragma unroll 1
+        for (int g = lane >> 3; g < 8; g += 4) {
+          const int64_t at0 = (int64_t)(64 * h + 32 * hw + g) * n;
+          // elements past 16 bytes at v0, the same for every i (8 n is a
+          // multiple of 4)
+          const int r = (int)((reinterpret_cast<uintptr_t>(p.levels + at0 + v0) >> 2) & 3u);
+          const int first = 4 * j - r;  // this thread's vertices are v0 + first ..
+          uint32_t lws[4], iws[4];
+          const int32_t *row[4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const int t = (before + first + c) & 31;
+            lws[c] = s_level[kStageRow * g + t];
+            iws[c] = s_index[kStageRow * g + t];
+            row[c] = tab + t * kTab;
+          }
+          const bool mine = 4 * j < own_tile;
+          int32_t *pl = p.levels + at0 + v0 + first, *pp = p.parents + at0 + v0 + first;
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            if (!decltype(checked)::value || l4 + i < lend) {
-              const int32_t lv = (int32_t)(int8_t)(uint8_t)(word >> (8 * i));
-              const int32_t pv = my_tab[(idx >> (8 * i)) & 0xFFu];
-              if (valid) {  // written once, never read here: evict-first
-                __stcs(pl, lv);
-                __stcs(pp, pv);
-              }
-              pl += n;
-              pp += n;
-            }
-          }
-        };
-        if (lend == 32) {
+            if (32 * hw + 8 * i >= lanes) break;  // uniform: no such lanes
+            int32_t lv[4], pv[4];
 #pragma unroll
-          for (int l4 = 0; l4 < 32; l4 += 4) group(l4, Flag<false>{});
-        } else {
-          for (int l4 = 0; l4 < lend; l4 += 4) group(l4, Flag<true>{});
+            for (int c = 0; c < 4; ++c) {
+              lv[c] = (int32_t)(int8_t)(uint8_t)(lws[c] >> (8 * i));
+              pv[c] = row[c][(iws[c] >> (8 * i)) & 0xFFu];
+            }
+            if (mine && 32 * hw + g + 8 * i < lanes) {
+              if (inner) {  // written once, never read here: evict-first
+                __stcs(reinterpret_cast<int4 *>(pl), make_int4(lv[0], lv[1], lv[2], lv[3]));
+                __stcs(reinterpret_cast<int4 *>(pp), make_int4(pv[0], pv[1], pv[2], pv[3]));
+              } else {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                  const int64_t x = v0 + first + c;
+                  if (x >= 0 && x < n) {
+                    __stcs(pl + c, lv[c]);
+                    __stcs(pp + c, pv[c]);
+                  }
+                }
+              }
+            }
+            pl += 8 * n;
+            pp += 8 * n;
+          }
         }
+        __syncwarp();  // the staged words are read
+      }
+      // (after the syncwarp, so after whichever thread wrote these elements; an
+      // overlapped vertex is in the tile that wrote the row's element)
+      for (uint64_t x = own; x; x &= x - 1) {
+        const int64_t at = (int64_t)(64 * h + __ffsll((long long)x) - 1) * n;
+        const int r =
+            (int)((reinterpret_cast<uintptr_t>(p.levels + at + tile * own_tile) >> 2) & 3u);
+        const int t = lane - before + r;
+        if (t >= 0 && t < own_tile) p.parents[at + v] = (int32_t)v;
       }
       __syncwarp();
     }
+  }
+#pragma unroll
+  for (int j = 0; j < kPre; ++j) {
+    const unsigned c = __reduce_add_sync(kMsFull, found[j]);
+    if (lane == 0 && c) atomicAdd(&s_cnt[j], c);
   }
   // the statistics: lane discoveries per round (level L came from round
   // L - 1) and in all; the last block out records the time since the last
@@ -1466,15 +1418,11 @@ int ledger_pass(cg_graph *g, MsState *s, const int64_t *roots, int k, int32_t *d
   CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&out_per_sm, msbfs_outputs<W>, kOutBlock,
                                                         smem));
   if (out_per_sm <= 0) return CG_ERR_NOT_SUPPORTED;
-  const int64_t tiles = (g->n + 31) / 32;
+  const int64_t tiles = (g->n + 3 + 27) / 28;  // of 28 vertices where rows are ragged, else 32
   int64_t blocks = (tiles + kOutWarps - 1) / kOutWarps;
   const int64_t cap = (int64_t)out_per_sm * g->num_sms;
   if (blocks > cap) blocks = cap;
   msbfs_outputs<W><<<(unsigned)blocks, kOutBlock, smem, g->stream>>>(p);
-  int fix_per_sm = 0;
-  CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fix_per_sm, msbfs_fixup<W>, kScanBlock, 0));
-  if (fix_per_sm <= 0) return CG_ERR_NOT_SUPPORTED;
-  msbfs_fixup<W><<<(unsigned)(fix_per_sm * g->num_sms), kScanBlock, 0, g->stream>>>(p);
   CG_CUDA(cudaGetLastError());
   return CG_OK;
 }
