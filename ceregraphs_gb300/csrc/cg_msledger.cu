@@ -274,6 +274,76 @@ __device__ __forceinline__ Mask<W> or_warp_first(const MsParams &p, int64_t s, i
   return got;
 }
 
+// Claimed vertices of out-degree > kLightMax on their way to the next queue
+// (light ones are found in the claim bitmap): a warp keeps them in shared
+// memory and queues 32 with one atomic, instead of one returning atomic on the
+// queue's counter per step with any -- the round's warps queue up there.
+struct HeavyQueue {
+  int32_t v[64];
+  uint32_t deg[64];
+};
+__shared__ HeavyQueue s_heavy[kMsBlock / 32];
+struct HeavyOut {
+  MsRound *Rn;                // the record of the next frontier
+  int parity;                 // its queue
+  unsigned count = 0;         // entries waiting, the same in every lane
+};
+
+// Queues entries [from, from + n), n <= 32.  All 32 lanes call.
+__device__ __forceinline__ void heavy_flush(const MsParams &p, HeavyOut &H, unsigned from,
+                                            unsigned n) {
+  const int lane = lane_id();
+  HeavyQueue &S = s_heavy[threadIdx.x >> 5];
+  const bool has = (unsigned)lane < n;
+  const uint32_t d = has ? S.deg[from + lane] : 0u;
+  uint32_t incl = d;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(kMsFull, incl, o);
+    if (lane >= o) incl += t;
+  }
+  const uint32_t total = __shfl_sync(kMsFull, incl, 31);
+  unsigned long long old = 0;
+  if (lane == 0) old = atomicAdd(&H.Rn->big, ((unsigned long long)n << 32) | total);
+  old = __shfl_sync(kMsFull, old, 0);
+  if (has) {
+    const unsigned idx = (unsigned)(old >> 32) + (unsigned)lane;
+    (H.parity ? p.queue1 : p.queue0)[p.n - 1 - (int64_t)idx] = S.v[from + lane];
+    (H.parity ? p.bigoff1 : p.bigoff0)[idx] = (uint32_t)old + incl - d;
+  }
+  __syncwarp();
+}
+
+// Counts the claims of one warp-wide step and keeps the heavy ones.  All 32
+// lanes call.
+__device__ __forceinline__ void claim_step(const MsParams &p, bool claimed, int32_t v, int64_t deg,
+                                           HeavyOut &H, MsAcc &acc) {
+  if (claimed) {
+    acc.nf += 1;
+    acc.mf += (unsigned long long)deg;
+  }
+  const bool heavy = claimed && deg > kLightMax;
+  const unsigned m = __ballot_sync(kMsFull, heavy);
+  if (!m) return;
+  HeavyQueue &S = s_heavy[threadIdx.x >> 5];
+  if (heavy) {
+    const unsigned at = H.count + __popc(m & ((1u << lane_id()) - 1u));
+    S.v[at] = v;
+    S.deg[at] = (uint32_t)deg;
+  }
+  H.count += __popc(m);
+  __syncwarp();
+  if (H.count >= 32) {
+    H.count -= 32;
+    heavy_flush(p, H, H.count, 32);
+  }
+}
+
+__device__ __forceinline__ void heavy_rest(const MsParams &p, HeavyOut &H) {
+  if (H.count) heavy_flush(p, H, 0, H.count);
+  H.count = 0;
+}
+
 // Claim bitmap T_L: one bit per vertex with a nonzero frontier mask F_L --
 // round L's frontier set.  Round L reads T_L (push rounds enumerate light
 // frontier vertices from it), sets T_{L+1}, and clears T_{L+2}; three rotate.
@@ -298,9 +368,7 @@ __device__ void lg_pull(const MsParams &p, int L, const uint64_t *cur, uint64_t 
   after_push = after_push && W == 1;
   const uint64_t *prev = after_push ? plane<W>(p, L - 1) : cur;
   const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
-  const int next_parity = (L + 1) & 1;
-  int32_t *q = next_parity ? p.queue1 : p.queue0;
-  uint32_t *boff = next_parity ? p.bigoff1 : p.bigoff0;
+  HeavyOut H{Rn, (L + 1) & 1};
   uint32_t *tnext = claims(p, L + 1);
   const int lane = lane_id();
   // a symmetric graph stores one list per vertex: out-degree = in-degree
@@ -394,7 +462,7 @@ __device__ void lg_pull(const MsParams &p, int L, const uint64_t *cur, uint64_t 
             if (cb) atomicOr(tnext + w0 + j, cb);
           }
         }
-        ms_enqueue<false>(claimed, (int32_t)v, deg, q, p.n, boff, &Rn->nlight, &Rn->big, acc);
+        claim_step(p, claimed, (int32_t)v, deg, H, acc);
       }
       if (finw != fin0) p.fin[w0 + lane] = finw;
     } else if (item < nlg + nmg) {
@@ -458,14 +526,14 @@ __device__ void lg_pull(const MsParams &p, int L, const uint64_t *cur, uint64_t 
         if (W == 1) {
           if (lane == t && got.any()) cq = true;
         } else {
-          ms_enqueue<false>(claimed, v, deg, q, p.n, boff, &Rn->nlight, &Rn->big, acc);
+          claim_step(p, claimed, v, deg, H, acc);
         }
       }
-      // the group's claimed vertices queued together: one atomic, not one each
+      // the group's claimed vertices together
       if (W == 1) {
         const int64_t dq =
             !cq ? 0 : (sym ? eq - sq : __ldg(p.out_off + vq + 1) - __ldg(p.out_off + vq));
-        ms_enqueue<false>(cq, vq, dq, q, p.n, boff, &Rn->nlight, &Rn->big, acc);
+        claim_step(p, cq, vq, dq, H, acc);
       }
     } else {
       const unsigned hi_item = item - nlg - nmg;
@@ -504,6 +572,7 @@ __device__ void lg_pull(const MsParams &p, int L, const uint64_t *cur, uint64_t 
     }
     item = __shfl_sync(kMsFull, nextitem, 0);
   }
+  heavy_rest(p, H);
 }
 
 // After the wait that ends a pull round's scans: hubs found this round get
@@ -513,9 +582,7 @@ __device__ void lg_hub_merge(const MsParams &p, int L, const uint64_t *cur, uint
                              MsRound *Rn, MsAcc &acc) {
   const int lane = lane_id();
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  const int next_parity = (L + 1) & 1;
-  int32_t *q = next_parity ? p.queue1 : p.queue0;
-  uint32_t *boff = next_parity ? p.bigoff1 : p.bigoff0;
+  HeavyOut H{Rn, (L + 1) & 1};
   uint32_t *tnext = claims(p, L + 1);
   for (int64_t h0 = (int64_t)warp_id_global() * 32; h0 < p.nhub; h0 += (int64_t)nwarps * 32) {
     const int64_t h = h0 + lane;
@@ -538,8 +605,9 @@ __device__ void lg_hub_merge(const MsParams &p, int L, const uint64_t *cur, uint
         claimed = true;
       }
     }
-    ms_enqueue<false>(claimed, v, deg, q, p.n, boff, &Rn->nlight, &Rn->big, acc);
+    claim_step(p, claimed, v, deg, H, acc);
   }
+  heavy_rest(p, H);
 }
 
 // Edge u -> v of a push round: the lanes of u's frontier that v has neither
@@ -551,25 +619,41 @@ __device__ void lg_hub_merge(const MsParams &p, int L, const uint64_t *cur, uint
 // Returns whether this thread claimed v (set its bit in the next claim
 // bitmap first).
 template <int W>
-__device__ __forceinline__ bool lg_relax(const MsParams &p, const Mask<W> &fu, int32_t u,
-                                         int32_t v, const uint64_t *cur, uint64_t *nxt,
-                                         uint32_t *tnext, const uint32_t *tfront, MsAcc &acc) {
-  const Mask<W> seen = ld_mask<W>(p.vis, v);
-  const Mask<W> have = ld_mask<W>(nxt, v);
-  const int slot = p.cand_slot[v];
-  const uint32_t tw = tnext[v >> 5];
+struct Target {
+  int32_t v = -1;             // -1: no edge
+  int32_t slot = -1;
+  uint32_t tw = 0;
+  Mask<W> f, add;             // new lanes, and those v's next mask lacks
+};
+
+template <int W>
+__device__ __forceinline__ void lg_load(const MsParams &p, Target<W> &t, const Mask<W> &fu,
+                                        const uint64_t *cur, const uint64_t *nxt,
+                                        const uint32_t *tnext, const uint32_t *tfront) {
+  t.f = t.add = Mask<W>::zero();
+  if (t.v < 0) return;
+  const Mask<W> seen = ld_mask<W>(p.vis, t.v);
+  const Mask<W> have = ld_mask<W>(nxt, t.v);
+  t.slot = p.cand_slot[t.v];
+  t.tw = tnext[t.v >> 5];
   Mask<W> now = Mask<W>::zero();
-  if (!tfront || ((tfront[v >> 5] >> (v & 31)) & 1u)) now = ld_mask<W>(cur, v);
-  const Mask<W> f = fu.andnot(seen | now);
-  if (!f.any()) return false;
-  acc_lanes<W>(acc, f);
-  if (slot >= 0) {
+  if (!tfront || ((tfront[t.v >> 5] >> (t.v & 31)) & 1u)) now = ld_mask<W>(cur, t.v);
+  t.f = fu.andnot(seen | now);
+  t.add = t.f.andnot(have);
+}
+
+template <int W>
+__device__ __forceinline__ bool lg_relax(const MsParams &p, int32_t u, const Target<W> &t,
+                                         uint64_t *nxt, uint32_t *tnext, MsAcc &acc) {
+  if (!t.f.any()) return false;
+  acc_lanes<W>(acc, t.f);
+  if (t.slot >= 0) {
     // lowest source per new lane: read first (a lower one is often there
     // already), four lanes' reads in flight at a time
-    uint32_t *cand = p.cand + (int64_t)slot * (64 * W);
+    uint32_t *cand = p.cand + (int64_t)t.slot * (64 * W);
 #pragma unroll
     for (int j = 0; j < W; ++j) {
-      uint64_t bits = f.w[j];
+      uint64_t bits = t.f.w[j];
       while (bits) {
         int b[4];
         uint32_t c[4];
@@ -586,40 +670,35 @@ __device__ __forceinline__ bool lg_relax(const MsParams &p, const Mask<W> &fu, i
       }
     }
   }
-  const Mask<W> add = f.andnot(have);
 #pragma unroll
   for (int i = 0; i < W; ++i)
-    if (add.w[i])
-      atomicOr(reinterpret_cast<unsigned long long *>(nxt + (int64_t)v * W + i),
-               (unsigned long long)add.w[i]);
-  const uint32_t tb = 1u << (v & 31);
-  if (tw & tb) return false;
-  return (atomicOr(tnext + (v >> 5), tb) & tb) == 0;
+    if (t.add.w[i])
+      atomicOr(reinterpret_cast<unsigned long long *>(nxt + (int64_t)t.v * W + i),
+               (unsigned long long)t.add.w[i]);
+  const uint32_t tb = 1u << (t.v & 31);
+  if (t.tw & tb) return false;
+  return (atomicOr(tnext + (t.v >> 5), tb) & tb) == 0;
 }
 
+// The claims of one warp-wide step of edges.
 template <int W>
-__device__ __forceinline__ void lg_step(const MsParams &p, bool valid, const Mask<W> &fu,
-                                        int32_t u, int64_t e, const uint64_t *cur, uint64_t *nxt,
-                                        uint32_t *tnext, const uint32_t *tfront, int32_t *q,
-                                        uint32_t *boff, MsRound *Rn, MsAcc &acc) {
-  bool claimed = false;
-  int32_t v = 0;
-  int64_t deg = 0;
-  if (valid) {
-    v = __ldg(p.out_idx + e);
-    claimed = lg_relax<W>(p, fu, u, v, cur, nxt, tnext, tfront, acc);
-    if (claimed) deg = __ldg(p.out_off + v + 1) - __ldg(p.out_off + v);
-  }
-  ms_enqueue<false>(claimed, v, deg, q, p.n, boff, &Rn->nlight, &Rn->big, acc);
+__device__ __forceinline__ void lg_apply(const MsParams &p, int32_t u, const Target<W> &t,
+                                         uint64_t *nxt, uint32_t *tnext, HeavyOut &H, MsAcc &acc) {
+  const bool claimed = lg_relax<W>(p, u, t, nxt, tnext, acc);
+  const int64_t deg = claimed ? __ldg(p.out_off + t.v + 1) - __ldg(p.out_off + t.v) : 0;
+  claim_step(p, claimed, t.v, deg, H, acc);
 }
 
 // Edge positions [x0, x1) of the big-vertex edge space (queue entries
-// q[cap-1-j] with prefix offsets boff[j], all of out-degree > kLightMax).
+// q[cap-1-j] with prefix offsets boff[j], all of out-degree > kLightMax).  With
+// 64 lanes two steps of 32 edges go together: their list entries, then their
+// targets' masks, are in flight at once (with 128 the registers would spill).
 template <int W>
 __device__ void lg_push_chunk(const MsParams &p, const uint64_t *cur, uint64_t *nxt,
                               uint32_t *tnext, const int32_t *bq, const uint32_t *boff,
                               unsigned nbig, unsigned x0, unsigned x1, const uint32_t *tfront,
-                              int32_t *q, uint32_t *qoff, MsRound *Rn, MsAcc &acc) {
+                              HeavyOut &H, MsAcc &acc) {
+  constexpr int U = W == 1 ? 2 : 1;
   const int lane = lane_id();
   const int64_t cap = p.n;
   unsigned lo = 0, hi = nbig - 1;
@@ -636,36 +715,54 @@ __device__ void lg_push_chunk(const MsParams &p, const uint64_t *cur, uint64_t *
   unsigned oj = boff[j];
   unsigned endj = oj + (unsigned)(__ldg(p.out_off + vj + 1) - sj);
   Mask<W> fj = ld_mask<W>(cur, vj);
-  for (unsigned base = x0; base < x1; base += 32) {
-    while (base >= endj) {
-      ++j;
-      vj = bq[cap - 1 - (int64_t)j];
-      sj = __ldg(p.out_off + vj);
-      oj = boff[j];
-      endj = oj + (unsigned)(__ldg(p.out_off + vj + 1) - sj);
-      fj = ld_mask<W>(cur, vj);
-    }
-    const unsigned x = base + lane;
-    const bool valid = x < x1;
-    int32_t u = vj;
-    int64_t e = sj + (int64_t)(x - oj);
-    Mask<W> fu = fj;
-    if (__ballot_sync(kMsFull, valid && x >= endj)) {
-      const int32_t vn = bq[cap - 1 - (int64_t)(j + 1)];
-      if (valid && x >= endj) {
-        u = vn;
-        e = __ldg(p.out_off + vn) + (int64_t)(x - endj);
-        fu = ld_mask<W>(cur, vn);
+  for (unsigned base = x0; base < x1; base += 32 * U) {
+    int32_t u[U];
+    Mask<W> fu[U];
+    Target<W> t[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const unsigned at = base + 32 * k;
+      if (at < x1) {  // uniform
+        while (at >= endj) {
+          ++j;
+          vj = bq[cap - 1 - (int64_t)j];
+          sj = __ldg(p.out_off + vj);
+          oj = boff[j];
+          endj = oj + (unsigned)(__ldg(p.out_off + vj + 1) - sj);
+          fj = ld_mask<W>(cur, vj);
+        }
       }
+      const unsigned x = at + lane;
+      const bool valid = x < x1 && x >= at;
+      u[k] = vj;
+      int64_t e = sj + (int64_t)(x - oj);
+      fu[k] = fj;
+      if (__ballot_sync(kMsFull, valid && x >= endj)) {
+        const int32_t vn = bq[cap - 1 - (int64_t)(j + 1)];
+        if (valid && x >= endj) {
+          u[k] = vn;
+          e = __ldg(p.out_off + vn) + (int64_t)(x - endj);
+          fu[k] = ld_mask<W>(cur, vn);
+        }
+      }
+      if (valid) t[k].v = __ldg(p.out_idx + e);
     }
-    lg_step<W>(p, valid, fu, u, e, cur, nxt, tnext, tfront, q, qoff, Rn, acc);
+#pragma unroll
+    for (int k = 0; k < U; ++k) lg_load<W>(p, t[k], fu[k], cur, nxt, tnext, tfront);
+#pragma unroll
+    for (int k = 0; k < U; ++k) lg_apply<W>(p, u[k], t[k], nxt, tnext, H, acc);
+    if (base + 32 * U < base) break;  // x1 within a step of 2^32
   }
 }
 
-// Push round.  Work items: the big vertices' edges in chunks (from the
-// queue, as in the direct kernel), then groups of 32 claim words (1024
-// vertices): the frontier vertices there merge their lanes into vis, and the
-// light ones (out-degree <= kLightMax) spread their edges over the warp.
+// Push round.  The big vertices' edges go in chunks (from the queue, as in the
+// direct kernel), handed out dynamically; then every warp takes 32 claim words
+// at a time, one a lane, a grid apart from each other -- neighbouring words are
+// alike, so this spreads them evenly without a counter: the frontier vertices
+// there merge their lanes into vis, and the light ones (out-degree <=
+// kLightMax) spread their edges over the warp.  A warp's steps follow one
+// another: 200,000 frontier vertices among 1 M took 116 us with 32 neighbouring
+// words to a warp, 42 us so.
 template <int W>
 __device__ void lg_push(const MsParams &p, int L, const uint64_t *cur, uint64_t *nxt,
                         bool sparse, MsRound *Rc, MsRound *Rn, MsAcc &acc) {
@@ -675,11 +772,10 @@ __device__ void lg_push(const MsParams &p, int L, const uint64_t *cur, uint64_t 
   const int lane = lane_id();
   const int wib = threadIdx.x >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  const int parity = L & 1, next_parity = parity ^ 1;
+  const int parity = L & 1;
   const int32_t *qc = parity ? p.queue1 : p.queue0;
   const uint32_t *bc = parity ? p.bigoff1 : p.bigoff0;
-  int32_t *qn = next_parity ? p.queue1 : p.queue0;
-  uint32_t *bn = next_parity ? p.bigoff1 : p.bigoff0;
+  HeavyOut H{Rn, parity ^ 1};
   const uint32_t *tcur = claims(p, L);
   uint32_t *tnext = claims(p, L + 1);
   // a frontier of under n/1024 vertices (few targets are in it): its claim
@@ -692,91 +788,93 @@ __device__ void lg_push(const MsParams &p, int L, const uint64_t *cur, uint64_t 
   unsigned chunk = ((big_edges / (unsigned)nwarps) + 31u) & ~31u;
   chunk = chunk < 32u ? 32u : (chunk > (unsigned)kPushChunk ? (unsigned)kPushChunk : chunk);
   const unsigned nb = (big_edges + chunk - 1) / chunk;
-  const unsigned ngroups = (unsigned)((p.words + 31) / 32);
-  const unsigned nitems = nb + ngroups;
   unsigned item = (unsigned)warp_id_global();
-  while (item < nitems) {
-    if (item < nb) {
-      const unsigned x0 = item * chunk;
-      lg_push_chunk<W>(p, cur, nxt, tnext, qc, bc, nbig, x0, min(x0 + chunk, big_edges), tfront,
-                       qn, bn, Rn, acc);
-    } else {
-      // the group's frontier vertices, compacted 32 at a time: lane j holds
-      // word j; the t-th frontier vertex is the (t - prefix)-th set bit of the
-      // word whose prefix count covers t
-      const int64_t w0 = (int64_t)(item - nb) * 32;
-      const uint32_t mine = w0 + lane < p.words ? tcur[w0 + lane] : 0u;
-      const int cnt = __popc(mine);
-      int incl_c = cnt;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(kMsFull, incl_c, o);
-        if (lane >= o) incl_c += t;
-      }
-      const int total_v = __shfl_sync(kMsFull, incl_c, 31);
-      for (int b0 = 0; b0 < total_v; b0 += 32) {
-        const int t = b0 + lane;
-        int32_t u = -1;
-        int64_t s = 0, d = 0;
-        // word holding the t-th vertex: the first lane whose inclusive count
-        // exceeds t (the counts never decrease)
-        int wsel = 0;
-#pragma unroll
-        for (int step = 16; step > 0; step >>= 1)
-          if (__shfl_sync(kMsFull, incl_c, wsel + step - 1) <= t) wsel += step;
-        const uint32_t wbits = __shfl_sync(kMsFull, mine, wsel);
-        const int before = __shfl_sync(kMsFull, incl_c - cnt, wsel);
-        if (t < total_v) {
-          const int bit = __fns(wbits, 0, t - before + 1);
-          const int64_t v = (w0 + wsel) * 32 + bit;
-          const Mask<W> fv = ld_mask<W>(cur, v);
-          st_mask<W>(p.vis, v, ld_mask<W>(p.vis, v) | fv);
-          s = __ldg(p.out_off + v);
-          d = __ldg(p.out_off + v + 1) - s;
-          if (d > kLightMax)
-            d = 0;  // big: its edges are in the chunks above
-          else
-            u = (int32_t)v;
-        }
-        int64_t incl = d;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int64_t tt = __shfl_up_sync(kMsFull, incl, o);
-          if (lane >= o) incl += tt;
-        }
-        const int64_t total = __shfl_sync(kMsFull, incl, 31);
-        s_u[wib][lane] = u;
-        s_s[wib][lane] = s;
-        s_x[wib][lane] = incl - d;
-        __syncwarp();
-        for (int64_t base = 0; base < total; base += 32) {
-          const int64_t t2 = base + lane;
-          const bool valid = t2 < total;
-          int64_t e = 0;
-          int32_t uu = 0;
-          Mask<W> fu = Mask<W>::zero();
-          if (valid) {
-            int lo = 0, hi = 31;
-            while (lo < hi) {
-              const int mid = (lo + hi + 1) >> 1;
-              if (s_x[wib][mid] <= t2)
-                lo = mid;
-              else
-                hi = mid - 1;
-            }
-            uu = s_u[wib][lo];
-            fu = ld_mask<W>(cur, uu);
-            e = s_s[wib][lo] + (t2 - s_x[wib][lo]);
-          }
-          lg_step<W>(p, valid, fu, uu, e, cur, nxt, tnext, tfront, qn, bn, Rn, acc);
-        }
-        __syncwarp();
-      }
-    }
+  while (item < nb) {
+    // the next item is claimed before this one is worked, hiding the atomic
     unsigned nextitem = 0;
     if (lane == 0) nextitem = (unsigned)nwarps + atomicAdd(&Rc->work, 1u);
+    const unsigned x0 = item * chunk;
+    lg_push_chunk<W>(p, cur, nxt, tnext, qc, bc, nbig, x0, min(x0 + chunk, big_edges), tfront, H,
+                     acc);
     item = __shfl_sync(kMsFull, nextitem, 0);
   }
+  for (int64_t w0 = warp_id_global(); w0 < p.words; w0 += 32 * (int64_t)nwarps) {
+    // the words' frontier vertices, compacted 32 at a time: lane j holds word
+    // w0 + j nwarps; the t-th frontier vertex is the (t - prefix)-th set bit
+    // of the word whose prefix count covers t
+    const int64_t wi = w0 + (int64_t)lane * nwarps;
+    const uint32_t mine = wi < p.words ? tcur[wi] : 0u;
+    const int cnt = __popc(mine);
+    int incl_c = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(kMsFull, incl_c, o);
+      if (lane >= o) incl_c += t;
+    }
+    const int total_v = __shfl_sync(kMsFull, incl_c, 31);
+    for (int b0 = 0; b0 < total_v; b0 += 32) {
+      const int t = b0 + lane;
+      int32_t u = -1;
+      int64_t s = 0, d = 0;
+      // word holding the t-th vertex: the first lane whose inclusive count
+      // exceeds t (the counts never decrease)
+      int wsel = 0;
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1)
+        if (__shfl_sync(kMsFull, incl_c, wsel + step - 1) <= t) wsel += step;
+      const uint32_t wbits = __shfl_sync(kMsFull, mine, wsel);
+      const int before = __shfl_sync(kMsFull, incl_c - cnt, wsel);
+      if (t < total_v) {
+        const int bit = __fns(wbits, 0, t - before + 1);
+        const int64_t v = (w0 + (int64_t)wsel * nwarps) * 32 + bit;
+        const Mask<W> fv = ld_mask<W>(cur, v);
+        st_mask<W>(p.vis, v, ld_mask<W>(p.vis, v) | fv);
+        s = __ldg(p.out_off + v);
+        d = __ldg(p.out_off + v + 1) - s;
+        if (d > kLightMax)
+          d = 0;  // big: its edges are in the chunks above
+        else
+          u = (int32_t)v;
+      }
+      int64_t incl = d;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int64_t tt = __shfl_up_sync(kMsFull, incl, o);
+        if (lane >= o) incl += tt;
+      }
+      const int64_t total = __shfl_sync(kMsFull, incl, 31);
+      s_u[wib][lane] = u;
+      s_s[wib][lane] = s;
+      s_x[wib][lane] = incl - d;
+      __syncwarp();
+      for (int64_t base = 0; base < total; base += 32) {
+        const int64_t t2 = base + lane;
+        const bool valid = t2 < total;
+        int64_t e = 0;
+        int32_t uu = 0;
+        Mask<W> fu = Mask<W>::zero();
+        if (valid) {
+          int lo = 0, hi = 31;
+          while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (s_x[wib][mid] <= t2)
+              lo = mid;
+            else
+              hi = mid - 1;
+          }
+          uu = s_u[wib][lo];
+          fu = ld_mask<W>(cur, uu);
+          e = s_s[wib][lo] + (t2 - s_x[wib][lo]);
+        }
+        Target<W> t;
+        if (valid) t.v = __ldg(p.out_idx + e);
+        lg_load<W>(p, t, fu, cur, nxt, tnext, tfront);
+        lg_apply<W>(p, uu, t, nxt, tnext, H, acc);
+      }
+      __syncwarp();
+    }
+  }
+  heavy_rest(p, H);
 }
 
 // End of round L (last block to arrive): termination, the next direction,
