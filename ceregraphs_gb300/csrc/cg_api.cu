@@ -37,6 +37,7 @@ static void free_graph(cg_graph *g) {
   cudaFree(g->in_off);
   cudaFree(g->in_idx);
   cudaFree(g->state);
+  cudaFree(g->head);
   cudaFree(g->tmp_levels);
   cudaFree(g->tmp_parents);
   cudaFree(g->orig);

@@ -43,15 +43,14 @@ constexpr int kBfsBlock = 512;
 // Pull rounds: in-list entries a thread loads at once (all in flight before
 // any is tested), and how many entries of its vertex's list a thread scans
 // before the whole warp takes over the rest of it.
-#ifndef CG_PULL_CHUNK
-#define CG_PULL_CHUNK 4
-#endif
-#ifndef CG_PULL_LANE_MAX
-#define CG_PULL_LANE_MAX 32
-#endif
-constexpr int kPullThreadScan = CG_PULL_CHUNK;
-constexpr unsigned kPullLaneMax = CG_PULL_LANE_MAX;
+constexpr int kPullThreadScan = 4;
+constexpr unsigned kPullLaneMax = 32;
 constexpr int kBfsWarps = kBfsBlock / 32;
+// Vertices a warp from which on a bitmap-wide round hands its items out from a
+// counter, two a warp; below, one item a warp takes fewer trips than the balance
+// is worth (525,000 unvisited vertices, 72 a warp, R-MAT scale 20: 16 us instead
+// of 21; scale 23, 500 a warp: 1.7 times slower without).
+constexpr unsigned long long kHeavyWork = 128;
 
 // Per-warp shared memory of the bitmap-wide rounds: a staged tile (its words
 // and the exclusive prefix of their popcounts, so that a lane can select the
@@ -62,7 +61,8 @@ struct __align__(16) WarpTile {  // 16-byte vector accesses to every member
   uint32_t found[kTileWords];
 };
 static_assert(sizeof(WarpTile) % 16 == 0 && kTileWords % 4 == 0, "16-byte tile rows");
-// Per-warp shared memory of a push round: the edge spreading of gather_expand
+// Per-warp shared memory of a push round (a pull round keeps the vertices whose
+// first in-neighbour was no parent here): the edge spreading of gather_expand
 // (list starts and prefix counts fit 32 bits, nnz being below 2^32), and the
 // claimed vertices not queued yet with their out-degrees.
 struct WarpExpand {
@@ -476,16 +476,30 @@ __device__ void push_round_bitmap(const BfsParams &p, const uint32_t *cur, uint3
 // Work items are (tile, slot) pairs of 4096-vertex bitmap tiles: one 16-byte
 // load per lane of each of vis, F_L and the map of vertices without in-edges
 // gives the tile's unvisited set, staged in shared memory, and the slot takes
-// an even range of it.  Each lane works on one vertex of the range at a time,
-// kPullThreadScan entries of its list a step (all loads in flight before any
-// test); a lane whose vertex is done (found, or its list exhausted) takes the
-// range's next vertex at once, so lanes do not wait for the slowest list of a
-// batch.  A list still unresolved after kPullLaneMax entries is finished by
-// the whole warp, 32 entries a step.  Found vertices set their bit in the
-// warp's shared copy of the tile's next-frontier words, ORed into F_{L+1} at
-// the end of the item.  Slot 0 of each tile also merges F_L into vis (the
-// union vis | F_L that other slots test is unchanged by it) and clears F_{L-1}
-// (the next round's output bitmap), so pull rounds need no sweep.
+// an even range of it.
+//
+// First the heads: a vertex's first in-neighbour and in-degree lie together in
+// an array by vertex (`head`), so a test of the first entry -- on R-MAT graphs,
+// a hub, the one that most vertices resolve at -- takes one coalesced 8-byte
+// load and one bit, where the list bounds and then the list are two dependent,
+// scattered trips.  An SM's scattered accesses, about 1.4 a ns, bound the big
+// pull rounds: R-MAT scale 23, 3.6 M vertices found, 78 -> 55 us.  Light rounds,
+// bound by the length of the chain, do without (n = 4096: 0.7 us a search).
+//
+// The misses are staged anew and scanned from their second entry on: each lane
+// works on one vertex of the range at a time, an aligned block of
+// kPullThreadScan entries of its list a step (one 16-byte load; all bit tests
+// in flight at once); a lane whose vertex is done (found, or its list
+// exhausted) takes the range's next vertex at once, so lanes do not wait for
+// the slowest list of a batch.  A list still unresolved after kPullLaneMax
+// entries is finished by the whole warp, 32 entries a step.  Found vertices set
+// their bit in the warp's shared copy of the tile's next-frontier words, ORed
+// into F_{L+1} at the end of the item.  Slot 0 of each tile also merges F_L into
+// vis (the union vis | F_L that other slots test is unchanged by it) and clears
+// F_{L-1} (the next round's output bitmap), so pull rounds need no sweep.
+// Without heads (graphs without hubs, see bfs_prepare; cg_bfs_noalloc, whose
+// arrays need not be aligned either; no memory for them) every vertex is scanned
+// from its first entry.
 __device__ void pull_round(const BfsParams &p, const uint32_t *cur, uint32_t *nxt, uint32_t *old,
                            int L, RoundRec *Rc, bool heavy, Acc &acc) {
   const int lane = lane_id();
@@ -516,16 +530,59 @@ __device__ void pull_round(const BfsParams &p, const uint32_t *cur, uint32_t *nx
     const uint4 un = make_uint4(~(vi.x | cu.x | dd.x), ~(vi.y | cu.y | dd.y),
                                 ~(vi.z | cu.z | dd.z), ~(vi.w | cu.w | dd.w));
     st4(T.found + 4 * lane, make_uint4(0u, 0u, 0u, 0u));
-    const unsigned total = stage_tile(un, T);
-    const unsigned k1 = (unsigned)((unsigned long long)total * (slot + 1) / S);
+    unsigned total = stage_tile(un, T);
+    unsigned k1 = (unsigned)((unsigned long long)total * (slot + 1) / S);
     unsigned cursor = (unsigned)((unsigned long long)total * slot / S);
+    const int64_t v0 = t * kTileWords * 32;  // the tile's first vertex
+    if (heavy && p.head) {
+      constexpr int U = 2;  // batches of 32 vertices in flight
+      uint32_t *miss = reinterpret_cast<uint32_t *>(&s_expand[wib]);
+      static_assert(sizeof(WarpExpand) >= 4 * kTileWords && sizeof(WarpExpand) % 16 == 0, "miss");
+      st4(miss + 4 * lane, make_uint4(0u, 0u, 0u, 0u));
+      __syncwarp();
+      for (unsigned b0 = cursor; b0 < k1; b0 += 32 * U) {
+        int at[U];   // vertex of the tile
+        uint2 h[U];  // its first in-neighbour and in-degree
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+          const unsigned k = b0 + 32 * q + lane;
+          at[q] = -1;
+          h[q] = make_uint2(0u, 0u);
+          if (k < k1) {
+            int j, bit;
+            select_bit(T, k, j, bit);
+            at[q] = 32 * j + bit;
+            h[q] = __ldg(p.head + v0 + at[q]);
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+          if (at[q] < 0) continue;
+          const uint32_t b = 1u << (at[q] & 31);
+          if ((cur[h[q].x >> 5] >> (h[q].x & 31)) & 1u) {
+            const int32_t ov = orig_id(p, v0 + at[q]);
+            p.parents[ov] = orig_id(p, (int32_t)h[q].x);
+            p.levels[ov] = L + 1;
+            atomicOr(&T.found[at[q] >> 5], b);
+            acc.nf += 1;
+            acc.visdeg += h[q].y;
+          } else if (h[q].y > 1) {
+            atomicOr(&miss[at[q] >> 5], b);
+          }
+        }
+      }
+      __syncwarp();
+      const uint4 m = ld4(miss + 4 * lane);
+      total = stage_tile(m, T);
+      cursor = 0;
+      k1 = total;
+    }
     // lane state: the vertex it works on (v, word j / bit of the tile), its
     // list [s, s + deg) and the next entry to scan
     bool has = false;
     int j = 0, bit = 0;
     int64_t s = 0;
     unsigned deg = 0, pos = 0;
-    const int64_t v0 = t * kTileWords * 32;  // the tile's first vertex
     bool refill = true;  // some lane has no vertex (warp-uniform)
     while (true) {
       if (refill) {
@@ -538,7 +595,7 @@ __device__ void pull_round(const BfsParams &p, const uint32_t *cur, uint32_t *nx
             const int64_t v = v0 + j * 32 + bit;
             s = __ldg(p.in_off + v);
             deg = (unsigned)(__ldg(p.in_off + v + 1) - s);
-            pos = 0;
+            pos = heavy && p.head ? 1 : 0;
           }
         }
         cursor += __popc(need);
@@ -546,10 +603,24 @@ __device__ void pull_round(const BfsParams &p, const uint32_t *cur, uint32_t *nx
       if (!__any_sync(kFull, has)) break;
       bool found = false;
       if (has && pos < kPullLaneMax) {
+        // the entries of the aligned block that holds entry pos (arrays of the
+        // library's own), or the next kPullThreadScan ones
         int32_t u[kPullThreadScan];
+        const int64_t e0 = s + pos;
+        unsigned skip = p.head ? (unsigned)e0 & 3u : 0u;
+        static_assert(kPullThreadScan == 4, "a 16-byte block");
+        if (p.head && e0 - skip + 4 <= p.nnz) {
+          const int4 x = __ldg(reinterpret_cast<const int4 *>(p.in_idx + (e0 - skip)));
+          u[0] = x.x, u[1] = x.y, u[2] = x.z, u[3] = x.w;
 #pragma unroll
-        for (int k = 0; k < kPullThreadScan; ++k)
-          u[k] = pos + k < deg ? __ldg(p.in_idx + s + pos + k) : -1;
+          for (int k = 0; k < kPullThreadScan; ++k)
+            if ((unsigned)k < skip || pos - skip + k >= deg) u[k] = -1;
+        } else {
+          skip = 0;
+#pragma unroll
+          for (int k = 0; k < kPullThreadScan; ++k)
+            u[k] = pos + k < deg ? __ldg(p.in_idx + e0 + k) : -1;
+        }
         uint32_t hit = 0;
 #pragma unroll
         for (int k = 0; k < kPullThreadScan; ++k)
@@ -565,7 +636,7 @@ __device__ void pull_round(const BfsParams &p, const uint32_t *cur, uint32_t *nx
           p.levels[ov] = L + 1;
           found = true;
         }
-        pos += kPullThreadScan;
+        pos += kPullThreadScan - skip;
       }
       // lists still open after kPullLaneMax entries: the whole warp scans the
       // rest, one vertex at a time
@@ -794,7 +865,7 @@ __device__ __forceinline__ unsigned close_round(const BfsParams &p, int L, int d
   const unsigned long long work =
       next == kPull ? (p.live > (int64_t)ss.visited ? (unsigned long long)p.live - ss.visited : 0ull)
                     : nf;
-  const bool heavy = work >= 32ull * (unsigned long long)((gridDim.x * blockDim.x) >> 5);
+  const bool heavy = work >= kHeavyWork * (unsigned long long)((gridDim.x * blockDim.x) >> 5);
   // (after a pull round of a directed graph the edges are not known: vd stands
   // for them)
   const bool solo = !done && next == kPush && nf <= solo_max &&
@@ -1273,7 +1344,7 @@ __global__ void __launch_bounds__(kBfsBlock, 3) bfs_persistent(BfsParams p) {
       queued = true;
       dir = (payload & kNextPull) ? kPull : kPush;
       heavy = (payload & kHeavy) != 0;
-      solo = false;
+        solo = false;
       __syncthreads();
       // all three bitmaps were cleared; fr0 holds F_L
     }
@@ -1415,24 +1486,38 @@ int64_t bfs_big_capacity(int64_t n, int64_t nnz) {
 // (bits past n are set too, through the tile padding: `words` = stride).  A
 // warp takes 32 words, a coalesced load of 33 offsets each.  *live: vertices
 // with in-edges.
+// hub_edges: entries of vertices of in-degree > kLightMax.
 __global__ void dead_map_kernel(int64_t n, int64_t words, const int64_t *__restrict__ in_off,
-                                uint32_t *dead, unsigned long long *live) {
+                                uint32_t *dead, unsigned long long *live,
+                                unsigned long long *hub_edges) {
   const int lane = lane_id();
-  unsigned long long alive = 0;
+  unsigned long long alive = 0, hubs = 0;
   const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t w0 = (int64_t)warp_id_global() * 32; w0 < words; w0 += warps * 32) {
     uint32_t mine = 0;
     for (int j = 0; j < 32 && w0 + j < words; ++j) {
       const int64_t v = (w0 + j) * 32 + lane;
-      const bool none = v >= n || __ldg(in_off + v) == __ldg(in_off + v + 1);
-      const uint32_t m = __ballot_sync(kFull, none);
+      const int64_t d = v < n ? __ldg(in_off + v + 1) - __ldg(in_off + v) : 0;
+      if (d > kLightMax) hubs += (unsigned long long)d;
+      const uint32_t m = __ballot_sync(kFull, d == 0);
       if (lane == j) mine = m;
     }
     if (w0 + lane < words) dead[w0 + lane] = mine;
     if (w0 + lane < words) alive += (unsigned)__popc(~mine);
   }
   alive = warp_sum(alive);
+  hubs = warp_sum(hubs);
   if (lane == 0 && alive) atomicAdd(live, alive);
+  if (lane == 0 && hubs) atomicAdd(hub_edges, hubs);
+}
+
+// Each vertex's first in-neighbour and in-degree (of one without, zeros).
+__global__ void head_kernel(int64_t n, const int64_t *__restrict__ in_off,
+                            const int32_t *__restrict__ in_idx, uint2 *__restrict__ head) {
+  const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= n) return;
+  const int64_t s = __ldg(in_off + v), e = __ldg(in_off + v + 1);
+  head[v] = s < e ? make_uint2((unsigned)__ldg(in_idx + s), (unsigned)(e - s)) : make_uint2(0u, 0u);
 }
 
 int refuse_setup_in_capture(cg_graph *g) {
@@ -1459,7 +1544,7 @@ int bfs_prepare(cg_graph *g) {
   };
   const size_t at_ctl = piece(sizeof(BfsCtl));
   const size_t at_stats = piece(sizeof(cg_stats));
-  const size_t at_live = piece(sizeof(unsigned long long));
+  const size_t at_live = piece(2 * sizeof(unsigned long long));  // and the hubs' entries
   const size_t zeroed = bytes;
   const size_t at_bitmaps = piece(sizeof(uint32_t) * 4 * (size_t)stride);
   const size_t at_dead = piece(sizeof(uint32_t) * (size_t)stride);
@@ -1481,16 +1566,48 @@ int bfs_prepare(cg_graph *g) {
   g->queue = reinterpret_cast<int32_t *>(base + at_queue);
   g->bigoff = reinterpret_cast<uint32_t *>(base + at_bigoff);
   unsigned long long *d_live = reinterpret_cast<unsigned long long *>(base + at_live);
-  unsigned long long live = 0;
+  unsigned long long live[2] = {0, 0};
   CG_CUDA(cudaMemsetAsync(base, 0, zeroed, g->stream));
   const int64_t blocks = (stride + 255) / 256;  // 8 warps of 32 words
   dead_map_kernel<<<(unsigned)(blocks < 4096 ? blocks : 4096), 256, 0, g->stream>>>(
-      g->n, stride, g->in_off, g->dead, d_live);
+      g->n, stride, g->in_off, g->dead, d_live, d_live + 1);
   CG_CUDA(cudaGetLastError());
-  CG_CUDA(cudaMemcpyAsync(&live, d_live, sizeof(live), cudaMemcpyDeviceToHost, g->stream));
+  CG_CUDA(cudaMemcpyAsync(live, d_live, sizeof(live), cudaMemcpyDeviceToHost, g->stream));
   CG_CUDA(cudaStreamSynchronize(g->stream));
-  g->live = (int64_t)live;
+  // Heads for graphs whose hubs hold half of the entries (R-MAT): the first
+  // entry of a list is then a hub, the one most vertices resolve at.  Without
+  // hubs the first entry is like any other, mostly a miss (directed ER of degree
+  // 8: its first pull round of 119 us took 127 with them).
+  if (2 * live[1] >= (unsigned long long)g->nnz && g->nnz > 0) {
+    if (cudaMalloc(&g->head, sizeof(uint2) * (size_t)g->n) == cudaSuccess) {
+      g->device_bytes += (int64_t)sizeof(uint2) * g->n;
+      head_kernel<<<(unsigned)((g->n + 255) / 256), 256, 0, g->stream>>>(g->n, g->in_off, g->in_idx,
+                                                                        g->head);
+      CG_CUDA(cudaGetLastError());
+    } else {
+      cudaGetLastError();  // searches do without
+      g->head = nullptr;
+    }
+  }
+  g->live = (int64_t)live[0];
   return CG_OK;
+}
+
+// Blocks per SM of a search whose options leave it open, at most what fits (3).
+// Fewer blocks make every round's barrier cheaper, and with one the searches of
+// three handles run side by side (R-MAT n = 4 K, three handles in turn: 55 -> 19
+// us a search); more keep more list reads in flight.  Measured, all rounds of
+// one search with 3 / 2 / 1 blocks, us: direction-optimizing R-MAT n = 4 K 47 / 46
+// / 45, 64 K 57 / 51 / 48, 256 K 67 / 63 / 61, 1 M 85 / 82 / 84, 2 M 127 / 122 /
+// 128, 4 M 177 / 183 / 230; directed ER 300 K 100 / 93 / 90, 1 M 139 / 136 / 147, 3
+// M 292 / 305 / 374; a 1000^2 grid is the same with all.  Top-down, which pushes
+// every edge: R-MAT 16 K (0.4 M entries) 56 / 56 / 57, 64 K (1.8 M) 76 / 77 / 92,
+// 256 K 136 / 159 / 204; ER 100 K (0.8 M) 94 / 90 / 94.
+static int blocks_for(const cg_graph *g) {
+  if (g->opt.direction == CG_DIR_TOPDOWN)
+    return g->nnz < (1 << 19) ? 1 : (g->nnz < (1 << 20) ? 2 : 3);
+  if (g->n <= 300000 || g->nnz < (1 << 22)) return 1;
+  return g->n <= (1 << 21) ? 2 : 3;
 }
 
 static int bfs_grid(cg_graph *g) {
@@ -1501,7 +1618,8 @@ static int bfs_grid(cg_graph *g) {
   int per_sm = 0;
   CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bfs_persistent, block, 0));
   if (per_sm <= 0) return CG_ERR_NOT_SUPPORTED;
-  if (g->opt.blocks_per_sm > 0 && g->opt.blocks_per_sm < per_sm) per_sm = g->opt.blocks_per_sm;
+  const int want = g->opt.blocks_per_sm > 0 ? g->opt.blocks_per_sm : blocks_for(g);
+  if (want < per_sm) per_sm = want;
   g->bfs_grid = per_sm * g->num_sms;
   g->bfs_block = block;
   return CG_OK;
@@ -1527,6 +1645,7 @@ int bfs_launch(cg_graph *g, int64_t root, int32_t *d_levels, int32_t *d_parents,
   p.fr2 = g->bitmaps + 3 * stride;
   p.dead = g->dead;
   p.live = g->live;
+  p.head = g->head;
   p.orig = g->orig;
   p.perm = g->perm;
   p.queue0 = g->queue;

@@ -108,6 +108,7 @@ struct BfsParams {
   const uint32_t *dead;  // vertices without in-edges (never reached), or null; bits
                          // past n are set, `stride` words
   int64_t live;          // vertices with in-edges (n when `dead` is null)
+  const uint2 *head;     // each vertex's first in-neighbour and in-degree, or null
   // Relabelled graph (cg_graph_reorder), or null: orig[v] is the original id
   // of resident vertex v and perm its inverse.  Roots come in original ids;
   // outputs are written at original positions with original parent ids.
@@ -152,6 +153,7 @@ struct cg_graph {
   uint32_t *bitmaps = nullptr;  // vis | fr0 | fr1 | fr2, 4 * bitmap_stride(n)
   uint32_t *dead = nullptr;     // 1 bit per vertex: no in-edges, bitmap_stride(n) words
   int64_t live = 0;             // vertices with in-edges
+  uint2 *head = nullptr;        // [n] first in-neighbour and in-degree (null: no memory)
   // cg_graph_reorder: resident vertex v is original vertex orig[v]; perm is
   // the inverse (both int32[n], null for a graph in its original order)
   int32_t *orig = nullptr;

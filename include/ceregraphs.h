@@ -70,7 +70,7 @@ typedef struct cg_options {
   float beta;               /* pull->push when frontier vertices < n / beta (and shrinking) */
   int64_t tau_switch_count; /* CG_DIR_TAU threshold; the reference uses round(0.15 n) */
   int32_t block_size;       /* threads per block of the persistent kernel (multiple of 32) */
-  int32_t blocks_per_sm;    /* 0 = as many as fit */
+  int32_t blocks_per_sm;    /* 0 = by the graph's size, at most as many as fit */
   int32_t level_cap;        /* stop with CG_ERR_LEVEL_CAP after this many rounds (0 = n + 1) */
   int32_t wait_timeout_ms;  /* bound on each grid-wide wait (default 1000) */
   int32_t lane_words;       /* multi-source: 1 = 64 lanes, 2 = 128 lanes per pass */
