@@ -64,14 +64,20 @@ static_assert(sizeof(WarpTile) % 16 == 0 && kTileWords % 4 == 0, "16-byte tile r
 // Per-warp shared memory of a push round (a pull round keeps the vertices whose
 // first in-neighbour was no parent here): the edge spreading of gather_expand
 // (list starts and prefix counts fit 32 bits, nnz being below 2^32), and the
-// claimed vertices not queued yet with their out-degrees.
+// light vertices claimed and not queued yet.  Big ones wait in the tile's
+// `found` words, which push rounds do not use.
 struct WarpExpand {
   int32_t u[32];
   uint32_t s[32];
   uint32_t x[32];
-  int32_t claim_v[64];
-  uint32_t claim_deg[64];
+  int32_t light[64];
 };
+struct BigClaims {
+  int32_t v[64];
+  uint32_t deg[64];
+};
+static_assert(sizeof(BigClaims) == sizeof(uint32_t) * kTileWords, "fits WarpTile::found");
+
 // Shared memory of block 0's runs of small rounds (solo_rounds): the frontier
 // and the next one (vertex, list start, out-degree), and the prefix of the
 // frontier's degrees.
@@ -212,80 +218,162 @@ __device__ __forceinline__ void enqueue_claims(const BfsParams &p, bool claimed,
   }
 }
 
-// Edge u -> v of a push round.  Returns true for the one thread that claims
-// v, with v's out-degree in deg (its offsets are loaded with the claim, so the
-// claimer does not wait for them afterwards).  A target claimed already gets
-// a read before its atomicMin: most of a big round's edges lead to vertices
-// that a lower source has reached, and a read costs the L2 less.
-__device__ __forceinline__ bool relax_push(const BfsParams &p, const uint32_t *cur,
-                                           uint32_t *nxt, int32_t u, int32_t v, int next_level,
-                                           uint32_t &deg) {
-  const uint32_t w = (uint32_t)v >> 5, bit = 1u << (v & 31);
-  // the three words in one round trip: a claim bit seen set stays set
-  const uint32_t seen = p.vis[w] | cur[w], claimed = nxt[w];
-  if (seen & bit) return false;
-  const int32_t ov = orig_id(p, v);
-  unsigned *par = reinterpret_cast<unsigned *>(p.parents) + ov;
-  const unsigned ou = (unsigned)orig_id(p, u);
-  if (claimed & bit) {
-    if (__ldcg(par) > ou) atomicMin(par, ou);
-    return false;
-  }
-  atomicMin(par, ou);
-  const int64_t o0 = __ldg(p.out_off + v), o1 = __ldg(p.out_off + v + 1);
-  const unsigned old = atomicOr(nxt + w, bit);
-  if (old & bit) return false;
-  p.levels[ov] = next_level;
-  deg = (uint32_t)(o1 - o0);
-  return true;
-}
-
-// Claimed vertices on their way to the next frontier's queue: a warp keeps
-// them in shared memory and queues 32 at a time, so a round makes one returning
-// atomic on the shared queue counter per 32 claims instead of one per step with
-// any claim -- at R-MAT scales that counter bounded the big push rounds -- and
-// the steps do not wait for it.  Rounds of 61,564
-// claims (R-MAT n = 100,003, top-down): 68 -> 37 us; of 862,250 (scale 23): 235
-// -> 174 us.
+// Claimed vertices on their way to the next frontier's queue.  A returning
+// atomic on one address takes about 2 ns however many blocks make them, and a
+// round that made one per step with claims, or one per warp at its end, was
+// bound by them.  So a warp keeps its claims in shared memory, light and big
+// ones apart, queues 32 of a kind with one atomic, and the block queues what its
+// warps have left together at the round's end.  Rounds of 61,564 claims (R-MAT n
+// = 100,003, top-down): FIG_A; of 202,765 (directed ER): FIG_B; of 862,250 (R-MAT
+// scale 23): FIG_C.
 struct Claims {
   WarpExpand &X;
-  unsigned count = 0;  // entries waiting (the same in every lane), < 32 between steps
+  BigClaims &B;
+  unsigned nl = 0, nb = 0;  // waiting (the same in every lane), < 32 between steps
 };
 
-__device__ __forceinline__ void queue_claims(const BfsParams &p, Claims &C, unsigned n,
-                                             unsigned from, int next_parity, RoundRec *Rn,
-                                             Acc &acc) {
-  const unsigned i = from + (unsigned)lane_id();
-  const bool has = (unsigned)lane_id() < n;
-  const int32_t v = has ? C.X.claim_v[i] : 0;
-  const uint32_t d = has ? C.X.claim_deg[i] : 0u;
-  enqueue_claims(p, has, v, (int64_t)d, next_parity, Rn, acc);
+// Big vertices B[from .. from + n), n <= 32, at queue index `idx` with edge
+// offset `edges` among the big vertices' lists.  All 32 lanes call.
+__device__ __forceinline__ void put_big(const BfsParams &p, const BigClaims &B, unsigned from,
+                                        unsigned n, unsigned idx, unsigned edges,
+                                        int next_parity) {
+  const int lane = lane_id();
+  const bool has = (unsigned)lane < n;
+  const uint32_t d = has ? B.deg[from + lane] : 0u;
+  uint32_t incl = d;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(kFull, incl, o);
+    if (lane >= o) incl += t;
+  }
+  if (!has) return;
+  (next_parity ? p.queue1 : p.queue0)[p.n - 1 - (int64_t)(idx + lane)] = B.v[from + lane];
+  (next_parity ? p.bigoff1 : p.bigoff0)[idx + lane] = edges + incl - d;
 }
 
-__device__ __forceinline__ void push_step(const BfsParams &p, const uint32_t *cur, uint32_t *nxt,
-                                          bool valid, int32_t u, int64_t e, int L,
-                                          int next_parity, RoundRec *Rn, Claims &C, Acc &acc) {
-  bool claimed = false;
-  int32_t v = 0;
-  uint32_t deg = 0;
-  if (valid) {
-    v = __ldg(p.out_idx + e);
-    claimed = relax_push(p, cur, nxt, u, v, L + 1, deg);
-  }
+// The claims of one warp-wide step.  All 32 lanes call.
+__device__ __forceinline__ void keep_claims(const BfsParams &p, bool claimed, int32_t v,
+                                            uint32_t deg, int next_parity, RoundRec *Rn, Claims &C,
+                                            Acc &acc) {
+  const int lane = lane_id();
+  const unsigned below = (1u << lane) - 1u;
   const unsigned m = __ballot_sync(kFull, claimed);
   if (!m) return;
   if (claimed) {
-    const unsigned at = C.count + __popc(m & ((1u << lane_id()) - 1u));
-    C.X.claim_v[at] = v;
-    C.X.claim_deg[at] = deg;
+    acc.nf += 1;
+    acc.mf += deg;
+    acc.visdeg += deg;
   }
-  C.count += __popc(m);
+  const bool big = claimed && deg > (uint32_t)kLightMax;
+  const unsigned mb = __ballot_sync(kFull, big), ml = m & ~mb;
+  if (big) {
+    const unsigned at = C.nb + __popc(mb & below);
+    C.B.v[at] = v;
+    C.B.deg[at] = deg;
+  } else if (claimed) {
+    C.X.light[C.nl + __popc(ml & below)] = v;
+  }
+  C.nb += __popc(mb);
+  C.nl += __popc(ml);
   __syncwarp();
-  if (C.count >= 32) {
-    C.count -= 32;  // the last 32: the entries below keep their places
-    queue_claims(p, C, 32, C.count, next_parity, Rn, acc);
+  // full groups: the last 32, the entries below keep their places
+  if (C.nl >= 32) {
+    C.nl -= 32;
+    unsigned base = 0;
+    if (lane == 0) base = atomicAdd(&Rn->nlight, 32u);
+    base = __shfl_sync(kFull, base, 0);
+    (next_parity ? p.queue1 : p.queue0)[base + lane] = C.X.light[C.nl + lane];
     __syncwarp();
   }
+  if (C.nb >= 32) {
+    C.nb -= 32;
+    const uint32_t edges = __reduce_add_sync(kFull, C.B.deg[C.nb + lane]);
+    unsigned long long old = 0;
+    if (lane == 0) old = atomicAdd(&Rn->big, (32ull << 32) | edges);
+    old = __shfl_sync(kFull, old, 0);
+    put_big(p, C.B, C.nb, 32, (unsigned)(old >> 32), (unsigned)old, next_parity);
+    __syncwarp();
+  }
+}
+
+// What the block's warps have left, one atomic of a kind.  All threads call.
+__device__ __forceinline__ void queue_rest(const BfsParams &p, Claims &C, int next_parity,
+                                           RoundRec *Rn) {
+  __shared__ unsigned s_nl[kBfsWarps], s_nb[kBfsWarps], s_edges[kBfsWarps];
+  const int lane = lane_id(), wib = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const uint32_t edges = __reduce_add_sync(kFull, (unsigned)lane < C.nb ? C.B.deg[lane] : 0u);
+  if (lane == 0) {
+    s_nl[wib] = C.nl;
+    s_nb[wib] = C.nb;
+    s_edges[wib] = edges;
+  }
+  __syncthreads();
+  if (wib == 0) {  // exclusive prefixes, from the queue's own counts
+    const unsigned l = lane < nw ? s_nl[lane] : 0u, b = lane < nw ? s_nb[lane] : 0u,
+                   e = lane < nw ? s_edges[lane] : 0u;
+    unsigned il = l, ib = b, ie = e;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned tl = __shfl_up_sync(kFull, il, o), tb = __shfl_up_sync(kFull, ib, o),
+                     te = __shfl_up_sync(kFull, ie, o);
+      if (lane >= o) il += tl, ib += tb, ie += te;
+    }
+    unsigned long long old = 0;
+    if (lane == 31 && il) old = atomicAdd(&Rn->nlight, il);
+    const unsigned base_l = (unsigned)__shfl_sync(kFull, old, 31);
+    if (lane == 31) old = ib ? atomicAdd(&Rn->big, ((unsigned long long)ib << 32) | ie) : 0ull;
+    old = __shfl_sync(kFull, old, 31);
+    if (lane < nw) {
+      s_nl[lane] = base_l + il - l;
+      s_nb[lane] = (unsigned)(old >> 32) + ib - b;
+      s_edges[lane] = (unsigned)old + ie - e;
+    }
+  }
+  __syncthreads();
+  if ((unsigned)lane < C.nl)
+    (next_parity ? p.queue1 : p.queue0)[s_nl[wib] + lane] = C.X.light[lane];
+  if (C.nb) put_big(p, C.B, 0, C.nb, s_nb[wib], s_edges[wib], next_parity);
+}
+
+constexpr uint32_t kNoEdge = 0xffffffffu;
+
+// Edge u -> out_idx[e] per lane of a push round (e = kNoEdge for none).  A
+// target claimed already gets a read before its atomicMin: most of a big
+// round's edges lead to vertices that a lower source has reached, and a read
+// costs the L2 less.
+__device__ __forceinline__ void push_step(const BfsParams &p, const uint32_t *cur, uint32_t *nxt,
+                                          int32_t u, uint32_t e, int L, int next_parity,
+                                          RoundRec *Rn, Claims &C, Acc &acc) {
+  const int32_t v = e != kNoEdge ? __ldg(p.out_idx + e) : -1;
+  bool open = false, mine = false;  // not visited; nor claimed by another edge before
+  if (v >= 0) {
+    const uint32_t w = (uint32_t)v >> 5, bit = 1u << (v & 31);
+    // the three words in one round trip: a claim bit seen set stays set (the
+    // L1's copy may lack it: reading the hot words from the L2 took 140 us where
+    // this takes 92, R-MAT n = 100,003, top-down)
+    const uint32_t seen = p.vis[w] | cur[w], claimed = nxt[w];
+    open = !(seen & bit);
+    mine = open && !(claimed & bit);
+  }
+  bool claimed = false;
+  uint32_t deg = 0;
+  if (open) {
+    const int32_t ov = orig_id(p, v);
+    const unsigned ou = (unsigned)orig_id(p, u);
+    unsigned *par = reinterpret_cast<unsigned *>(p.parents) + ov;
+    if (mine) {
+      atomicMin(par, ou);
+      // the target's list bounds go out with its claim
+      const int64_t o = __ldg(p.out_off + v);
+      deg = (uint32_t)(__ldg(p.out_off + v + 1) - o);
+      const uint32_t bit = 1u << (v & 31);
+      claimed = !(atomicOr(nxt + ((uint32_t)v >> 5), bit) & bit);
+      if (claimed) p.levels[ov] = L + 1;
+    } else if (__ldcg(par) > ou) {
+      atomicMin(par, ou);
+    }
+  }
+  keep_claims(p, claimed, v, deg, next_parity, Rn, C, acc);
 }
 
 // Expands up to 32 frontier vertices (one per lane, u < 0 for none) with the
@@ -315,23 +403,13 @@ __device__ __forceinline__ void gather_expand(const BfsParams &p, const uint32_t
   __syncwarp();
   for (uint32_t base = 0; base < total; base += 32) {
     const uint32_t t = base + lane;
-    const bool valid = t < total;
-    int32_t uu = 0;
-    int64_t e = 0;
-    if (valid) {
-      int lo = 0, hi = 31;
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (X.x[mid] <= t)
-          lo = mid;
-        else
-          hi = mid - 1;
-      }
-      uu = X.u[lo];
-      e = (int64_t)(X.s[lo] + (t - X.x[lo]));
-    }
-    push_step(p, cur, nxt, valid, uu, e, L, next_parity, Rn, C, acc);
-    if (base + 32 < base) break;  // total within 32 of 2^32
+    int lo = 0;  // the last of the 32 whose prefix is <= t
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1)
+      if (X.x[lo + step] <= t) lo += step;
+    const uint32_t e = t < total && t >= base ? X.s[lo] + (t - X.x[lo]) : kNoEdge;
+    push_step(p, cur, nxt, X.u[lo], e, L, next_parity, Rn, C, acc);
+    if (base + 32 < base) break;  // total within a step of 2^32
   }
   __syncwarp();
 }
@@ -364,12 +442,14 @@ __device__ void push_round_queue(const BfsParams &p, const uint32_t *cur, uint32
   unsigned group = 1;
   while (group < 32u && nlight > group * (unsigned)nwarps) group <<= 1;
   const unsigned nitems = nchunks + (nlight + group - 1) / group;
-  Claims C{s_expand[wib]};
+  Claims C{s_expand[wib], reinterpret_cast<BigClaims &>(s_tiles[wib].found)};
   unsigned item = (unsigned)warp_id_global();
   while (item < nitems) {
-    // the next item is claimed before this one is worked, hiding the atomic
-    unsigned nextitem = 0;
-    if (lane == 0) nextitem = (unsigned)nwarps + atomicAdd(&Rc->work, 1u);
+    // the next item is claimed before this one is worked, hiding the atomic;
+    // with no more items than warps there is none
+    unsigned nextitem = nitems;
+    if (nitems > (unsigned)nwarps && lane == 0)
+      nextitem = (unsigned)nwarps + atomicAdd(&Rc->work, 1u);
     if (item < nchunks) {
       const unsigned x0 = item * chunk;
       const unsigned x1 = min(x0 + chunk, big_edges);
@@ -384,29 +464,29 @@ __device__ void push_round_queue(const BfsParams &p, const uint32_t *cur, uint32
       }
       unsigned j = lo;
       int32_t vj = q[p.n - 1 - (int64_t)j];
-      int64_t sj = __ldg(p.out_off + vj);
+      uint32_t sj = (uint32_t)__ldg(p.out_off + vj);
       unsigned oj = boff[j];
-      unsigned endj = oj + (unsigned)(__ldg(p.out_off + vj + 1) - sj);
+      unsigned endj = oj + ((uint32_t)__ldg(p.out_off + vj + 1) - sj);
       for (unsigned base = x0; base < x1; base += 32) {
         while (base >= endj) {  // the next big vertex (degrees exceed 32)
           ++j;
           vj = q[p.n - 1 - (int64_t)j];
-          sj = __ldg(p.out_off + vj);
+          sj = (uint32_t)__ldg(p.out_off + vj);
           oj = boff[j];
-          endj = oj + (unsigned)(__ldg(p.out_off + vj + 1) - sj);
+          endj = oj + ((uint32_t)__ldg(p.out_off + vj + 1) - sj);
         }
         const unsigned x = base + lane;
         const bool valid = x < x1;
         int32_t u = vj;
-        int64_t e = sj + (int64_t)(x - oj);
+        uint32_t e = valid ? sj + (x - oj) : kNoEdge;
         if (__ballot_sync(kFull, valid && x >= endj)) {  // lanes past vertex j's end
           const int32_t vn = q[p.n - 1 - (int64_t)(j + 1)];
           if (valid && x >= endj) {
             u = vn;
-            e = __ldg(p.out_off + vn) + (int64_t)(x - endj);
+            e = (uint32_t)__ldg(p.out_off + vn) + (x - endj);
           }
         }
-        push_step(p, cur, nxt, valid, u, e, L, next_parity, Rn, C, acc);
+        push_step(p, cur, nxt, u, e, L, next_parity, Rn, C, acc);
       }
     } else {
       const unsigned idx = (item - nchunks) * group + lane;
@@ -415,7 +495,7 @@ __device__ void push_round_queue(const BfsParams &p, const uint32_t *cur, uint32
     }
     item = __shfl_sync(kFull, nextitem, 0);
   }
-  if (C.count) queue_claims(p, C, C.count, 0, next_parity, Rn, acc);
+  queue_rest(p, C, next_parity, Rn);
 }
 
 // Work items of a bitmap-wide round: (tile, slot) pairs; a tile holds 4096
@@ -448,7 +528,7 @@ __device__ void push_round_bitmap(const BfsParams &p, const uint32_t *cur, uint3
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int next_parity = (L + 1) & 1;
   WarpTile &T = s_tiles[wib];
-  Claims C{s_expand[wib]};
+  Claims C{s_expand[wib], reinterpret_cast<BigClaims &>(s_tiles[wib].found)};
   const unsigned S = tile_slots(p.tiles, nwarps, heavy);
   const int64_t items = p.tiles * S;
   for (int64_t item = warp_id_global(); item < items; item = next_item(item, nwarps, Rc, heavy)) {
@@ -468,7 +548,7 @@ __device__ void push_round_bitmap(const BfsParams &p, const uint32_t *cur, uint3
     }
     __syncwarp();  // T is restaged by the next item
   }
-  if (C.count) queue_claims(p, C, C.count, 0, next_parity, Rn, acc);
+  queue_rest(p, C, next_parity, Rn);
 }
 
 // Bottom-up round: every unvisited vertex scans its ascending in-list and

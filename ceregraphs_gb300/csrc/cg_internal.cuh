@@ -64,14 +64,19 @@ __host__ __device__ constexpr int64_t bitmap_stride(int64_t n) {
 }
 
 // Statistics of frontier F_k (the vertices at level k) and the queue holding it.
-struct RoundRec {
+// The three counters that many warps add to with a result (about 2 ns each, one
+// after another) have a 128-byte line of their own.
+struct alignas(128) RoundRec {
   unsigned long long nf[kCounterShards];      // |F_k|
   unsigned long long mf[kCounterShards];      // sum of out-degrees over F_k
   unsigned long long visdeg[kCounterShards];  // sum of degrees over F_k (unexplored edges)
+  unsigned long long pad0[8];
   unsigned long long big;      // (count << 32) | total edges of the big vertices of F_k
+  unsigned long long pad1[15];
   unsigned int nlight;         // light vertices, queue front
+  unsigned int pad2[31];
   unsigned int work;           // dynamic work counter used while F_k is expanded
-  unsigned long long pad[6];
+  unsigned int pad3[31];
 };
 
 // What block 0 hands the other blocks when its run of small rounds ends (or,

@@ -633,9 +633,11 @@ __device__ __forceinline__ void lg_load(const MsParams &p, Target<W> &t, const M
   t.f = t.add = Mask<W>::zero();
   if (t.v < 0) return;
   const Mask<W> seen = ld_mask<W>(p.vis, t.v);
-  const Mask<W> have = ld_mask<W>(nxt, t.v);
+  Mask<W> have;
+#pragma unroll
+  for (int i = 0; i < W; ++i) have.w[i] = __ldcg(nxt + (int64_t)t.v * W + i);
   t.slot = p.cand_slot[t.v];
-  t.tw = tnext[t.v >> 5];
+  t.tw = __ldcg(tnext + (t.v >> 5));
   Mask<W> now = Mask<W>::zero();
   if (!tfront || ((tfront[t.v >> 5] >> (t.v & 31)) & 1u)) now = ld_mask<W>(cur, t.v);
   t.f = fu.andnot(seen | now);
@@ -663,7 +665,7 @@ __device__ __forceinline__ bool lg_relax(const MsParams &p, int32_t u, const Tar
           bits &= bits ? bits - 1 : 0ull;
         }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) c[k] = b[k] >= 0 ? cand[j * 64 + b[k]] : 0u;
+        for (int k = 0; k < 4; ++k) c[k] = b[k] >= 0 ? __ldcg(cand + j * 64 + b[k]) : 0u;
 #pragma unroll
         for (int k = 0; k < 4; ++k)
           if (b[k] >= 0 && (unsigned)u < c[k]) atomicMin(cand + j * 64 + b[k], (unsigned)u);
