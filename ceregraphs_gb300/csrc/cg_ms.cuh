@@ -88,6 +88,9 @@ struct MsParams {
   // rounds stay below 255 and chunks below 2^24 (nnz < 2^32, 1024 per chunk)
   unsigned *hub_done;
   int nhub;
+  // pull rounds of ledger batches: things handed out together, and items of
+  // each kind (light words, medium vertices, hub chunks; pull_grabs)
+  unsigned hub_chunks, light_grab, med_grab, hub_grab, light_items, med_items, hub_items;
   int32_t *levels, *parents;  // batch mode: lane l at levels + l * n (start round 0)
   const LaneTable *lanes;     // serving pool: per-lane outputs and start rounds
   MsCtl *ctl;
@@ -545,6 +548,7 @@ struct MsState {
   uint32_t *lightfin = nullptr;  // [2][words]: the light map, then the finished map
   int64_t bcap = 0;
   int nhub = 0;
+  unsigned hub_chunks = 0;    // chunks of all hubs' in-lists
   int lane_words = 0;
   int hist_planes = 0;        // frontier planes after vis: 3, or the round history
   int hist_opt = 0;           // the ms_history option the state was sized for
@@ -600,6 +604,9 @@ inline MsParams ms_params(const cg_graph *g, const MsState *s) {
   p.hub_found = s->hub_found;
   p.hub_done = s->hub_done;
   p.nhub = s->nhub;
+  p.hub_chunks = s->hub_chunks;
+  p.light_grab = p.med_grab = p.hub_grab = 1;
+  p.light_items = p.med_items = p.hub_items = 0;
   p.levels = p.parents = nullptr;
   p.lanes = nullptr;
   p.ctl = s->ctl;

@@ -716,6 +716,7 @@ static int ms_build_hubs(cg_graph *g, MsState *s) {
       for (unsigned h = 0; h < nhub; ++h) h_chunks[h + 1] += h_chunks[h];
       // chunk -> hub, so a work item finds its hub with one load
       nchunks = h_chunks[nhub];
+      s->hub_chunks = (unsigned)nchunks;
       h_owner = new uint32_t[2 * (nchunks ? nchunks : 1)];
       uint32_t *h_order = h_owner + (nchunks ? nchunks : 1);
       for (unsigned h = 0; h < nhub; ++h)

@@ -373,30 +373,25 @@ __device__ void lg_pull(const MsParams &p, int L, const uint64_t *cur, uint64_t 
   const int lane = lane_id();
   // a symmetric graph stores one list per vertex: out-degree = in-degree
   const bool sym = p.out_off == p.in_off;
-  // light vertex groups (kLightGrab x 32 vertices), then medium vertices
-  // (groups of kMedGrab), then hub chunks (groups of kHubGrab), handed out
+  // light vertices by groups of p.light_grab bitmap words, then medium vertices
+  // by p.med_grab, then hub chunks by p.hub_grab (pull_grabs), handed out
   // dynamically -- one item per warp, then a counter -- so that the round's
   // last warps are not the ones with the longest lists
-  constexpr unsigned kLightGrab = 8, kMedGrab = 8, kHubGrab = 4;
   const unsigned nwarps = (unsigned)(nthreads >> 5);
-  const unsigned nlg = (unsigned)((p.n + 32 * kLightGrab - 1) / (32 * kLightGrab));
-  const unsigned nmg = (unsigned)((p.nmed + kMedGrab - 1) / kMedGrab);
-  const unsigned nchunks = p.nhub > 0 ? p.hub_choff[p.nhub] : 0u;
-  const unsigned nhg = (nchunks + kHubGrab - 1) / kHubGrab;
   unsigned item = (unsigned)warp_id_global();
-  while (item < nlg + nmg + nhg) {
+  while (item < p.light_items + p.med_items + p.hub_items) {
     // the next item is claimed before this one is worked, hiding the atomic
     unsigned nextitem = 0;
     if (lane == 0) nextitem = nwarps + atomicAdd(&Rc->work, 1u);
-    if (item < nlg) {
-      // the light vertices of kLightGrab words not yet finished, compacted 32
+    if (item < p.light_items) {
+      // the light vertices of a group's words not yet finished, compacted 32
       // at a time (vertices without in-edges are not light: none can reach
-      // them).  Lane j < kLightGrab holds word j; the t-th vertex is the
+      // them).  Lane j holds word j; the t-th vertex is the
       // (t - prefix)-th set bit of the first word whose inclusive count
       // exceeds t.  Only this warp touches these words of fin this round.
-      const int64_t w0 = (int64_t)item * kLightGrab;
+      const int64_t w0 = (int64_t)item * p.light_grab;
       uint32_t finw = 0, mine = 0;
-      if (lane < kLightGrab && w0 + lane < p.words) {
+      if ((unsigned)lane < p.light_grab && w0 + lane < p.words) {
         finw = p.fin[w0 + lane];
         mine = __ldg(p.light + w0 + lane) & ~finw;
       }
@@ -404,16 +399,16 @@ __device__ void lg_pull(const MsParams &p, int L, const uint64_t *cur, uint64_t 
       const int cnt = __popc(mine);
       int incl = cnt;
 #pragma unroll
-      for (int o = 1; o < kLightGrab; o <<= 1) {
+      for (int o = 1; o < 32; o <<= 1) {
         const int t = __shfl_up_sync(kMsFull, incl, o);
         if (lane >= o) incl += t;
       }
-      const int total = __shfl_sync(kMsFull, incl, kLightGrab - 1);
+      const int total = __shfl_sync(kMsFull, incl, 31);
       for (int b0 = 0; b0 < total; b0 += 32) {
         const int t = b0 + lane;
         int wsel = 0;
 #pragma unroll
-        for (int step = kLightGrab / 2; step > 0; step >>= 1)
+        for (int step = 16; step > 0; step >>= 1)
           if (__shfl_sync(kMsFull, incl, wsel + step - 1) <= t) wsel += step;
         const uint32_t wbits = __shfl_sync(kMsFull, mine, wsel);
         const int before = __shfl_sync(kMsFull, incl - cnt, wsel);
@@ -465,11 +460,11 @@ __device__ void lg_pull(const MsParams &p, int L, const uint64_t *cur, uint64_t 
         claim_step(p, claimed, (int32_t)v, deg, H, acc);
       }
       if (finw != fin0) p.fin[w0 + lane] = finw;
-    } else if (item < nlg + nmg) {
-      const unsigned mi = item - nlg;
-      const int64_t j0 = (int64_t)mi * kMedGrab;
-      const int64_t j1 = min(j0 + kMedGrab, p.nmed);
-      // 64 lanes: lanes 0 .. kMedGrab-1 look at the group's vertices at once
+    } else if (item < p.light_items + p.med_items) {
+      const unsigned mi = item - p.light_items;
+      const int64_t j0 = (int64_t)mi * p.med_grab;
+      const int64_t j1 = min(j0 + (int64_t)p.med_grab, p.nmed);
+      // 64 lanes: the first lanes look at the group's vertices at once
       // (the lanes each still wants and its in-list) and the warp then scans
       // those wanting any; 128 lanes (more registers): one vertex at a time
       int32_t vq = 0;
@@ -488,7 +483,7 @@ __device__ void lg_pull(const MsParams &p, int L, const uint64_t *cur, uint64_t 
         eq = __ldg(p.in_off + vq + 1);
       }
       unsigned pend = W == 1 ? __ballot_sync(kMsFull, wq.any())
-                             : (1u << (unsigned)(j1 - j0)) - 1u;
+                             : kMsFull >> (32u - (unsigned)(j1 - j0));
       while (pend) {
         const int t = __ffs(pend) - 1;
         pend &= pend - 1;
@@ -536,14 +531,14 @@ __device__ void lg_pull(const MsParams &p, int L, const uint64_t *cur, uint64_t 
         claim_step(p, cq, vq, dq, H, acc);
       }
     } else {
-      const unsigned hi_item = item - nlg - nmg;
-      const unsigned c1 = min((hi_item + 1) * kHubGrab, nchunks);
+      const unsigned hi_item = item - p.light_items - p.med_items;
+      const unsigned c1 = min((hi_item + 1) * p.hub_grab, p.hub_chunks);
       // a hub whose chunk c' < c found every wanted lane: chunk c holds only
       // higher-index entries, which could not be parents (known to this item
       // at once, to others through hub_done, tagged with the round)
       const unsigned tag = (unsigned)(L + 1) << 24;
       int done_h = -1;
-      for (unsigned ci = hi_item * kHubGrab; ci < c1; ++ci) {
+      for (unsigned ci = hi_item * p.hub_grab; ci < c1; ++ci) {
         const unsigned c = p.hub_chunk_order[ci];  // by rank within the hub, then hub
         const int h = (int)p.hub_of_chunk[c];
         if (h == done_h) continue;
@@ -1085,7 +1080,7 @@ __global__ void __launch_bounds__(kMsBlock, 2) msbfs_ledger(MsParams p) {
 // ---- scan pass, output pass ---------------------------------------------------
 
 constexpr int kScanBlock = 256;  // scan pass: threads a block
-constexpr int kScanWords = 4;    // scan pass: scanmap words a warp takes at a time
+constexpr int kScanWords = 16;   // scan pass: scanmap words a warp takes at a time, at most
 constexpr int kScanG = 2;        // in-list entries loaded together (most lanes resolve at the first)
 constexpr int kPre = 8;          // history planes loaded together (the output pass needs 8)
 
@@ -1112,14 +1107,15 @@ __device__ __forceinline__ uint64_t open_levels(const MsParams &p, int rounds) {
 
 // Scan pass, between the rounds and the output pass, over the light vertices
 // (in-degree 1 .. kPullLight; heavier ones have candidate slots) that the
-// rounds marked in scanmap.  A warp takes kScanWords words of the map at a time
+// rounds marked in scanmap.  A warp takes `grab` words of the map at a time
 // (the first by its index, the next from a counter, claimed before the current
-// chunk is worked), compacts their marked vertices in shared memory, and gives
+// chunk is worked; at 4 words a time the counter's 65,536 atomics took the whole
+// 60 us at R-MAT scale 23, 35 us at 16), compacts their marked vertices in shared memory, and gives
 // each thread one, whose in-list it scans for the parents of up to kOutLevels
 // open levels at once: the first entry u holding a lane of F_L in F_{L-1} is
 // its parent, and its position joins the vertex's slices.
 template <int W>
-__global__ void __launch_bounds__(kScanBlock) msbfs_scan(MsParams p) {
+__global__ void __launch_bounds__(kScanBlock) msbfs_scan(MsParams p, int grab) {
   __shared__ int32_t s_list[kScanBlock / 32][kScanWords * 32];
   if (*(volatile int *)p.flag || *(volatile int *)&p.ctl->status != 0) return;
   const uint64_t open = open_levels<W>(p, history_rounds(p));
@@ -1127,15 +1123,15 @@ __global__ void __launch_bounds__(kScanBlock) msbfs_scan(MsParams p) {
   const int lane = lane_id();
   int32_t *list = s_list[threadIdx.x >> 5];
   const unsigned nwarps = gridDim.x * (kScanBlock / 32);
-  const unsigned nchunks = (unsigned)((p.words + kScanWords - 1) / kScanWords);
+  const unsigned nchunks = (unsigned)((p.words + grab - 1) / grab);
   unsigned chunk = (unsigned)warp_id_global();
   while (chunk < nchunks) {
     unsigned next = 0;
     if (lane == 0) next = nwarps + atomicAdd(&p.ctl->scan_work, 1u);
-    const int64_t w0 = (int64_t)chunk * kScanWords;
+    const int64_t w0 = (int64_t)chunk * grab;
     const int64_t wi = w0 + lane;
     uint32_t bits =
-        lane < kScanWords && wi < p.words ? p.scanmap[wi] & __ldg(p.light + wi) : 0u;
+        lane < grab && wi < p.words ? p.scanmap[wi] & __ldg(p.light + wi) : 0u;
     const int c = __popc(bits);
     int incl = c;
 #pragma unroll
@@ -1475,6 +1471,25 @@ __global__ void __launch_bounds__(kOutBlock, 5) msbfs_outputs(MsParams p) {
     p.stats->finish_ns = global_ns() - *(volatile long long *)&ctl->t_round;
 }
 
+// What warps take at a time: the largest power of two that still leaves two
+// items for every warp.  More items than that only add atomics on
+// the round's work counter (one each, about 1 ns apart: the last pull round of 64
+// lanes on R-MAT scale 23 spent 220 us on 190,000 items, 171 us on 53,000), fewer
+// leave warps idle (scale 18: 4,864 warps shared 1,024 groups of 8 words; rounds
+// 125 / 84 us, 80 / 58 us now).
+unsigned grab_of(int64_t things, unsigned least, unsigned most, int64_t warps, unsigned *items) {
+  unsigned g = least;
+  while (g < most && things >= 4 * (int64_t)g * warps) g <<= 1;
+  *items = (unsigned)((things + g - 1) / g);
+  return g;
+}
+
+void pull_grabs(MsParams &p, int64_t warps) {
+  p.light_grab = grab_of(p.words, 1, 32, warps, &p.light_items);
+  p.med_grab = grab_of(p.nmed, 1, 32, warps, &p.med_items);
+  p.hub_grab = grab_of(p.hub_chunks, 1, 4, warps, &p.hub_items);
+}
+
 template <int W>
 int ledger_pass(cg_graph *g, MsState *s, const int64_t *roots, int k, int32_t *d_levels,
                 int32_t *d_parents) {
@@ -1503,14 +1518,17 @@ int ledger_pass(cg_graph *g, MsState *s, const int64_t *roots, int k, int32_t *d
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  pull_grabs(p, per_sm * g->num_sms * (block / 32));
   CG_CUDA(cudaLaunchKernelEx(&cfg, msbfs_ledger<W>, p));
   int scan_per_sm = 0;
   CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&scan_per_sm, msbfs_scan<W>, kScanBlock, 0));
   if (scan_per_sm <= 0) return CG_ERR_NOT_SUPPORTED;
-  const int64_t chunks = ((g->n + 31) / 32 + kScanWords - 1) / kScanWords;
-  int64_t scan_blocks = (chunks + kScanBlock / 32 - 1) / (kScanBlock / 32);
+  unsigned scan_items = 0;
+  const int64_t scan_warps = (int64_t)scan_per_sm * g->num_sms * (kScanBlock / 32);
+  const int scan_words = (int)grab_of(p.words, 4, kScanWords, scan_warps, &scan_items);
+  int64_t scan_blocks = ((int64_t)scan_items + kScanBlock / 32 - 1) / (kScanBlock / 32);
   if (scan_blocks > (int64_t)scan_per_sm * g->num_sms) scan_blocks = (int64_t)scan_per_sm * g->num_sms;
-  msbfs_scan<W><<<(unsigned)scan_blocks, kScanBlock, 0, g->stream>>>(p);
+  msbfs_scan<W><<<(unsigned)scan_blocks, kScanBlock, 0, g->stream>>>(p, scan_words);
   const int smem = kOutWarps * kOutWarpBytes;
   CG_CUDA(cudaFuncSetAttribute(msbfs_outputs<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                smem));
