@@ -53,6 +53,8 @@ namespace {
 
 constexpr int kOutBlock = 128;                 // output pass: 4 warps a block
 constexpr int kOutWarps = kOutBlock / 32;
+constexpr size_t kSmemOfSm = 228 * 1024;       // shared memory of an SM at most, and what
+constexpr size_t kSmemReserved = 1024;         // the system takes of it for a block
 constexpr int kOutLevels = 4;                  // levels resolved per in-list scan
 // A warp's shared tile: one parent table of kTab words per thread.  A vertex
 // with a candidate slot has its 64 parents there, lane l at column (l - 8 t) mod
@@ -1513,11 +1515,23 @@ int ledger_pass(cg_graph *g, MsState *s, const int64_t *roots, int k, int32_t *d
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = g->stream;
-  cudaLaunchAttribute attr[1];
+  // The rounds gather through the L1, which is what shared memory leaves of an
+  // SM.  Without a stated share the SM keeps the split of the kernel before it
+  // where that is large enough, and started right behind another handle's
+  // output pass (209 KB of shared memory a block set) every round ran on 20 KB
+  // of L1: three handles taking turns, n = 1,000,003, 100 lanes, rounds 829 us
+  // for 566; R-MAT scale 23, 64 lanes, 8.1 ms for 3.5.  Whole batches there:
+  // 1,223 -> 970 us and 4.5 to 5.4 -> 3.9 ms.
+  cudaFuncAttributes fa;
+  CG_CUDA(cudaFuncGetAttributes(&fa, msbfs_ledger<W>));
+  const size_t shared = (fa.sharedSizeBytes + kSmemReserved) * (size_t)per_sm;
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
+  attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+  attr[1].val.sharedMemCarveout = (unsigned)((shared * 100 + kSmemOfSm - 1) / kSmemOfSm);
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   pull_grabs(p, per_sm * g->num_sms * (block / 32));
   CG_CUDA(cudaLaunchKernelEx(&cfg, msbfs_ledger<W>, p));
   int scan_per_sm = 0;
