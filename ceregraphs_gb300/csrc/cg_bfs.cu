@@ -84,6 +84,16 @@ static_assert(sizeof(BigClaims) == sizeof(uint32_t) * kTileWords, "fits WarpTile
 constexpr int kSoloMax = 1280;             // vertices of a frontier kept here
 constexpr unsigned kSoloEdges = 4096;      // edges of a round run by one block
 constexpr unsigned kSoloEnter = 2048;      // edges of the first round of a run
+// A run that goes on above kTeamEnter edges a round is taken by a team of
+// blocks (team_rounds) in the kernel for graphs where that happens.
+constexpr int kTeamBlock = 384;            // threads of a block of that kernel, at most
+constexpr unsigned kTeam = 16;             // blocks
+constexpr unsigned kTeamEdges = 32768;     // edges of a round of the team
+constexpr unsigned kTeamEnter = 1024, kTeamLeave = 512;
+constexpr int64_t kTeamVertices = 1 << 16; // of a graph, at least
+constexpr int64_t kTeamDegree = 8;         // in-degree that all but 1/1024 of the entries keep to
+constexpr int kTeamAfter = 4;              // rounds above kTeamEnter before the hand-over
+constexpr int kTeamSession = 64;           // rounds of one hand-over, at most
 struct SoloShared {
   int32_t v[2][kSoloMax];
   uint32_t s[2][kSoloMax];
@@ -103,6 +113,7 @@ union __align__(16) RoundShared {
   SoloShared solo;
 };
 __shared__ RoundShared s_round;
+__shared__ unsigned s_commands;  // the team lead's commands that this block has served
 #define s_tiles s_round.grid.tiles
 #define s_expand s_round.grid.expand
 
@@ -838,6 +849,9 @@ __device__ __forceinline__ int next_direction(const BfsParams &p, int dir, unsig
 constexpr unsigned kDone = 1u, kNextPull = 2u, kHeavy = 4u;
 // ... is small enough for one block (solo_rounds)
 constexpr unsigned kSolo = 8u;
+// ... or for a team
+constexpr unsigned kHandOver = 16u;
+__device__ __forceinline__ unsigned team_size() { return gridDim.x >= 2 * kTeam ? kTeam : 0u; }
 
 // Flat grid-wide barrier of the per-root kernel, called by thread 0 of each
 // block after a __syncthreads: one fire-and-forget release add on the launch's
@@ -958,6 +972,7 @@ __device__ __forceinline__ unsigned close_round(const BfsParams &p, int L, int d
 // 0-23 each load one sharded counter of the round record (one L2 round trip),
 // lane 0 takes the decision (close_round), the same in every block.  All 32
 // lanes call; lane 0's return value is the payload.
+template <bool kTeamed>
 __device__ unsigned round_decision(const BfsParams &p, int L, int dir, SearchState &ss) {
   BfsCtl *ctl = p.ctl;
   const RoundRec *Rn = &ctl->rec[(L + 1) % kRing];
@@ -983,6 +998,16 @@ __device__ unsigned round_decision(const BfsParams &p, int L, int dir, SearchSta
   ss.next_light = (unsigned)qlight;
   // one block takes over well below what it can hold, so that a frontier near
   // the line does not go back and forth
+  if constexpr (kTeamed) {
+    // a team takes over where the frontier changes slowly (elsewhere it would be
+    // handed out for a round or two)
+    const bool steady = 4 * nf >= 3 * ss.prev_nf && 4 * nf <= 5 * ss.prev_nf;
+    if (dir == kPush && steady && (nf > (unsigned)kSoloMax / 2 || mf > kSoloEnter) &&
+        team_size()) {
+      const unsigned x = close_round(p, L, dir, nf, mf, vd, kTeam * kSoloMax / 4, kTeamEdges / 2, ss);
+      return (x & kSolo) ? x | kHandOver : x;
+    }
+  }
   return close_round(p, L, dir, nf, mf, vd, kSoloMax / 2, kSoloEnter, ss);
 }
 
@@ -1044,6 +1069,7 @@ __device__ __forceinline__ uint32_t solo_scan(SoloShared &S, int c, unsigned cnt
 // kSoloMax vertices the rest goes to `spill`).  A thread's U edges go through
 // every stage together: the searches' shared loads, the list entries, the
 // claims and the claimed targets' list bounds are in flight at once.
+template <bool kListed>
 __device__ __forceinline__ void solo_expand(const BfsParams &p, SoloShared &S, int c, unsigned cnt,
                                             uint32_t E, int L, int32_t *spill) {
   constexpr int U = 4;  // edges a thread has in flight
@@ -1115,10 +1141,245 @@ __device__ __forceinline__ void solo_expand(const BfsParams &p, SoloShared &S, i
         S.s[c ^ 1][at] = s[k];
         S.d[c ^ 1][at] = d[k];
       } else {
-        spill[at] = v[k];
+        spill[kListed ? atomicAdd(&p.ctl->team.listed, 1u) : at] = v[k];
       }
       ++at;
     }
+  }
+}
+
+// ---- small rounds on a team of blocks -----------------------------------------
+// One SM makes about 1.5 requests a ns past its L1, so that a grid graph's
+// round of 2,400 edges takes the lead block 7 us, 2.5 of it latency.  Sixteen
+// blocks share such rounds: each keeps the vertices it claims in its own shared
+// memory (the compare-and-swap on the level is the same), and a round ends with
+// one wait on a sum that carries the frontier's totals, about 2.5 us.  The
+// lead hands its frontier out as a list in memory and gets one back, at least
+// every kTeamSession rounds, which also evens out the shares.  A search of a
+// 1000^2 grid 9.9 -> 6.8 ms, of a 4000^2 grid 51.4 -> 42.7 ms; three handles
+// taking turns on a 1000^2 grid 5.5 -> 3.3 ms a search (with 4 blocks 4.7, 8 3.95,
+// 12 3.7, 16 3.55, 24 3.5, all with 512 threads a block).
+// This block's place in the team (the lead's is 0), kTeam or more outside it.
+// Members are spread over the grid: neighbours may share an SM.
+__device__ __forceinline__ unsigned team_rank() {
+  const unsigned stride = gridDim.x / kTeam;
+  return team_size() && blockIdx.x % stride == 0 ? blockIdx.x / stride : kTeam;
+}
+__device__ __forceinline__ bool in_team() { return team_rank() < kTeam; }
+
+// F_L's list while the team runs: the queue that F_L is not put in.
+__device__ __forceinline__ int32_t *team_list(const BfsParams &p, int L) {
+  return (L & 1) ? p.queue0 : p.queue1;
+}
+
+// Bounded wait of thread 0 until *at satisfies `ready`; its value, or ~0 after
+// the time limit (or another block's error).
+template <class Ready>
+__device__ __forceinline__ unsigned long long team_wait(const unsigned long long *at, int *status,
+                                                        long long timeout_ns, Ready ready) {
+  long long t0 = 0;
+  unsigned spins = 0;
+  unsigned long long x;
+  while (true) {
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(x) : "l"(at) : "memory");
+    if (ready(x)) break;
+    if ((++spins & 255u) == 0) {
+      if (t0 == 0) t0 = global_ns();
+      if (*(volatile int *)status != 0 || global_ns() - t0 > timeout_ns) {
+        atomicCAS(status, 0, (int)CG_ERR_TIMEOUT);
+        return ~0ull;
+      }
+    }
+  }
+  asm volatile("fence.acq_rel.gpu;" ::: "memory");
+  return x;
+}
+
+// The team's rounds from L on, its frontier the first cnt entries of
+// team_list(L).  Every block of the team calls with the same ss, and all take
+// the same decisions from the sums of TeamRound; ends with the frontier of the
+// round to run next listed again.  Returns its payload (all threads), with the
+// frontier's edges (saturated) and L in S.warp_total[1] and [2].
+__device__ __noinline__ unsigned team_rounds(const BfsParams &p, SearchState &ss, unsigned cnt,
+                                             int L) {
+  SoloShared &S = s_round.solo;
+  TeamCtl *T = &p.ctl->team;
+  const unsigned team = team_size(), rank = team_rank();
+  const bool leader = threadIdx.x == 0;
+  // sum: 8 bits of arrivals, 8 of blocks that overflowed, 8 of blocks with too
+  // many out-degrees for their 20 bits, 23 of out-degrees, 17 of vertices
+  constexpr unsigned kMfBits = 23, kNfBits = 17;
+  static_assert(kTeamEdges < (1u << kNfBits), "a round's claims fit");
+  static_assert(kMfBits + kNfBits <= 40, "flags above");
+  const unsigned lo = (unsigned)((unsigned long long)cnt * rank / team);
+  unsigned mine = (unsigned)((unsigned long long)cnt * (rank + 1) / team) - lo;
+  {
+    const int32_t *list = team_list(p, L) + lo;
+    for (unsigned i = threadIdx.x; i < mine; i += blockDim.x) solo_load(p, S, i, __ldcg(list + i));
+  }
+  __syncthreads();
+  int c = 0;
+  unsigned payload;
+  for (int ran = 1;; ++ran) {
+    const uint32_t E = solo_scan(S, c, mine);
+    if (leader) S.n = S.mf = 0;
+    __syncthreads();
+    solo_expand<true>(p, S, c, mine, E, L, team_list(p, L + 1));
+    __syncthreads();
+    if (leader) {
+      const unsigned nf = S.n, mf = S.mf;
+      const bool over = nf > (unsigned)kSoloMax, many = mf >= (1u << kMfBits) / kTeam;
+      TeamRound *R = &T->round[L & 3];
+      if (rank == 0) {  // its readers were done before the last round's arrivals
+        TeamRound *Z = &T->round[(L + 2) & 3];
+        Z->sum = Z->mf = 0;
+      }
+      if (many) atomicAdd(&R->mf, (unsigned long long)mf);
+      const unsigned long long add = (1ull << 56) | ((unsigned long long)over << 48) |
+                                     ((unsigned long long)many << 40) |
+                                     ((unsigned long long)(many ? 0u : mf) << kNfBits) | nf;
+      asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&R->sum), "l"(add) : "memory");
+      const unsigned long long x =
+          team_wait(&R->sum, &p.ctl->status, p.timeout_ns,
+                    [&](unsigned long long s) { return (unsigned)(s >> 56) >= team; });
+      unsigned pay = kWaitFailed;
+      if (x != ~0ull) {
+        const unsigned long long nfs = x & ((1ull << kNfBits) - 1);
+        unsigned long long mfs = (x >> kNfBits) & ((1ull << kMfBits) - 1);
+        if ((x >> 40) & 0xffu) mfs += __ldcg(&R->mf);
+        const bool lists_fit = ((x >> 48) & 0xffu) == 0;
+        pay = close_round(p, L, kPush, nfs, mfs, mfs, lists_fit ? kTeam * kSoloMax / 2 : 0u,
+                          kTeamEdges, ss);
+        S.d[c][0] = (uint32_t)min(mfs, 0xffffffffull);  // F_L's degrees are done with
+        // hand back what one block runs faster
+        S.x[0] = mfs < kTeamLeave && nfs <= (unsigned)kSoloMax / 2;
+      }
+      S.payload = pay;
+    }
+    __syncthreads();
+    payload = S.payload;
+    const uint32_t mf = S.d[c][0];
+    const bool small = S.x[0] != 0;
+    mine = min(S.n, (unsigned)kSoloMax);
+    c ^= 1;
+    ++L;
+    __syncthreads();  // S is read
+    if (payload == kWaitFailed || !(payload & kSolo) || small || ran >= kTeamSession) {
+      if (leader) {
+        S.warp_total[1] = mf;
+        S.warp_total[2] = (uint32_t)L;
+      }
+      break;
+    }
+  }
+  if (payload == kWaitFailed) return payload;
+  // list what this block claimed (past kSoloMax it is listed already)
+  if (leader) S.n = atomicAdd(&T->listed, mine);
+  __syncthreads();
+  int32_t *list = team_list(p, L) + S.n;
+  for (unsigned i = threadIdx.x; i < mine; i += blockDim.x) list[i] = S.v[c][i];
+  __syncthreads();
+  return payload;
+}
+
+// The lead's side of one hand-over: F_L (cnt vertices) is in team_list(L).
+// Returns the payload, with the next frontier's vertices, edges and round in
+// S.warp_total[0 .. 2].
+__device__ __noinline__ unsigned team_lead(const BfsParams &p, SearchState &ss, unsigned cnt, int L) {
+  SoloShared &S = s_round.solo;
+  BfsCtl *ctl = p.ctl;
+  TeamCtl *T = &ctl->team;
+  if (threadIdx.x == 0) {
+    SoloExit *x = &ctl->solo;
+    x->visited = ss.visited;
+    x->prev_nf = ss.prev_nf;
+    x->explored = ss.explored;
+    x->pull_rounds = ss.pull_rounds;
+    x->switches = ss.switches;
+    T->L = L;
+    T->cnt = cnt;
+    T->listed = T->back = 0;
+    // the first round's record; the second's is cleared by the first, and so on
+    for (int k = 0; k < 2; ++k) T->round[(L + k) & 3].sum = T->round[(L + k) & 3].mf = 0;
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&T->command) : "memory");
+  }
+  __syncthreads();
+  const unsigned payload = team_rounds(p, ss, cnt, L);
+  if (payload == kWaitFailed || (payload & kDone)) return payload;
+  if (threadIdx.x == 0) {
+    // every member's part of the list is written
+    const unsigned others = team_size() - 1;
+    const unsigned long long x = team_wait(
+        reinterpret_cast<const unsigned long long *>(&T->listed), &ctl->status, p.timeout_ns,
+        [&](unsigned long long w) { return (unsigned)(w >> 32) >= others; });
+    S.warp_total[0] = (unsigned)x;
+    S.payload = x == ~0ull ? kWaitFailed : payload;
+  }
+  __syncthreads();
+  return S.payload;
+}
+
+// A member's side of the lead block's run of small rounds: arrives at the
+// run's grid-wide waits, and serves the lead's commands while it waits.
+// False after a time limit (all threads).
+__device__ __noinline__ bool team_member(const BfsParams &p, SearchState &ss,
+                                         unsigned long long &target, unsigned &commands) {
+  SoloShared &S = s_round.solo;
+  BfsCtl *ctl = p.ctl;
+  TeamCtl *T = &ctl->team;
+  enum : unsigned { kPassed, kCommand, kFailed };
+  bool arrive = true;
+  while (true) {
+    if (threadIdx.x == 0) {
+      if (arrive) {
+        target += gridDim.x;
+        flat_arrive(&ctl->arrive);
+      }
+      const unsigned long long goal = target;
+      const unsigned seen = commands;
+      unsigned got = kFailed, spins = 0;
+      long long t0 = 0;
+      while (true) {
+        unsigned long long a;
+        unsigned w;
+        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(a) : "l"(&ctl->arrive) : "memory");
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(w) : "l"(&T->command) : "memory");
+        if (w != seen) { got = kCommand; break; }
+        if (a >= goal) { got = kPassed; break; }
+        __nanosleep(50);
+        if ((++spins & 255u) == 0) {
+          if (t0 == 0) t0 = global_ns();
+          if (*(volatile int *)&ctl->status != 0 || global_ns() - t0 > p.timeout_ns) {
+            atomicCAS(&ctl->status, 0, (int)CG_ERR_TIMEOUT);
+            break;
+          }
+        }
+      }
+      asm volatile("fence.acq_rel.gpu;" ::: "memory");
+      if (got == kCommand) {
+        const SoloExit *x = &ctl->solo;
+        commands = seen + 1;
+        ss.visited = __ldcg(&x->visited);
+        ss.prev_nf = __ldcg(&x->prev_nf);
+        ss.explored = __ldcg(&x->explored);
+        ss.pull_rounds = __ldcg(&x->pull_rounds);
+        ss.switches = __ldcg(&x->switches);
+        S.n = __ldcg(&T->cnt);
+        S.mf = (unsigned)__ldcg(&T->L);
+      }
+      // a wait of a run that goes on: the next one
+      S.payload = got == kPassed && __ldcg(&ctl->solo.still) != 0 ? ~0u : got;
+    }
+    __syncthreads();
+    const unsigned got = S.payload, cnt = S.n;
+    const int L = (int)S.mf;
+    __syncthreads();
+    arrive = got == ~0u;
+    if (arrive) continue;
+    if (got != kCommand) return got == kPassed;
+    if (team_rounds(p, ss, cnt, L) == kWaitFailed) return false;
+    if (threadIdx.x == 0)
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&T->back) : "memory");
   }
 }
 
@@ -1126,50 +1387,101 @@ __device__ __forceinline__ void solo_expand(const BfsParams &p, SoloShared &S, i
 // vertices, loaded and synchronised).  Ends with SoloExit written and the
 // barrier arrived at; returns the payload of the round to run next (every
 // thread), L being that round.
+template <bool kTeamed>
 __device__ __forceinline__ unsigned solo_rounds(const BfsParams &p, SoloShared &S, SearchState &ss,
                                                 unsigned long long &target, unsigned cnt, int &L,
-                                                uint32_t *cur) {
+                                                uint32_t *cur, unsigned payload) {
   BfsCtl *ctl = p.ctl;
   const bool leader = threadIdx.x == 0;
   const long long session_ns = p.timeout_ns / 4;
   long long t0 = leader ? global_ns() : 0;
   int c = 0, ran = 0;
-  unsigned payload = 0;
-  uint32_t E = solo_scan(S, c, cnt);
-  // a first frontier whose edges were not known may hold too many
-  bool stay = E <= kSoloEdges;
-  while (stay) {
-    if (leader) S.n = S.mf = 0;
-    __syncthreads();
-    // what does not fit goes to the queue F_{L+1} is not put in
-    solo_expand(p, S, c, cnt, E, L, (L & 1) ? p.queue1 : p.queue0);
-    __syncthreads();
-    if (leader) {
-      const unsigned nf = S.n, mf = S.mf;
-      // a frontier that more than doubled is left to the grid: the next one
-      // would be too large anyway, and the lists of new parts of the graph are
-      // cold (directed ER, 3,363 claims from 3,320 edges: 17 us here, 11 there)
-      const unsigned room = min(kSoloEdges, max(kSoloEdges / 4, 2 * E));
-      const unsigned x = close_round(p, L, kPush, nf, mf, mf, kSoloMax, room, ss);
-      if ((x & kSolo) && (++ran >= kSoloSession || ss.t_mark - t0 > session_ns)) {
-        // the waiting blocks' time limit: let them through to the next wait
-        ctl->solo.still = 1;
-        target += gridDim.x;
-        flat_arrive(&ctl->arrive);
-        ran = 0;
-        t0 = ss.t_mark;
-      }
-      S.payload = x;
-    }
-    __syncthreads();
-    payload = S.payload;
-    cnt = S.n;
-    c ^= 1;
-    ++L;
-    stay = (payload & kSolo) != 0;
-    if (stay) E = solo_scan(S, c, cnt);
+  [[maybe_unused]] int large = 0;  // rounds in a row of more than kTeamEnter edges
+  // F_L is in team_list(L), not in S
+  [[maybe_unused]] bool listed = kTeamed && (payload & kHandOver);
+  uint32_t E = 0;
+  bool stay = false;
+  if (!listed) {
+    payload = 0;
+    E = solo_scan(S, c, cnt);
+    // a first frontier whose edges were not known may hold too many
+    stay = E <= kSoloEdges;
   }
-  payload &= ~kSolo;
+  while (true) {
+    while (stay) {
+      if (leader) S.n = S.mf = 0;
+      __syncthreads();
+      // what does not fit goes to the queue F_{L+1} is not put in
+      solo_expand<false>(p, S, c, cnt, E, L, (L & 1) ? p.queue1 : p.queue0);
+      __syncthreads();
+      if (leader) {
+        const unsigned nf = S.n, mf = S.mf;
+        // a frontier that more than doubled is left to the grid: the next one
+        // would be too large anyway, and the lists of new parts of the graph are
+        // cold (directed ER, 3,363 claims from 3,320 edges: 17 us here, 11 there)
+        const unsigned room = min(kSoloEdges, max(kSoloEdges / 4, 2 * E));
+        unsigned x = close_round(p, L, kPush, nf, mf, mf, kSoloMax, room, ss);
+        if ((x & kSolo) && (++ran >= kSoloSession || ss.t_mark - t0 > session_ns)) {
+          // the waiting blocks' time limit: let them through to the next wait
+          ctl->solo.still = 1;
+          target += gridDim.x;
+          flat_arrive(&ctl->arrive);
+          ran = 0;
+          t0 = ss.t_mark;
+        }
+        if constexpr (kTeamed) {
+          large = mf > kTeamEnter ? large + 1 : 0;
+          if ((x & kSolo) && large >= kTeamAfter && team_size()) {
+            x |= kHandOver;
+            large = 0;
+          }
+        }
+        S.payload = x;
+      }
+      __syncthreads();
+      payload = S.payload;
+      cnt = S.n;
+      c ^= 1;
+      ++L;
+      stay = (payload & (kSolo | kHandOver)) == kSolo;
+      if (stay) E = solo_scan(S, c, cnt);
+    }
+    if constexpr (!kTeamed) {
+      break;
+    } else {
+      if (!(payload & kHandOver)) break;
+      if (!listed) {
+        int32_t *list = team_list(p, L);
+        for (unsigned i = threadIdx.x; i < cnt; i += blockDim.x) list[i] = S.v[c][i];
+        listed = true;
+      }
+      do {
+        __syncthreads();
+        payload = team_lead(p, ss, cnt, L);
+        if (payload == kWaitFailed) return kWaitFailed;
+        cnt = S.warp_total[0];
+        E = S.warp_total[1];
+        L = (int)S.warp_total[2];
+        if (leader && (payload & kSolo) && ss.t_mark - t0 > session_ns) {
+          ctl->solo.still = 1;
+          target += gridDim.x;
+          flat_arrive(&ctl->arrive);
+          ran = 0;
+          t0 = ss.t_mark;
+        }
+      } while ((payload & kSolo) && !(E < kTeamLeave && cnt <= (unsigned)kSoloMax / 2));
+      if (!(payload & kSolo)) break;
+      // small again: back to this block alone
+      const int32_t *list = team_list(p, L);
+      c = 0;
+      for (unsigned i = threadIdx.x; i < cnt; i += blockDim.x) solo_load(p, S, i, __ldcg(list + i));
+      __syncthreads();
+      E = solo_scan(S, c, cnt);
+      listed = false;
+      stay = true;
+    }
+  }
+  payload &= ~(kSolo | kHandOver);
   // every other block has arrived: the bitmaps are clear, the records unread
   if (leader)
     S.payload = flat_wait(&ctl->arrive, target + gridDim.x - 1, &ctl->status, p.timeout_ns)
@@ -1190,7 +1502,10 @@ __device__ __forceinline__ unsigned solo_rounds(const BfsParams &p, SoloShared &
       int32_t v = 0;
       int64_t d = 0;
       if (has) {
-        v = i < (unsigned)kSoloMax ? S.v[c][i] : spill[i];
+        if constexpr (kTeamed)
+          v = !listed && i < (unsigned)kSoloMax ? S.v[c][i] : __ldcg(spill + i);
+        else
+          v = i < (unsigned)kSoloMax ? S.v[c][i] : spill[i];
         d = __ldg(p.out_off + v + 1) - __ldg(p.out_off + v);
         atomicOr(cur + ((uint32_t)v >> 5), 1u << (v & 31));
       }
@@ -1267,7 +1582,8 @@ __device__ __noinline__ void copy_to_host(const BfsParams &p) {
   }
 }
 
-__global__ void __launch_bounds__(kBfsBlock, 3) bfs_persistent(BfsParams p) {
+template <bool kTeamed>
+__device__ __forceinline__ void search(const BfsParams &p) {
   __shared__ unsigned s_payload;
   __shared__ int s_L;
   BfsCtl *ctl = p.ctl;
@@ -1325,6 +1641,7 @@ __global__ void __launch_bounds__(kBfsBlock, 3) bfs_persistent(BfsParams p) {
   if (threadIdx.x == 0) {
     const unsigned long long target = gridDim.x;
     s_target = target;
+    if constexpr (kTeamed) s_commands = 0;
     // the test hook expects one arrival more than the grid has: it must time out
     const bool ok0 = flat_barrier(&ctl->arrive, target + (p.unmatched_wait ? 1u : 0u),
                                   &ctl->status, p.timeout_ns);
@@ -1349,6 +1666,7 @@ __global__ void __launch_bounds__(kBfsBlock, 3) bfs_persistent(BfsParams p) {
   uint32_t *fr0 = p.fr0, *fr1 = p.fr1, *fr2 = p.fr2;
   int dir = kPush;
   bool heavy = false;
+  [[maybe_unused]] bool hand = false;  // a small round for the team
   bool queued = true;  // F_L is in a queue (a pull round leaves it in the bitmap only)
   int L = 0;
   Acc acc;
@@ -1378,9 +1696,15 @@ __global__ void __launch_bounds__(kBfsBlock, 3) bfs_persistent(BfsParams p) {
         if (from_queue) {
           const int32_t *q = (L & 1) ? p.queue1 : p.queue0;
           const unsigned nl = ss.next_light, nb = (unsigned)(ss.next_big >> 32);
-          cnt = nl + nb;  // at most kSoloMax / 2
-          for (unsigned i = threadIdx.x; i < cnt; i += blockDim.x)
-            solo_load(p, S, i, i < nl ? q[i] : q[p.n - 1 - (int64_t)(i - nl)]);
+          cnt = nl + nb;  // at most kSoloMax / 2 (kTeam * kSoloMax / 4 handed over)
+          int32_t *list = team_list(p, L);
+          for (unsigned i = threadIdx.x; i < cnt; i += blockDim.x) {
+            const int32_t v = i < nl ? q[i] : q[p.n - 1 - (int64_t)(i - nl)];
+            if (kTeamed && hand)
+              list[i] = v;
+            else
+              solo_load(p, S, i, v);
+          }
         } else if (fold) {
           cnt = __ldcg(&ctl->solo.listed);
           for (unsigned i = threadIdx.x; i < cnt; i += blockDim.x)
@@ -1389,14 +1713,24 @@ __global__ void __launch_bounds__(kBfsBlock, 3) bfs_persistent(BfsParams p) {
           solo_load(p, S, 0, root);
         }
         __syncthreads();
-        const unsigned payload = solo_rounds(p, S, ss, s_target, cnt, L, fr0);
+        const unsigned payload = solo_rounds<kTeamed>(p, S, ss, s_target, cnt, L, fr0, hand ? kHandOver : 0u);
         if (threadIdx.x == 0) s_payload = payload;
         __syncthreads();
       } else {
+        if (kTeamed && in_team()) {
+          // (ends with the last wait of the run still to make)
+          const bool served = team_member(p, ss, s_target, s_commands);
+          __syncthreads();
+          if (!served) {
+            if (threadIdx.x == 0) s_payload = kWaitFailed;
+            __syncthreads();
+            break;
+          }
+        }
         if (threadIdx.x == 0) {
           const SoloExit *x = &ctl->solo;
-          bool arrived;
-          do {
+          bool arrived = true;
+          if (!(kTeamed && in_team())) do {
             const unsigned long long target = s_target + gridDim.x;
             s_target = target;
             flat_arrive(&ctl->arrive);
@@ -1474,7 +1808,7 @@ __global__ void __launch_bounds__(kBfsBlock, 3) bfs_persistent(BfsParams p) {
       // lane 0's acquire fence, then this warp barrier, order the other lanes'
       // counter loads after every block's arrival
       arrived = __shfl_sync(kFull, arrived, 0);
-      const unsigned payload = arrived ? round_decision(p, L, dir, ss) : kWaitFailed;
+      const unsigned payload = arrived ? round_decision<kTeamed>(p, L, dir, ss) : kWaitFailed;
       if (threadIdx.x == 0) s_payload = payload;
     }
     __syncthreads();
@@ -1484,6 +1818,7 @@ __global__ void __launch_bounds__(kBfsBlock, 3) bfs_persistent(BfsParams p) {
     dir = (payload & kNextPull) ? kPull : kPush;
     heavy = (payload & kHeavy) != 0;
     solo = (payload & kSolo) != 0;
+    if constexpr (kTeamed) hand = (payload & kHandOver) != 0;
     uint32_t *t = fr2;  // rotate: F_{L+1} becomes the frontier
     fr2 = fr0;
     fr0 = fr1;
@@ -1493,6 +1828,17 @@ __global__ void __launch_bounds__(kBfsBlock, 3) bfs_persistent(BfsParams p) {
   if (leader && s_payload == kWaitFailed) p.stats->status = *(volatile int *)&ctl->status;
   // after the last wait every output is final
   if (s_payload != kWaitFailed && (p.host_levels || p.host_parents)) copy_to_host(p);
+}
+
+__global__ void __launch_bounds__(kBfsBlock, 3) bfs_persistent(BfsParams p) { search<false>(p); }
+
+// The same search with rounds that a team runs.  A kernel of its own, so that
+// the other keeps its registers (with the team in it R-MAT and random graphs took
+// 2 to 3% longer), and of fewer threads, so that it has 56 without spills and
+// three handles' blocks still fit an SM: 512 threads and 64 registers are as fast
+// for one handle, 4.6 ms a search for three taking turns where this takes 3.3.
+__global__ void __launch_bounds__(kTeamBlock, 3) bfs_persistent_team(BfsParams p) {
+  search<true>(p);
 }
 
 // A vertex's share of Graph500's m (bfs_timing.py:379-398): its entries c <= v
@@ -1569,9 +1915,9 @@ int64_t bfs_big_capacity(int64_t n, int64_t nnz) {
 // hub_edges: entries of vertices of in-degree > kLightMax.
 __global__ void dead_map_kernel(int64_t n, int64_t words, const int64_t *__restrict__ in_off,
                                 uint32_t *dead, unsigned long long *live,
-                                unsigned long long *hub_edges) {
+                                unsigned long long *hub_edges, unsigned long long *wide_edges) {
   const int lane = lane_id();
-  unsigned long long alive = 0, hubs = 0;
+  unsigned long long alive = 0, hubs = 0, wide = 0;
   const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t w0 = (int64_t)warp_id_global() * 32; w0 < words; w0 += warps * 32) {
     uint32_t mine = 0;
@@ -1579,6 +1925,7 @@ __global__ void dead_map_kernel(int64_t n, int64_t words, const int64_t *__restr
       const int64_t v = (w0 + j) * 32 + lane;
       const int64_t d = v < n ? __ldg(in_off + v + 1) - __ldg(in_off + v) : 0;
       if (d > kLightMax) hubs += (unsigned long long)d;
+      if (d > kTeamDegree) wide += (unsigned long long)d;
       const uint32_t m = __ballot_sync(kFull, d == 0);
       if (lane == j) mine = m;
     }
@@ -1587,8 +1934,10 @@ __global__ void dead_map_kernel(int64_t n, int64_t words, const int64_t *__restr
   }
   alive = warp_sum(alive);
   hubs = warp_sum(hubs);
+  wide = warp_sum(wide);
   if (lane == 0 && alive) atomicAdd(live, alive);
   if (lane == 0 && hubs) atomicAdd(hub_edges, hubs);
+  if (lane == 0 && wide) atomicAdd(wide_edges, wide);
 }
 
 // Each vertex's first in-neighbour and in-degree (of one without, zeros).
@@ -1624,7 +1973,7 @@ int bfs_prepare(cg_graph *g) {
   };
   const size_t at_ctl = piece(sizeof(BfsCtl));
   const size_t at_stats = piece(sizeof(cg_stats));
-  const size_t at_live = piece(2 * sizeof(unsigned long long));  // and the hubs' entries
+  const size_t at_live = piece(3 * sizeof(unsigned long long));  // and entries by in-degree
   const size_t zeroed = bytes;
   const size_t at_bitmaps = piece(sizeof(uint32_t) * 4 * (size_t)stride);
   const size_t at_dead = piece(sizeof(uint32_t) * (size_t)stride);
@@ -1646,11 +1995,11 @@ int bfs_prepare(cg_graph *g) {
   g->queue = reinterpret_cast<int32_t *>(base + at_queue);
   g->bigoff = reinterpret_cast<uint32_t *>(base + at_bigoff);
   unsigned long long *d_live = reinterpret_cast<unsigned long long *>(base + at_live);
-  unsigned long long live[2] = {0, 0};
+  unsigned long long live[3] = {0, 0, 0};
   CG_CUDA(cudaMemsetAsync(base, 0, zeroed, g->stream));
   const int64_t blocks = (stride + 255) / 256;  // 8 warps of 32 words
   dead_map_kernel<<<(unsigned)(blocks < 4096 ? blocks : 4096), 256, 0, g->stream>>>(
-      g->n, stride, g->in_off, g->dead, d_live, d_live + 1);
+      g->n, stride, g->in_off, g->dead, d_live, d_live + 1, d_live + 2);
   CG_CUDA(cudaGetLastError());
   CG_CUDA(cudaMemcpyAsync(live, d_live, sizeof(live), cudaMemcpyDeviceToHost, g->stream));
   CG_CUDA(cudaStreamSynchronize(g->stream));
@@ -1669,6 +2018,13 @@ int bfs_prepare(cg_graph *g) {
       g->head = nullptr;
     }
   }
+  // Meshes, grids and road networks, which take hundreds of rounds of slowly
+  // changing frontiers: bounded degrees, and enough vertices for a frontier of
+  // kTeamEnter edges that is as deep as it is wide (below, one block runs every
+  // round: a 200^2 grid takes 1,090 us with either kernel, 1,125 on some GPUs
+  // with the team's).
+  g->team = g->n >= kTeamVertices && g->nnz > 0 &&
+            1024 * live[2] <= (unsigned long long)g->nnz;
   g->live = (int64_t)live[0];
   return CG_OK;
 }
@@ -1693,10 +2049,12 @@ static int blocks_for(const cg_graph *g) {
 static int bfs_grid(cg_graph *g) {
   int block = g->opt.block_size > 0 ? g->opt.block_size : kBfsBlock;
   if (block > kBfsBlock) block = kBfsBlock;
+  if (g->team && block > kTeamBlock) block = kTeamBlock;
   block = (block / 32) * 32;
   if (block < 64) block = 64;
   int per_sm = 0;
-  CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bfs_persistent, block, 0));
+  CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+      &per_sm, g->team ? bfs_persistent_team : bfs_persistent, block, 0));
   if (per_sm <= 0) return CG_ERR_NOT_SUPPORTED;
   const int want = g->opt.blocks_per_sm > 0 ? g->opt.blocks_per_sm : blocks_for(g);
   if (want < per_sm) per_sm = want;
@@ -1759,7 +2117,7 @@ int bfs_launch(cg_graph *g, int64_t root, int32_t *d_levels, int32_t *d_parents,
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  CG_CUDA(cudaLaunchKernelEx(&cfg, bfs_persistent, p));
+  CG_CUDA(cudaLaunchKernelEx(&cfg, g->team ? bfs_persistent_team : bfs_persistent, p));
   return CG_OK;
 }
 

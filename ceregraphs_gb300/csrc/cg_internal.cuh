@@ -90,6 +90,23 @@ struct SoloExit {
   unsigned pad[17];
 };
 
+// The team of blocks that runs small rounds too large for one block: the lead's
+// command (a count that members compare with theirs), the frontier list's
+// length, and per round (four records in turn) the members' sums.
+struct TeamRound {
+  unsigned long long sum;      // arrivals, flags, out-degrees, vertices (team_rounds)
+  unsigned long long mf;       // out-degrees, exact
+  unsigned long long pad[14];
+};
+struct TeamCtl {
+  unsigned command, cnt;       // runs handed out; vertices of the frontier in the list
+  int L;
+  unsigned pad0[29];
+  unsigned listed, back;       // vertices listed for the next hand-out; members done
+  unsigned pad1[30];
+  TeamRound round[4];
+};
+
 // Control block of one per-root search, zeroed before every launch.  The
 // search-wide bookkeeping (visited total, explored edges, ...) is not here:
 // every block keeps its own copy, updated from the same round totals.
@@ -99,6 +116,7 @@ struct BfsCtl {
   int status;                  // first error (CG_ERR_TIMEOUT, CG_ERR_LEVEL_CAP), else 0
   int pad1[31];
   SoloExit solo;
+  TeamCtl team;
   RoundRec rec[kRing];
 };
 
@@ -158,6 +176,7 @@ struct cg_graph {
   uint32_t *bitmaps = nullptr;  // vis | fr0 | fr1 | fr2, 4 * bitmap_stride(n)
   uint32_t *dead = nullptr;     // 1 bit per vertex: no in-edges, bitmap_stride(n) words
   int64_t live = 0;             // vertices with in-edges
+  bool team = false;            // searches run bfs_persistent_team
   uint2 *head = nullptr;        // [n] first in-neighbour and in-degree (null: no memory)
   // cg_graph_reorder: resident vertex v is original vertex orig[v]; perm is
   // the inverse (both int32[n], null for a graph in its original order)
