@@ -39,7 +39,7 @@ METRIC = "per-root BFS GTEPS, harmonic mean over the Graph500 roots"
 # DRAM bytes (read + write) per launch of bfs_persistent measured with ncu
 # (dram__bytes_read.sum + dram__bytes_write.sum, mean over the timed step's
 # launches) for (scale, edgefactor, seed, root seed); roofline.traffic.
-NCU_TRAFFIC_BYTES = {(21, 16, 0, 1): 80.5e6, (23, 16, 2, 3): 541.0e6}
+NCU_TRAFFIC_BYTES = {(21, 16, 0, 1): 50.8e6, (23, 16, 2, 3): 413.7e6}
 FALLBACK_HBM_GBS = 6800.0
 
 
@@ -461,11 +461,11 @@ def run_ours(args):
                "lanes": lanes, "rounds": stb["rounds"],
                "pull_rounds": stb["pull_rounds"], "bit_exact_vs_per_root": same,
                "roofline": roofline(bk / (batch_ms * 1e-3) / 1e9, None,
-                                    "msbfs_ledger + msbfs_scan + msbfs_outputs + msbfs_fixup",
+                                    "msbfs_ledger + msbfs_scan + msbfs_outputs",
                                     "B_k = 4*nnz + 8*(n+1) + rounds*2*n*lanes/8 + 8*n*k per "
                                     "batch"),
                "launch": "per 64/128 roots: the rounds (one cooperative kernel), then the "
-                         "scan, output and fix-up passes, replayed as one CUDA graph"}
+                         "scan and output passes, replayed as one CUDA graph"}
   clocks = sampler.stop()
 
   gteps_dev = m / (per_root_ms * 1e-3) / 1e9
@@ -574,7 +574,7 @@ def run_uneven(args):
     torch.cuda.synchronize()
     st = g.last_stats()
     batch_ms = e0.elapsed_time(e1) / args.steps
-    launches += args.steps * ((k + lanes - 1) // lanes) * 5
+    launches += args.steps * ((k + lanes - 1) // lanes) * 4
     m = g.count_edges(d_lv, k)
     # every lane of the first batch through the device tree checks
     first = min(k, lanes)
