@@ -1872,7 +1872,7 @@ __global__ void edge_weight_kernel(int64_t n, int symmetric, const int64_t *__re
 // search, and kept with it (`w`; null when there was no memory for them: then
 // they are found here).  A sum of weights stays below nnz < 2^32.  The rest is
 // one read of the levels.  R-MAT scale 20, 16 searches: 158 us with a
-// search per vertex and search, 64 us now.
+// search per vertex and search, 64 us with kept weights, 21 us now.
 constexpr int kCountGroup = 16;
 __global__ void __launch_bounds__(256) count_edges_kernel(
     int64_t n, int k, int symmetric, const int64_t *__restrict__ in_off,
@@ -1896,10 +1896,21 @@ __global__ void __launch_bounds__(256) count_edges_kernel(
     for (int s = 0; s < kCountGroup; ++s)
       if (lv[s] >= 0) local[s] += x;
   }
+  // (32 bits hold the sums: a search's m is at most nnz.)  One atomic a block and
+  // search, a block's in one request: the totals share a line, and one from each
+  // warp, about 1 ns apart, took 43 of the 64 us
+  __shared__ unsigned part[8][kCountGroup];
 #pragma unroll
   for (int s = 0; s < kCountGroup; ++s) {
     const unsigned x = __reduce_add_sync(kFull, local[s]);
-    if ((threadIdx.x & 31) == 0 && x) atomicAdd(m_out + s0 + s, (unsigned long long)x);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5][s] = x;
+  }
+  __syncthreads();
+  if (threadIdx.x < (unsigned)ks) {
+    unsigned x = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x += part[i][threadIdx.x];
+    if (x) atomicAdd(m_out + s0 + threadIdx.x, (unsigned long long)x);
   }
 }
 
@@ -2136,7 +2147,7 @@ int count_edges_launch(cg_graph *g, const int32_t *d_levels, int32_t k,
     }
   }
   CG_CUDA(cudaMemsetAsync(d_m, 0, sizeof(unsigned long long) * (size_t)k, g->stream));
-  const int64_t blocks = (g->n + 255) / 256, cap = (int64_t)g->num_sms * 4;
+  const int64_t blocks = (g->n + 255) / 256, cap = (int64_t)g->num_sms * 8;
   count_edges_kernel<<<dim3((unsigned)(blocks < cap ? blocks : cap),
                             (k + kCountGroup - 1) / kCountGroup),
                        256, 0, g->stream>>>(g->n, k, sym, g->in_off, g->in_idx, g->out_off,
