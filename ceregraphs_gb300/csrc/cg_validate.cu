@@ -77,7 +77,7 @@ __device__ __forceinline__ bool contains(const int32_t *__restrict__ idx, int64_
 // instructions per 32 entries and 16 searches, and lists of uneven lengths in a
 // warp) and by the latency of the 4 * NW byte gathers, which the L2 serves.
 // R-MAT scale 20, 16 searches, device time: 6670 us for the two per-search
-// kernels, 540 us for these (packing 12, vertices 331, long lists 196).
+// kernels, 535 us for these (packing 12, vertices 330, long lists 193).
 constexpr uint32_t kHigh = 0x80808080u, kOnes = 0x01010101u;
 constexpr int kUnreached = 127, kMaxLevel = 125;
 constexpr int kGroup = 16;          // searches of a group at most
@@ -127,6 +127,11 @@ __device__ __forceinline__ uint32_t bound_of(uint32_t b) {
   return (b - kOnes + unreached) | kHigh;
 }
 
+// The low four bits of m as bit 7 of a byte each.
+__device__ __forceinline__ uint32_t byte_flags(unsigned m) {
+  return ((m & 0xfu) * 0x00204081u & kOnes) << 7;
+}
+
 template <int NW>
 __global__ void __launch_bounds__(kBlock) pack_levels_kernel(GroupArgs a) {
   const int64_t v = (int64_t)blockIdx.x * kBlock + threadIdx.x;
@@ -156,12 +161,54 @@ __device__ __noinline__ void flag_edges(const GroupArgs &a, const uint32_t (&m)[
     if ((m[s >> 2] >> (8 * (s & 3) + 7)) & 1u) flag(a.tally + s, CG_CHECK_EDGES, v);
 }
 
+// Searches in which v is reached, below its root (bit 7 of each byte), from
+// bound_of: t is 1 .. 126.
+__device__ __forceinline__ uint32_t below_root(uint32_t th) {
+  const uint32_t t = th & ~kHigh;
+  return (t + ~kHigh) & ~(t + kOnes) & kHigh;
+}
+
+// v's t (level, or 127) in search s, s the lane's own.
+template <int NW>
+__device__ __forceinline__ int level_of(const uint32_t (&th)[NW], int s) {
+  uint32_t x = 0;
+#pragma unroll
+  for (int w = 0; w < NW; ++w)
+    if ((s >> 2) == w) x = th[w];
+  return (int)((x >> (8 * (s & 3))) & 0x7fu);
+}
+
+// The checks of v's own level t and parent p in search s (SPAN, ROOT and what
+// TREE needs no other vertex for).  True if p is a vertex to look for among v's
+// in-neighbours.
+__device__ __forceinline__ bool check_vertex(const GroupArgs &a, int s, int64_t v, int t,
+                                             int32_t p) {
+  const bool reached = t != kUnreached;
+  if (reached != (p >= 0)) flag(a.tally + s, CG_CHECK_SPAN, v);
+  if (v == __ldg(a.roots + s)) {
+    if (p != (int32_t)v || t != 0) flag(a.tally + s, CG_CHECK_ROOT, v);
+    return false;
+  }
+  if (p >= 0 && reached && t > 0 && p < a.n) return true;
+  if (p >= 0 || p < -1) flag(a.tally + s, CG_CHECK_TREE, v);
+  return false;
+}
+
+// p is one level up from v in search s (TREE).
+template <int NW>
+__device__ __forceinline__ bool one_up(const GroupArgs &a, int s, int64_t v, int t, int32_t p) {
+  if (__ldg(reinterpret_cast<const uint8_t *>(a.lv) + (int64_t)p * (4 * NW) + s) == t) return true;
+  flag(a.tally + s, CG_CHECK_TREE, v);
+  return false;
+}
+
 // The first in-neighbour of v one level up in search s is u (-1: none), its
-// parent is p, and p is one level up: u is p unless p is not in the list or a
-// lower one precedes it.
+// parent is p: where they are the same, p is one level up, in the list and the
+// lowest, and its level is not read.
+template <int NW>
 __device__ __forceinline__ void check_first(const GroupArgs &a, int s, int64_t v, int64_t b,
-                                            int64_t e, int32_t u, int32_t p) {
-  if (u == p) return;
+                                            int64_t e, int t, int32_t u, int32_t p) {
+  if (u == p || !one_up<NW>(a, s, v, t, p)) return;
   flag(a.tally + s, CG_CHECK_LOWEST, v);
   if (!contains(a.in_idx, b, e, p)) flag(a.tally + s, CG_CHECK_TREE_EDGE, v);
 }
@@ -229,9 +276,10 @@ __device__ __forceinline__ int32_t warp_entries(const GroupArgs &a, int64_t v, i
 }
 
 // Every check of the group's searches, one warp per 32 consecutive vertices:
-// the per-vertex checks by a lane each, short in-lists by their lane (four
-// entries' loads in flight), middling ones by the warp; long ones go on a
-// list for check_long_kernel.
+// short in-lists by their lane (four entries' loads in flight), middling ones by
+// the warp; long ones go on a list for check_long_kernel.  Parents are read
+// once, after the list: the level of one that is the list's first vertex a level
+// up needs no look (16 M byte gathers less, 338 -> 330 us).
 template <int NW>
 __global__ void __launch_bounds__(kBlock, 4) check_vertices_kernel(GroupArgs a) {
   if (*(volatile int *)a.wide) return;
@@ -240,7 +288,7 @@ __global__ void __launch_bounds__(kBlock, 4) check_vertices_kernel(GroupArgs a) 
   uint32_t th[NW], pend[NW];
   int64_t b = 0, e = 0;
 #pragma unroll
-  for (int w = 0; w < NW; ++w) th[w] = kHigh, pend[w] = 0;
+  for (int w = 0; w < NW; ++w) th[w] = ~0u, pend[w] = 0;
   if (v < a.n) {
     uint32_t mine[NW];
     ld_words<NW>(a.lv, v, mine);
@@ -249,47 +297,16 @@ __global__ void __launch_bounds__(kBlock, 4) check_vertices_kernel(GroupArgs a) 
 #pragma unroll
     for (int w = 0; w < NW; ++w) {
       th[w] = bound_of(mine[w]);
-      int32_t p[4];
-      int up[4];  // the parent's level byte (0: out of range)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int s = 4 * w + j;
-        p[j] = s < a.searches ? __ldg(a.parents + (int64_t)s * a.n + v) : -1;
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        up[j] = p[j] >= 0 && p[j] < a.n
-                    ? __ldg(reinterpret_cast<const uint8_t *>(a.lv) + (int64_t)p[j] * (4 * NW) +
-                            4 * w + j)
-                    : 0;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int s = 4 * w + j;
-        if (s >= a.searches) continue;
-        const int bv = (int)((mine[w] >> (8 * j)) & 0xffu);  // level + 1, 127 unreached
-        const bool reached = bv != kUnreached;
-        if (reached != (p[j] >= 0)) flag(a.tally + s, CG_CHECK_SPAN, v);
-        if (v == __ldg(a.roots + s)) {
-          if (p[j] != (int32_t)v || bv != 1) flag(a.tally + s, CG_CHECK_ROOT, v);
-        } else if (p[j] >= 0) {
-          // level >= 1 and the parent one level up: b(p) = level(v) = b(v) - 1
-          if (!reached || bv < 2 || up[j] != bv - 1)
-            flag(a.tally + s, CG_CHECK_TREE, v);
-          else
-            pend[w] |= 0x80u << (8 * j);
-        } else if (p[j] < -1) {
-          flag(a.tally + s, CG_CHECK_TREE, v);
-        }
-      }
+      pend[w] = below_root(th[w]);
     }
   }
   const int64_t deg = e - b;
   if (deg <= kLaneList) {
     // each search's first entry one level up, as a list position in its byte
     // (no branch: every lane would take it at an entry of its own)
-    uint32_t at[NW], found[NW];
+    uint32_t at[NW];
 #pragma unroll
-    for (int w = 0; w < NW; ++w) at[w] = 0, found[w] = pend[w];
+    for (int w = 0; w < NW; ++w) at[w] = 0;
     for (int64_t j = b; j < e; j += 4) {
       int32_t u[4];
       uint32_t x[4][NW];
@@ -323,15 +340,27 @@ __global__ void __launch_bounds__(kBlock, 4) check_vertices_kernel(GroupArgs a) 
         }
       }
     }
+    if (v < a.n) {
 #pragma unroll
-    for (int w = 0; w < NW; ++w) {
-      found[w] &= ~pend[w];
+      for (int w = 0; w < NW; ++w) {
+        const uint32_t found = below_root(th[w]) & ~pend[w];
+        int32_t p[4], u[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int s = 4 * w + j;
-        if ((found[w] >> (8 * j + 7)) & 1u) {
-          const int32_t u = __ldg(a.in_idx + b + ((at[w] >> (8 * j)) & 0xffu));
-          check_first(a, s, v, b, e, u, __ldg(a.parents + (int64_t)s * a.n + v));
+        for (int j = 0; j < 4; ++j) {
+          const int s = 4 * w + j;
+          p[j] = s < a.searches ? __ldg(a.parents + (int64_t)s * a.n + v) : -1;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          u[j] = (found >> (8 * j + 7)) & 1u
+                     ? __ldg(a.in_idx + b + ((at[w] >> (8 * j)) & 0xffu))
+                     : -1;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int s = 4 * w + j;
+          const int t = (int)((th[w] >> (8 * j)) & 0x7fu);
+          if (s < a.searches && check_vertex(a, s, v, t, p[j]))
+            check_first<NW>(a, s, v, b, e, t, u[j], p[j]);
         }
       }
     }
@@ -349,43 +378,41 @@ __global__ void __launch_bounds__(kBlock, 4) check_vertices_kernel(GroupArgs a) 
       sth[w] = __shfl_sync(0xffffffffu, th[w], src);
       sp[w] = __shfl_sync(0xffffffffu, pend[w], src);
     }
-    // lane s: search s's parent and whether it is to be checked
+    // lane s: search s's parent
     const int32_t p = lane < a.searches ? __ldg(a.parents + (int64_t)lane * a.n + vv) : -1;
-    bool want = false;
-#pragma unroll
-    for (int w = 0; w < NW; ++w)
-      if ((lane >> 2) == w) want = (sp[w] >> (8 * (lane & 3) + 7)) & 1u;
     const int32_t u = warp_entries<NW>(a, vv, vb, ve, sth, sp);
-    if (want) check_first(a, lane, vv, vb, ve, u, p);
-    if (lane == src) {
-#pragma unroll
-      for (int w = 0; w < NW; ++w) pend[w] = 0;
-    }
-  }
-  if (deg <= kLaneList) {
-    // no in-neighbour one level up was seen: the parent is not in the list
-#pragma unroll
-    for (int w = 0; w < NW; ++w)
-      for (uint32_t m = pend[w]; m; m &= m - 1) {
-        const int s = 4 * w + ((__ffs(m) - 1) >> 3);
-        check_first(a, s, v, b, e, -1, __ldg(a.parents + (int64_t)s * a.n + v));
-      }
+    const int t = level_of<NW>(sth, lane);
+    if (lane < a.searches && check_vertex(a, lane, vv, t, p))
+      check_first<NW>(a, lane, vv, vb, ve, t, u, p);
   }
   const unsigned ml = __ballot_sync(0xffffffffu, deg > kWarpList);
-  if (!ml) return;
-  if (deg > kWarpList) {
-    // a parent that is not in a long list is found here; its chunks then only
-    // look for a lower one (the binary search is rare: few vertices)
+  // long lists: lane s checks search s's parent, in the list or not; the chunks
+  // then only look for a lower one
+  for (unsigned m = ml; m; m &= m - 1) {
+    const int src = __ffs(m) - 1;
+    const int64_t vb = __shfl_sync(0xffffffffu, b, src), ve = __shfl_sync(0xffffffffu, e, src);
+    const int64_t vv = v - lane + src;
+    uint32_t sth[NW];
 #pragma unroll
-    for (int w = 0; w < NW; ++w)
-      for (uint32_t m = pend[w]; m; m &= m - 1) {
-        const int s = 4 * w + ((__ffs(m) - 1) >> 3);
-        if (!contains(a.in_idx, b, e, __ldg(a.parents + (int64_t)s * a.n + v))) {
-          flag(a.tally + s, CG_CHECK_LOWEST, v);
-          flag(a.tally + s, CG_CHECK_TREE_EDGE, v);
-          pend[w] &= ~(m & (0u - m));
-        }
+    for (int w = 0; w < NW; ++w) sth[w] = __shfl_sync(0xffffffffu, th[w], src);
+    bool want = false;
+    if (lane < a.searches) {
+      const int32_t p = __ldg(a.parents + (int64_t)lane * a.n + vv);
+      const int t = level_of<NW>(sth, lane);
+      want = check_vertex(a, lane, vv, t, p) && one_up<NW>(a, lane, vv, t, p);
+      if (want && !contains(a.in_idx, vb, ve, p)) {
+        flag(a.tally + lane, CG_CHECK_LOWEST, vv);
+        flag(a.tally + lane, CG_CHECK_TREE_EDGE, vv);
+        want = false;
       }
+    }
+    const unsigned wanted = __ballot_sync(0xffffffffu, want);
+    if (lane == src) {
+#pragma unroll
+      for (int w = 0; w < NW; ++w) pend[w] = byte_flags(wanted >> (4 * w));
+    }
+  }
+  if (deg > kWarpList) {
     const unsigned chunks = (unsigned)((deg + kChunkList - 1) / kChunkList);
     // one packed add gives the entry's place and its first chunk, so the list
     // is sorted by first chunk
@@ -432,8 +459,7 @@ __global__ void __launch_bounds__(kBlock, 4) check_long_kernel(GroupArgs a) {
 #pragma unroll
     for (int w = 0; w < NW; ++w) {
       th[w] = bound_of(th[w]);
-      const uint32_t four = (below >> (4 * w)) & 0xfu;  // to bit 7 of a byte each
-      pend[w] = a.pend[(int64_t)lo * NW + w] & ((four * 0x00204081u & kOnes) << 7);
+      pend[w] = a.pend[(int64_t)lo * NW + w] & byte_flags(below >> (4 * w));
     }
     const int32_t u = warp_entries<NW>(a, v, b, e, th, pend);
     if (u < 0 || u >= par) continue;
