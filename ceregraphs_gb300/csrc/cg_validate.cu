@@ -82,8 +82,14 @@ constexpr uint32_t kHigh = 0x80808080u, kOnes = 0x01010101u;
 constexpr int kUnreached = 127, kMaxLevel = 125;
 constexpr int kGroup = 16;          // searches of a group at most
 constexpr int64_t kLaneList = 32;   // in-lists up to this: one thread
-constexpr int64_t kWarpList = 128;  // up to this: the warp that owns the vertex; above: chunks
-constexpr int64_t kChunkList = 512; // entries of a longer list per warp
+// Lists up to warp_list: the warp that owns the vertex; longer ones in chunks of
+// 1 << chunk_bits entries, a warp each.  Large graphs have warps enough for
+// longer pieces, whose set-up then counts less (16 searches, R-MAT, us with 128 and
+// 512 / 512 and 1024: 1 M 693 / 658, degree 32 693 / 601, 256 K 369 / 371, 16 K 198 /
+// 230).
+constexpr int64_t kWarpList = 128, kWarpListLarge = 512;
+constexpr int kChunkBits = 9, kChunkBitsLarge = 10;
+constexpr int64_t kLargeGraph = 1 << 19;
 
 // A vertex whose in-list is scanned in chunks: `base` is its first chunk.
 struct LongVertex {
@@ -106,6 +112,8 @@ struct GroupArgs {
   LongVertex *longs;
   uint32_t *pend;            // [longs][NW] searches whose parent is still to be checked
   uint32_t *bad;             // [longs][NW] searches already counted as LOWEST failures
+  int64_t warp_list;
+  int chunk_bits;
 };
 
 template <int NW>
@@ -365,8 +373,8 @@ __global__ void __launch_bounds__(kBlock, 4) check_vertices_kernel(GroupArgs a) 
       }
     }
   }
-  // lists of kLaneList + 1 .. kWarpList entries: the whole warp, one at a time
-  unsigned todo = __ballot_sync(0xffffffffu, deg > kLaneList && deg <= kWarpList);
+  // lists of kLaneList + 1 .. warp_list entries: the whole warp, one at a time
+  unsigned todo = __ballot_sync(0xffffffffu, deg > kLaneList && deg <= a.warp_list);
   while (todo) {
     const int src = __ffs(todo) - 1;
     todo &= todo - 1;
@@ -385,7 +393,7 @@ __global__ void __launch_bounds__(kBlock, 4) check_vertices_kernel(GroupArgs a) 
     if (lane < a.searches && check_vertex(a, lane, vv, t, p))
       check_first<NW>(a, lane, vv, vb, ve, t, u, p);
   }
-  const unsigned ml = __ballot_sync(0xffffffffu, deg > kWarpList);
+  const unsigned ml = __ballot_sync(0xffffffffu, deg > a.warp_list);
   // long lists: lane s checks search s's parent, in the list or not; the chunks
   // then only look for a lower one
   for (unsigned m = ml; m; m &= m - 1) {
@@ -412,8 +420,8 @@ __global__ void __launch_bounds__(kBlock, 4) check_vertices_kernel(GroupArgs a) 
       for (int w = 0; w < NW; ++w) pend[w] = byte_flags(wanted >> (4 * w));
     }
   }
-  if (deg > kWarpList) {
-    const unsigned chunks = (unsigned)((deg + kChunkList - 1) / kChunkList);
+  if (deg > a.warp_list) {
+    const unsigned chunks = (unsigned)((deg - 1) >> a.chunk_bits) + 1u;
     // one packed add gives the entry's place and its first chunk, so the list
     // is sorted by first chunk
     const unsigned long long old = atomicAdd(a.nlong, (1ull << 32) | chunks);
@@ -427,7 +435,7 @@ __global__ void __launch_bounds__(kBlock, 4) check_vertices_kernel(GroupArgs a) 
   }
 }
 
-// The listed vertices' in-lists, a warp per chunk of kChunkList entries.  The
+// The listed vertices' in-lists, a warp per chunk.  The
 // parents are known to be in the lists, so LOWEST fails exactly when a chunk
 // holds an entry one level up below the parent; `bad` counts it once.
 template <int NW>
@@ -447,9 +455,9 @@ __global__ void __launch_bounds__(kBlock, 4) check_long_kernel(GroupArgs a) {
         hi = mid - 1;
     }
     const int64_t v = a.longs[lo].v;
-    const int64_t b = __ldg(a.in_off + v) + (int64_t)(c - a.longs[lo].base) * kChunkList;
+    const int64_t b = __ldg(a.in_off + v) + ((int64_t)(c - a.longs[lo].base) << a.chunk_bits);
     const int64_t end = __ldg(a.in_off + v + 1);
-    const int64_t e = b + kChunkList < end ? b + kChunkList : end;
+    const int64_t e = min(b + ((int64_t)1 << a.chunk_bits), end);
     uint32_t th[NW], pend[NW];
     ld_words<NW>(a.lv, v, th);
     // lane s holds search s's parent; only the chunks that start below it can
@@ -690,6 +698,8 @@ extern "C" int cg_validate_device(cg_graph *g, const int64_t *roots, int32_t k,
       a.n = g->n;
       a.in_off = g->in_off;
       a.in_idx = g->in_idx;
+      a.warp_list = g->n >= kLargeGraph ? kWarpListLarge : kWarpList;
+      a.chunk_bits = g->n >= kLargeGraph ? kChunkBitsLarge : kChunkBits;
       for (int i = 0; i < groups; ++i) {
         const int64_t s0 = (int64_t)i * kGroup;
         a.roots = d_roots + s0;

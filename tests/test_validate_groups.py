@@ -81,3 +81,32 @@ def test_edge_counts_of_groups(built_lib, k):
       seen = L[i] >= 0
       want = int(np.sum(seen[dst] & (a.in_idx <= dst))) if a.symmetric else int(seen[a.in_idx].sum())
       assert got[i] == want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k", [4, 7, 16])
+def test_large_graph_matches_oracle(built_lib, oracle_mod, k):
+  # from 2^19 vertices on lists go to chunks later, and chunks are longer
+  import torch
+  from ceregraphs_gb300.engine import Graph
+  a = _degrees_graph((1 << 19) + 3, 5)
+  rng = np.random.default_rng(k)
+  out_off, out_idx = a.out_lists()
+  special = [v * 37 + 5 for v in range(13)]
+  roots = [0] + rng.integers(0, a.n, k - 1).tolist()
+  L, P = np.empty((k, a.n), np.int32), np.empty((k, a.n), np.int32)
+  for i, r in enumerate(roots):
+    L[i], P[i], _ = oracle_mod.bfs(out_off, out_idx, a.in_off, a.in_idx, r)
+    if i % 3 == 1:
+      continue
+    L[i], P[i] = _damage(L[i], P[i], a.n, rng, 20)
+    for j, v in enumerate(special):  # any in-neighbour, the last one, none of them
+      nb = a.in_idx[a.in_off[v]:a.in_off[v + 1]]
+      P[i][v] = (int(rng.choice(nb)), int(nb[-1]), int(rng.integers(0, a.n)))[(i + j) % 3]
+      L[i][int(rng.choice(nb))] = int(rng.integers(0, 9))
+  with Graph(a) as g:
+    got = g.validate(roots, torch.from_numpy(L).cuda(), torch.from_numpy(P).cuda())
+    for i, r in enumerate(roots):
+      want = oracle_mod.validation_counts(a.in_off, a.in_idx, r, L[i], P[i])
+      for c in CHECKS:
+        assert (got[i][c]["failures"], got[i][c]["first"]) == want[c], (i, c, got[i], want)
