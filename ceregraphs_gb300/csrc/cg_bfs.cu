@@ -905,6 +905,7 @@ struct SearchState {
   unsigned long long visited, prev_nf, explored;
   int pull_rounds, switches;
   long long t_mark;  // block 0: end of the previous round on the device clock
+  long long t_session;  // team lead: when the other blocks began their bounded wait
   unsigned long long next_big;  // the next frontier's queue sizes (record big, nlight)
   unsigned next_light;
 };
@@ -1206,7 +1207,8 @@ __device__ __noinline__ unsigned team_rounds(const BfsParams &p, SearchState &ss
   TeamCtl *T = &p.ctl->team;
   const unsigned team = team_size(), rank = team_rank();
   const bool leader = threadIdx.x == 0;
-  // sum: 8 bits of arrivals, 8 of blocks that overflowed, 8 of blocks with too
+  // sum: 8 bits of arrivals, the lead's word that the session's time is over, 7
+  // bits of blocks that overflowed, 8 of blocks with too
   // many out-degrees for their 20 bits, 23 of out-degrees, 17 of vertices
   constexpr unsigned kMfBits = 23, kNfBits = 17;
   static_assert(kTeamEdges < (1u << kNfBits), "a round's claims fit");
@@ -1235,7 +1237,9 @@ __device__ __noinline__ unsigned team_rounds(const BfsParams &p, SearchState &ss
         Z->sum = Z->mf = 0;
       }
       if (many) atomicAdd(&R->mf, (unsigned long long)mf);
-      const unsigned long long add = (1ull << 56) | ((unsigned long long)over << 48) |
+      const bool late = rank == 0 && ss.t_mark - ss.t_session > p.timeout_ns / 4;
+      const unsigned long long add = (1ull << 56) | ((unsigned long long)late << 55) |
+                                     ((unsigned long long)over << 48) |
                                      ((unsigned long long)many << 40) |
                                      ((unsigned long long)(many ? 0u : mf) << kNfBits) | nf;
       asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&R->sum), "l"(add) : "memory");
@@ -1247,24 +1251,24 @@ __device__ __noinline__ unsigned team_rounds(const BfsParams &p, SearchState &ss
         const unsigned long long nfs = x & ((1ull << kNfBits) - 1);
         unsigned long long mfs = (x >> kNfBits) & ((1ull << kMfBits) - 1);
         if ((x >> 40) & 0xffu) mfs += __ldcg(&R->mf);
-        const bool lists_fit = ((x >> 48) & 0xffu) == 0;
+        const bool lists_fit = ((x >> 48) & 0x7fu) == 0;
         pay = close_round(p, L, kPush, nfs, mfs, mfs, lists_fit ? kTeam * kSoloMax / 2 : 0u,
                           kTeamEdges, ss);
         S.d[c][0] = (uint32_t)min(mfs, 0xffffffffull);  // F_L's degrees are done with
-        // hand back what one block runs faster
-        S.x[0] = mfs < kTeamLeave && nfs <= (unsigned)kSoloMax / 2;
+        // hand back what one block runs faster, and before the waits' time limit
+        S.x[0] = (mfs < kTeamLeave && nfs <= (unsigned)kSoloMax / 2) || ((x >> 55) & 1u);
       }
       S.payload = pay;
     }
     __syncthreads();
     payload = S.payload;
     const uint32_t mf = S.d[c][0];
-    const bool small = S.x[0] != 0;
+    const bool back = S.x[0] != 0;
     mine = min(S.n, (unsigned)kSoloMax);
     c ^= 1;
     ++L;
     __syncthreads();  // S is read
-    if (payload == kWaitFailed || !(payload & kSolo) || small || ran >= kTeamSession) {
+    if (payload == kWaitFailed || !(payload & kSolo) || back || ran >= kTeamSession) {
       if (leader) {
         S.warp_total[1] = mf;
         S.warp_total[2] = (uint32_t)L;
@@ -1456,6 +1460,7 @@ __device__ __forceinline__ unsigned solo_rounds(const BfsParams &p, SoloShared &
         listed = true;
       }
       do {
+        if (leader) ss.t_session = t0;
         __syncthreads();
         payload = team_lead(p, ss, cnt, L);
         if (payload == kWaitFailed) return kWaitFailed;
