@@ -582,9 +582,11 @@ int fifo_state(cg_graph *g, FifoState **out) {
     bytes = (bytes + size + 255) & ~(size_t)255;
     return at;
   };
+  // (what a call clears together lies together: sums, nlong and counts; lr and
+  // pl; rk and best)
   const size_t at_sums = piece(sizeof(FifoSums)), at_nlong = piece(sizeof(unsigned long long)),
-               at_longs = piece(sizeof(FifoLong) * nlongs), at_temp = piece(f->temp_bytes),
                at_counts = piece(sizeof(unsigned) * (n + 1)),
+               at_longs = piece(sizeof(FifoLong) * nlongs), at_temp = piece(f->temp_bytes),
                at_offs = piece(sizeof(unsigned) * (n + 2)), at_lr = piece(8 * n),
                at_pl = piece(8 * n);
   size_t at4[9];  // 4 bytes a vertex each
@@ -637,9 +639,12 @@ int fifo_parents(cg_graph *g, int64_t root, const int32_t *d_levels, int32_t *d_
   const int64_t n = g->n;
   const int sms = g->num_sms;
   cudaStream_t st = g->stream;
-  CG_CUDA(cudaMemsetAsync(f->sums, 0, sizeof(FifoSums), st));
-  CG_CUDA(cudaMemsetAsync(f->nlong, 0, sizeof(unsigned long long), st));
-  CG_CUDA(cudaMemsetAsync(f->counts, 0, sizeof(unsigned) * (size_t)(n + 1), st));
+  auto fill = [&](void *first, void *last, size_t last_bytes, int value) {
+    return cudaMemsetAsync(first, value,
+                           (size_t)(static_cast<unsigned char *>(last) -
+                                    static_cast<unsigned char *>(first)) + last_bytes, st);
+  };
+  CG_CUDA(fill(f->sums, f->counts, sizeof(unsigned) * (size_t)(n + 1), 0));
   const unsigned hist_blocks = grid_for(n, kFifoBlock, sms);
   fifo_hist_kernel<<<hist_blocks < 4u * sms ? hist_blocks : 4u * sms, kFifoBlock, 0, st>>>(
       n, d_levels, g->in_off, g->out_off, f->counts, f->sums);
@@ -668,8 +673,7 @@ int fifo_parents(cg_graph *g, int64_t root, const int32_t *d_levels, int32_t *d_
                                           reinterpret_cast<const uint32_t *>(d_levels), f->best,
                                           reinterpret_cast<const int32_t *>(f->rk), f->order, n, 0,
                                           bits_for((uint64_t)maxlevel + 1), st));
-  CG_CUDA(cudaMemsetAsync(f->rk, 0xff, sizeof(uint32_t) * (size_t)n, st));
-  CG_CUDA(cudaMemsetAsync(f->best, 0xff, sizeof(uint32_t) * (size_t)n, st));
+  CG_CUDA(fill(f->rk, f->best, sizeof(uint32_t) * (size_t)n, 0xff));
   auto small = [&](int L) {  // level L to L + 1 suits a run of small levels
     return counts[(size_t)L] <= (unsigned)kSmallLevel &&
            counts[(size_t)L + 1] <= (unsigned)kSmallLevel && counts[(size_t)L + 1] > 0 &&
@@ -687,8 +691,7 @@ int fifo_parents(cg_graph *g, int64_t root, const int32_t *d_levels, int32_t *d_
     if (L1 - L >= kSmallRun) {
       // levels L .. L1 in one launch of one block
       if (!small_ready) {
-        CG_CUDA(cudaMemsetAsync(f->lr, 0xff, sizeof(unsigned long long) * (size_t)n, st));
-        CG_CUDA(cudaMemsetAsync(f->pl, 0xff, sizeof(unsigned long long) * (size_t)n, st));
+        CG_CUDA(fill(f->lr, f->pl, sizeof(unsigned long long) * (size_t)n, 0xff));
         CG_CUDA(cudaMemcpyAsync(f->offs, offs.data(), sizeof(unsigned) * offs.size(),
                                 cudaMemcpyHostToDevice, st));
         small_ready = true;
