@@ -33,6 +33,8 @@
 // merging F_L into vis during round L races with nothing.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "cg_internal.cuh"
 
 namespace cg {
@@ -63,7 +65,8 @@ struct __align__(16) WarpTile {  // 16-byte vector accesses to every member
 static_assert(sizeof(WarpTile) % 16 == 0 && kTileWords % 4 == 0, "16-byte tile rows");
 // Per-warp shared memory of a push round (a pull round keeps the vertices whose
 // first in-neighbour was no parent here): the edge spreading of gather_expand
-// (list starts and prefix counts fit 32 bits, nnz being below 2^32), and the
+// (a resident graph's list starts and prefix counts fit 32 bits, its nnz being
+// below 2^32; larger ones: s_start_high), and the
 // light vertices claimed and not queued yet.  Big ones wait in the tile's
 // `found` words, which push rounds do not use.
 struct WarpExpand {
@@ -77,6 +80,22 @@ struct BigClaims {
   uint32_t deg[64];
 };
 static_assert(sizeof(BigClaims) == sizeof(uint32_t) * kTileWords, "fits WarpTile::found");
+
+// Graphs of 2^32 - 2^16 list entries and more (kWide: only a caller's own arrays
+// can be so large, cg_bfs_noalloc): list starts take 64 bits, their high words
+// here, and a round record's `big` has its count from bit 43 on (at most 2^20 big
+// vertices there).  A frontier of kEdges32 big edges or more is expanded from the
+// bitmap, where edges are counted per 32 vertices.
+__shared__ uint32_t s_start_high[kBfsWarps][32];
+constexpr unsigned long long kEdges32 = (1ull << 32) - (1ull << 16);
+template <bool kWide>
+struct BigWord {
+  static constexpr int kShift = kWide ? 43 : 32;
+  static constexpr unsigned long long kEdges = (1ull << kShift) - 1ull;
+  static __device__ __forceinline__ unsigned long long pack(unsigned count, unsigned edges) {
+    return ((unsigned long long)count << kShift) | edges;
+  }
+};
 
 // Shared memory of block 0's runs of small rounds (solo_rounds): the frontier
 // and the next one (vertex, list start, out-degree), and the prefix of the
@@ -263,6 +282,7 @@ __device__ __forceinline__ void put_big(const BfsParams &p, const BigClaims &B, 
 }
 
 // The claims of one warp-wide step.  All 32 lanes call.
+template <bool kWide>
 __device__ __forceinline__ void keep_claims(const BfsParams &p, bool claimed, int32_t v,
                                             uint32_t deg, int next_parity, RoundRec *Rn, Claims &C,
                                             Acc &acc) {
@@ -300,14 +320,16 @@ __device__ __forceinline__ void keep_claims(const BfsParams &p, bool claimed, in
     C.nb -= 32;
     const uint32_t edges = __reduce_add_sync(kFull, C.B.deg[C.nb + lane]);
     unsigned long long old = 0;
-    if (lane == 0) old = atomicAdd(&Rn->big, (32ull << 32) | edges);
+    if (lane == 0) old = atomicAdd(&Rn->big, BigWord<kWide>::pack(32, edges));
     old = __shfl_sync(kFull, old, 0);
-    put_big(p, C.B, C.nb, 32, (unsigned)(old >> 32), (unsigned)old, next_parity);
+    put_big(p, C.B, C.nb, 32, (unsigned)(old >> BigWord<kWide>::kShift), (unsigned)old,
+            next_parity);
     __syncwarp();
   }
 }
 
 // What the block's warps have left, one atomic of a kind.  All threads call.
+template <bool kWide>
 __device__ __forceinline__ void queue_rest(const BfsParams &p, Claims &C, int next_parity,
                                            RoundRec *Rn) {
   __shared__ unsigned s_nl[kBfsWarps], s_nb[kBfsWarps], s_edges[kBfsWarps];
@@ -332,11 +354,11 @@ __device__ __forceinline__ void queue_rest(const BfsParams &p, Claims &C, int ne
     unsigned long long old = 0;
     if (lane == 31 && il) old = atomicAdd(&Rn->nlight, il);
     const unsigned base_l = (unsigned)__shfl_sync(kFull, old, 31);
-    if (lane == 31) old = ib ? atomicAdd(&Rn->big, ((unsigned long long)ib << 32) | ie) : 0ull;
+    if (lane == 31) old = ib ? atomicAdd(&Rn->big, BigWord<kWide>::pack(ib, ie)) : 0ull;
     old = __shfl_sync(kFull, old, 31);
     if (lane < nw) {
       s_nl[lane] = base_l + il - l;
-      s_nb[lane] = (unsigned)(old >> 32) + ib - b;
+      s_nb[lane] = (unsigned)(old >> BigWord<kWide>::kShift) + ib - b;
       s_edges[lane] = (unsigned)old + ie - e;
     }
   }
@@ -346,16 +368,21 @@ __device__ __forceinline__ void queue_rest(const BfsParams &p, Claims &C, int ne
   if (C.nb) put_big(p, C.B, 0, C.nb, s_nb[wib], s_edges[wib], next_parity);
 }
 
-constexpr uint32_t kNoEdge = 0xffffffffu;
+// Position of a list entry; all bits set for none.
+template <bool kWide>
+using EdgePos = std::conditional_t<kWide, uint64_t, uint32_t>;
+template <bool kWide>
+constexpr EdgePos<kWide> kNoEdge = ~EdgePos<kWide>(0);
 
 // Edge u -> out_idx[e] per lane of a push round (e = kNoEdge for none).  A
 // target claimed already gets a read before its atomicMin: most of a big
 // round's edges lead to vertices that a lower source has reached, and a read
 // costs the L2 less.
+template <bool kWide>
 __device__ __forceinline__ void push_step(const BfsParams &p, const uint32_t *cur, uint32_t *nxt,
-                                          int32_t u, uint32_t e, int L, int next_parity,
+                                          int32_t u, EdgePos<kWide> e, int L, int next_parity,
                                           RoundRec *Rn, Claims &C, Acc &acc) {
-  const int32_t v = e != kNoEdge ? __ldg(p.out_idx + e) : -1;
+  const int32_t v = e != kNoEdge<kWide> ? __ldg(p.out_idx + e) : -1;
   bool open = false, mine = false;  // not visited; nor claimed by another edge before
   if (v >= 0) {
     const uint32_t w = (uint32_t)v >> 5, bit = 1u << (v & 31);
@@ -384,20 +411,22 @@ __device__ __forceinline__ void push_step(const BfsParams &p, const uint32_t *cu
       atomicMin(par, ou);
     }
   }
-  keep_claims(p, claimed, v, deg, next_parity, Rn, C, acc);
+  keep_claims<kWide>(p, claimed, v, deg, next_parity, Rn, C, acc);
 }
 
 // Expands up to 32 frontier vertices (one per lane, u < 0 for none) with the
 // warp's combined edge list spread evenly over its lanes.
+template <bool kWide>
 __device__ __forceinline__ void gather_expand(const BfsParams &p, const uint32_t *cur,
                                               uint32_t *nxt, int32_t u, int L, int next_parity,
                                               RoundRec *Rn, Claims &C, Acc &acc) {
   const int lane = lane_id();
   WarpExpand &X = C.X;
-  uint32_t s = 0, d = 0;
+  EdgePos<kWide> s = 0;
+  uint32_t d = 0;
   if (u >= 0) {
     const int64_t o = __ldg(p.out_off + u);
-    s = (uint32_t)o;
+    s = (EdgePos<kWide>)o;
     d = (uint32_t)(__ldg(p.out_off + u + 1) - o);
   }
   uint32_t incl = d;
@@ -409,7 +438,8 @@ __device__ __forceinline__ void gather_expand(const BfsParams &p, const uint32_t
   const uint32_t total = __shfl_sync(kFull, incl, 31);
   if (total == 0) return;
   X.u[lane] = u;
-  X.s[lane] = s;
+  X.s[lane] = (uint32_t)s;
+  if constexpr (kWide) s_start_high[threadIdx.x >> 5][lane] = (uint32_t)(s >> 32);
   X.x[lane] = incl - d;
   __syncwarp();
   for (uint32_t base = 0; base < total; base += 32) {
@@ -418,8 +448,13 @@ __device__ __forceinline__ void gather_expand(const BfsParams &p, const uint32_t
 #pragma unroll
     for (int step = 16; step > 0; step >>= 1)
       if (X.x[lo + step] <= t) lo += step;
-    const uint32_t e = t < total && t >= base ? X.s[lo] + (t - X.x[lo]) : kNoEdge;
-    push_step(p, cur, nxt, X.u[lo], e, L, next_parity, Rn, C, acc);
+    EdgePos<kWide> e = kNoEdge<kWide>;
+    if (t < total && t >= base) {
+      e = X.s[lo];
+      if constexpr (kWide) e |= (uint64_t)s_start_high[threadIdx.x >> 5][lo] << 32;
+      e += t - X.x[lo];
+    }
+    push_step<kWide>(p, cur, nxt, X.u[lo], e, L, next_parity, Rn, C, acc);
     if (base + 32 < base) break;  // total within a step of 2^32
   }
   __syncwarp();
@@ -434,6 +469,7 @@ __device__ __forceinline__ void gather_expand(const BfsParams &p, const uint32_t
 // 16 us).  Item i goes to warp i first; warps that finish take the rest from a counter.
 // bigw / nlight: F_L's queue sizes ((big count << 32) | big edges, light
 // count), handed over with the barrier that ended round L - 1.
+template <bool kWide>
 __device__ void push_round_queue(const BfsParams &p, const uint32_t *cur, uint32_t *nxt, int L,
                                  RoundRec *Rc, RoundRec *Rn, unsigned long long bigw,
                                  unsigned nlight, Acc &acc) {
@@ -475,38 +511,38 @@ __device__ void push_round_queue(const BfsParams &p, const uint32_t *cur, uint32
       }
       unsigned j = lo;
       int32_t vj = q[p.n - 1 - (int64_t)j];
-      uint32_t sj = (uint32_t)__ldg(p.out_off + vj);
+      EdgePos<kWide> sj = (EdgePos<kWide>)__ldg(p.out_off + vj);
       unsigned oj = boff[j];
-      unsigned endj = oj + ((uint32_t)__ldg(p.out_off + vj + 1) - sj);
+      unsigned endj = oj + (uint32_t)((EdgePos<kWide>)__ldg(p.out_off + vj + 1) - sj);
       for (unsigned base = x0; base < x1; base += 32) {
         while (base >= endj) {  // the next big vertex (degrees exceed 32)
           ++j;
           vj = q[p.n - 1 - (int64_t)j];
-          sj = (uint32_t)__ldg(p.out_off + vj);
+          sj = (EdgePos<kWide>)__ldg(p.out_off + vj);
           oj = boff[j];
-          endj = oj + ((uint32_t)__ldg(p.out_off + vj + 1) - sj);
+          endj = oj + (uint32_t)((EdgePos<kWide>)__ldg(p.out_off + vj + 1) - sj);
         }
         const unsigned x = base + lane;
         const bool valid = x < x1;
         int32_t u = vj;
-        uint32_t e = valid ? sj + (x - oj) : kNoEdge;
+        EdgePos<kWide> e = valid ? sj + (x - oj) : kNoEdge<kWide>;
         if (__ballot_sync(kFull, valid && x >= endj)) {  // lanes past vertex j's end
           const int32_t vn = q[p.n - 1 - (int64_t)(j + 1)];
           if (valid && x >= endj) {
             u = vn;
-            e = (uint32_t)__ldg(p.out_off + vn) + (x - endj);
+            e = (EdgePos<kWide>)__ldg(p.out_off + vn) + (x - endj);
           }
         }
-        push_step(p, cur, nxt, u, e, L, next_parity, Rn, C, acc);
+        push_step<kWide>(p, cur, nxt, u, e, L, next_parity, Rn, C, acc);
       }
     } else {
       const unsigned idx = (item - nchunks) * group + lane;
-      gather_expand(p, cur, nxt, (unsigned)lane < group && idx < nlight ? q[idx] : -1, L,
-                    next_parity, Rn, C, acc);
+      gather_expand<kWide>(p, cur, nxt, (unsigned)lane < group && idx < nlight ? q[idx] : -1, L,
+                           next_parity, Rn, C, acc);
     }
     item = __shfl_sync(kFull, nextitem, 0);
   }
-  queue_rest(p, C, next_parity, Rn);
+  queue_rest<kWide>(p, C, next_parity, Rn);
 }
 
 // Work items of a bitmap-wide round: (tile, slot) pairs; a tile holds 4096
@@ -532,6 +568,7 @@ __device__ __forceinline__ int64_t next_item(int64_t item, int nwarps, RoundRec 
 // Push round right after a pull round: the frontier is only in the bitmap, so
 // warps stage it a tile at a time (one 16-byte load per lane) and expand its
 // set bits 32 at a time (lane i takes the i-th bit of its batch).
+template <bool kWide>
 __device__ void push_round_bitmap(const BfsParams &p, const uint32_t *cur, uint32_t *nxt, int L,
                                   RoundRec *Rc, RoundRec *Rn, bool heavy, Acc &acc) {
   const int lane = lane_id();
@@ -555,11 +592,11 @@ __device__ void push_round_bitmap(const BfsParams &p, const uint32_t *cur, uint3
         select_bit(T, b + lane, j, bit);
         u = (int32_t)((t * kTileWords + j) * 32 + bit);
       }
-      gather_expand(p, cur, nxt, u, L, next_parity, Rn, C, acc);
+      gather_expand<kWide>(p, cur, nxt, u, L, next_parity, Rn, C, acc);
     }
     __syncwarp();  // T is restaged by the next item
   }
-  queue_rest(p, C, next_parity, Rn);
+  queue_rest<kWide>(p, C, next_parity, Rn);
 }
 
 // Bottom-up round: every unvisited vertex scans its ascending in-list and
@@ -851,6 +888,8 @@ constexpr unsigned kDone = 1u, kNextPull = 2u, kHeavy = 4u;
 constexpr unsigned kSolo = 8u;
 // ... or for a team
 constexpr unsigned kHandOver = 16u;
+// ... expands its frontier from the bitmap, although it was queued (kWide)
+constexpr unsigned kUnqueued = 32u;
 __device__ __forceinline__ unsigned team_size() { return gridDim.x >= 2 * kTeam ? kTeam : 0u; }
 
 // Flat grid-wide barrier of the per-root kernel, called by thread 0 of each
@@ -973,7 +1012,7 @@ __device__ __forceinline__ unsigned close_round(const BfsParams &p, int L, int d
 // 0-23 each load one sharded counter of the round record (one L2 round trip),
 // lane 0 takes the decision (close_round), the same in every block.  All 32
 // lanes call; lane 0's return value is the payload.
-template <bool kTeamed>
+template <bool kTeamed, bool kWide>
 __device__ unsigned round_decision(const BfsParams &p, int L, int dir, SearchState &ss) {
   BfsCtl *ctl = p.ctl;
   const RoundRec *Rn = &ctl->rec[(L + 1) % kRing];
@@ -995,8 +1034,13 @@ __device__ unsigned round_decision(const BfsParams &p, int L, int dir, SearchSta
   const unsigned long long mf = __shfl_sync(kFull, x, 8);
   const unsigned long long vd = __shfl_sync(kFull, x, 16);
   if (lane != 0) return 0u;
-  ss.next_big = qbig;
   ss.next_light = (unsigned)qlight;
+  if constexpr (kWide) {
+    const unsigned long long edges = qbig & BigWord<true>::kEdges;
+    ss.next_big = ((qbig >> BigWord<true>::kShift) << 32) | (uint32_t)edges;
+    return close_round(p, L, dir, nf, mf, vd, 0u, 0u, ss) | (edges >= kEdges32 ? kUnqueued : 0u);
+  }
+  ss.next_big = qbig;
   // one block takes over well below what it can hold, so that a frontier near
   // the line does not go back and forth
   if constexpr (kTeamed) {
@@ -1587,7 +1631,7 @@ __device__ __noinline__ void copy_to_host(const BfsParams &p) {
   }
 }
 
-template <bool kTeamed>
+template <bool kTeamed, bool kWide>
 __device__ __forceinline__ void search(const BfsParams &p) {
   __shared__ unsigned s_payload;
   __shared__ int s_L;
@@ -1612,7 +1656,7 @@ __device__ __forceinline__ void search(const BfsParams &p) {
   // a root of few edges starts on block 0 alone: it is in vis then, and the
   // frontier bitmaps are clear
   const int64_t root_deg = __ldg(p.out_off + root + 1) - __ldg(p.out_off + root);
-  bool solo = root_deg <= (int64_t)kSoloEnter;
+  bool solo = !kWide && root_deg <= (int64_t)kSoloEnter;
   for (int64_t i = gtid; i < p.tiles * (kTileWords / 4); i += nthreads) {
     uint4 f0 = zero4;
     if (i == (root_word >> 2)) {  // F_0 = {root}, seeded by the thread that clears its word
@@ -1637,7 +1681,7 @@ __device__ __forceinline__ void search(const BfsParams &p) {
     } else {
       p.queue0[p.n - 1] = root;
       p.bigoff0[0] = 0;
-      R0->big = (1ull << 32) | (unsigned long long)deg;
+      R0->big = BigWord<kWide>::pack(1, (unsigned)deg);
     }
   }
   // barrier b of this launch completes at (b + 1) * gridDim.x arrivals
@@ -1676,7 +1720,7 @@ __device__ __forceinline__ void search(const BfsParams &p) {
   int L = 0;
   Acc acc;
   while (ok) {
-    if (solo) {
+    if (!kWide && solo) {
       // L = 0: the root alone, in vis already (phase 0)
       const bool fold = L > 0, from_queue = L > 0 && queued;
       if (fold && !queued) {
@@ -1763,7 +1807,7 @@ __device__ __forceinline__ void search(const BfsParams &p) {
       queued = true;
       dir = (payload & kNextPull) ? kPull : kPush;
       heavy = (payload & kHeavy) != 0;
-        solo = false;
+      solo = false;
       __syncthreads();
       // all three bitmaps were cleared; fr0 holds F_L
     }
@@ -1774,9 +1818,9 @@ __device__ __forceinline__ void search(const BfsParams &p) {
     uint32_t *old = fr2;        // F_{L-1}
     if (dir == kPush) {
       if (queued)
-        push_round_queue(p, cur, nxt, L, Rc, Rn, ss.next_big, ss.next_light, acc);
+        push_round_queue<kWide>(p, cur, nxt, L, Rc, Rn, ss.next_big, ss.next_light, acc);
       else
-        push_round_bitmap(p, cur, nxt, L, Rc, Rn, heavy, acc);
+        push_round_bitmap<kWide>(p, cur, nxt, L, Rc, Rn, heavy, acc);
       // vis |= F_L (readers test vis | F_L, so this races with nothing) and
       // clear F_{L-1}, which becomes the next round's output bitmap; a pull
       // round does both in its own tile pass
@@ -1813,13 +1857,14 @@ __device__ __forceinline__ void search(const BfsParams &p) {
       // lane 0's acquire fence, then this warp barrier, order the other lanes'
       // counter loads after every block's arrival
       arrived = __shfl_sync(kFull, arrived, 0);
-      const unsigned payload = arrived ? round_decision<kTeamed>(p, L, dir, ss) : kWaitFailed;
+      const unsigned payload = arrived ? round_decision<kTeamed, kWide>(p, L, dir, ss) : kWaitFailed;
       if (threadIdx.x == 0) s_payload = payload;
     }
     __syncthreads();
     const unsigned payload = s_payload;
     if (payload == kWaitFailed || (payload & kDone)) break;
     queued = dir == kPush;  // a push round queued F_{L+1}; a pull round did not
+    if constexpr (kWide) queued = queued && !(payload & kUnqueued);
     dir = (payload & kNextPull) ? kPull : kPush;
     heavy = (payload & kHeavy) != 0;
     solo = (payload & kSolo) != 0;
@@ -1835,7 +1880,15 @@ __device__ __forceinline__ void search(const BfsParams &p) {
   if (s_payload != kWaitFailed && (p.host_levels || p.host_parents)) copy_to_host(p);
 }
 
-__global__ void __launch_bounds__(kBfsBlock, 3) bfs_persistent(BfsParams p) { search<false>(p); }
+__global__ void __launch_bounds__(kBfsBlock, 3) bfs_persistent(BfsParams p) {
+  search<false, false>(p);
+}
+
+// The same search without small rounds on one block, its list positions in 64
+// bits: graphs of kEdges32 entries and more.
+__global__ void __launch_bounds__(kBfsBlock, 3) bfs_persistent_wide(BfsParams p) {
+  search<false, true>(p);
+}
 
 // The same search with rounds that a team runs.  A kernel of its own, so that
 // the other keeps its registers (with the team in it R-MAT and random graphs took
@@ -1843,7 +1896,7 @@ __global__ void __launch_bounds__(kBfsBlock, 3) bfs_persistent(BfsParams p) { se
 // three handles' blocks still fit an SM: 512 threads and 64 registers are as fast
 // for one handle, 4.6 ms a search for three taking turns where this takes 3.3.
 __global__ void __launch_bounds__(kTeamBlock, 3) bfs_persistent_team(BfsParams p) {
-  search<true>(p);
+  search<true, false>(p);
 }
 
 // A vertex's share of Graph500's m (bfs_timing.py:379-398): its entries c <= v

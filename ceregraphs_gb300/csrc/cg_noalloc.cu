@@ -23,6 +23,7 @@
 namespace cg {
 
 __global__ void bfs_persistent(BfsParams p);
+__global__ void bfs_persistent_wide(BfsParams p);
 void set_error_text(const char *text);
 
 int64_t bfs_big_capacity(int64_t n, int64_t nnz);
@@ -44,7 +45,7 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
 constexpr int kMaxDevices = 64;
 static std::mutex g_setup_mu;
-static int g_grid[kMaxDevices] = {};
+static int g_grid[kMaxDevices][2] = {};  // by the kernel: 32-bit list positions, 64-bit
 
 // With the device current: the device address of the scratch array (host code
 // cannot use the symbol itself, whose host-side name is only a stand-in) and
@@ -52,23 +53,24 @@ static int g_grid[kMaxDevices] = {};
 // host-side table read -- so a cudaDeviceReset between calls, which reloads
 // the module and may move the array, leaves no stale address behind.  The
 // grid size (SM count times resident blocks per SM) is fixed per device and
-// computed once.
-static int noalloc_setup(int dev, void **scratch, int *grid) {
+// kernel and computed once.
+static int noalloc_setup(int dev, bool wide, void **scratch, int *grid) {
   void *addr = nullptr;
   cudaError_t e = cudaGetSymbolAddress(&addr, g_noalloc_scratch);
   if (e != cudaSuccess) return cuda_fail(e, "cudaGetSymbolAddress(g_noalloc_scratch)");
   std::lock_guard<std::mutex> lock(g_setup_mu);
-  if (!g_grid[dev]) {
+  if (!g_grid[dev][wide]) {
     int sms = 0, per_sm = 0;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return cuda_fail(e, "cudaDeviceGetAttribute");
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bfs_persistent, 512, 0);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &per_sm, wide ? bfs_persistent_wide : bfs_persistent, 512, 0);
     if (e != cudaSuccess) return cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
     if (per_sm <= 0) return CG_ERR_NOT_SUPPORTED;
-    g_grid[dev] = per_sm * sms;
+    g_grid[dev][wide] = per_sm * sms;
   }
   *scratch = addr;
-  *grid = g_grid[dev];
+  *grid = g_grid[dev][wide];
   return CG_OK;
 }
 
@@ -109,7 +111,10 @@ extern "C" int cg_bfs_noalloc(int64_t n, int64_t nnz, const int64_t *d_in_off,
   if (dev < 0 || dev >= kMaxDevices) return CG_ERR_NOT_SUPPORTED;
   void *scratch = nullptr;
   int grid = 0;
-  int rc = noalloc_setup(dev, &scratch, &grid);
+  // the caller's arrays may hold more entries than a resident graph does: the
+  // kernel then keeps list positions in 64 bits
+  const bool wide = nnz >= (1ll << 32) - (1ll << 16);
+  int rc = noalloc_setup(dev, wide, &scratch, &grid);
   if (rc) return rc;
   unsigned char *base = static_cast<unsigned char *>(scratch);
   const int64_t words = (n + 31) / 32;
@@ -184,7 +189,7 @@ extern "C" int cg_bfs_noalloc(int64_t n, int64_t nnz, const int64_t *d_in_off,
     }
   }
   CG_CUDA(cudaMemsetAsync(p.ctl, 0, sizeof(BfsCtl), st));
-  CG_CUDA(cudaLaunchKernelEx(&cfg, bfs_persistent, p));
+  CG_CUDA(cudaLaunchKernelEx(&cfg, wide ? bfs_persistent_wide : bfs_persistent, p));
   if (!stats) return CG_OK;
   CG_CUDA(cudaMemcpyAsync(stats, p.stats, sizeof(cg_stats), cudaMemcpyDeviceToHost, st));
   if (async_stats) return CG_OK;  // valid once the stream has reached this point

@@ -338,6 +338,7 @@ int cg_graph_reorder(const cg_graph *g, int32_t order, cg_graph **out);
  * Limits: n <= CG_NOALLOC_MAX_VERTICES and min(n, nnz / 65 + 1) (the bound on
  * vertices of out-degree > 64) <= CG_NOALLOC_MAX_BIG; larger graphs are
  * rejected with CG_ERR_INVALID_ARG and a message in cg_last_error_string.
+ * Within them nnz may be 2^32 and more, which a resident graph's may not.
  * Every call on a GPU shares the array and it keeps the last call's contents:
  * calls that overlap on that GPU (other streams or threads) race and give
  * wrong results.  The first call on each device computes the grid size; the

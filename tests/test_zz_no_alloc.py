@@ -128,3 +128,70 @@ def test_noalloc_partial_last_word_and_stats_modes(built_lib, stats):
     if st is not None:
       assert st["status"] == 0
       assert st["rounds"] == wst["rounds"] and st["pull_rounds"] == wst["pull_rounds"]
+
+
+@pytest.mark.parametrize("lists", [32766, 32772])
+def test_noalloc_more_than_2_32_entries(built_lib, lists):
+  """A caller's own arrays may hold more entries than 32 bits count: 131,072
+  vertices, the first `lists` of them with edges to all.  The others' lists start
+  past entry 2^32 (32,772 lists), or just below it (32,766)."""
+  torch = pytest.importorskip("torch")
+  n, path, fan = 1 << 17, 60, 100
+  if torch.cuda.mem_get_info()[0] < 60 << 30:
+    pytest.skip("needs 60 GB of device memory")
+  first, last = lists, n - 1
+  # last -> first .. first + fan - 1 (a list longer than 64), and a path behind them
+  chain = torch.arange(first + fan - 1, first + fan + path, device="cuda", dtype=torch.int32)
+  out_deg = torch.zeros(n, dtype=torch.int64, device="cuda")
+  out_deg[:lists] = n
+  out_deg[chain[:-1].long()] = 1
+  out_deg[last] = fan
+  out_off = torch.zeros(n + 1, dtype=torch.int64, device="cuda")
+  torch.cumsum(out_deg, 0, out=out_off[1:])
+  every = torch.arange(n, device="cuda", dtype=torch.int32)
+  out_idx = torch.cat([every.repeat(lists), chain[1:], every[first:first + fan]])
+  nnz = int(out_off[-1])
+  assert len(out_idx) == nnz and (nnz > 1 << 32) == (lists > 32768)
+  # in-lists: the first `lists` vertices, then a path's or the fan's source
+  in_deg = torch.full((n,), lists, dtype=torch.int64, device="cuda")
+  in_deg[chain[1:].long()] += 1
+  in_deg[first:first + fan] += 1
+  in_off = torch.zeros(n + 1, dtype=torch.int64, device="cuda")
+  torch.cumsum(in_deg, 0, out=in_off[1:])
+  in_idx = torch.empty(nnz, dtype=torch.int32, device="cuda")
+  at, end = first, first + fan + path  # vertices with one more source
+  in_idx[:at * lists] = every[:lists].repeat(at)
+  for v in range(at, end):
+    b = int(in_off[v])
+    in_idx[b:b + lists] = every[:lists]
+    in_idx[b + lists] = last if v < first + fan else v - 1
+  in_idx[int(in_off[end]):] = every[:lists].repeat(n - end)
+
+  lv, pa = (torch.empty(n, dtype=torch.int32, device="cuda") for _ in range(2))
+
+  def search(root):
+    st = _lib.CgStats()
+    rc = built_lib.cg_bfs_noalloc(n, nnz, _ptr(in_off), _ptr(in_idx), _ptr(out_off),
+                                  _ptr(out_idx), root, _ptr(lv), _ptr(pa), ctypes.byref(st), None)
+    assert rc == 0, (rc, built_lib.cg_last_error_string())
+    return lv.cpu().numpy(), pa.cpu().numpy(), st.as_dict()
+
+  want_l, want_p = np.full((2, n), -1, dtype=np.int32)
+  want_l[last], want_p[last] = 0, last
+  want_l[first:first + fan], want_p[first:first + fan] = 1, last
+  for i, v in enumerate(range(first + fan, end)):
+    want_l[v], want_p[v] = 2 + i, v - 1
+  got_l, got_p, st = search(last)
+  assert np.array_equal(got_l, want_l) and np.array_equal(got_p, want_p)
+  assert st["rounds"] == path + 2 and st["visited"] == 1 + fan + path
+  # a root with edges to all: the next frontier's lists hold over 2^32 entries
+  got_l, got_p, st = search(5)
+  want_l[:], want_p[:] = 1, 5
+  want_l[5] = 0
+  assert np.array_equal(got_l, want_l) and np.array_equal(got_p, want_p)
+  assert st["rounds"] == 2 and st["visited"] == n
+  # from a vertex of the path only the path's rest is reached
+  v = first + fan + 10
+  got_l, got_p, st = search(v)
+  assert st["visited"] == path - 10 and int(got_l[end - 1]) == end - 1 - v
+  assert (got_l >= 0).sum() == path - 10 and (got_p[v + 1:end] == np.arange(v, end - 1)).all()
