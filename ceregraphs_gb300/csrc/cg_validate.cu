@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(kBlock) vertex_checks_kernel(
     const int32_t *__restrict__ parents_all, const int *wide, Tally *tallies) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (kBlock / 32);
-  for (int s = 0; s < k; ++s) {
+  for (int s = blockIdx.y; s < k; s += gridDim.y) {
     if (wide && !wide[s / kGroup]) continue;
     const int32_t *__restrict__ level = levels_all + (int64_t)s * n;
     const int32_t *__restrict__ parent = parents_all + (int64_t)s * n;
@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(kBlock) edge_checks_kernel(
     int k, const int32_t *__restrict__ levels_all, const int *wide, Tally *tallies) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (kBlock / 32);
-  for (int s = 0; s < k; ++s) {
+  for (int s = blockIdx.y; s < k; s += gridDim.y) {
     if (wide && !wide[s / kGroup]) continue;
     const int32_t *__restrict__ level = levels_all + (int64_t)s * n;
     Tally *t = tallies + s;
@@ -653,6 +653,20 @@ void launch_group(const cg_graph *g, const GroupArgs &a) {
   check_long_kernel<NW><<<(unsigned)g->num_sms * 6, kBlock, 0, g->stream>>>(a);
 }
 
+// Grid of a per-search kernel, one search filling `blocks` blocks: at most 8
+// blocks an SM for a search, and as many searches side by side (blockIdx.y, the
+// rest in turn) as come to four times that.  One after another, the searches of a
+// small deep graph leave the GPU idle: 64 of a 200^2 grid took 2,960 us a call, 336
+// so; of a caterpillar of 3,000 vertices with 30 leaves each 9,760 and 495.  No
+// more, so that the launch stays short where the groups have done all of it.
+constexpr int64_t kSideBySide = 4;
+dim3 search_grid(const cg_graph *g, int64_t blocks, int k) {
+  const int64_t cap = (int64_t)g->num_sms * 8;
+  const int64_t x = blocks < cap ? blocks : cap;
+  const int64_t side = (kSideBySide * cap + x - 1) / x;
+  return dim3((unsigned)x, (unsigned)(side < k ? side : k));
+}
+
 }  // namespace
 }  // namespace cg
 
@@ -714,18 +728,16 @@ extern "C" int cg_validate_device(cg_graph *g, const int64_t *roots, int32_t k,
         else launch_group<4>(g, a);
       }
     }
-    // the searches the groups left (levels past a byte), or all of them;
-    // about 8 warps' worth of work per SM
-    const int64_t vblocks = (g->n + kBlock - 1) / kBlock;
-    const int64_t cap = (int64_t)g->num_sms * 8;
+    // the searches the groups left (levels past a byte), or all of them
     const int *wide = grouped ? d_wide : nullptr;
-    vertex_checks_kernel<<<(unsigned)(vblocks < cap ? vblocks : cap), kBlock, 0, g->stream>>>(
-        g->n, g->in_off, g->in_idx, d_roots, k, d_levels, d_parents, wide, d_t);
+    vertex_checks_kernel<<<search_grid(g, (g->n + kBlock - 1) / kBlock, k), kBlock, 0,
+                           g->stream>>>(g->n, g->in_off, g->in_idx, d_roots, k, d_levels,
+                                        d_parents, wide, d_t);
     if (g->nnz > 0) {
-      const int64_t eblocks = (g->nnz + (int64_t)kEdgesPerWarp * (kBlock / 32) - 1) /
-                              ((int64_t)kEdgesPerWarp * (kBlock / 32));
-      edge_checks_kernel<<<(unsigned)(eblocks < cap ? eblocks : cap), kBlock, 0, g->stream>>>(
-          g->n, g->nnz, g->in_off, g->in_idx, k, d_levels, wide, d_t);
+      const int64_t per_block = (int64_t)kEdgesPerWarp * (kBlock / 32);
+      edge_checks_kernel<<<search_grid(g, (g->nnz + per_block - 1) / per_block, k), kBlock, 0,
+                           g->stream>>>(g->n, g->nnz, g->in_off, g->in_idx, k, d_levels, wide,
+                                        d_t);
     }
     e = cudaGetLastError();
     if (e == cudaSuccess)

@@ -110,3 +110,38 @@ def test_large_graph_matches_oracle(built_lib, oracle_mod, k):
       want = oracle_mod.validation_counts(a.in_off, a.in_idx, r, L[i], P[i])
       for c in CHECKS:
         assert (got[i][c]["failures"], got[i][c]["first"]) == want[c], (i, c, got[i], want)
+
+
+def _caterpillar(spine, leaves):
+  i, j = np.arange(spine - 1), np.arange(spine * leaves)
+  return from_edges(spine * (leaves + 1), np.concatenate([i, j // leaves]),
+                    np.concatenate([i + 1, spine + j]), symmetrize=True)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["grid200", "caterpillar"])
+def test_deep_searches_side_by_side(built_lib, kind):
+  """The checks of a small deep graph, whose levels pass a byte, fill the GPU with
+  several searches at once: eight times the searches, which take nearly eight
+  times as long one after another, take less than half of that."""
+  import time
+  import torch
+  from ceregraphs_gb300.engine import Graph
+  a = generators.grid2d(200) if kind == "grid200" else _caterpillar(3000, 30)
+  with Graph(a) as g:
+    took = {}
+    for k in (8, 64):
+      roots = list(range(k))
+      lv, pa = (torch.empty((k, a.n), dtype=torch.int32, device="cuda") for _ in range(2))
+      for i, r in enumerate(roots):
+        g.bfs_device(r, lv[i], pa[i])
+      g.last_stats()
+      assert int(lv.max()) > 126
+      times = []
+      for _ in range(15):
+        t0 = time.perf_counter()
+        found = g.validate(roots, lv, pa)  # waits
+        times.append(time.perf_counter() - t0)
+      took[k] = sorted(times)[len(times) // 2]
+      assert all(f[c]["failures"] == 0 for f in found for c in CHECKS)
+  assert took[64] < 4 * took[8], took
