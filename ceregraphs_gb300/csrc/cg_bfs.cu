@@ -48,12 +48,6 @@ constexpr int kBfsBlock = 512;
 constexpr int kPullThreadScan = 4;
 constexpr unsigned kPullLaneMax = 32;
 constexpr int kBfsWarps = kBfsBlock / 32;
-// Vertices a warp from which on a bitmap-wide round hands its items out from a
-// counter, two a warp; below, one item a warp takes fewer trips than the balance
-// is worth (525,000 unvisited vertices, 72 a warp, R-MAT scale 20: 16 us instead
-// of 21; scale 23, 500 a warp: 1.7 times slower without).
-constexpr unsigned long long kHeavyWork = 128;
-
 // Per-warp shared memory of the bitmap-wide rounds: a staged tile (its words
 // and the exclusive prefix of their popcounts, so that a lane can select the
 // k-th set bit) and the tile's next-frontier words found by a pull round.
@@ -953,11 +947,13 @@ struct SearchState {
 // the search), the direction of round L + 1, and block 0's record of the
 // round.  nf, mf, vd: the next frontier's vertices, their out-degrees and (in
 // a pull round) in-degrees summed.  solo_max, solo_edges: the largest frontier
-// block 0 takes alone.  Thread 0 of a block calls; returns the payload.
+// block 0 takes alone.  heavy_work: kHeavyWork or the search's own.  Thread 0 of a
+// block calls; returns the payload.
 __device__ __forceinline__ unsigned close_round(const BfsParams &p, int L, int dir,
                                                 unsigned long long nf, unsigned long long mf,
                                                 unsigned long long vd, unsigned solo_max,
-                                                unsigned solo_edges, SearchState &ss) {
+                                                unsigned solo_edges, unsigned long long heavy_work,
+                                                SearchState &ss) {
   BfsCtl *ctl = p.ctl;
   ss.pull_rounds += dir == kPull ? 1 : 0;
   ss.visited += nf;
@@ -999,7 +995,7 @@ __device__ __forceinline__ unsigned close_round(const BfsParams &p, int L, int d
   const unsigned long long work =
       next == kPull ? (p.live > (int64_t)ss.visited ? (unsigned long long)p.live - ss.visited : 0ull)
                     : nf;
-  const bool heavy = work >= kHeavyWork * (unsigned long long)((gridDim.x * blockDim.x) >> 5);
+  const bool heavy = work >= heavy_work * (unsigned long long)((gridDim.x * blockDim.x) >> 5);
   // (after a pull round of a directed graph the edges are not known: vd stands
   // for them)
   const bool solo = !done && next == kPush && nf <= solo_max &&
@@ -1038,7 +1034,8 @@ __device__ unsigned round_decision(const BfsParams &p, int L, int dir, SearchSta
   if constexpr (kWide) {
     const unsigned long long edges = qbig & BigWord<true>::kEdges;
     ss.next_big = ((qbig >> BigWord<true>::kShift) << 32) | (uint32_t)edges;
-    return close_round(p, L, dir, nf, mf, vd, 0u, 0u, ss) | (edges >= kEdges32 ? kUnqueued : 0u);
+    return close_round(p, L, dir, nf, mf, vd, 0u, 0u, kHeavyWork, ss) |
+           (edges >= kEdges32 ? kUnqueued : 0u);
   }
   ss.next_big = qbig;
   // one block takes over well below what it can hold, so that a frontier near
@@ -1049,11 +1046,13 @@ __device__ unsigned round_decision(const BfsParams &p, int L, int dir, SearchSta
     const bool steady = 4 * nf >= 3 * ss.prev_nf && 4 * nf <= 5 * ss.prev_nf;
     if (dir == kPush && steady && (nf > (unsigned)kSoloMax / 2 || mf > kSoloEnter) &&
         team_size()) {
-      const unsigned x = close_round(p, L, dir, nf, mf, vd, kTeam * kSoloMax / 4, kTeamEdges / 2, ss);
+      const unsigned x = close_round(p, L, dir, nf, mf, vd, kTeam * kSoloMax / 4, kTeamEdges / 2,
+                                     kHeavyWork, ss);
       return (x & kSolo) ? x | kHandOver : x;
     }
   }
-  return close_round(p, L, dir, nf, mf, vd, kSoloMax / 2, kSoloEnter, ss);
+  return close_round(p, L, dir, nf, mf, vd, kSoloMax / 2, kSoloEnter,
+                     kTeamed ? kHeavyWork : p.heavy_work, ss);
 }
 
 // ---- small rounds on one block -------------------------------------------------
@@ -1297,7 +1296,7 @@ __device__ __noinline__ unsigned team_rounds(const BfsParams &p, SearchState &ss
         if ((x >> 40) & 0xffu) mfs += __ldcg(&R->mf);
         const bool lists_fit = ((x >> 48) & 0x7fu) == 0;
         pay = close_round(p, L, kPush, nfs, mfs, mfs, lists_fit ? kTeam * kSoloMax / 2 : 0u,
-                          kTeamEdges, ss);
+                          kTeamEdges, kHeavyWork, ss);
         S.d[c][0] = (uint32_t)min(mfs, 0xffffffffull);  // F_L's degrees are done with
         // hand back what one block runs faster, and before the waits' time limit
         S.x[0] = (mfs < kTeamLeave && nfs <= (unsigned)kSoloMax / 2) || ((x >> 55) & 1u);
@@ -1468,7 +1467,8 @@ __device__ __forceinline__ unsigned solo_rounds(const BfsParams &p, SoloShared &
         // would be too large anyway, and the lists of new parts of the graph are
         // cold (directed ER, 3,363 claims from 3,320 edges: 17 us here, 11 there)
         const unsigned room = min(kSoloEdges, max(kSoloEdges / 4, 2 * E));
-        unsigned x = close_round(p, L, kPush, nf, mf, mf, kSoloMax, room, ss);
+        unsigned x = close_round(p, L, kPush, nf, mf, mf, kSoloMax, room,
+                                 kTeamed ? kHeavyWork : p.heavy_work, ss);
         if ((x & kSolo) && (++ran >= kSoloSession || ss.t_mark - t0 > session_ns)) {
           // the waiting blocks' time limit: let them through to the next wait
           ctl->solo.still = 1;
@@ -2098,6 +2098,12 @@ int bfs_prepare(cg_graph *g) {
   return CG_OK;
 }
 
+// The search pulls from its first rounds on.
+static bool pulls_early(const cg_graph *g) {
+  return g->opt.direction == CG_DIR_BOTTOMUP ||
+         (g->opt.direction == CG_DIR_TAU && g->opt.tau_switch_count < g->n / 256);
+}
+
 // Blocks per SM of a search whose options leave it open, at most what fits (3).
 // Fewer blocks make every round's barrier cheaper, and with one the searches of
 // three handles run side by side (R-MAT n = 4 K, three handles in turn: 55 -> 19
@@ -2107,10 +2113,18 @@ int bfs_prepare(cg_graph *g) {
 // 128, 4 M 177 / 183 / 230; directed ER 300 K 100 / 93 / 90, 1 M 139 / 136 / 147, 3
 // M 292 / 305 / 374; a 1000^2 grid is the same with all.  Top-down, which pushes
 // every edge: R-MAT 16 K (0.4 M entries) 56 / 56 / 57, 64 K (1.8 M) 76 / 77 / 92,
-// 256 K 136 / 159 / 204; ER 100 K (0.8 M) 94 / 90 / 94.
+// 256 K 136 / 159 / 204; ER 100 K (0.8 M) 94 / 90 / 94.  Searches that pull from the
+// start scan whole lists, a hub's by one warp together with its neighbours' (the
+// more warps, the fewer of them): bottom-up R-MAT 64 K of degree 16 93 / 84 / 79, 128
+// K of degree 128 789 / 769 / 746, 256 K of 32 122 / 116 / 124, 1 M of 4 876 / 1,076 /
+// 1,618, 2 M of 16 5,560 / 7,446 / 12,211; ER 250 K of 64 203 / 172 / 239.  A one-way
+// switch at 15% of the vertices pushes most edges first: R-MAT 128 K of degree 128
+// 158 / 168 / 220, 1 M of 32 149 / 203 / 247, but 256 K of 32 (14 M entries) 76 / 72 / 71.
 static int blocks_for(const cg_graph *g) {
   if (g->opt.direction == CG_DIR_TOPDOWN)
     return g->nnz < (1 << 19) ? 1 : (g->nnz < (1 << 20) ? 2 : 3);
+  if (pulls_early(g)) return g->n <= (1 << 17) ? 1 : (g->n <= (1 << 18) ? 2 : 3);
+  if (g->opt.direction == CG_DIR_TAU && g->nnz >= (1 << 24)) return 3;
   if (g->n <= 300000 || g->nnz < (1 << 22)) return 1;
   return g->n <= (1 << 21) ? 2 : 3;
 }
@@ -2174,6 +2188,7 @@ int bfs_launch(cg_graph *g, int64_t root, int32_t *d_levels, int32_t *d_parents,
                                      : (int)((g->n + 1) < 0x7fffffff ? g->n + 1 : 0x7fffffff);
   p.timeout_ns = (long long)(g->opt.wait_timeout_ms > 0 ? g->opt.wait_timeout_ms : 1000) * 1000000ll;
   p.unmatched_wait = g->opt.test_unmatched_wait;
+  p.heavy_work = g->head && pulls_early(g) ? kHeavyWorkEarly : kHeavyWork;
   // every launch starts from a clean control block (round records, wait counter)
   CG_CUDA(cudaMemsetAsync(g->ctl, 0, sizeof(BfsCtl), g->stream));
   cudaLaunchConfig_t cfg = {};

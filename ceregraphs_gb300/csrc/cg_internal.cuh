@@ -151,7 +151,20 @@ struct BfsParams {
   int level_cap;
   long long timeout_ns;
   int unmatched_wait;
+  unsigned heavy_work;   // vertices a warp of a heavy bitmap-wide round (kHeavyWork)
 };
+
+// Vertices a warp from which on a bitmap-wide round hands its items out from a
+// counter, two a warp; below, one item a warp takes fewer trips than the balance
+// is worth (525,000 unvisited vertices, 72 a warp, R-MAT scale 20: 16 us instead
+// of 21; scale 23, 500 a warp: 1.7 times slower without).
+constexpr unsigned kHeavyWork = 128;
+// The same for a search that pulls before its time on a graph with hubs: no list
+// ends early, so the hubs' lists, next to each other in one item, are a round's
+// length, and smaller items halve it (R-MAT scale 20 of degree 4, all rounds
+// pulled: 1,313 us with 128, 876 with 32; without hubs 128 stays better, directed
+// ER of 1 M vertices and degree 2: 627 and 708).
+constexpr unsigned kHeavyWorkEarly = 32;
 
 }  // namespace cg
 

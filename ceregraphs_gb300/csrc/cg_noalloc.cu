@@ -163,6 +163,7 @@ extern "C" int cg_bfs_noalloc(int64_t n, int64_t nnz, const int64_t *d_in_off,
   p.level_cap = (int)((n + 1) < 0x7fffffff ? n + 1 : 0x7fffffff);
   p.timeout_ns = 1000ll * 1000000ll;
   p.unmatched_wait = 0;
+  p.heavy_work = kHeavyWork;
   // The array keeps the previous call's contents: the round records and the
   // grid-wait counter must start at zero (bitmaps and outputs are reset by the
   // kernel itself); the memset is enqueued below, after the argument checks.
