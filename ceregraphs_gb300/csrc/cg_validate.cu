@@ -141,7 +141,7 @@ __device__ __forceinline__ uint32_t byte_flags(unsigned m) {
 }
 
 template <int NW>
-__global__ void __launch_bounds__(kBlock) pack_levels_kernel(GroupArgs a) {
+__device__ __forceinline__ void pack_levels(const GroupArgs &a) {
   const int64_t v = (int64_t)blockIdx.x * kBlock + threadIdx.x;
   if (v >= a.n) return;
   uint32_t x[NW];
@@ -289,7 +289,7 @@ __device__ __forceinline__ int32_t warp_entries(const GroupArgs &a, int64_t v, i
 // once, after the list: the level of one that is the list's first vertex a level
 // up needs no look (16 M byte gathers less, 338 -> 330 us).
 template <int NW>
-__global__ void __launch_bounds__(kBlock, 4) check_vertices_kernel(GroupArgs a) {
+__device__ __forceinline__ void check_vertices(const GroupArgs &a) {
   if (*(volatile int *)a.wide) return;
   const int lane = threadIdx.x & 31;
   const int64_t v = (int64_t)blockIdx.x * kBlock + threadIdx.x;
@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(kBlock, 4) check_vertices_kernel(GroupArgs a) 
 // parents are known to be in the lists, so LOWEST fails exactly when a chunk
 // holds an entry one level up below the parent; `bad` counts it once.
 template <int NW>
-__global__ void __launch_bounds__(kBlock, 4) check_long_kernel(GroupArgs a) {
+__device__ __forceinline__ void check_long(const GroupArgs &a) {
   if (*(volatile int *)a.wide) return;
   const unsigned long long total = *(volatile unsigned long long *)a.nlong;
   const unsigned nv = (unsigned)(total >> 32), nchunks = (unsigned)total;
@@ -475,6 +475,44 @@ __global__ void __launch_bounds__(kBlock, 4) check_long_kernel(GroupArgs a) {
     if (!(atomicOr(a.bad + (int64_t)lo * NW + (lane >> 2), bit) & bit))
       flag(a.tally + lane, CG_CHECK_LOWEST, v);
   }
+}
+
+template <int NW>
+__global__ void __launch_bounds__(kBlock) pack_levels_kernel(GroupArgs a) { pack_levels<NW>(a); }
+template <int NW>
+__global__ void __launch_bounds__(kBlock, 4) check_vertices_kernel(GroupArgs a) {
+  check_vertices<NW>(a);
+}
+template <int NW>
+__global__ void __launch_bounds__(kBlock, 4) check_long_kernel(GroupArgs a) { check_long<NW>(a); }
+
+// The same for full groups side by side, group `a` + blockIdx.y; long_cap: entries
+// of each one's longs, pend and bad.
+__device__ __forceinline__ GroupArgs beside(const GroupArgs &first, int64_t long_cap) {
+  GroupArgs a = first;
+  const int64_t y = blockIdx.y;
+  a.roots += y * kGroup;
+  a.levels += y * kGroup * a.n;
+  a.parents += y * kGroup * a.n;
+  a.tally += y * kGroup;
+  a.wide += y;
+  a.nlong += y;
+  a.lv += y * a.n * (kGroup / 4);
+  a.longs += y * long_cap;
+  a.pend += y * long_cap * (kGroup / 4);
+  a.bad += y * long_cap * (kGroup / 4);
+  return a;
+}
+__global__ void __launch_bounds__(kBlock) pack_levels_beside_kernel(GroupArgs a, int64_t long_cap) {
+  pack_levels<kGroup / 4>(beside(a, long_cap));
+}
+__global__ void __launch_bounds__(kBlock, 4) check_vertices_beside_kernel(GroupArgs a,
+                                                                          int64_t long_cap) {
+  check_vertices<kGroup / 4>(beside(a, long_cap));
+}
+__global__ void __launch_bounds__(kBlock, 4) check_long_beside_kernel(GroupArgs a,
+                                                                      int64_t long_cap) {
+  check_long<kGroup / 4>(beside(a, long_cap));
 }
 
 // ---- one search at a time, any level ------------------------------------------
@@ -616,12 +654,20 @@ int64_t long_capacity(const cg_graph *g) {
   return c < g->n ? c : g->n;
 }
 
-// The handle's workspace for `nw` level words per vertex (kept for later
-// calls, freed with the handle); false when it cannot be had, and the
+// Full groups side by side: as many as fill the GPU, 8 blocks an SM, one vertex a
+// thread.
+int groups_beside(const cg_graph *g, int full) {
+  const int64_t blocks = (g->n + kBlock - 1) / kBlock, most = (int64_t)g->num_sms * 8 / blocks;
+  const int64_t side = most < full ? most : full;
+  return side < 1 ? 1 : (int)side;
+}
+
+// The handle's workspace for `groups` groups of `nw` level words per vertex (kept
+// for later calls, freed with the handle); false when it cannot be had, and the
 // per-search kernels, which need none, do the work.
-bool check_workspace(cg_graph *g, int nw, GroupArgs *a) {
-  const size_t nl = (size_t)long_capacity(g);
-  const size_t lv = round256(sizeof(uint32_t) * nw * (size_t)g->n);
+bool check_workspace(cg_graph *g, int nw, int groups, GroupArgs *a) {
+  const size_t nl = (size_t)long_capacity(g) * groups;
+  const size_t lv = round256(sizeof(uint32_t) * nw * (size_t)g->n * groups);
   const size_t longs = round256(sizeof(LongVertex) * nl), mask = round256(sizeof(uint32_t) * nw * nl);
   const size_t bytes = lv + longs + 2 * mask;
   if (g->check_bytes < bytes) {
@@ -653,17 +699,29 @@ void launch_group(const cg_graph *g, const GroupArgs &a) {
   check_long_kernel<NW><<<(unsigned)g->num_sms * 6, kBlock, 0, g->stream>>>(a);
 }
 
+// Groups a .. a + groups - 1, 16 searches each, at once: a small graph's group
+// leaves most of the GPU idle (64 searches of R-MAT scale 12: 553 us a call with the
+// groups in turn, 288 so; scale 16: 597 and 366).
+void launch_groups(const cg_graph *g, const GroupArgs &a, int groups) {
+  const dim3 vb((unsigned)((g->n + kBlock - 1) / kBlock), (unsigned)groups);
+  const int64_t cap = long_capacity(g);
+  pack_levels_beside_kernel<<<vb, kBlock, 0, g->stream>>>(a, cap);
+  check_vertices_beside_kernel<<<vb, kBlock, 0, g->stream>>>(a, cap);
+  const dim3 lb((unsigned)((g->num_sms * 6 + groups - 1) / groups), (unsigned)groups);
+  check_long_beside_kernel<<<lb, kBlock, 0, g->stream>>>(a, cap);
+}
+
 // Grid of a per-search kernel, one search filling `blocks` blocks: at most 8
-// blocks an SM for a search, and as many searches side by side (blockIdx.y, the
-// rest in turn) as come to four times that.  One after another, the searches of a
-// small deep graph leave the GPU idle: 64 of a 200^2 grid took 2,960 us a call, 336
-// so; of a caterpillar of 3,000 vertices with 30 leaves each 9,760 and 495.  No
-// more, so that the launch stays short where the groups have done all of it.
-constexpr int64_t kSideBySide = 4;
+// blocks an SM for a search, and searches side by side (blockIdx.y, the rest in
+// turn) up to four times that, k / 8 times from 32 searches on.  One after another,
+// the searches of a small deep graph leave the GPU idle: 64 of a 200^2 grid took
+// 2,960 us a call, 302 so; of a caterpillar of 3,000 vertices with 30 leaves each
+// 9,760 and 460.  No more, so that the launch stays short where the groups have done
+// all of it (16 searches of R-MAT scale 20, 665 us: 8 us longer with 16 times).
 dim3 search_grid(const cg_graph *g, int64_t blocks, int k) {
   const int64_t cap = (int64_t)g->num_sms * 8;
   const int64_t x = blocks < cap ? blocks : cap;
-  const int64_t side = (kSideBySide * cap + x - 1) / x;
+  const int64_t side = ((k / 8 > 4 ? k / 8 : 4) * cap + x - 1) / x;
   return dim3((unsigned)x, (unsigned)(side < k ? side : k));
 }
 
@@ -707,14 +765,15 @@ extern "C" int cg_validate_device(cg_graph *g, const int64_t *roots, int32_t k,
     tally_init_kernel<<<(k * kChecks + 255) / 256, 256, 0, g->stream>>>(d_t, k);
     GroupArgs a{};
     const int most = k < kGroup ? k : kGroup;
-    const bool grouped = check_workspace(g, most <= 4 ? 1 : (most <= 8 ? 2 : 4), &a);
+    const int side = groups_beside(g, k / kGroup);
+    const bool grouped = check_workspace(g, most <= 4 ? 1 : (most <= 8 ? 2 : 4), side, &a);
     if (grouped) {
       a.n = g->n;
       a.in_off = g->in_off;
       a.in_idx = g->in_idx;
       a.warp_list = g->n >= kLargeGraph ? kWarpListLarge : kWarpList;
       a.chunk_bits = g->n >= kLargeGraph ? kChunkBitsLarge : kChunkBits;
-      for (int i = 0; i < groups; ++i) {
+      for (int i = 0, now; i < groups; i += now) {
         const int64_t s0 = (int64_t)i * kGroup;
         a.roots = d_roots + s0;
         a.levels = d_levels + s0 * g->n;
@@ -723,9 +782,17 @@ extern "C" int cg_validate_device(cg_graph *g, const int64_t *roots, int32_t k,
         a.tally = d_t + s0;
         a.wide = d_wide + i;
         a.nlong = d_nlong + i;
-        if (a.searches <= 4) launch_group<1>(g, a);
-        else if (a.searches <= 8) launch_group<2>(g, a);
-        else launch_group<4>(g, a);
+        now = 1;
+        if (side > 1 && a.searches == kGroup) {
+          now = k / kGroup - i < side ? k / kGroup - i : side;
+          launch_groups(g, a, now);
+        } else if (a.searches <= 4) {
+          launch_group<1>(g, a);
+        } else if (a.searches <= 8) {
+          launch_group<2>(g, a);
+        } else {
+          launch_group<4>(g, a);
+        }
       }
     }
     // the searches the groups left (levels past a byte), or all of them

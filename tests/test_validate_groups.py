@@ -145,3 +145,53 @@ def test_deep_searches_side_by_side(built_lib, kind):
       took[k] = sorted(times)[len(times) // 2]
       assert all(f[c]["failures"] == 0 for f in found for c in CHECKS)
   assert took[64] < 4 * took[8], took
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,k", [(3001, 32), (3001, 70), (100_003, 64)])
+def test_groups_side_by_side_match_oracle(built_lib, oracle_mod, n, k):
+  """Full groups of 16 searches run side by side on small graphs: all of them, the
+  last of fewer searches alone, and (100,003 vertices) three at a time."""
+  import torch
+  from ceregraphs_gb300.engine import Graph
+  a = _degrees_graph(n, 9)
+  rng = np.random.default_rng(k)
+  out_off, out_idx = a.out_lists()
+  roots = [0] + rng.integers(0, a.n, k - 1).tolist()
+  L, P = np.empty((k, a.n), np.int32), np.empty((k, a.n), np.int32)
+  for i, r in enumerate(roots):
+    L[i], P[i], _ = oracle_mod.bfs(out_off, out_idx, a.in_off, a.in_idx, r)
+    if i % 3 != 1:
+      L[i], P[i] = _damage(L[i], P[i], a.n, rng, 1 + 7 * (i % 3))
+  L[20, 7] = 126  # past a byte: the second group's searches one at a time
+  with Graph(a) as g:
+    for _ in range(2):
+      got = g.validate(roots, torch.from_numpy(L).cuda(), torch.from_numpy(P).cuda())
+      for i, r in enumerate(roots):
+        want = oracle_mod.validation_counts(a.in_off, a.in_idx, r, L[i], P[i])
+        for c in CHECKS:
+          assert (got[i][c]["failures"], got[i][c]["first"]) == want[c], (i, c, got[i], want)
+
+
+@pytest.mark.gpu
+def test_groups_of_a_small_graph_take_little_longer_than_one(built_lib):
+  """Four groups in turn take more than three times as long as one; the GPU has
+  room for all of a small graph's at once."""
+  import time
+  import torch
+  from ceregraphs_gb300.engine import Graph
+  a = generators.rmat(12, 16, 4)
+  with Graph(a) as g:
+    took = {}
+    for k in (16, 64):
+      roots = np.nonzero(np.diff(a.in_off))[0][:k].tolist()
+      lv, pa = (torch.empty((k, a.n), dtype=torch.int32, device="cuda") for _ in range(2))
+      g.msbfs_device(roots, lv, pa)
+      g.last_stats()
+      times = []
+      for _ in range(15):
+        t0 = time.perf_counter()
+        g.validate(roots, lv, pa)  # waits
+        times.append(time.perf_counter() - t0)
+      took[k] = sorted(times)[len(times) // 2]
+  assert took[64] < 2.5 * took[16], took
