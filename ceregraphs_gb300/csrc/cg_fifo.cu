@@ -7,8 +7,8 @@
 // (rank of the parent, vertex id).
 //
 // Given the levels of a finished search, this pass recomputes the parents
-// level by level.  A stable sort of the vertices by level (one 8-bit pass up to
-// 254 levels) lists each level in id order.  Level L's ranks reach level L+1
+// level by level.  The vertices are first listed by level, each level in id order
+// (fifo_list_kernel).  Level L's ranks reach level L+1
 // from whichever side has fewer list entries -- each vertex takes the minimum
 // over its in-list of a 4-byte rank map, or level L's out-lists push their ranks
 // by atomicMin -- and a stable sort of level L+1 by parent rank, as few bits as
@@ -18,9 +18,9 @@
 // stream (and is refused inside a graph capture).
 //
 // Bound by the dependent launches of a level (about nine, 3 to 10 us each) and
-// by the rank gathers of the widest levels.  R-MAT scale 20, device time with
-// the search: 1319 us with a warp per vertex, 64-bit sorts and one block for
-// levels of few vertices but long lists, 418 us now.
+// by the rank gathers of the widest levels.  R-MAT scale 20, a call with its
+// search: 1,296 us with a warp per vertex, 64-bit sorts and one block for levels of
+// few vertices but long lists, 414 us now.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -59,6 +59,7 @@ struct FifoState {
   uint32_t *key[2] = {nullptr, nullptr};  // [n] sort keys
   int32_t *queue[3] = {nullptr, nullptr, nullptr};  // [n] a level in queue order, and sort values
   unsigned *counts = nullptr;     // [n + 1] vertices per level
+  unsigned *block_counts = nullptr;  // [kListDigits][list_blocks + 1] of the listing passes
   FifoLong *longs = nullptr;
   void *temp = nullptr;           // radix sort scratch
   size_t temp_bytes = 0;
@@ -78,15 +79,27 @@ constexpr int64_t kFifoLane = 32;    // in-lists up to this: one thread
 constexpr int64_t kFifoWarp = 1024;  // lists up to this: the warp that meets them; above: chunks
 constexpr int64_t kFifoChunk = 512;
 
+// A listing pass's blocks have a run of items each, of the graph's vertices 4 blocks
+// an SM.
+constexpr int kListDigits = 256;
+static_assert(kFifoSums <= kListDigits && kFifoBlock == kListDigits, "a thread per digit");
+int64_t list_run(int64_t n, int sms) {
+  const int64_t run = (n + 4 * (int64_t)sms - 1) / (4 * (int64_t)sms);
+  return (run + kFifoBlock - 1) / kFifoBlock * kFifoBlock;
+}
+unsigned list_blocks(int64_t items, int64_t run) { return (unsigned)((items + run - 1) / run); }
+
 // Vertices per level (levels >= 0), their degrees summed (the first kFifoSums
-// levels), and the deepest level.  One round of shared atomics per level
+// levels), and the deepest level; block_counts: the first kFifoSums levels' counts
+// by block, for fifo_list_kernel (the same grid and run).  One round of shared atomics per level
 // present in a warp, then one global atomic a block and value: a maximum from
 // each of 9,700 warps to one address, and the sums of 2,400 blocks, were most of its
 // 20 us on R-MAT scale 20 (the whole call 294 -> 282 us with 4 blocks an SM; 286 with
 // 2, 288 with 8 or 16).
 __global__ void __launch_bounds__(kFifoBlock) fifo_hist_kernel(
-    int64_t n, const int32_t *__restrict__ levels, const int64_t *__restrict__ in_off,
-    const int64_t *__restrict__ out_off, unsigned *counts, FifoSums *sums) {
+    int64_t n, int64_t run, const int32_t *__restrict__ levels,
+    const int64_t *__restrict__ in_off, const int64_t *__restrict__ out_off, unsigned *counts,
+    unsigned *block_counts, FifoSums *sums) {
   __shared__ unsigned s_count[kFifoSums];
   __shared__ unsigned long long s_out[kFifoSums], s_in[kFifoSums];
   __shared__ int s_max;
@@ -95,10 +108,10 @@ __global__ void __launch_bounds__(kFifoBlock) fifo_hist_kernel(
   __syncthreads();
   const int lane = lane_id();
   int mx = -1;
-  for (int64_t base = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~31ll; base < n;
-       base += (int64_t)gridDim.x * blockDim.x) {
+  const int64_t end = min(n, (blockIdx.x + 1) * run);
+  for (int64_t base = blockIdx.x * run + (threadIdx.x & ~31u); base < end; base += kFifoBlock) {
     const int64_t v = base + lane;
-    const int L = v < n ? levels[v] : -1;
+    const int L = v < end ? levels[v] : -1;
     unsigned din = 0, dout = 0;
     if (L >= 0 && L < kFifoSums) {
       din = (unsigned)(__ldg(in_off + v + 1) - __ldg(in_off + v));
@@ -127,19 +140,161 @@ __global__ void __launch_bounds__(kFifoBlock) fifo_hist_kernel(
   if (lane == 0 && mx >= 0) atomicMax(&s_max, mx);
   __syncthreads();
   if (threadIdx.x == 0 && s_max >= 0) atomicMax(&sums->maxlevel, s_max);
-  for (int i = threadIdx.x; i < kFifoSums; i += blockDim.x)
+  for (int i = threadIdx.x; i < kFifoSums; i += blockDim.x) {
+    block_counts[i * gridDim.x + blockIdx.x] = s_count[i];
     if (s_count[i]) {
       atomicAdd(&counts[i], s_count[i]);
       atomicAdd(&sums->counts[i], s_count[i]);
       atomicAdd(&sums->in[i], s_in[i]);
       atomicAdd(&sums->out[i], s_out[i]);
     }
+  }
 }
 
-__global__ void fifo_iota_kernel(int64_t n, int32_t *x) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    x[i] = (int32_t)i;
+// One pass of the listing: the items (in[0 .. count), or all vertices below `count`
+// that were reached) in the order of digit (level >> shift) & 255, items of one
+// digit in the order they came in.  Up to kFifoSums levels fifo_hist_kernel has
+// counted the blocks' digits and one pass lists them; deeper searches take a pass
+// per 8 bits of the level, lowest first, with fifo_digits_kernel and
+// fifo_scan_kernel before each.
+__device__ __forceinline__ int list_digit(const int32_t *__restrict__ in,
+                                          const int32_t *__restrict__ levels, int shift, int64_t i,
+                                          int64_t end, int32_t &v) {
+  v = i < end ? (in ? __ldg(in + i) : (int32_t)i) : -1;
+  const int L = v >= 0 ? __ldg(levels + v) : -1;
+  return L < 0 ? -1 : (L >> shift) & (kListDigits - 1);
+}
+
+__global__ void __launch_bounds__(kFifoBlock) fifo_digits_kernel(
+    int64_t count, int64_t run, const int32_t *__restrict__ in,
+    const int32_t *__restrict__ levels, int shift, unsigned *__restrict__ block_counts) {
+  __shared__ unsigned s[kListDigits];
+  s[threadIdx.x] = 0;
+  __syncthreads();
+  const int64_t end = min(count, (blockIdx.x + 1) * run);
+  const int lane = lane_id();
+  for (int64_t base = blockIdx.x * run + (threadIdx.x & ~31u); base < end; base += kFifoBlock) {
+    int32_t v;
+    const int d = list_digit(in, levels, shift, base + lane, end, v);
+    const unsigned peers = __match_any_sync(kAll, d);
+    if (d >= 0 && lane == __ffs(peers) - 1) atomicAdd(&s[d], (unsigned)__popc(peers));
+  }
+  __syncthreads();
+  block_counts[threadIdx.x * gridDim.x + blockIdx.x] = s[threadIdx.x];
+}
+
+// Each digit's counts become the items of that digit in the blocks before; totals:
+// in all of them.  A warp per digit.
+__global__ void __launch_bounds__(kFifoBlock) fifo_scan_kernel(unsigned blocks, int digits,
+                                                               unsigned *block_counts,
+                                                               unsigned *__restrict__ totals) {
+  const int lane = lane_id(), d = (int)warp_id_global();
+  if (d >= digits) return;
+  unsigned *row = block_counts + d * blocks, carry = 0;
+  for (unsigned b0 = 0; b0 < blocks; b0 += 32) {
+    const unsigned b = b0 + lane, mine = b < blocks ? row[b] : 0u;
+    unsigned incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned x = __shfl_up_sync(kAll, incl, o);
+      if (lane >= o) incl += x;
+    }
+    if (b < blocks) row[b] = carry + incl - mine;
+    carry += __shfl_sync(kAll, incl, 31);
+  }
+  if (lane == 0) totals[d] = carry;
+}
+
+// A warp has a run of items of its own: it counts their digits, learns where each
+// digit's items of this block begin (after those of lower digits, and of the same
+// digit in the blocks before: totals and block_counts after fifo_scan_kernel, or, for
+// few digits, `totals` null, each block sums the counts for itself), and goes through
+// its items again.  digits: that occur, at most.  Bound by its chain of dependent
+// steps and the scattered stores: R-MAT scale 20 (1 M vertices, 8 levels) 12 us, where
+// a radix sort of (level, id) pairs took 27; 93,000 vertices on 1,552 levels, two
+// passes of three kernels, 27 us for 30.
+__global__ void __launch_bounds__(kFifoBlock) fifo_list_kernel(
+    int64_t count, int64_t run, const int32_t *__restrict__ in,
+    const int32_t *__restrict__ levels, int shift, int digits,
+    const unsigned *__restrict__ block_counts, const unsigned *__restrict__ totals,
+    int32_t *__restrict__ out) {
+  constexpr int kWarps = kFifoBlock / 32;
+  __shared__ unsigned s_at[kWarps][kListDigits];
+  __shared__ unsigned s_all[kListDigits], s_before[kListDigits], s_warp[kWarps];
+  const int lane = lane_id(), wib = threadIdx.x >> 5, t = threadIdx.x;
+  for (int d = lane; d < digits; d += 32) s_at[wib][d] = 0;
+  __syncwarp();
+  const int64_t first = blockIdx.x * run + wib * (run / kWarps);
+  const int64_t end = min(count, first + run / kWarps);
+  for (int64_t base = first; base < end; base += 32) {
+    int32_t v;
+    const int d = list_digit(in, levels, shift, base + lane, end, v);
+    const unsigned peers = __match_any_sync(kAll, d);
+    if (d >= 0 && lane == __ffs(peers) - 1) s_at[wib][d] += (unsigned)__popc(peers);
+    __syncwarp();
+  }
+  if (totals) {
+    if (t < digits) {
+      s_all[t] = __ldg(totals + t);
+      s_before[t] = __ldg(block_counts + t * gridDim.x + blockIdx.x);
+    }
+  } else {
+    for (int d = wib; d < digits; d += kWarps) {
+      unsigned all = 0, before = 0;
+      for (unsigned b0 = lane; b0 < gridDim.x; b0 += 128) {
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {  // in flight at once
+          const unsigned b = b0 + 32 * h;
+          const unsigned x = b < gridDim.x ? __ldg(block_counts + d * gridDim.x + b) : 0u;
+          all += x;
+          before += b < blockIdx.x ? x : 0u;
+        }
+      }
+      all = __reduce_add_sync(kAll, all);
+      before = __reduce_add_sync(kAll, before);
+      if (lane == 0) {
+        s_all[d] = all;
+        s_before[d] = before;
+      }
+    }
+  }
+  __syncthreads();
+  {  // a thread per digit: its first place, and each warp's
+    const unsigned mine = t < digits ? s_all[t] : 0u;
+    unsigned incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned x = __shfl_up_sync(kAll, incl, o);
+      if (lane >= o) incl += x;
+    }
+    if (lane == 31) s_warp[wib] = incl;
+    __syncthreads();
+    unsigned at = incl - mine;
+    for (int w = 0; w < wib; ++w) at += s_warp[w];
+    if (t < digits) {
+      at += s_before[t];
+      for (int w = 0; w < kWarps; ++w) {
+        const unsigned x = s_at[w][t];
+        s_at[w][t] = at;
+        at += x;
+      }
+    }
+  }
+  __syncthreads();
+  for (int64_t base = first; base < end; base += 32) {
+    int32_t v;
+    const int d = list_digit(in, levels, shift, base + lane, end, v);
+    const unsigned peers = __match_any_sync(kAll, d);
+    const int leader = __ffs(peers) - 1;
+    unsigned at = 0;
+    if (d >= 0 && lane == leader) {
+      at = s_at[wib][d];
+      s_at[wib][d] = at + (unsigned)__popc(peers);
+    }
+    at = __shfl_sync(kAll, at, leader);
+    if (d >= 0) out[at + __popc(peers & ((1u << lane) - 1u))] = v;
+    __syncwarp();
+  }
 }
 
 // The rank map of level L (rk is ~0 elsewhere).
@@ -352,6 +507,7 @@ __global__ void fifo_leave_kernel(const int32_t *__restrict__ seg, unsigned coun
 }
 
 // Runs of levels of at most kSmallLevel vertices and kSmallEdges list entries
+// (counted for the first kFifoSums levels only; the vertices bound those behind)
 // are handled by one block, many levels to a launch, with no sort: level L+1's queue is level L's queue in
 // order with each vertex's children (the out-neighbours whose FIFO parent it
 // is) appended in out-list order, which is ascending -- the same order the
@@ -568,12 +724,7 @@ int fifo_state(cg_graph *g, FifoState **out) {
   {
     cub::DoubleBuffer<uint32_t> k(nullptr, nullptr);
     cub::DoubleBuffer<int32_t> v(nullptr, nullptr);
-    size_t by_rank = 0, by_level = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, by_rank, k, v, (int64_t)n, 0, 32, g->stream);
-    cub::DeviceRadixSort::SortPairs(nullptr, by_level, (const uint32_t *)nullptr,
-                                    (uint32_t *)nullptr, (const int32_t *)nullptr,
-                                    (int32_t *)nullptr, (int64_t)n, 0, 32, g->stream);
-    f->temp_bytes = by_rank > by_level ? by_rank : by_level;
+    cub::DeviceRadixSort::SortPairs(nullptr, f->temp_bytes, k, v, (int64_t)n, 0, 32, g->stream);
   }
   const size_t nlongs = (size_t)(g->nnz / (kFifoWarp + 1) + 1);
   size_t bytes = 0;
@@ -588,7 +739,9 @@ int fifo_state(cg_graph *g, FifoState **out) {
                at_counts = piece(sizeof(unsigned) * (n + 1)),
                at_longs = piece(sizeof(FifoLong) * nlongs), at_temp = piece(f->temp_bytes),
                at_offs = piece(sizeof(unsigned) * (n + 2)), at_lr = piece(8 * n),
-               at_pl = piece(8 * n);
+               at_pl = piece(8 * n),
+               at_blocks = piece(sizeof(unsigned) * kListDigits *
+                                 (list_blocks((int64_t)n, list_run((int64_t)n, g->num_sms)) + 1));
   size_t at4[9];  // 4 bytes a vertex each
   for (size_t &x : at4) x = piece(4 * n);
   if (cudaMalloc(&f->base, bytes) != cudaSuccess ||
@@ -603,6 +756,7 @@ int fifo_state(cg_graph *g, FifoState **out) {
   f->longs = reinterpret_cast<FifoLong *>(f->base + at_longs);
   f->temp = f->base + at_temp;
   f->counts = reinterpret_cast<unsigned *>(f->base + at_counts);
+  f->block_counts = reinterpret_cast<unsigned *>(f->base + at_blocks);
   f->offs = reinterpret_cast<unsigned *>(f->base + at_offs);
   f->lr = reinterpret_cast<unsigned long long *>(f->base + at_lr);
   f->pl = reinterpret_cast<unsigned long long *>(f->base + at_pl);
@@ -645,9 +799,9 @@ int fifo_parents(cg_graph *g, int64_t root, const int32_t *d_levels, int32_t *d_
                                     static_cast<unsigned char *>(first)) + last_bytes, st);
   };
   CG_CUDA(fill(f->sums, f->counts, sizeof(unsigned) * (size_t)(n + 1), 0));
-  const unsigned hist_blocks = grid_for(n, kFifoBlock, sms);
-  fifo_hist_kernel<<<hist_blocks < 4u * sms ? hist_blocks : 4u * sms, kFifoBlock, 0, st>>>(
-      n, d_levels, g->in_off, g->out_off, f->counts, f->sums);
+  const int64_t run = list_run(n, sms);
+  fifo_hist_kernel<<<list_blocks(n, run), kFifoBlock, 0, st>>>(
+      n, run, d_levels, g->in_off, g->out_off, f->counts, f->block_counts, f->sums);
   CG_CUDA(cudaGetLastError());
   FifoSums sums;
   CG_CUDA(cudaMemcpyAsync(&sums, f->sums, sizeof(sums), cudaMemcpyDeviceToHost, st));
@@ -663,16 +817,29 @@ int fifo_parents(cg_graph *g, int64_t root, const int32_t *d_levels, int32_t *d_
   }
   std::vector<unsigned> offs((size_t)maxlevel + 2, 0u);
   for (int L = 0; L <= maxlevel; ++L) offs[(size_t)L + 1] = offs[(size_t)L] + counts[(size_t)L];
-  // the vertices by level, in id order within one (unreached ones, -1, last:
-  // all bits set is past maxlevel); rk and best hold the values and the keys
-  // on their way
-  fifo_iota_kernel<<<grid_for(n, kFifoBlock, sms), kFifoBlock, 0, st>>>(
-      n, reinterpret_cast<int32_t *>(f->rk));
-  size_t tb = f->temp_bytes;
-  CG_CUDA(cub::DeviceRadixSort::SortPairs(f->temp, tb,
-                                          reinterpret_cast<const uint32_t *>(d_levels), f->best,
-                                          reinterpret_cast<const int32_t *>(f->rk), f->order, n, 0,
-                                          bits_for((uint64_t)maxlevel + 1), st));
+  // the reached vertices by level, in id order within one
+  if (maxlevel < kFifoSums) {
+    fifo_list_kernel<<<list_blocks(n, run), kFifoBlock, 0, st>>>(
+        n, run, nullptr, d_levels, 0, maxlevel + 1, f->block_counts, nullptr, f->order);
+  } else {
+    const int passes = (bits_for((uint64_t)maxlevel) + 7) / 8;
+    const int32_t *in = nullptr;
+    for (int q = 0; q < passes; ++q) {
+      const int64_t items = q ? (int64_t)offs.back() : n;
+      const unsigned blocks = list_blocks(items, run);
+      const int top = maxlevel >> (8 * q), digits = top < kListDigits ? top + 1 : kListDigits;
+      unsigned *totals = f->block_counts + (size_t)kListDigits * blocks;
+      int32_t *out = (passes - q) & 1 ? f->order : f->queue[0];
+      fifo_digits_kernel<<<blocks, kFifoBlock, 0, st>>>(items, run, in, d_levels, 8 * q,
+                                                        f->block_counts);
+      fifo_scan_kernel<<<(digits + 7) / 8, kFifoBlock, 0, st>>>(blocks, digits, f->block_counts,
+                                                                totals);
+      fifo_list_kernel<<<blocks, kFifoBlock, 0, st>>>(items, run, in, d_levels, 8 * q, digits,
+                                                      f->block_counts, totals, out);
+      in = out;
+    }
+  }
+  CG_CUDA(cudaGetLastError());
   CG_CUDA(fill(f->rk, f->best, sizeof(uint32_t) * (size_t)n, 0xff));
   auto small = [&](int L) {  // level L to L + 1 suits a run of small levels
     return counts[(size_t)L] <= (unsigned)kSmallLevel &&
@@ -739,7 +906,7 @@ int fifo_parents(cg_graph *g, int64_t root, const int32_t *d_levels, int32_t *d_
     if (L + 1 == maxlevel) break;  // the last level's order is not needed
     cub::DoubleBuffer<uint32_t> kb(f->key[0], f->key[1]);
     cub::DoubleBuffer<int32_t> vb(vals[0], vals[1]);
-    tb = f->temp_bytes;
+    size_t tb = f->temp_bytes;
     CG_CUDA(cub::DeviceRadixSort::SortPairs(f->temp, tb, kb, vb, (int64_t)c, 0, bits_for(p - 1),
                                             st));
     queue = vb.Current();

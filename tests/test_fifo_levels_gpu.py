@@ -51,3 +51,59 @@ def test_fifo_parents_of_layered_graphs(built_lib, oracle_mod, name, both):
       rl, _, _ = oracle_mod.bfs(*a.out_lists(), a.in_off, a.in_idx, r)
       assert st["status"] == 0 and np.array_equal(lv, rl)
       assert np.array_equal(pa, oracle_mod.fifo_parents(a.in_off, a.in_idx, rl, r))
+
+
+@pytest.mark.parametrize("levels", [2, 63, 64, 65, 255, 256, 257, 4000])
+def test_levels_listed_in_id_order(built_lib, oracle_mod, levels):
+  """The listing's passes (one up to 64 levels, one for each 8 bits beyond), on a
+  ragged number of vertices with levels all over the ids and half of them unreached."""
+  rng = np.random.default_rng(levels)
+  per = max(1, 12_345 // levels)
+  widths = [1] + [int(w) for w in rng.integers(1, 2 * per + 1, levels - 1)]
+  a, root = _layers(widths, 2, rng, False)
+  src = np.repeat(np.arange(a.n), np.diff(a.out_lists()[0]))
+  n = 2 * a.n + 77
+  ids = rng.permutation(n)
+  a = from_edges(n, ids[src], ids[a.out_lists()[1]])
+  root = int(ids[root])
+  rl, _, _ = oracle_mod.bfs(*a.out_lists(), a.in_off, a.in_idx, root)
+  assert rl.max() == levels - 1
+  with Graph(a) as g:
+    g.set_options(parent_rule=_lib.CG_PARENT_FIFO)
+    for _ in range(2):
+      lv, pa, _ = g.bfs(root)
+      assert np.array_equal(lv, rl)
+      assert np.array_equal(pa, oracle_mod.fifo_parents(a.in_off, a.in_idx, rl, root))
+
+
+def test_more_levels_than_two_bytes(built_lib):
+  """Two vertices a level, each with edges to both of the next: all of a level have
+  the same parent, the lower vertex of the level before."""
+  rng = np.random.default_rng(8)
+  depth = 66_000
+  n = 2 * depth + 1000
+  ids = rng.permutation(n)
+  root, pairs = int(ids[0]), ids[1:2 * depth + 1].reshape(depth, 2)
+  src = np.concatenate([[root, root]] + [pairs[:-1, i] for i in (0, 0, 1, 1)])
+  dst = np.concatenate([pairs[0]] + [pairs[1:, i] for i in (0, 1, 0, 1)])
+  want = np.full(n, -1, dtype=np.int32)
+  want[root], want[pairs[0]] = root, root
+  want[pairs[1:]] = pairs[:-1].min(axis=1)[:, None]
+  with Graph(from_edges(n, src, dst)) as g:
+    g.set_options(parent_rule=_lib.CG_PARENT_FIFO)
+    lv, pa, st = g.bfs(root)
+    assert st["rounds"] == depth + 1
+    assert np.array_equal(lv[pairs], np.repeat(np.arange(1, depth + 1), 2).reshape(depth, 2))
+    assert np.array_equal(pa, want)
+
+
+def test_hubs_past_the_counted_levels(built_lib, oracle_mod):
+  """Long lists on levels whose entries are not counted (from 64 on)."""
+  rng = np.random.default_rng(3)
+  a, root = _layers([1] + [5] * 70 + [6000, 12, 6000, 3, 5000, 40, 40, 40, 2000], 3, rng, True)
+  with Graph(a) as g:
+    g.set_options(parent_rule=_lib.CG_PARENT_FIFO)
+    lv, pa, _ = g.bfs(root)
+    rl, _, _ = oracle_mod.bfs(*a.out_lists(), a.in_off, a.in_idx, root)
+    assert rl.max() > 70 and np.array_equal(lv, rl)
+    assert np.array_equal(pa, oracle_mod.fifo_parents(a.in_off, a.in_idx, rl, root))
