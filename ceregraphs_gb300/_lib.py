@@ -125,6 +125,7 @@ SIGNATURES = {
     "cg_bfs": ([_P, ctypes.c_int64, _P, _P, ctypes.POINTER(CgStats)], ctypes.c_int),
     "cg_bfs_device": ([_P, ctypes.c_int64, _P, _P], ctypes.c_int),
     "cg_graph_last_stats": ([_P, ctypes.POINTER(CgStats)], ctypes.c_int),
+    "cg_test_team_runs": ([_P, ctypes.POINTER(ctypes.c_int32)], ctypes.c_int),
     "cg_msbfs": ([_P, _P, ctypes.c_int32, _P, _P, ctypes.POINTER(CgStats)], ctypes.c_int),
     "cg_msbfs_device": ([_P, _P, ctypes.c_int32, _P, _P], ctypes.c_int),
     "cg_count_edges": ([_P, _P, ctypes.c_int32, _I64P], ctypes.c_int),

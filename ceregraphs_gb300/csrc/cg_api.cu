@@ -287,6 +287,15 @@ int cg_graph_last_stats(cg_graph *g, cg_stats *stats) {
   return CG_OK;
 }
 
+int cg_test_team_runs(cg_graph *g, int32_t *runs) {
+  if (!g || !runs) return CG_ERR_INVALID_ARG;
+  // the control block keeps its contents until the next search clears it
+  CG_CUDA(cudaMemcpyAsync(runs, &g->ctl->team.command, sizeof(*runs), cudaMemcpyDeviceToHost,
+                          g->stream));
+  CG_CUDA(cudaStreamSynchronize(g->stream));
+  return CG_OK;
+}
+
 // Device-visible address of a page-locked host buffer, or NULL for pageable
 // memory (which is then filled by an ordinary copy).
 static int32_t *pinned_device_ptr(int32_t *host) {

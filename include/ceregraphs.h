@@ -156,6 +156,9 @@ int cg_bfs_device(cg_graph *g, int64_t root, int32_t *d_levels, int32_t *d_paren
 /* Waits for the handle's stream, then reports the last search's device
  * statistics (rounds_completed, nf_history, direction_history, status). */
 int cg_graph_last_stats(cg_graph *g, cg_stats *stats);
+/* Test hook: how often the last per-root search handed small rounds to a team of
+ * blocks (0 on graphs whose searches have none).  Waits for the handle's stream. */
+int cg_test_team_runs(cg_graph *g, int32_t *runs);
 
 /* ---- Kernel 2, batched: k searches in one pass ------------------------
  * Multi-source BFS: roots packed as bit lanes per vertex (64 or 128 lanes a
