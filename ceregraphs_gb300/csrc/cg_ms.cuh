@@ -110,10 +110,7 @@ struct MsParams {
   int *flag;                  // set when a search outgrows the history
   // parent candidates of the output pass: vertices of in-degree > kPullLight
   const int32_t *cand_slot;   // [n], -1 for light vertices
-  const int32_t *cand_vtx;    // [ncand]
-  const uint32_t *cand_choff; // [ncand + 1] prefix of in-list chunks
-  uint32_t *cand;             // [ncand][64 W], 0xFFFFFFFF = none yet
-  int ncand;
+  uint32_t *cand;             // [slots][64 W], 0xFFFFFFFF = none yet
   // ledger batches: the in-list position of each lane's parent, for light
   // vertices, as bit slices -- bit l of pos[b][v] is bit b of lane l's position.
   // Slice b of v counts only once bit b of pos_used[v] is set (it is stored
@@ -539,8 +536,6 @@ struct MsState {
   MsCtl *ctl = nullptr;
   int *flag = nullptr;        // history overflow flag of the last batch
   int32_t *cand_slot = nullptr;
-  int32_t *cand_vtx = nullptr;
-  uint32_t *cand_choff = nullptr;
   uint32_t *cand = nullptr;
   int ncand = 0;
   uint64_t *pos = nullptr;
@@ -575,10 +570,7 @@ inline MsParams ms_params(const cg_graph *g, const MsState *s) {
   p.flag = s->flag;
   p.gate = 0;
   p.cand_slot = s->cand_slot;
-  p.cand_vtx = s->cand_vtx;
-  p.cand_choff = s->cand_choff;
   p.cand = s->cand;
-  p.ncand = s->ncand;
   p.pos = s->pos;
   p.pos_used = s->pos_used;
   p.light = s->lightfin;

@@ -153,31 +153,6 @@ __device__ __forceinline__ Mask<W> thread_scan(const MsParams &p, int64_t v, int
   return got;
 }
 
-// Scans a warp's 32 non-hub vertices: short in-lists one per thread, the
-// others by the whole warp in turn.  want must be zero where no scan is due.
-template <int W>
-__device__ __forceinline__ Mask<W> scan_group(const MsParams &p, int64_t v, int64_t s, int64_t e,
-                                              const Mask<W> &want, const uint64_t *cur,
-                                              int level) {
-  const bool need = want.any();
-  const bool longer = need && (e - s) > kPullLight;
-  Mask<W> got = Mask<W>::zero();
-  if (need && !longer) got = thread_scan<W>(p, v, s, e, want, cur, level);
-  unsigned hm = __ballot_sync(kMsFull, longer);
-  while (hm) {
-    const int j = __ffs(hm) - 1;
-    hm &= hm - 1;
-    const int64_t vj = __shfl_sync(kMsFull, v, j);
-    const int64_t sj = __shfl_sync(kMsFull, s, j), ej = __shfl_sync(kMsFull, e, j);
-    Mask<W> wj;
-#pragma unroll
-    for (int i = 0; i < W; ++i) wj.w[i] = __shfl_sync(kMsFull, want.w[i], j);
-    const Mask<W> gj = warp_scan<W>(p, vj, sj, ej, wj, cur, level, -1);
-    if (lane_id() == j) got = gj;
-  }
-  return got;
-}
-
 // Hub in-list chunks of a round: chunk c of hub h scans its slice for the
 // wanted lanes (frozen for the round: nothing writes a hub's vis before its
 // finalize), min-combining winners into the candidate buffer.
@@ -642,8 +617,6 @@ static void ms_free_state(MsState *s) {
   cudaFree(s->ctl);
   cudaFree(s->flag);
   cudaFree(s->cand_slot);
-  cudaFree(s->cand_vtx);
-  cudaFree(s->cand_choff);
   cudaFree(s->cand);
   cudaFree(s->pos);
   cudaFree(s->pos_used);
@@ -762,9 +735,10 @@ static int ms_build_hubs(cg_graph *g, MsState *s) {
   return rc;
 }
 
-__global__ void slot_map_kernel(int count, const int32_t *__restrict__ vtx, int32_t *slot) {
+__global__ void slot_map_kernel(int count, const int32_t *__restrict__ vtx, int first,
+                                int32_t *slot) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
-    slot[vtx[i]] = i;
+    slot[vtx[i]] = first + i;
 }
 
 // Bit v of light[w]: vertex v = 32 w + b has in-degree 1 .. kPullLight (the
@@ -786,14 +760,12 @@ __global__ void light_map_kernel(int64_t n, int64_t words, const int64_t *__rest
 
 // Parent-candidate slots of the output pass of a ledger batch: every vertex of
 // in-degree > kPullLight (the medium list, then the hubs) gets a slot of 64 W
-// candidates and its in-list is cut into kHubChunk-entry chunks.
+// candidates.
 static int ms_build_cands(cg_graph *g, MsState *s) {
   const int64_t ncand = s->nmed + s->nhub;
   s->ncand = (int)ncand;
   const size_t nc = ncand > 0 ? (size_t)ncand : 1;
   if (cudaMalloc(&s->cand_slot, sizeof(int32_t) * (size_t)g->n) != cudaSuccess ||
-      cudaMalloc(&s->cand_vtx, sizeof(int32_t) * nc) != cudaSuccess ||
-      cudaMalloc(&s->cand_choff, sizeof(uint32_t) * (nc + 1)) != cudaSuccess ||
       cudaMalloc(&s->cand, sizeof(uint32_t) * nc * 64 * s->lane_words) != cudaSuccess ||
       cudaMalloc(&s->pos, sizeof(uint64_t) * kPosBits * (size_t)g->n * s->lane_words) !=
           cudaSuccess ||
@@ -810,40 +782,17 @@ static int ms_build_cands(cg_graph *g, MsState *s) {
     CG_CUDA(cudaGetLastError());
   }
   CG_CUDA(cudaMemsetAsync(s->cand_slot, 0xff, sizeof(int32_t) * (size_t)g->n, g->stream));
-  if (s->nmed)
-    CG_CUDA(cudaMemcpyAsync(s->cand_vtx, s->med_vtx, sizeof(int32_t) * (size_t)s->nmed,
-                            cudaMemcpyDeviceToDevice, g->stream));
-  if (s->nhub)
-    CG_CUDA(cudaMemcpyAsync(s->cand_vtx + s->nmed, s->hub_vtx, sizeof(int32_t) * (size_t)s->nhub,
-                            cudaMemcpyDeviceToDevice, g->stream));
-  uint32_t *chunks = nullptr;
-  CG_CUDA(cudaMalloc(&chunks, sizeof(uint32_t) * nc));
-  int rc = CG_OK;
-  uint32_t *h = new (std::nothrow) uint32_t[nc + 1];
-  do {
-    if (!h) { rc = CG_ERR_OUT_OF_MEMORY; break; }
-    h[0] = 0;
-    if (ncand > 0) {
-      const int blocks = (int)((ncand + 255) / 256 < g->num_sms * 16 ? (ncand + 255) / 256
-                                                                      : g->num_sms * 16);
-      slot_map_kernel<<<blocks, 256, 0, g->stream>>>((int)ncand, s->cand_vtx, s->cand_slot);
-      hub_chunks_kernel<<<blocks, 256, 0, g->stream>>>((int)ncand, g->in_off, s->cand_vtx, chunks);
-      cudaError_t e = cudaMemcpyAsync(h + 1, chunks, sizeof(uint32_t) * (size_t)ncand,
-                                      cudaMemcpyDeviceToHost, g->stream);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-      if (e != cudaSuccess) { rc = cuda_fail(e, "candidate chunks"); break; }
-      for (int64_t i = 0; i < ncand; ++i) h[i + 1] += h[i];
-    }
-    cudaError_t e = cudaMemcpyAsync(s->cand_choff, h, sizeof(uint32_t) * (size_t)(ncand + 1),
-                                    cudaMemcpyHostToDevice, g->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-    if (e != cudaSuccess) { rc = cuda_fail(e, "candidate chunks"); break; }
-    g->device_bytes += sizeof(int32_t) * (g->n + nc) + sizeof(uint32_t) * (nc + 1) +
-                       sizeof(uint32_t) * nc * 64 * s->lane_words;
-  } while (0);
-  delete[] h;
-  cudaFree(chunks);
-  return rc;
+  auto slots = [&](int64_t count, const int32_t *vtx, int64_t first) {
+    if (count == 0) return;
+    const int64_t blocks = (count + 255) / 256, cap = (int64_t)g->num_sms * 16;
+    slot_map_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, g->stream>>>(
+        (int)count, vtx, (int)first, s->cand_slot);
+  };
+  slots(s->nmed, s->med_vtx, 0);
+  slots(s->nhub, s->hub_vtx, s->nmed);
+  CG_CUDA(cudaGetLastError());
+  g->device_bytes += sizeof(int32_t) * g->n + sizeof(uint32_t) * nc * 64 * s->lane_words;
+  return CG_OK;
 }
 
 // Lane state for one batched search stream (a graph's batch state or a pool).

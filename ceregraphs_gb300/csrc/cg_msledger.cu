@@ -91,25 +91,6 @@ __device__ __forceinline__ uint64_t *plane(const MsParams &p, int L) {
   return p.hist + (int64_t)L * p.n * W;
 }
 
-// OR of the frontier masks of in-list entries [s, e) restricted to `want`,
-// one thread, four entries' loads in flight; stops once all of want is found.
-template <int W>
-__device__ __forceinline__ Mask<W> or_thread(const MsParams &p, int64_t s, int64_t e,
-                                             const Mask<W> &want, const uint64_t *cur) {
-  constexpr int G = 4;
-  Mask<W> got = Mask<W>::zero();
-  for (int64_t i0 = s; i0 < e; i0 += G) {
-    int32_t u[G];
-#pragma unroll
-    for (int k = 0; k < G; ++k) u[k] = i0 + k < e ? __ldg(p.in_idx + i0 + k) : -1;
-#pragma unroll
-    for (int k = 0; k < G; ++k)
-      if (u[k] >= 0) got = got | (ld_mask<W>(cur, u[k]) & want);
-    if (got == want) break;
-  }
-  return got;
-}
-
 // Adds lanes to slice b of light vertex v's positions; `used` is its pos_used.
 template <int W>
 __device__ __forceinline__ void add_slice(const MsParams &p, int64_t v, int b, const Mask<W> &a,
@@ -201,7 +182,8 @@ __device__ __forceinline__ uint32_t warp_transpose32(uint32_t x) {
   return x;
 }
 
-// or_warp that also records, per lane of `want`, the first in-list entry
+// OR of the frontier masks of in-list entries [s, e) restricted to `want`, by the
+// whole warp, recording per lane of `want` the first in-list entry
 // holding it -- the lowest-index parent -- into row[lane] (plain stores when
 // the warp scans the whole in-list, atomicMin when other warps scan other
 // chunks of it).  The hits of 32 entries form a 32 x 64 W bit matrix that is
