@@ -329,9 +329,14 @@ int cg_bfs(cg_graph *g, int64_t root, int32_t *levels, int32_t *parents, cg_stat
     g->h_stats = static_cast<cg_stats *>(h);
   }
   // page-locked outputs are written by the search kernel itself at its end
-  // (the GPU's own SMs over the host link); pageable ones by a copy after it
+  // (the GPU's own SMs over the host link, 16 bytes a store where n allows);
+  // pageable ones, and those off the 16 bytes, by a copy after it
   const bool fifo = g->opt.parent_rule == CG_PARENT_FIFO;
-  int32_t *hl = pinned_device_ptr(levels), *hp = fifo ? nullptr : pinned_device_ptr(parents);
+  auto stored = [&](int32_t *host) -> int32_t * {
+    const bool aligned = (reinterpret_cast<uintptr_t>(host) & 15u) == 0;
+    return (g->n & 3) == 0 && !aligned ? nullptr : pinned_device_ptr(host);
+  };
+  int32_t *hl = stored(levels), *hp = fifo ? nullptr : stored(parents);
   CG_CUDA(cudaEventRecord(g->ev0, g->stream));
   int rc = bfs_launch(g, root, g->tmp_levels, g->tmp_parents, hl, hp);
   if (rc) return rc;
