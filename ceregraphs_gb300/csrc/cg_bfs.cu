@@ -1892,8 +1892,8 @@ __global__ void __launch_bounds__(kBfsBlock, 3) bfs_persistent_wide(BfsParams p)
 
 // The same search with rounds that a team runs.  A kernel of its own, so that
 // the other keeps its registers (with the team in it R-MAT and random graphs took
-// 2 to 3% longer), and of fewer threads, so that it has 56 without spills and
-// three handles' blocks still fit an SM: 512 threads and 64 registers are as fast
+// 2 to 3% longer), and of fewer threads, so that it has 56 (one is spilled)
+// and three handles' blocks still fit an SM: 512 threads and 64 registers are as fast
 // for one handle, 4.6 ms a search for three taking turns where this takes 3.3.
 __global__ void __launch_bounds__(kTeamBlock, 3) bfs_persistent_team(BfsParams p) {
   search<true, false>(p);
@@ -2089,9 +2089,14 @@ int bfs_prepare(cg_graph *g) {
   }
   // Meshes, grids and road networks, which take hundreds of rounds of slowly
   // changing frontiers: bounded degrees, and enough vertices for a frontier of
-  // kTeamEnter edges that is as deep as it is wide (below, one block runs every
-  // round: a 200^2 grid takes 1,090 us with either kernel, 1,125 on some GPUs
-  // with the team's).
+  // kTeamEnter edges that is as deep as it is wide.  Below, one block runs every
+  // round; at the line the team's kernel pays only for several handles in turn
+  // (256^2 grid: one handle 1,684 us without and 1,786 with it, three in turn 850 and
+  // 704; 500^2: 4,496 and 3,749, 2,424 and 1,488).  The degrees alone do not tell a
+  // mesh from a random graph of few edges, which it makes slower (1 M vertices,
+  // three random in- and out-edges each 181 -> 193 us, a binary tree of 256 K 250 ->
+  // 302; 292 and 441 before there were small rounds); what does, how fast a frontier
+  // grows, is known only to a search.
   g->team = g->n >= kTeamVertices && g->nnz > 0 &&
             1024 * live[2] <= (unsigned long long)g->nnz;
   g->live = (int64_t)live[0];
@@ -2129,15 +2134,25 @@ static int blocks_for(const cg_graph *g) {
   return g->n <= (1 << 21) ? 2 : 3;
 }
 
+// The team's kernel has 1,152 threads an SM where the common one has 1,536: rounds
+// that only pull want those from 4 M vertices on (bottom-up, us with the team's / the
+// common kernel: a ring of 4 M with few long edges 31,300 / 28,200, a 3000^2 grid
+// 327,800 / 291,600, directed ER of 4 M vertices and degree 1.2 79 / 73; but a 2000^2
+// grid 100,200 / 101,200 and the ring of 1 M 11,000 / 12,100).
+using BfsKernel = void (*)(BfsParams);
+static BfsKernel kernel_for(const cg_graph *g) {
+  return g->team && !(pulls_early(g) && g->n >= (1 << 22)) ? bfs_persistent_team : bfs_persistent;
+}
+
 static int bfs_grid(cg_graph *g) {
+  const BfsKernel kernel = kernel_for(g);
   int block = g->opt.block_size > 0 ? g->opt.block_size : kBfsBlock;
   if (block > kBfsBlock) block = kBfsBlock;
-  if (g->team && block > kTeamBlock) block = kTeamBlock;
+  if (kernel == bfs_persistent_team && block > kTeamBlock) block = kTeamBlock;
   block = (block / 32) * 32;
   if (block < 64) block = 64;
   int per_sm = 0;
-  CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      &per_sm, g->team ? bfs_persistent_team : bfs_persistent, block, 0));
+  CG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0));
   if (per_sm <= 0) return CG_ERR_NOT_SUPPORTED;
   const int want = g->opt.blocks_per_sm > 0 ? g->opt.blocks_per_sm : blocks_for(g);
   if (want < per_sm) per_sm = want;
@@ -2201,7 +2216,7 @@ int bfs_launch(cg_graph *g, int64_t root, int32_t *d_levels, int32_t *d_parents,
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  CG_CUDA(cudaLaunchKernelEx(&cfg, g->team ? bfs_persistent_team : bfs_persistent, p));
+  CG_CUDA(cudaLaunchKernelEx(&cfg, kernel_for(g), p));
   return CG_OK;
 }
 

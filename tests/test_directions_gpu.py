@@ -64,3 +64,30 @@ def test_early_pull_rounds_split_the_hubs(built_lib, options):
     want = lv.clone(), pa.clone()
     assert _searched(g, root, lv, pa, **options) < 10 * auto
     assert torch.equal(lv, want[0]) and torch.equal(pa, want[1])
+
+
+def test_large_graphs_of_bounded_degree(built_lib):
+  """Bottom-up searches of 4 M vertices of bounded degree, which run in the common
+  kernel, against direction-optimizing ones, which run in the team's."""
+  import ctypes
+  import torch
+  n, m = 1 << 22, 5_000_000
+  gen = torch.Generator(device="cuda").manual_seed(1)
+  src, dst = (torch.randint(0, n, (m,), generator=gen, device="cuda", dtype=torch.int32)
+              for _ in range(2))
+  torch.cuda.synchronize()
+  h = ctypes.c_void_p()
+  _lib.check(_lib.load().cg_graph_from_edges(n, m, ctypes.c_void_p(src.data_ptr()),
+                                             ctypes.c_void_p(dst.data_ptr()),
+                                             _lib.CG_EDGES_DROP_LOOPS, ctypes.byref(h)), "build")
+  with Graph.from_handle(h) as g:
+    lv, pa = (torch.empty(n, dtype=torch.int32, device="cuda") for _ in range(2))
+    for root in range(0, n, n // 7):
+      g.set_options(direction=_lib.CG_DIR_AUTO)
+      g.bfs_device(root, lv, pa)
+      rounds = g.last_stats()["rounds"]
+      want = lv.clone(), pa.clone()
+      g.set_options(direction=_lib.CG_DIR_BOTTOMUP)
+      g.bfs_device(root, lv, pa)
+      assert g.last_stats()["rounds"] == rounds
+      assert torch.equal(lv, want[0]) and torch.equal(pa, want[1])
