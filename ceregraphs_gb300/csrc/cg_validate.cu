@@ -77,7 +77,7 @@ __device__ __forceinline__ bool contains(const int32_t *__restrict__ idx, int64_
 // instructions per 32 entries and 16 searches, and lists of uneven lengths in a
 // warp) and by the latency of the 4 * NW byte gathers, which the L2 serves.
 // R-MAT scale 20, 16 searches, device time: 6670 us for the two per-search
-// kernels, 535 us for these (packing 12, vertices 330, long lists 193).
+// kernels, 510 us for these (packing 12, vertices 417, long lists 81).
 constexpr uint32_t kHigh = 0x80808080u, kOnes = 0x01010101u;
 constexpr int kUnreached = 127, kMaxLevel = 125;
 constexpr int kGroup = 16;          // searches of a group at most
